@@ -6,23 +6,54 @@
 // computed once per device for all 4096 patterns by k_init_tables and looked
 // up afterwards. Corner cutting and the ear clip of the cut polygon depend on
 // neighbours and on the image, and are computed per cell.
+#include <array>
+#include <cstring>
+#include <map>
+#include <memory>
+#include <new>
+#include <vector>
+
 #include "depix_internal.h"
 
 namespace depix {
 
 __device__ uint64_t g_hull_lut[4096];
 __device__ uint64_t g_tri_lut[4096];
-// Per pattern and hull vertex v: the corner-cutting case of v (bits 0-1:
-// 0 both adjacent edges linked, 1 both border, 2 only the previous edge
-// linked, 3 only the current edge linked) and, for 2 and 3, that edge's link
-// direction (bits 2-4); 5 bits per vertex.
-__device__ uint64_t g_vk_lut[4096];
-// Per pattern and hull vertex v: Q on edge v -> v+1 near v and R on edge
-// v-1 -> v near v (getQ_i(v), getR_i(v-1)), as int8 x, y, x, y in 1/64 cell.
-__device__ __align__(16) uint32_t g_qr_lut[4096 * 8];
-// Per pattern: bit e set when the hull reaches into the open square of
-// neighbour e (hull bounding box test).
-__device__ uint8_t g_spill_lut[4096];
+
+// ---- cut polygons by pieces
+//
+// One corner-cutting round changes a hull edge by edge, so the boundary of a
+// cut polygon is made of pieces (subdivision, subdivision_functions.cu:564-669):
+//  - what the cell's own pattern decides: border edges from Q_v to R_v+1, cut
+//    corners R_v -> Q_v, linked edges between two linked ones;
+//  - per linked edge with a border edge at one end or both: the path over the
+//    midpoint(s) with the linked neighbour's R or Q, which the edge's geometry
+//    and the neighbour's pattern decide;
+//  - per corner that the T-junction test keeps: the triangle R, P, Q.
+// Coverage by crossing number is the XOR of the pieces' coverages, so a cut
+// cell's mask is a few table entries XORed (k_build_scale_masks), with no
+// polygon built. Over all 4096 patterns there are 16 geometries of such
+// linked edges, at most 4 of them in a pattern, 7924 pairs of an edge's own
+// cut ends and a neighbour's points, and 68 corner triangles.
+constexpr int kGeoms = 16, kMaxPaths = 8192, kMaxCorners = 128;
+struct CutPath { // an open path of n points in 1/64 cell
+    int8_t n, x[4], y[4];
+};
+struct CutCorner { // hull vertex P between two border edges, R before and Q after it
+    int8_t px, py, rx, ry, qx, qy;
+};
+struct CutTables {
+    // per pattern its linked edges with a border edge beside them: first path
+    // of the edge's own class (bits 0-15), geometry (16-19), link (20-22),
+    // present (23)
+    uint4 edges[4096];
+    uint64_t verts[4096];   // per hull vertex between border edges (byte v): its corner class, else 0xFF
+    uint32_t corners[4096]; // the same for the vertices at the cell's corners (0,0), (1,0), (1,1), (0,1)
+    uint8_t nb_class[kGeoms * 4096]; // per geometry and neighbour pattern: the neighbour's class
+    CutPath paths[kMaxPaths];        // [own class first path + neighbour's class]
+    CutCorner tris[kMaxCorners];
+};
+__device__ __align__(16) CutTables g_cut;
 
 // ------------------------------------------------------ pattern tables
 
@@ -148,44 +179,120 @@ __global__ void k_init_tables()
     uint64_t te = 0;
     for (int q = 0; q < 3 * nt; q++) te |= (uint64_t)tri[q] << (3 * q);
     g_tri_lut[pat] = te;
-    // vertex cases and corner-cutting points
-    int links[kMaxHull];
-    for (int v = 0; v < k; v++) links[v] = hull_edge_link(e, k, node, v);
-    uint64_t vk = 0;
-    for (int v = 0; v < kMaxHull; v++) {
-        uint32_t qr = 0;
-        if (v < k) {
-            const int lc = links[v], lp = links[v == 0 ? k - 1 : v - 1];
-            const bool cur = lc >= 0, prev = lp >= 0;
-            const int kind = cur == prev ? (cur ? 0 : 1) : (prev ? 2 : 3);
-            const int L = kind == 2 ? lp : (kind == 3 ? lc : 0);
-            vk |= (uint64_t)(kind | (L << 2)) << (5 * v);
-            int qx, qy, rx, ry;
-            hull_qr(e, k, v, false, qx, qy);
-            hull_qr(e, k, v - 1, true, rx, ry);
-            qr = (uint32_t)(uint8_t)qx | ((uint32_t)(uint8_t)qy << 8) | ((uint32_t)(uint8_t)rx << 16) |
-                 ((uint32_t)(uint8_t)ry << 24);
+}
+
+// The tables of g_cut from the hull table; false when a class count does not
+// fit (it cannot: the patterns are fixed).
+static bool build_cut_tables(const uint64_t* hull, CutTables& T)
+{
+    using Key = std::array<int, 9>;
+    std::map<std::array<int, 5>, int> geoms; // link, P_v, P_v+1
+    std::map<int, std::map<std::array<int, 4>, int>> nb; // per geometry: (Q at P_v, R at P_v+1) -> class
+    std::map<Key, int> own;                  // geometry, R_v, Q_v+1 where cut -> first path
+    std::map<std::array<int, 6>, int> tris;
+    int npaths = 0;
+    memset(&T, 0, sizeof(T));
+    for (int pat = 0; pat < 4096; pat++) {
+        const uint64_t e = hull[pat];
+        const int n = (int)(e & 0xF);
+        int link[kMaxHull];
+        for (int v = 0; v < n; v++) link[v] = hull_edge_link(e, n, (unsigned)pat & 0xFFu, v);
+        T.verts[pat] = ~0ull;
+        T.corners[pat] = ~0u;
+        uint32_t ed[4] = {0, 0, 0, 0};
+        int ne = 0;
+        for (int v = 0; v < n; v++) {
+            const int v1 = v + 1 == n ? 0 : v + 1;
+            const bool prev = link[v == 0 ? n - 1 : v - 1] >= 0, cur = link[v] >= 0;
+            const int px = hx(e, v), py = hy(e, v), p1x = hx(e, v1), p1y = hy(e, v1);
+            int rx, ry, qx, qy;
+            hull_qr(e, n, v - 1, true, rx, ry);
+            if (!cur && !prev) {
+                hull_qr(e, n, v, false, qx, qy);
+                const auto it = tris.emplace(std::array<int, 6>{px, py, rx, ry, qx, qy}, (int)tris.size()).first;
+                if (it->second >= kMaxCorners) return false;
+                T.tris[it->second] = CutCorner{(int8_t)px, (int8_t)py, (int8_t)rx, (int8_t)ry, (int8_t)qx, (int8_t)qy};
+                const uint64_t id = (uint64_t)it->second;
+                T.verts[pat] = (T.verts[pat] & ~(0xFFull << (8 * v))) | id << (8 * v);
+                if ((px == 0 || px == kUnit) && (py == 0 || py == kUnit)) {
+                    const int c = py == 0 ? (px == 0 ? 0 : 1) : (px == 0 ? 3 : 2);
+                    T.corners[pat] = (T.corners[pat] & ~(0xFFu << (8 * c))) | (uint32_t)id << (8 * c);
+                }
+            }
+            const bool cut0 = !prev, cut1 = link[v1] < 0; // R_v -> M_v, M_v+1 -> Q_v+1
+            if (!cur || (!cut0 && !cut1)) continue;
+            const int L = link[v];
+            hull_qr(e, n, v1, false, qx, qy);
+            const int g = geoms.emplace(std::array<int, 5>{L, px, py, p1x, p1y}, (int)geoms.size()).first->second;
+            if (g >= kGeoms || ne == 4) return false;
+            auto& cls = nb[g];
+            if (cls.empty()) {
+                for (int np = 0; np < 4096; np++) {
+                    const uint64_t he = hull[np];
+                    const int hn = (int)(he & 0xF);
+                    // the neighbour's vertex at this position, else its vertex 0 (getPointIndex)
+                    auto at = [&](int x, int y) {
+                        for (int t = 0; t < hn; t++)
+                            if (hx(he, t) == x - kUnit * dir_di(L) && hy(he, t) == y - kUnit * dir_dj(L)) return t;
+                        return 0;
+                    };
+                    int ax, ay, bx, by;
+                    hull_qr(he, hn, at(px, py), false, ax, ay);
+                    hull_qr(he, hn, at(p1x, p1y) - 1, true, bx, by);
+                    const int id = cls.emplace(std::array<int, 4>{ax + kUnit * dir_di(L), ay + kUnit * dir_dj(L),
+                                                                  bx + kUnit * dir_di(L), by + kUnit * dir_dj(L)},
+                                               (int)cls.size()).first->second;
+                    if (id > 255) return false;
+                    T.nb_class[g * 4096 + np] = (uint8_t)id;
+                }
+            }
+            const Key key{g, cut0, cut0 ? rx : 0, cut0 ? ry : 0, cut1, cut1 ? qx : 0, cut1 ? qy : 0, 0, 0};
+            const auto it = own.emplace(key, npaths).first;
+            if (it->second == npaths) {
+                if (npaths + (int)cls.size() > kMaxPaths) return false;
+                for (const auto& c : cls) {
+                    CutPath& p = T.paths[npaths + c.second];
+                    auto put = [&](int x, int y) {
+                        p.x[p.n] = (int8_t)x;
+                        p.y[p.n++] = (int8_t)y;
+                    };
+                    if (cut0) {
+                        put(rx, ry);
+                        put((rx + c.first[0]) / 2, (ry + c.first[1]) / 2);
+                    } else {
+                        put(px, py);
+                    }
+                    if (cut1) {
+                        put((qx + c.first[2]) / 2, (qy + c.first[3]) / 2);
+                        put(qx, qy);
+                    } else {
+                        put(p1x, p1y);
+                    }
+                }
+                npaths += (int)cls.size();
+            }
+            ed[ne++] = (uint32_t)it->second | (uint32_t)g << 16 | (uint32_t)L << 20 | 1u << 23;
         }
-        g_qr_lut[pat * 8 + v] = qr;
+        T.edges[pat] = make_uint4(ed[0], ed[1], ed[2], ed[3]);
     }
-    g_vk_lut[pat] = vk;
-    int mnx = 1 << 20, mny = 1 << 20, mxx = -(1 << 20), mxy = -(1 << 20);
-    for (int t = 0; t < k; t++) {
-        mnx = min(mnx, hx(e, t)); mxx = max(mxx, hx(e, t));
-        mny = min(mny, hy(e, t)); mxy = max(mxy, hy(e, t));
-    }
-    unsigned sp = 0;
-    for (int d = 0; d < 8; d++) {
-        int sx = kUnit * dir_di(d), sy = kUnit * dir_dj(d);
-        if (mxx > sx && mnx < sx + kUnit && mxy > sy && mny < sy + kUnit) sp |= 1u << d;
-    }
-    g_spill_lut[pat] = (uint8_t)sp;
+    return true;
 }
 
 cudaError_t init_tables(cudaStream_t s)
-{
+try {
+    std::vector<uint64_t> hull(4096);
+    std::unique_ptr<CutTables> T(new CutTables);
     k_init_tables<<<16, 256, 0, s>>>();
-    return cudaGetLastError();
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess)
+        e = cudaMemcpyFromSymbolAsync(hull.data(), g_hull_lut, sizeof(g_hull_lut), 0, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return e;
+    if (!build_cut_tables(hull.data(), *T)) return cudaErrorUnknown;
+    e = cudaMemcpyToSymbolAsync(g_cut, T.get(), sizeof(CutTables), 0, cudaMemcpyHostToDevice, s);
+    return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+} catch (const std::bad_alloc&) {
+    return cudaErrorMemoryAllocation;
 }
 
 cudaError_t hull_table_address(const uint64_t** out)
@@ -529,19 +636,32 @@ cudaError_t launch_raster(const RasterBatch& b, int nframes, cudaStream_t s)
 //    lie in [-0.25, 1.25], subdivision adds midpoints of an own point and a
 //    neighbour's point (neighbour hull shifted by one cell);
 //  - footprint: output samples (X+0.5)/s in that box, offsets m = X - i*s in
-//    [mlo, mlo + F); one 32-bit row word per footprint row (F <= 32, s <= 12);
-//  - plain cells (no subdivision) take their rows from a per-scale table over
-//    the 4096 hull patterns; subdivided cells are gathered into a list and
-//    cut, ear-clipped and masked one per thread;
+//    [mlo, mlo + F), F <= 30 for s <= 12;
+//  - plain cells take their mask from a per-scale table over the 4096 hull
+//    patterns, subdivided cells XOR theirs from table entries (CutTables);
 //  - an output block (the s x s samples of one cell) takes, per sample, the
-//    latest covering cell in VBO order among the 3x3 cells around it. A cell
-//    whose block its own mask fills and no neighbour polygon reaches is
-//    filled without per-sample work.
+//    latest covering cell in VBO order among the 3x3 cells around it.
+//
+// Mask layouts: up to scale 8 a mask is nine parts, one per cell of the 3x3
+// around it (the cell itself is part 4), each part the s*s samples of that
+// cell in s rows of s bits, so that a block reads one part of each of its
+// nine candidates and resolves all its samples at once. A part is 16 bits up
+// to scale 4 and 64 bits up to scale 8. Above, a mask is one word per
+// footprint row (parts would need up to 144 bits each, twice the shared
+// memory of the rows).
+//
+// What bounds it: a 32x32 tile's phases (tile load, plain cells, cut cells,
+// fills, shared blocks) take 22, 22, 28, 20 and 8 % of a block's time, each a
+// short chain of shared-memory accesses; cut cells wait on table loads. 1024
+// frames of 256x224 at x4: 2605 us when a cell per distinct neighbourhood
+// built its polygon from dependent table lookups and masked it by crossing
+// number (hash tables found the distinct ones), 886 us now (4.6 TB/s of
+// input and output, 0.67 of the measured copy rate). 16 frames of 640x480 at
+// x8: 597 us before, 305 us now (4.2 TB/s).
 
 struct MaskGeom {
     int s;
-    int mlo, F;   // footprint of any cell polygon
-    int hlo, HF;  // footprint of a hull (no subdivision): [-0.25, 1.25]
+    int mlo, F; // footprint of any cell polygon
 };
 
 __host__ __device__ __forceinline__ MaskGeom mask_geom(int s)
@@ -550,16 +670,31 @@ __host__ __device__ __forceinline__ MaskGeom mask_geom(int s)
     g.s = s;
     g.mlo = -((3 * s + 2) / 4);
     g.F = (7 * s - 2) / 4 - g.mlo + 1;
-    g.hlo = -((s + 2) / 4);
-    g.HF = (5 * s - 2) / 4 - g.hlo + 1;
     return g;
 }
+
+enum MaskLayout { ML_U16, ML_U64, ML_ROWS };
+__host__ __device__ constexpr MaskLayout mask_layout(int s) { return s <= 4 ? ML_U16 : (s <= 8 ? ML_U64 : ML_ROWS); }
+// words of a mask, of a table entry (mask, then 16 flag bits: above part 8
+// for ML_U16, in a word of their own else) and between masks in shared memory
+// (odd, so that a warp's cells fall into different banks)
+__host__ __device__ __forceinline__ int mask_words(int s)
+{
+    return s <= 4 ? 5 : (s <= 8 ? 18 : mask_geom(s).F);
+}
+__host__ __device__ __forceinline__ int entry_words(int s) { return s <= 4 ? 8 : (s <= 8 ? 20 : ((mask_geom(s).F + 4) & ~3)); }
+__host__ __device__ __forceinline__ int mask_stride(int s) { return mask_words(s) | 1; }
+
+// a scale's table: plain hulls, cut cells' own pieces (per pattern), paths
+// over a linked neighbour, corner triangles
+constexpr int kPlainEntry = 0, kCutEntry = 4096, kPathEntry = 8192, kCornerEntry = kPathEntry + kMaxPaths;
+constexpr int kScaleEntries = kCornerEntry + kMaxCorners;
+size_t scale_mask_words(int s) { return (size_t)kScaleEntries * entry_words(s); }
 
 // Sets the footprint samples (offsets mlo.. in both axes, F of them) that the
 // triangle covers under the top-left rule. Vertices in 1/256 output pixel
 // relative to the cell origin.
-__device__ __forceinline__ void tri_mask(int ax, int ay, int bx, int by, int cx, int cy, int mlo, int F,
-                                         uint32_t* rows, int rstride = 1)
+__device__ __forceinline__ void tri_mask(int ax, int ay, int bx, int by, int cx, int cy, int mlo, int F, uint32_t* rows)
 {
     int area = (bx - ax) * (cy - ay) - (by - ay) * (cx - ax);
     if (area == 0) return;
@@ -590,32 +725,137 @@ __device__ __forceinline__ void tri_mask(int ax, int ay, int bx, int by, int cx,
             int px = 256 * m + 128;
             if (A0 * px + e0 >= b0 && A1 * px + e1 >= b1 && A2 * px + e2 >= b2) bits |= 1u << (m - mlo);
         }
-        if (bits) rows[(n - mlo) * rstride] |= bits;
+        if (bits) rows[n - mlo] |= bits;
     }
 }
 
-// Per-scale table: for each hull pattern, HF row words over the hull window.
+// Crossing-number coverage of one directed edge (1/64 cell): on every sample
+// row it crosses, the samples left of the crossing toggle. The sample point
+// is shifted by (+e, -e^2), so that the XOR over a simple polygon's edges is
+// what the top-left rule gives for any exact triangulation of it.
+__device__ void edge_mask(int x0, int y0, int x1, int y1, const MaskGeom& G, uint32_t* rows)
+{
+    const int u = 4 * G.s;
+    int lx = x0 * u, ly = y0 * u, hxx = x1 * u, hyy = y1 * u;
+    if (ly == hyy) return;
+    if (ly > hyy) {
+        int t = lx; lx = hxx; hxx = t;
+        t = ly; ly = hyy; hyy = t;
+    }
+    // rows whose sample height py = 256 row + 128 has ly < py <= hyy
+    const int r0 = max(((ly - 128) >> 8) + 1, G.mlo), r1 = min((hyy - 128) >> 8, G.mlo + G.F - 1);
+    const int D = hyy - ly, den = 256 * D;
+    for (int row = r0; row <= r1; row++) {
+        // samples left of the crossing: 256 m + 128 < x_cross  <=>  m < num / den
+        const int num = lx * D + (256 * row + 128 - ly) * (hxx - lx) - 128 * D;
+        int q = num / den;
+        if (num % den > 0) q++; // ceil; the division truncates toward zero
+        const int k = q - G.mlo;
+        rows[row - G.mlo] ^= k <= 0 ? 0u : (k >= 32 ? 0xFFFFFFFFu : ((1u << k) - 1u));
+    }
+}
+
+// An edge's part in the test that the polygon is star-shaped about the cell
+// centre (every edge turns strictly counter-clockwise around it and the
+// polygon winds around it once; it is then simple, the reference's ear clip
+// never gives up on it and tiles it exactly): 64 when the edge does not turn
+// counter-clockwise, 1 when it passes angle 0. Sums to 1 over the edges of a
+// star-shaped polygon.
+__device__ __forceinline__ int edge_flags(int x0, int y0, int x1, int y1)
+{
+    const int ax = x0 - kUnit / 2, ay = y0 - kUnit / 2, bx = x1 - kUnit / 2, by = y1 - kUnit / 2;
+    const bool up0 = ay > 0 || (ay == 0 && ax > 0), up1 = by > 0 || (by == 0 && bx > 0);
+    return (ax * by - ay * bx > 0 ? 0 : 64) + (!up0 && up1 ? 1 : 0);
+}
+
+// footprint rows to a mask in the scale's layout
+__device__ __forceinline__ void pack_mask(const MaskGeom& G, const uint32_t* rows, uint32_t* dst)
+{
+    const int s = G.s;
+    if (mask_layout(s) == ML_ROWS) {
+        for (int r = 0; r < G.F; r++) dst[r] = rows[r];
+        return;
+    }
+    const uint32_t blockbits = (1u << s) - 1u;
+    uint64_t part[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    for (int rr = 0; rr < G.F; rr++) {
+        const int m = rr + G.mlo, dj = m < 0 ? -1 : (m >= s ? 1 : 0);
+        const uint64_t x = (uint64_t)rows[rr] << (s + G.mlo);
+        for (int di = -1; di <= 1; di++)
+            part[(dj + 1) * 3 + di + 1] |= ((x >> ((di + 1) * s)) & blockbits) << ((m - dj * s) * s);
+    }
+    if (mask_layout(s) == ML_U16) {
+        for (int p = 0; p < 4; p++) dst[p] = (uint32_t)part[2 * p] | (uint32_t)part[2 * p + 1] << 16;
+        dst[4] = (uint32_t)part[8];
+    } else {
+        for (int p = 0; p < 9; p++) {
+            dst[2 * p] = (uint32_t)part[p];
+            dst[2 * p + 1] = (uint32_t)(part[p] >> 32);
+        }
+    }
+}
+
 __global__ void k_build_scale_masks(int s, uint32_t* lut)
 {
-    int pat = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pat >= 4096) return;
-    MaskGeom g = mask_geom(s);
-    Poly c;
-    hull_from_lut(g_hull_lut[pat], c);
-    uint64_t te = g_tri_lut[pat];
+    const int id = blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= kScaleEntries) return;
+    const MaskGeom G = mask_geom(s);
     uint32_t rows[32];
-    for (int r = 0; r < g.HF; r++) rows[r] = 0;
-    const int u = 4 * s;
-    for (int t = 0; t < c.n - 2; t++) {
-        int a = (int)((te >> (9 * t)) & 7), b = (int)((te >> (9 * t + 3)) & 7), d = (int)((te >> (9 * t + 6)) & 7);
-        tri_mask(c.x[a] * u, c.y[a] * u, c.x[b] * u, c.y[b] * u, c.x[d] * u, c.y[d] * u, g.hlo, g.HF, rows);
+    for (int r = 0; r < 32; r++) rows[r] = 0;
+    int flags = 0;
+    auto edge = [&](int x0, int y0, int x1, int y1) {
+        edge_mask(x0, y0, x1, y1, G, rows);
+        flags += edge_flags(x0, y0, x1, y1);
+    };
+    if (id < kCutEntry) {
+        Poly c;
+        hull_from_lut(g_hull_lut[id], c);
+        const uint64_t te = g_tri_lut[id];
+        const int u = 4 * s;
+        for (int t = 0; t < c.n - 2; t++) {
+            int a = (int)((te >> (9 * t)) & 7), b = (int)((te >> (9 * t + 3)) & 7), d = (int)((te >> (9 * t + 6)) & 7);
+            tri_mask(c.x[a] * u, c.y[a] * u, c.x[b] * u, c.y[b] * u, c.x[d] * u, c.y[d] * u, G.mlo, G.F, rows);
+        }
+    } else if (id < kPathEntry) {
+        const int pat = id - kCutEntry;
+        const uint64_t e = g_hull_lut[pat];
+        const int n = (int)(e & 0xF);
+        for (int v = 0; v < n; v++) {
+            const int v1 = v + 1 == n ? 0 : v + 1;
+            const bool prev = hull_edge_link(e, n, (unsigned)pat & 0xFFu, v == 0 ? n - 1 : v - 1) >= 0;
+            const bool cur = hull_edge_link(e, n, (unsigned)pat & 0xFFu, v) >= 0;
+            const bool next = hull_edge_link(e, n, (unsigned)pat & 0xFFu, v1) >= 0;
+            int qx, qy, rx, ry, r1x, r1y;
+            hull_qr(e, n, v, false, qx, qy);
+            hull_qr(e, n, v - 1, true, rx, ry);
+            hull_qr(e, n, v, true, r1x, r1y); // R before vertex v + 1
+            if (!cur && !prev) edge(rx, ry, qx, qy);
+            if (!cur) edge(qx, qy, r1x, r1y);
+            else if (prev && next) edge(hx(e, v), hy(e, v), hx(e, v1), hy(e, v1));
+        }
+    } else if (id < kCornerEntry) {
+        const CutPath& p = g_cut.paths[id - kPathEntry];
+        for (int k = 0; k + 1 < p.n; k++) edge(p.x[k], p.y[k], p.x[k + 1], p.y[k + 1]);
+    } else {
+        // a kept corner: R -> P -> Q in place of R -> Q
+        const CutCorner& t = g_cut.tris[id - kCornerEntry];
+        edge(t.rx, t.ry, t.px, t.py);
+        edge(t.px, t.py, t.qx, t.qy);
+        edge_mask(t.rx, t.ry, t.qx, t.qy, G, rows);
+        flags -= edge_flags(t.rx, t.ry, t.qx, t.qy);
     }
-    for (int r = 0; r < g.HF; r++) lut[(size_t)pat * g.HF + r] = rows[r];
+    for (int r = 0; r < G.F; r++) rows[r] &= (1u << G.F) - 1u; // F <= 30
+    uint32_t* dst = lut + (size_t)id * entry_words(s);
+    for (int k = 0; k < entry_words(s); k++) dst[k] = 0;
+    pack_mask(G, rows, dst);
+    const uint32_t f = (uint32_t)flags & 0xFFFFu;
+    if (mask_layout(s) == ML_U16) dst[4] |= f << 16;
+    else dst[mask_words(s)] = f;
 }
 
 cudaError_t build_scale_masks(int s, uint32_t* lut, cudaStream_t st)
 {
-    k_build_scale_masks<<<16, 256, 0, st>>>(s, lut);
+    k_build_scale_masks<<<(kScaleEntries + 127) / 128, 128, 0, st>>>(s, lut);
     return cudaGetLastError();
 }
 
@@ -623,231 +863,263 @@ cudaError_t build_scale_masks(int s, uint32_t* lut, cudaStream_t st)
 // its tile unwritten); read and cleared by depix_take_device_faults
 __device__ int g_raster_fault;
 
-// slots of a tile's table of distinct cut polygons (bounded probing: a
-// polygon that finds no slot makes its own mask)
-constexpr int kPolyTable = 1024, kPolyProbes = 16;
+// Compile-time scale of a raster kernel: 1..4 and 8 themselves, 0 the scales
+// 5 to 7 (64-bit parts), -1 the scales above 8 (rows).
+__host__ __device__ constexpr int raster_mode(int s) { return (s <= 4 || s == 8) ? s : (s < 8 ? 0 : -1); }
+__host__ __device__ constexpr MaskLayout mode_layout(int S) { return S < 0 ? ML_ROWS : (S == 0 ? ML_U64 : mask_layout(S)); }
 
-template <int TW, int TH>
+// Threads of a raster block, and the blocks per SM that its registers leave
+// room for: 48 registers and five blocks up to x4, whose masks take 23 KB of a
+// 32x32 tile (1024 frames of 256x224 at x4: 128 threads and six blocks 965 us,
+// 256 and four 956, 256 and five 886); above, the masks allow three.
+constexpr int kRT = 256;
+constexpr int raster_blocks(int S) { return S > 0 && S <= 4 ? 5 : 3; }
+
+template <int S, int TW, int TH>
 struct MaskTile {
     static constexpr int GW = TW + 2, GH = TH + 2, GN = GW * GH; // cells with their ring
     static constexpr int BW = TW + 6, BH = TH + 6;               // graph, halo 3
     static constexpr int CW = TW + 4, CH = TH + 4;               // pixels, halo 2
-    // pixels with halo 2, stored from two columns further left (x0 - 4) so
-    // that a TMA box can start on a 16-byte boundary: pixel (lx, ly) of the
-    // halo-2 window is pix[ly][lx + 2]
+    // pixels (RGBA words; the alpha byte may hold anything) with halo 2,
+    // stored from two columns further left (x0 - 4) so that a TMA box can
+    // start on a 16-byte boundary: pixel (lx, ly) of the halo-2 window is
+    // pix[ly][lx + 2]
     __align__(128) uint32_t pix[CH][CW + 4];
-    uint64_t bar;      // completion of the TMA pixel load
+    uint64_t bar;      // completion of the TMA loads
     int tma_ok;
     // graph bytes with halo 3, stored from 13 columns further left (x0 - 16)
     // so that a TMA box starts on a 16-byte boundary: graph byte (bx, by) of
     // the halo-3 window is graph[by][bx + kGOff]
     static constexpr int kGOff = 13, GRW = TW + 32;
     __align__(128) uint8_t graph[BH][GRW];
-    uint8_t spill[GN]; // bit e: the polygon reaches into the open square of neighbour e
-    uint8_t live[GN];  // the cell exists (inside the image)
-    uint16_t list[GN]; // subdivided cells of the tile, then the blocks that need owner resolution
-    uint16_t rep[GN];  // per subdivided cell: the list entry whose key, then whose polygon, it shares
-    uint16_t reps[GN]; // list entries that build a polygon (one per distinct key)
-    // distinct keys (first half), then distinct polygons (second half): hash
-    // tag | (list entry + 1), 0 empty; the first half later holds the list
-    // entries that make a mask
-    unsigned long long table[kPolyTable];
-    int count;
-    int slow;          // blocks in list for the owner-resolution pass
-    int nreps;
-    int nmakers;
+    // sample groups of a block that are resolved at once (at most 16 samples):
+    // the whole block up to x4, two of its rows at x8
+    static constexpr int NG = S == 8 ? 4 : 1;
+    static constexpr uint32_t kFull = S == 4 || S == 8 ? 0xFFFFu : (S > 0 && S < 4 ? (1u << (S * S & 15)) - 1u : 0u);
+    static constexpr int NL = GN > TW * TH * NG ? GN : TW * TH * NG;
+    uint16_t list[NL]; // subdivided cells of the tile, then the sample groups that need owner resolution
+    int count;         // cells in list
+    int slow;          // groups in list
 };
 
-__device__ __forceinline__ uint32_t rgba_of(uint32_t p)
+// RGBA word of one pixel with alpha 255
+template <int LAYOUT>
+__device__ __forceinline__ uint32_t load_rgba(const uint8_t* img, int ws, int i, int j)
 {
-    return ((p >> 16) & 0xFFu) | (p & 0xFF00u) | ((p & 0xFFu) << 16) | 0xFF000000u;
+    if (LAYOUT == DEPIX_LAYOUT_RGBA) return __ldg(reinterpret_cast<const uint32_t*>(img + (size_t)j * ws) + i);
+    const uint32_t p = load_bgr(img, ws, LAYOUT, i, j);
+    return ((p >> 16) & 0xFFu) | (p & 0xFF00u) | ((p & 0xFFu) << 16);
 }
 
-// bit e set when the box [x0,x1]x[y0,y1] (1/64 units) overlaps the open unit
-// square of neighbour e
-__device__ __forceinline__ unsigned spill_bits(int x0, int y0, int x1, int y1)
+// a slot in a shared list for every lane with pred, one atomic per warp (all
+// lanes call it)
+__device__ __forceinline__ int list_slot(int* counter, bool pred)
 {
-    unsigned m = 0;
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-        int sx = kUnit * dir_di(e), sy = kUnit * dir_dj(e);
-        if (x1 > sx && x0 < sx + kUnit && y1 > sy && y0 < sy + kUnit) m |= 1u << e;
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, pred);
+    const int lane = threadIdx.x & 31;
+    int base = 0;
+    if (m && lane == __ffs(m) - 1) base = atomicAdd(counter, __popc(m));
+    base = __shfl_sync(0xFFFFFFFFu, base, m ? __ffs(m) - 1 : 0);
+    return base + __popc(m & ((1u << lane) - 1u));
+}
+
+// Mask of a cut polygon that is not star-shaped about its cell centre: built
+// and ear-clipped as the reference does, triangle by triangle. g: the cell's
+// graph byte in the tile window (rows of `pitch` bytes); keep: bit c the
+// corner test at corner c (as CutTables::corners), bit 4 every vertex kept.
+__device__ __noinline__ void ear_clip_cell_mask(const uint8_t* g, int pitch, unsigned keep, int s, uint32_t* dst)
+{
+    const MaskGeom G = mask_geom(s);
+    auto pattern = [&](const uint8_t* q) { return cell_pattern(q[0], q[-1], q[1]); };
+    Poly c, p;
+    hull_from_lut(__ldg(&g_hull_lut[pattern(g)]), c);
+    subdivide_cell(
+        c, g[0], [&](int L, Poly& nb) { hull_from_lut(__ldg(&g_hull_lut[pattern(g + dir_dj(L) * pitch + dir_di(L))]), nb); },
+        [&](int px, int py) -> bool {
+            if (keep & 16u) return true;
+            if (px == 0 && py == 0) return keep & 1u;
+            if (px == kUnit && py == 0) return keep & 2u;
+            if (px == kUnit && py == kUnit) return keep & 4u;
+            if (px == 0 && py == kUnit) return keep & 8u;
+            return false;
+        },
+        p);
+    uint8_t tri[3 * kMaxPoly];
+    bool ok;
+    const int nt = ear_clip(p, tri, ok), u = 4 * s;
+    uint32_t rows[32];
+    for (int r = 0; r < 32; r++) rows[r] = 0;
+    for (int t = 0; t < nt; t++) {
+        const int a = tri[3 * t], b = tri[3 * t + 1], d = tri[3 * t + 2];
+        tri_mask(p.x[a] * u, p.y[a] * u, p.x[b] * u, p.y[b] * u, p.x[d] * u, p.y[d] * u, G.mlo, G.F, rows);
     }
-    return m;
+    pack_mask(G, rows, dst);
 }
 
-// One corner-cutting round (subdivision, subdivision_functions.cu:564-669)
-// read off the per-pattern tables: each hull vertex's case, its own Q and R
-// points and, on a linked/border transition, the linked neighbour's R (or Q)
-// around the vertex matching this one (getPointIndex falls back to vertex 0).
-// NbPattern(L) is the pattern of the neighbour in direction L; TJ(px, py) the
-// corner test of a vertex between two border edges; Emit(t, x, y) receives
-// cut vertex t. Returns the vertex count.
-template <typename NbPattern, typename TJ, typename Emit>
-__device__ __forceinline__ int subdivide_tables(int pat, uint64_t e, NbPattern nb_pattern, TJ tj, Emit emit)
-{
-    const int n = (int)(e & 0xF);
-    const uint64_t vk = __ldg(&g_vk_lut[pat]);
-    const uint32_t* qrs = g_qr_lut + pat * 8;
-    int m = 0;
-    for (int v = 0; v < n; v++) {
-        const int code = (int)((vk >> (5 * v)) & 31u), kind = code & 3;
-        const int px = hx(e, v), py = hy(e, v);
-        const uint32_t qr = __ldg(qrs + v);
-        const int qx = (int8_t)(qr & 0xFF), qy = (int8_t)((qr >> 8) & 0xFF);
-        const int rx = (int8_t)((qr >> 16) & 0xFF), ry = (int8_t)(qr >> 24);
-        if (kind == 0 || (kind == 1 && tj(px, py))) {
-            emit(m++, px, py);
-        } else if (kind == 1) {
-            emit(m++, rx, ry);
-            emit(m++, qx, qy);
+// XOR of table entries: in registers for the part layouts, straight in the
+// cell's mask for the rows
+template <MaskLayout ML>
+struct MaskAcc {
+    static constexpr int W = ML == ML_U16 ? 5 : 18;
+    uint32_t w[W];
+    unsigned flags;
+    uint32_t* dst;
+    __device__ __forceinline__ MaskAcc(uint32_t* d, int) : flags(0), dst(d)
+    {
+#pragma unroll
+        for (int k = 0; k < W; k++) w[k] = 0;
+    }
+    __device__ __forceinline__ void add(const uint32_t* e)
+    {
+        const uint4* q = reinterpret_cast<const uint4*>(e);
+        if constexpr (ML == ML_U16) {
+            const uint4 a = __ldg(q);
+            const uint32_t b = __ldg(e + 4);
+            w[0] ^= a.x; w[1] ^= a.y; w[2] ^= a.z; w[3] ^= a.w;
+            w[4] ^= b & 0xFFFFu;
+            flags += b >> 16;
         } else {
-            const int L = code >> 2, ddx = dir_di(L), ddy = dir_dj(L);
-            const int np = nb_pattern(L);
-            const uint64_t ne = __ldg(&g_hull_lut[np]);
-            const int nn = (int)(ne & 0xF);
-            // index of the neighbour hull vertex at this vertex's position
-            // (quarter units in the neighbour's frame), else 0
-            const int tqx = (px - kUnit * ddx) / (kUnit / 4) + 1, tqy = (py - kUnit * ddy) / (kUnit / 4) + 1;
-            int op = 0;
-            if (tqx >= 0 && tqx < 8 && tqy >= 0 && tqy < 8) {
-                const uint64_t key = (uint64_t)(tqx | (tqy << 3)) * 0x041041041041ull;
-                const uint64_t x = ((ne >> 4) & 0xFFFFFFFFFFFFull) ^ key;
-                uint64_t zero = (x - 0x041041041041ull) & ~x & 0x820820820820ull;
-                zero &= (1ull << (6 * nn)) - 1ull; // only the hull's own vertices
-                if (zero) op = (__ffsll((long long)zero) - 1) / 6;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const uint4 a = __ldg(q + k);
+                w[4 * k] ^= a.x; w[4 * k + 1] ^= a.y; w[4 * k + 2] ^= a.z; w[4 * k + 3] ^= a.w;
             }
-            const uint32_t nq = __ldg(&g_qr_lut[np * 8 + op]);
-            int ax, ay;
-            if (kind == 2) { // previous edge linked: the neighbour's R
-                ax = (int8_t)((nq >> 16) & 0xFF);
-                ay = (int8_t)(nq >> 24);
-            } else { // current edge linked: the neighbour's Q
-                ax = (int8_t)(nq & 0xFF);
-                ay = (int8_t)((nq >> 8) & 0xFF);
-            }
-            ax += kUnit * ddx;
-            ay += kUnit * ddy;
-            if (kind == 2) {
-                emit(m++, (qx + ax) / 2, (qy + ay) / 2);
-                emit(m++, qx, qy);
-            } else {
-                emit(m++, rx, ry);
-                emit(m++, (rx + ax) / 2, (ry + ay) / 2);
-            }
+            const uint4 a = __ldg(q + 4);
+            w[16] ^= a.x; w[17] ^= a.y;
+            flags += a.z;
         }
     }
-    return m;
-}
-
-// Coverage of a polygon that is not star-shaped around its cell centre: the
-// reference's own ear clip, triangle by triangle. Returns the ear count.
-__device__ __noinline__ int ear_clip_mask(const Packed& P, int u, int mlo, int F, uint32_t* rows, int rstride)
-{
-    bool ok;
-    return ear_clip_packed(
-        P,
-        [&](int ax, int ay, int bx, int by, int cx, int cy) {
-            tri_mask(ax * u, ay * u, bx * u, by * u, cx * u, cy * u, mlo, F, rows, rstride);
-        },
-        ok);
-}
-
-// Footprint mask rows (F words at rows[r * rstride]) and spill bits of one
-// subdivided cell. G(dx, dy) is the graph byte of the cell at that offset
-// (0 outside the image, bits toward outside cleared); TJ(px, py) the corner
-// test.
-// The cut polygon of a subdivided cell (G(dx, dy): graph byte of the cell at
-// that offset, 0 outside the image, bits toward outside cleared; TJ(px, py):
-// the corner test).
-template <typename GraphAt, typename TJ, typename Emit>
-__device__ __forceinline__ int cell_polygon_emit(GraphAt G, TJ tj, Emit emit)
-{
-    const unsigned node = G(0, 0);
-    const int pat = cell_pattern(node, G(-1, 0), G(1, 0));
-    const uint64_t e = __ldg(&g_hull_lut[pat]);
-    auto nb_pattern = [&](int L) -> int {
-        const int dx = dir_di(L), dy = dir_dj(L);
-        return cell_pattern(G(dx, dy), G(dx - 1, dy), G(dx + 1, dy));
-    };
-    return subdivide_tables(pat, e, nb_pattern, tj, emit);
-}
-
-// The cut polygon in registers.
-template <typename GraphAt, typename TJ>
-__device__ __forceinline__ void cell_polygon(GraphAt G, TJ tj, Packed& sp)
-{
-    sp.x0 = sp.x1 = sp.y0 = sp.y1 = 0;
-    sp.n = cell_polygon_emit(G, tj, [&](int t, int x, int y) { pk_put(sp, t, x, y); });
-}
-
-// The cut polygon written straight into 9 parked words (rows[0..3] the x
-// bytes, rows[4..7] the y bytes, rows[8] the count: park_polygon's layout),
-// one byte store per coordinate.
-template <typename GraphAt, typename TJ>
-__device__ __forceinline__ void cell_polygon_parked(GraphAt G, TJ tj, uint32_t* rows)
-{
+    __device__ __forceinline__ void store() const
+    {
 #pragma unroll
-    for (int r = 0; r < 8; r++) rows[r] = 0u;
-    uint8_t* xb = reinterpret_cast<uint8_t*>(rows);
-    uint8_t* yb = xb + 16;
-    rows[8] = (uint32_t)cell_polygon_emit(G, tj, [&](int t, int x, int y) {
-        xb[t] = (uint8_t)x;
-        yb[t] = (uint8_t)y;
-    });
-}
-
-// Coverage rows of a cut polygon and its spill bits (0 when the ear clip
-// gives up, as the reference then draws nothing for the cell).
-__device__ __forceinline__ unsigned polygon_mask(const Packed& sp, const MaskGeom& Gm, uint32_t* rows, int rstride)
-{
-    for (int r = 0; r < Gm.F; r++) rows[r * rstride] = 0;
-    const int u = 4 * Gm.s;
-    int mnx, mny, mxx, mxy;
-    // a star-shaped polygon is simple: the reference's ear clip would tile it
-    // exactly, so its crossing-number mask is the coverage
-    if (!star_crossing_mask(sp, u, Gm.mlo, Gm.F, rows, rstride, mnx, mny, mxx, mxy)) {
-        for (int r = 0; r < Gm.F; r++) rows[r * rstride] = 0;
-        if (ear_clip_mask(sp, u, Gm.mlo, Gm.F, rows, rstride) == 0) return 0;
+        for (int k = 0; k < W; k++) dst[k] = w[k];
     }
-    return spill_bits(mnx, mny, mxx, mxy);
+};
+template <>
+struct MaskAcc<ML_ROWS> {
+    uint32_t* dst;
+    int F;
+    unsigned flags;
+    __device__ __forceinline__ MaskAcc(uint32_t* d, int F_) : dst(d), F(F_), flags(0)
+    {
+        for (int r = 0; r < F; r++) dst[r] = 0;
+    }
+    __device__ __forceinline__ void add(const uint32_t* e)
+    {
+        for (int r = 0; r < F; r++) dst[r] ^= __ldg(e + r);
+        flags += __ldg(e + F);
+    }
+    __device__ __forceinline__ void store() const {}
+};
+
+// Mask of a subdivided cell as the XOR of its pieces. pat, g: its pattern and
+// its graph byte in the tile window (rows of `pitch` bytes); keep_of(corner
+// classes) the corners (bits 0-3, as CutTables::corners) that the T-junction
+// test keeps, bit 4 when it keeps every vertex.
+template <MaskLayout ML, typename Keep>
+__device__ __forceinline__ void cut_cell_mask(MaskAcc<ML>& acc, int pat, const uint8_t* g, int pitch, const uint32_t* lut,
+                                              int ES, Keep keep_of)
+{
+    const uint4 ed = __ldg(&g_cut.edges[pat]);
+    const uint32_t corners = __ldg(&g_cut.corners[pat]);
+    acc.add(lut + (size_t)(kCutEntry + pat) * ES);
+    // the edges' loads in two rounds, each round's in flight together
+    const uint32_t e4[4] = {ed.x, ed.y, ed.z, ed.w};
+    int cls[4];
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+        cls[t] = 0;
+        if (e4[t]) {
+            const int L = (int)(e4[t] >> 20) & 7;
+            const uint8_t* nb = g + dir_dj(L) * pitch + dir_di(L);
+            cls[t] = __ldg(&g_cut.nb_class[((e4[t] >> 16) & 15u) * 4096 + cell_pattern(nb[0], nb[-1], nb[1])]);
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < 4; t++)
+        if (e4[t]) acc.add(lut + (size_t)(kPathEntry + (int)(e4[t] & 0xFFFFu) + cls[t]) * ES);
+    const unsigned keep = keep_of(corners);
+    if (keep & 16u) {
+        const uint64_t verts = __ldg(&g_cut.verts[pat]);
+#pragma unroll 1
+        for (int v = 0; v < 8; v++) {
+            const int id = (int)(verts >> (8 * v)) & 0xFF;
+            if (id != 0xFF) acc.add(lut + (size_t)(kCornerEntry + id) * ES);
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int id = (int)(corners >> (8 * c)) & 0xFF;
+            if (((keep >> c) & 1u) && id != 0xFF) acc.add(lut + (size_t)(kCornerEntry + id) * ES);
+        }
+    }
 }
 
-// A cut polygon parked in its own cell's mask rows until the mask is made
-// (rows[0..3] the x bytes, rows[4..7] the y bytes, rows[8] the count, as
-// cell_polygon_parked writes it), and a 64-bit mix of it for the tile's table
-// of distinct polygons.
-__device__ __forceinline__ void unpark_polygon(const uint32_t* rows, Packed& sp)
+// The four corner tests (checkTJunction, subdivision_functions.cu:170-242) of
+// a cell off the image's edge, px its pixel in the tile (rows of PW words):
+// bit c set when the corner's neighbour colours differ.
+__device__ __forceinline__ unsigned corner_tests(const uint32_t* px, int PW)
 {
-    sp.x0 = rows[0] | (uint64_t)rows[1] << 32;
-    sp.x1 = rows[2] | (uint64_t)rows[3] << 32;
-    sp.y0 = rows[4] | (uint64_t)rows[5] << 32;
-    sp.y1 = rows[6] | (uint64_t)rows[7] << 32;
-    sp.n = (int)rows[8];
+    auto ne = [&](int a, int b) -> unsigned { return ((px[a] ^ px[b]) & 0x00FFFFFFu) != 0; };
+    return (ne(-1, -PW - 1) | ne(-PW - 1, -PW)) | (ne(1, -PW + 1) | ne(-PW + 1, -PW)) << 1 |
+           (ne(PW, PW + 1) | ne(PW + 1, 1)) << 2 | (ne(PW - 1, PW) | ne(PW, -1)) << 3;
 }
 
-__device__ __forceinline__ uint64_t polygon_hash(const Packed& sp)
+// Colour (B | G << 8 | R << 16) that the reference's linear addressing reads
+// at the pixel (i, j) one column outside the image (i = -1 or w) or above it:
+// bytes of the rows before and after, of a row's padding (for RGBA input that
+// of the 4-byte aligned BGR rows the reference would have loaded: zeros), or
+// zero outside the buffer.
+template <int LAYOUT>
+__device__ uint32_t wrapped_colour(const uint8_t* img, int ws, int w, int h, int i, int j)
 {
-    uint64_t h = sp.x0 ^ (sp.x1 * 0x9E3779B97F4A7C15ull) ^ ((sp.y0 << 1 | sp.y0 >> 63) * 0xC2B2AE3D27D4EB4Full) ^
-                 ((sp.y1 << 7 | sp.y1 >> 57) * 0x165667B19E3779F9ull) ^ (uint64_t)sp.n;
-    h ^= h >> 33;
-    h *= 0xFF51AFD7ED558CCDull;
-    h ^= h >> 33;
-    h *= 0xC4CEB9FE1A85EC53ull;
-    h ^= h >> 33;
-    return h;
+    if (LAYOUT == DEPIX_LAYOUT_BGR) {
+        uint32_t c = 0;
+        const long long off = (long long)j * ws + 3LL * i, end = (long long)h * ws;
+        for (int b = 0; b < 3; b++)
+            if (off + b >= 0 && off + b < end) c |= (uint32_t)__ldg(img + off + b) << (8 * b);
+        return c;
+    }
+    const int pad = 8 * (((3 * w + 3) & ~3) - 3 * w); // bits of padding after a row
+    if (i < 0) return j >= 1 && j <= h ? load_bgr(img, ws, LAYOUT, w - 1, j - 1) >> pad : 0u;
+    if (i >= w) return j + 1 < h ? (load_bgr(img, ws, LAYOUT, 0, j + 1) << pad) & 0x00FFFFFFu : 0u;
+    return 0u; // above the last row
+}
+
+// The corner tests of a cell on the image's edge (as corner_tests), bit 4 when
+// the reference's bounds test keeps every vertex. Neighbours outside the image
+// as its linear addressing reads them, the others from the tile's pixels px
+// (rows of PW words).
+template <int LAYOUT>
+__device__ __noinline__ unsigned edge_corner_tests(const uint32_t* px, int PW, const uint8_t* img, int ws, int w, int h,
+                                                   int ci, int cj)
+{
+    const long long st = LAYOUT == DEPIX_LAYOUT_BGR ? ws : ((3 * w + 3) & ~3);
+    const long long index = (long long)cj * st + (long long)ci * 3;
+    if ((index - st - 1) < 0 || (index + w + 1) > ((long long)h * st - 1)) return 16u;
+    auto at = [&](int dx, int dy) -> uint32_t {
+        const int i = ci + dx, j = cj + dy;
+        if (i < 0 || i >= w || j >= h) return wrapped_colour<LAYOUT>(img, ws, w, h, i, j);
+        const uint32_t c = px[dy * PW + dx];
+        return ((c >> 16) & 0xFFu) | (c & 0xFF00u) | ((c & 0xFFu) << 16);
+    };
+    const uint32_t l = at(-1, 0), r = at(1, 0), d = at(0, -1), u = at(0, 1);
+    const uint32_t dl = at(-1, -1), dr = at(1, -1), ul = at(-1, 1), ur = at(1, 1);
+    return (unsigned)(l != dl || dl != d) | (unsigned)(r != dr || dr != d) << 1 | (unsigned)(u != ur || ur != r) << 2 |
+           (unsigned)(ul != u || u != l) << 3;
 }
 
 template <int LAYOUT, int S, int TW, int TH, bool TMA = false>
-__device__ void mask_raster_tile(MaskTile<TW, TH>& M, uint32_t* masks, const uint8_t* img, int ws, const uint8_t* g,
+__device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const uint8_t* img, int ws, const uint8_t* g,
                                  uint8_t* out, int w, int h, int scale, bool subdivide, const uint32_t* lut, int x0,
                                  int y0, const CUtensorMap* pix_map = nullptr, int frame = 0,
                                  const CUtensorMap* graph_map = nullptr)
 {
-    using T = MaskTile<TW, TH>;
+    using T = MaskTile<S, TW, TH>;
+    constexpr MaskLayout ML = mode_layout(S);
     const int s = S > 0 ? S : scale;
-    const MaskGeom G = mask_geom(s);
-    const int F = G.F;
+    const int MS = mask_stride(s), ES = entry_words(s), MW = mask_words(s);
+    constexpr uint32_t kAlpha = 0xFF000000u;
     // ---- phase A
     if constexpr (TMA) {
         // the pixel window (x0 - 4 .. x0 + TW + 4) x (y0 - 2 .. y0 + TH + 2)
@@ -863,10 +1135,7 @@ __device__ void mask_raster_tile(MaskTile<TW, TH>& M, uint32_t* masks, const uin
     if (threadIdx.x == 0) {
         M.count = 0;
         M.slow = 0;
-        M.nreps = 0;
-        M.nmakers = 0;
     }
-    for (int k = threadIdx.x; k < kPolyTable; k += blockDim.x) M.table[k] = 0ull;
     if (!(TMA && graph_map)) {
         for (int k = threadIdx.x; k < T::BW * T::BH; k += blockDim.x) {
             int gx = x0 - 3 + k % T::BW, gy = y0 - 3 + k / T::BW;
@@ -876,17 +1145,11 @@ __device__ void mask_raster_tile(MaskTile<TW, TH>& M, uint32_t* masks, const uin
         }
     }
     if constexpr (TMA) {
-        // the box holds RGBA words; the tile works on the reference's byte
-        // order (b0, b1, b2) = (B, G, R), as load_bgr gives it
         if (threadIdx.x == 0) {
             M.tma_ok = tma_wait_or_flag(&M.bar, &g_raster_fault) ? 1 : 0;
         }
         __syncthreads();
         if (!M.tma_ok) return;
-        for (int k = threadIdx.x; k < T::CH * (T::CW + 4); k += blockDim.x) {
-            uint32_t& v = M.pix[k / (T::CW + 4)][k % (T::CW + 4)];
-            v = ((v >> 16) & 0xFFu) | (v & 0xFF00u) | ((v & 0xFFu) << 16);
-        }
         // graph bytes on the image's edge lose their bits toward outside (the
         // box reads zero beyond the image); only tiles that reach an edge
         if (graph_map && (x0 < 3 || y0 < 3 || x0 + TW + 3 > w || y0 + TH + 3 > h)) {
@@ -895,295 +1158,217 @@ __device__ void mask_raster_tile(MaskTile<TW, TH>& M, uint32_t* masks, const uin
                 if (gx >= 0 && gy >= 0 && gx < w && gy < h)
                     M.graph[k / T::BW][k % T::BW + T::kGOff] &= (uint8_t)inside_mask(gx, gy, w, h);
             }
+            __syncthreads();
         }
     } else {
         for (int k = threadIdx.x; k < T::CW * T::CH; k += blockDim.x) {
             int gx = x0 - 2 + k % T::CW, gy = y0 - 2 + k / T::CW;
             uint32_t v = 0;
-            if (gx >= 0 && gy >= 0 && gx < w && gy < h) v = load_bgr(img, ws, LAYOUT, gx, gy);
+            if (gx >= 0 && gy >= 0 && gx < w && gy < h) v = load_rgba<LAYOUT>(img, ws, gx, gy);
             M.pix[k / T::CW][k % T::CW + 2] = v;
         }
+        __syncthreads();
     }
-    __syncthreads();
 
     // ---- phase B: plain cells from the table, subdivided cells to the list
-    for (int k = threadIdx.x; k < T::GN; k += blockDim.x) {
-        int lx = k % T::GW, ly = k / T::GW;
-        int ci = x0 - 1 + lx, cj = y0 - 1 + ly;
-        uint32_t* rows = masks + (size_t)k * F;
-        bool live = ci >= 0 && cj >= 0 && ci < w && cj < h;
-        M.live[k] = live;
-        M.spill[k] = 0;
-        if (!live) {
-            for (int r = 0; r < F; r++) rows[r] = 0;
-            continue;
+    for (int k0 = 0; k0 < T::GN; k0 += blockDim.x) {
+        const int k = k0 + threadIdx.x;
+        bool cut = false;
+        if (k < T::GN) {
+            const int lx = k % T::GW, ly = k / T::GW;
+            const int ci = x0 - 1 + lx, cj = y0 - 1 + ly;
+            uint32_t* dst = masks + k * MS;
+            if (ci < 0 || cj < 0 || ci >= w || cj >= h) {
+                for (int r = 0; r < MW; r++) dst[r] = 0;
+            } else {
+                const uint8_t* gb = &M.graph[ly + 2][lx + 2 + T::kGOff];
+                const unsigned node = gb[0];
+                cut = subdivide && node != 90;
+                if (!cut) {
+                    if (ML == ML_U16 && node == 90) {
+                        // linked on its four sides only: its own square
+                        dst[0] = dst[1] = dst[3] = dst[4] = 0;
+                        dst[2] = T::kFull; // part 4
+                    } else {
+                        MaskAcc<ML> acc(dst, MW);
+                        acc.add(lut + (size_t)(kPlainEntry + cell_pattern(node, gb[-1], gb[1])) * ES);
+                        acc.store();
+                    }
+                }
+            }
         }
-        const int bx = lx + 2, by = ly + 2;
-        unsigned node = M.graph[by][bx + T::kGOff];
-        if (subdivide && node != 90) {
-            int slot = atomicAdd(&M.count, 1);
-            M.list[slot] = (uint16_t)k;
-            continue;
-        }
-        int pat = cell_pattern(node, M.graph[by][bx - 1 + T::kGOff], M.graph[by][bx + 1 + T::kGOff]);
-        const int dr = G.hlo - G.mlo; // hull window row/column offset inside the footprint
-        const uint32_t* src = lut + (size_t)pat * G.HF;
-        for (int r = 0; r < F; r++) {
-            int q = r - dr;
-            rows[r] = (q >= 0 && q < G.HF) ? (__ldg(src + q) << dr) : 0u;
-        }
-        M.spill[k] = __ldg(&g_spill_lut[pat]);
+        const int slot = list_slot(&M.count, cut);
+        if (cut) M.list[slot] = (uint16_t)k;
     }
     __syncthreads();
 
-    // ---- phase B2: subdivided cells
-    // A cut polygon is a function of the 5x3 graph bytes around its cell and
-    // of the corner tests (tj) at the four cell corners, and its mask is a
-    // function of the polygon. So (B2a) each cell keys itself by those inputs
-    // and one cell per distinct key builds the polygon (B2b), one builder per
-    // distinct polygon makes the mask (B2c), and the others copy (B2d). Cells
-    // whose corner test goes through the reference's bounds test or linear
-    // addressing (image edges) build on their own.
+    // ---- phase B2: subdivided cells, XORed from their pieces
     const int nlist = M.count;
-    auto cell_at = [&](int k, int& lx, int& ly, int& ci, int& cj, bool& border) {
-        lx = k % T::GW;
-        ly = k / T::GW;
-        ci = x0 - 1 + lx;
-        cj = y0 - 1 + ly;
-        const long long st = LAYOUT == DEPIX_LAYOUT_BGR ? ws : ((3 * w + 3) & ~3);
-        const long long index = (long long)cj * st + (long long)ci * 3;
-        border = (index - st - 1) < 0 || (index + w + 1) > ((long long)h * st - 1) || ci == 0 || ci == w - 1 ||
-                 cj >= h - 1;
-    };
-    // corner test at vertex (px, py) of the cell at tile position (lx, ly)
-    auto tj_of = [&](int lx, int ly, int ci, int cj, bool border, int px, int py) -> bool {
-        if (border) {
-            const long long st = LAYOUT == DEPIX_LAYOUT_BGR ? ws : ((3 * w + 3) & ~3);
-            const long long index = (long long)cj * st + (long long)ci * 3;
-            if ((index - st - 1) < 0 || (index + w + 1) > ((long long)h * st - 1)) return true;
-            return t_junction_global(img, w, h, ws, LAYOUT, ci, cj, px, py);
-        }
-        const int qx = lx + 1, qy = ly + 1;
-        auto C = [&](int dx, int dy) { return M.pix[qy + dy][qx + dx + 2]; };
-        if (px == 0 && py == 0) return C(-1, 0) != C(-1, -1) || C(-1, -1) != C(0, -1);
-        if (px == kUnit && py == 0) return C(1, 0) != C(1, -1) || C(1, -1) != C(0, -1);
-        if (px == kUnit && py == kUnit) return C(0, 1) != C(1, 1) || C(1, 1) != C(1, 0);
-        if (px == 0 && py == kUnit) return C(-1, 1) != C(0, 1) || C(0, 1) != C(-1, 0);
-        return false;
-    };
-    // insert-or-find in one half of the table: the list entry whose parked
-    // words equal this entry's (same(rq)), or q when q took a free slot or
-    // the probes ran out
-    auto dedupe = [&](uint64_t hs, int half, int q, auto same) -> int {
-        const unsigned long long tag = hs & ~0xFFFFull;
-        constexpr int kHalf = kPolyTable / 2;
-        int slot = (int)(hs >> 16) & (kHalf - 1);
-        for (int probe = 0; probe < kPolyProbes; probe++, slot = (slot + 1) & (kHalf - 1)) {
-            unsigned long long* e = &M.table[half * kHalf + slot];
-            unsigned long long cur = *e;
-            if (cur == 0ull) {
-                cur = atomicCAS(e, 0ull, tag | (unsigned long long)(q + 1));
-                if (cur == 0ull) return q;
-            }
-            if ((cur & ~0xFFFFull) == tag) {
-                const int rq = (int)(cur & 0xFFFFull) - 1;
-                if (same(rq)) return rq;
-            }
-        }
-        return q;
-    };
-    // B2a
     for (int q = threadIdx.x; q < nlist; q += blockDim.x) {
-        const int k = M.list[q];
-        int lx, ly, ci, cj;
-        bool border;
-        cell_at(k, lx, ly, ci, cj, border);
-        const int bx = lx + 2, by = ly + 2;
-        uint32_t* rows = masks + (size_t)k * F;
-        if (F < 10) { // no room to park keys or polygons: every cell makes its mask
-            auto Gs = [&](int dx, int dy) -> unsigned { return M.graph[by + dy][bx + dx + T::kGOff]; };
-            auto tj = [&](int px, int py) -> bool { return tj_of(lx, ly, ci, cj, border, px, py); };
-            Packed sp;
-            cell_polygon(Gs, tj, sp);
-            M.spill[k] = (uint8_t)polygon_mask(sp, G, rows, 1);
-            continue;
-        }
-        int rep = q;
-        if (!border) {
-            auto B = [&](int dx, int dy) -> uint32_t { return M.graph[by + dy][bx + dx + T::kGOff]; };
-            const uint32_t corners = (uint32_t)tj_of(lx, ly, ci, cj, false, 0, 0) |
-                                     (uint32_t)tj_of(lx, ly, ci, cj, false, kUnit, 0) << 1 |
-                                     (uint32_t)tj_of(lx, ly, ci, cj, false, kUnit, kUnit) << 2 |
-                                     (uint32_t)tj_of(lx, ly, ci, cj, false, 0, kUnit) << 3;
-            const uint32_t w0 = B(-2, -1) | B(-1, -1) << 8 | B(0, -1) << 16 | B(1, -1) << 24;
-            const uint32_t w1 = B(2, -1) | B(-2, 0) << 8 | B(-1, 0) << 16 | B(0, 0) << 24;
-            const uint32_t w2 = B(1, 0) | B(2, 0) << 8 | B(-2, 1) << 16 | B(-1, 1) << 24;
-            const uint32_t w3 = B(0, 1) | B(1, 1) << 8 | B(2, 1) << 16 | corners << 24;
-            rows[0] = w0;
-            rows[1] = w1;
-            rows[2] = w2;
-            rows[3] = w3;
-            __threadfence_block();
-            Packed kp;
-            kp.x0 = w0 | (uint64_t)w1 << 32;
-            kp.x1 = w2 | (uint64_t)w3 << 32;
-            kp.y0 = kp.y1 = 0;
-            kp.n = 0;
-            rep = dedupe(polygon_hash(kp), 0, q, [&](int rq) {
-                const uint32_t* o = masks + (size_t)M.list[rq] * F;
-                return o[0] == w0 && o[1] == w1 && o[2] == w2 && o[3] == w3;
-            });
-        }
-        M.rep[q] = (uint16_t)rep;
-        if (rep == q) M.reps[atomicAdd(&M.nreps, 1)] = (uint16_t)q;
+        const int k = M.list[q], lx = k % T::GW, ly = k / T::GW;
+        const int ci = x0 - 1 + lx, cj = y0 - 1 + ly;
+        const uint8_t* gb = &M.graph[ly + 2][lx + 2 + T::kGOff];
+        const uint32_t* px = &M.pix[ly + 1][lx + 3];
+        constexpr int PW = T::CW + 4;
+        const int pat = cell_pattern(gb[0], gb[-1], gb[1]);
+        const bool edge = ci == 0 || cj == 0 || ci == w - 1 || cj == h - 1;
+        unsigned keep = edge ? edge_corner_tests<LAYOUT>(px, PW, img, ws, w, h, ci, cj) : 0u;
+        MaskAcc<ML> acc(masks + k * MS, MW);
+        cut_cell_mask(acc, pat, gb, T::GRW, lut, ES, [&](uint32_t corners) {
+            if (!edge && corners != 0xFFFFFFFFu) keep = corner_tests(px, PW);
+            return keep;
+        });
+        if ((acc.flags & 0xFFFFu) == 1u) acc.store();
+        else ear_clip_cell_mask(gb, T::GRW, keep, s, masks + k * MS); // not star-shaped
     }
     __syncthreads();
-    if (F >= 10) {
-        // B2b: one polygon per distinct key, parked in its cell's rows; the
-        // builder's rep becomes the builder whose polygon (and mask) it shares
-        const int nb = M.nreps;
-        uint16_t* makers = reinterpret_cast<uint16_t*>(M.table); // the key half, free now
-        for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-            const int q = M.reps[i], k = M.list[q];
-            int lx, ly, ci, cj;
-            bool border;
-            cell_at(k, lx, ly, ci, cj, border);
-            const int bx = lx + 2, by = ly + 2;
-            auto Gs = [&](int dx, int dy) -> unsigned { return M.graph[by + dy][bx + dx + T::kGOff]; };
-            auto tj = [&](int px, int py) -> bool { return tj_of(lx, ly, ci, cj, border, px, py); };
-            cell_polygon_parked(Gs, tj, masks + (size_t)k * F);
-            Packed sp;
-            unpark_polygon(masks + (size_t)k * F, sp);
-            __threadfence_block();
-            const int rp = dedupe(polygon_hash(sp), 1, q, [&](int rq) {
-                Packed o;
-                unpark_polygon(masks + (size_t)M.list[rq] * F, o);
-                return o.n == sp.n && o.x0 == sp.x0 && o.x1 == sp.x1 && o.y0 == sp.y0 && o.y1 == sp.y1;
-            });
-            M.rep[q] = (uint16_t)rp;
-            if (rp == q) makers[atomicAdd(&M.nmakers, 1)] = (uint16_t)q;
-        }
-        __syncthreads();
-        // B2c: the masks
-        const int nm = M.nmakers;
-        for (int i = threadIdx.x; i < nm; i += blockDim.x) {
-            const int k = M.list[makers[i]];
-            uint32_t* rows = masks + (size_t)k * F;
-            Packed sp;
-            unpark_polygon(rows, sp);
-            M.spill[k] = (uint8_t)polygon_mask(sp, G, rows, 1);
-        }
-        __syncthreads();
-        // B2d: copies (key rep -> its polygon's mask maker)
-        for (int q = threadIdx.x; q < nlist; q += blockDim.x) {
-            const int rq = M.rep[M.rep[q]];
-            if (rq == q) continue;
-            const int k = M.list[q], rk = M.list[rq];
-            const uint32_t* src = masks + (size_t)rk * F;
-            uint32_t* dst = masks + (size_t)k * F;
-            for (int r = 0; r < F; r++) dst[r] = src[r];
-            M.spill[k] = M.spill[rk];
-        }
-        __syncthreads();
-    }
 
-    // ---- phase C: one output block per tile cell
+    // ---- phase C: output blocks (one per tile cell). Candidate q = 0..8 of a
+    // block is the cell at (1 - q % 3, 1 - q / 3) from it: VBO order from the
+    // latest (row above, right to left) to the earliest; its part over the
+    // block is part q of its mask.
     const int ow = w * s;
-    const bool vec = ((S == 4 || S == 8) && (ow % 4) == 0 && ((reinterpret_cast<uintptr_t>(out) & 15) == 0));
-    const uint32_t blockbits = (s >= 32) ? 0xFFFFFFFFu : ((1u << s) - 1u);
-    for (int q = threadIdx.x; q < TW * TH; q += blockDim.x) {
-        int tx = q % TW, ty = q / TW;
-        int ci = x0 + tx, cj = y0 + ty;
-        if (ci >= w || cj >= h) continue;
-        const int k0 = (ty + 1) * T::GW + (tx + 1);
-        unsigned intr = 0;
+    const bool vec = (S == 4 || S == 8) && (ow % 4) == 0 && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
+    const uint32_t blockbits = (1u << s) - 1u;
+    auto cand = [&](int k, int q) -> const uint32_t* { return masks + (k + (1 - q / 3) * T::GW + 1 - q % 3) * MS; };
+    // row r of the block as candidate q covers it
+    auto part_row = [&](int k, int q, int r) -> uint32_t {
+        const uint32_t* m = cand(k, q);
+        if constexpr (ML == ML_U16) {
+            return (reinterpret_cast<const uint16_t*>(m)[q] >> (r * s)) & blockbits;
+        } else if constexpr (ML == ML_U64) {
+            return (uint32_t)(((uint64_t)m[2 * q + 1] << 32 | m[2 * q]) >> (r * s)) & blockbits;
+        } else {
+            const MaskGeom G = mask_geom(s);
+            const int rr = r - s * (1 - q / 3) - G.mlo, sh = s * (1 - q % 3) + G.mlo;
+            if (rr < 0 || rr >= G.F) return 0u;
+            const uint64_t b = m[rr];
+            return (uint32_t)(sh >= 0 ? b << sh : b >> -sh) & blockbits;
+        }
+    };
+    constexpr int NG = T::NG;
+    constexpr int GR = S == 8 ? 2 : (S > 0 ? S : 1); // rows of a group
+    constexpr uint32_t kFull = T::kFull;
+    auto group = [&](int k, int q, int gr) -> uint32_t { // candidate q's part over the group
+        const uint16_t* m = reinterpret_cast<const uint16_t*>(cand(k, q));
+        return m[S == 8 ? 4 * q + gr : q];
+    };
+    for (int i = threadIdx.x; i < TW * TH * NG; i += blockDim.x) {
+        const int q = i % (TW * TH), gr = i / (TW * TH);
+        const int tx = q % TW, ty = q / TW;
+        const int ci = x0 + tx, cj = y0 + ty;
+        const bool in = ci < w && cj < h;
+        const int k = (ty + 1) * T::GW + tx + 1;
+        // filled at once: its own cell covers all of it and no later one any
+        bool fill = false;
+        if (in) {
+            if constexpr (S > 0) {
+                fill = group(k, 4, gr) == kFull &&
+                       (group(k, 0, gr) | group(k, 1, gr) | group(k, 2, gr) | group(k, 3, gr)) == 0;
+            } else {
+                fill = true;
+                for (int r = 0; r < s && fill; r++)
+                    fill = part_row(k, 4, r) == blockbits &&
+                           (part_row(k, 0, r) | part_row(k, 1, r) | part_row(k, 2, r) | part_row(k, 3, r)) == 0;
+            }
+        }
+        const int slot = list_slot(&M.slow, in && !fill);
+        if (in && !fill) M.list[slot] = (uint16_t)i; // resolved after the barrier, over a compacted list
+        if (!fill) continue;
+        const uint32_t col = M.pix[ty + 2][tx + 4] | kAlpha;
+        uint8_t* orow = out + (((size_t)cj * s + gr * GR) * ow + (size_t)ci * s) * 4;
+        const int rows = S > 0 ? GR : s;
 #pragma unroll
-        for (int e = 0; e < 8; e++) {
-            int kn = k0 + dir_dj(e) * T::GW + dir_di(e);
-            intr |= (unsigned)bitof(M.spill[kn], 7 - e);
-        }
-        const uint32_t* own = masks + (size_t)k0 * F;
-        bool full = true;
-        for (int r = 0; r < s; r++) full &= ((own[r - G.mlo] >> (-G.mlo)) & blockbits) == blockbits;
-        if (!full || intr) {
-            // owner resolution after the barrier, over a compacted list, so
-            // that warps do not run it beside blocks that need none
-            M.list[atomicAdd(&M.slow, 1)] = (uint16_t)q;
-            continue;
-        }
-        const uint32_t own_col = rgba_of(M.pix[ty + 2][tx + 4]);
-        uint8_t* orow = out + ((size_t)cj * s * ow + (size_t)ci * s) * 4;
-        for (int r = 0; r < s; r++) {
+        for (int r = 0; r < rows; r++) {
             uint32_t* o = reinterpret_cast<uint32_t*>(orow + (size_t)r * ow * 4);
             if (vec) {
-                for (int c4 = 0; c4 < s; c4 += 4)
-                    __stcs(reinterpret_cast<uint4*>(o + c4), make_uint4(own_col, own_col, own_col, own_col));
+#pragma unroll
+                for (int c4 = 0; c4 < S; c4 += 4) __stcs(reinterpret_cast<uint4*>(o + c4), make_uint4(col, col, col, col));
             } else {
-                for (int c = 0; c < s; c++) o[c] = own_col;
+                for (int c = 0; c < s; c++) o[c] = col;
             }
         }
     }
     __syncthreads();
     const int nslow = M.slow;
     for (int qs = threadIdx.x; qs < nslow; qs += blockDim.x) {
-        const int q = M.list[qs];
+        const int i = M.list[qs], q = i % (TW * TH), gr = i / (TW * TH);
         const int tx = q % TW, ty = q / TW;
         const int ci = x0 + tx, cj = y0 + ty;
-        const int k0 = (ty + 1) * T::GW + (tx + 1);
-        uint8_t* orow = out + ((size_t)cj * s * ow + (size_t)ci * s) * 4;
-        // the nine candidates' colours, in priority order
-        uint32_t cand_col[9];
+        const int k = (ty + 1) * T::GW + tx + 1;
+        uint8_t* orow = out + (((size_t)cj * s + gr * GR) * ow + (size_t)ci * s) * 4;
+        const uint32_t* px = &M.pix[ty + 2][tx + 4];
+        auto colour = [&](int q) -> uint32_t { return px[(1 - q / 3) * (T::CW + 4) + 1 - q % 3] | kAlpha; };
+        if constexpr (S > 0) {
+            // candidates from the latest on until every sample has its owner
+            // (each lane walks its own block's owners, so that a warp's trips
+            // are the most owners of a block, not the nine candidates)
+            constexpr int NS = S == 8 ? 16 : S * S, RL = S;
+            uint32_t col[NS], claimed = 0;
+            unsigned owners = 0;
 #pragma unroll
-        for (int z = 0; z < 9; z++) cand_col[z] = rgba_of(M.pix[ty + 2 + 1 - z / 3][tx + 4 + 1 - z % 3]);
-        for (int r = 0; r < s; r++) {
-            // per candidate (priority order q = 0..8: rows above first, then
-            // right to left) the samples of this row it covers and no
-            // earlier candidate does; candidates are one cell apart so the
-            // nine masks are disjoint and each sample has at most one owner
-            uint32_t claimed = 0;
-            uint32_t take[9];
-            int qq = 0;
+            for (int q = 0; q < 9; q++) {
+                const uint32_t m = group(k, q, gr);
+                if (m & ~claimed) owners |= 1u << q;
+                claimed |= m;
+            }
 #pragma unroll
-            for (int dj = 1; dj >= -1; dj--) {
-                const int rr = r - s * dj - G.mlo;
+            for (int c = 0; c < NS; c++) col[c] = kAlpha; // no owner: the clear colour
+            claimed = 0;
+            while (owners) {
+                const int q = __ffs(owners) - 1;
+                owners &= owners - 1;
+                const int dj = 1 - q / 3, di = 1 - q % 3;
+                const uint16_t* mp = reinterpret_cast<const uint16_t*>(masks + (k + dj * T::GW + di) * MS);
+                const uint32_t m = mp[S == 8 ? 4 * q + gr : q], take = m & ~claimed;
+                const uint32_t c0 = px[dj * (T::CW + 4) + di] | kAlpha;
+                claimed |= m;
 #pragma unroll
-                for (int di = 1; di >= -1; di--, qq++) {
-                    take[qq] = 0;
-                    if (rr < 0 || rr >= F) continue;
-                    const int kn = k0 + dj * T::GW + di; // cells outside the image have zero rows
-                    const uint64_t wbits = masks[(size_t)kn * F + rr];
-                    const int sh = s * di + G.mlo; // block column c = footprint column + sh
-                    const uint32_t bits =
-                        (uint32_t)((sh >= 0 ? (wbits << sh) : (wbits >> (-sh))) & blockbits) & ~claimed;
-                    claimed |= bits;
-                    take[qq] = bits;
+                for (int c = 0; c < NS; c++)
+                    if ((take >> c) & 1u) col[c] = c0;
+            }
+#pragma unroll
+            for (int r = 0; r < GR; r++) {
+                uint32_t* o = reinterpret_cast<uint32_t*>(orow + (size_t)r * ow * 4);
+                if (vec) {
+#pragma unroll
+                    for (int c4 = 0; c4 + 3 < RL; c4 += 4)
+                        __stcs(reinterpret_cast<uint4*>(o + c4), make_uint4(col[r * RL + c4], col[r * RL + c4 + 1],
+                                                                            col[r * RL + c4 + 2], col[r * RL + c4 + 3]));
+                } else {
+#pragma unroll
+                    for (int c = 0; c < RL; c++) o[c] = col[r * RL + c];
                 }
             }
-            uint32_t* o = reinterpret_cast<uint32_t*>(orow + (size_t)r * ow * 4);
-            auto owner_colour = [&](int c) -> uint32_t {
-                uint32_t col = 0xFF000000u; // no owner: the clear colour
+        } else {
+            for (int r = 0; r < s; r++) {
+                uint32_t col[12], claimed = 0;
 #pragma unroll
-                for (int q = 0; q < 9; q++)
-                    if ((take[q] >> c) & 1u) col = cand_col[q];
-                return col;
-            };
-            if (vec) {
+                for (int c = 0; c < 12; c++) col[c] = kAlpha;
+#pragma unroll 1
+                for (int q = 0; q < 9; q++) {
+                    const uint32_t m = part_row(k, q, r), take = m & ~claimed;
+                    if (!take) continue;
+                    const uint32_t c0 = colour(q);
 #pragma unroll
-                for (int c4 = 0; c4 < (S > 0 ? S : 16); c4 += 4)
-                    if (c4 < s)
-                        __stcs(reinterpret_cast<uint4*>(o + c4), make_uint4(owner_colour(c4), owner_colour(c4 + 1),
-                                                                            owner_colour(c4 + 2), owner_colour(c4 + 3)));
-            } else {
-                for (int c = 0; c < s; c++) o[c] = owner_colour(c);
+                    for (int c = 0; c < 12; c++)
+                        if ((take >> c) & 1u) col[c] = c0;
+                    claimed |= m;
+                    if (claimed == blockbits) break;
+                }
+                uint32_t* o = reinterpret_cast<uint32_t*>(orow + (size_t)r * ow * 4);
+#pragma unroll
+                for (int c = 0; c < 12; c++)
+                    if (c < s) o[c] = col[c];
             }
         }
     }
 }
 
 template <int LAYOUT, int S, int TH>
-__global__ void __launch_bounds__(256) k_mask_raster(RasterBatch b, const uint32_t* lut)
+__global__ void __launch_bounds__(kRT, raster_blocks(S)) k_mask_raster(RasterBatch b, const uint32_t* lut)
 {
-    __shared__ MaskTile<32, TH> M;
+    __shared__ MaskTile<S, 32, TH> M;
     extern __shared__ uint32_t masks[];
     size_t z = blockIdx.z;
     mask_raster_tile<LAYOUT, S, 32, TH>(M, masks, b.img + b.img_stride * z, b.ws, b.graph + b.graph_stride * z,
@@ -1194,11 +1379,11 @@ __global__ void __launch_bounds__(256) k_mask_raster(RasterBatch b, const uint32
 // The equal-size batch raster with its pixel windows loaded by TMA (RGBA
 // frames whose base, rows and frame stride are 16-byte aligned).
 template <int S, int TH>
-__global__ void __launch_bounds__(256, 3) k_mask_raster_tma(RasterBatch b, const uint32_t* lut,
+__global__ void __launch_bounds__(kRT, raster_blocks(S)) k_mask_raster_tma(RasterBatch b, const uint32_t* lut,
                                                          const __grid_constant__ CUtensorMap pix_map,
                                                          const __grid_constant__ CUtensorMap graph_map, int with_graph)
 {
-    __shared__ MaskTile<32, TH> M;
+    __shared__ MaskTile<S, 32, TH> M;
     extern __shared__ uint32_t masks[];
     size_t z = blockIdx.z;
     mask_raster_tile<DEPIX_LAYOUT_RGBA, S, 32, TH, true>(M, masks, b.img + b.img_stride * z, b.ws,
@@ -1277,15 +1462,21 @@ static bool pixel_tensor_map(const RasterBatch& b, int nframes, int TH, CUtensor
     return rgba_tensor_map(b.img, b.w, b.h, b.ws, b.img_stride, nframes, 32 + 8, TH + 4, map);
 }
 
+// dynamic shared memory: the cells' masks
+template <int S, int TW, int TH>
+static size_t mask_smem(int scale)
+{
+    return (size_t)MaskTile<S, TW, TH>::GN * mask_stride(scale) * sizeof(uint32_t);
+}
+
 template <int LAYOUT, int S, int TH>
 static cudaError_t launch_mask_raster_t(const RasterBatch& b, int nframes, const uint32_t* lut, cudaStream_t s)
 {
     if constexpr (LAYOUT == DEPIX_LAYOUT_RGBA) {
         CUtensorMap map;
         if (pixel_tensor_map(b, nframes, TH, &map)) {
-            MaskGeom g = mask_geom(b.scale);
-            size_t smem = (size_t)MaskTile<32, TH>::GN * g.F * sizeof(uint32_t);
-            if (smem + sizeof(MaskTile<32, TH>) > 48 * 1024) {
+            size_t smem = mask_smem<S, 32, TH>(b.scale);
+            if (smem + sizeof(MaskTile<S, 32, TH>) > 48 * 1024) {
                 cudaError_t e = cudaFuncSetAttribute(k_mask_raster_tma<S, TH>,
                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
                 if (e != cudaSuccess) return e;
@@ -1295,30 +1486,27 @@ static cudaError_t launch_mask_raster_t(const RasterBatch& b, int nframes, const
             const bool with_graph = u8_tensor_map(b.graph, b.w, b.h, b.graph_stride, nframes, 32 + 32, TH + 6, &gmap);
             if (!with_graph) gmap = map; // unused
             dim3 grid((b.w + 32 - 1) / 32, (b.h + TH - 1) / TH, nframes);
-            k_mask_raster_tma<S, TH><<<grid, 256, smem, s>>>(b, lut, map, gmap, with_graph ? 1 : 0);
+            k_mask_raster_tma<S, TH><<<grid, kRT, smem, s>>>(b, lut, map, gmap, with_graph ? 1 : 0);
             return cudaGetLastError();
         }
     }
-    MaskGeom g = mask_geom(b.scale);
-    size_t smem = (size_t)MaskTile<32, TH>::GN * g.F * sizeof(uint32_t);
-    if (smem + sizeof(MaskTile<32, TH>) > 48 * 1024) {
+    size_t smem = mask_smem<S, 32, TH>(b.scale);
+    if (smem + sizeof(MaskTile<S, 32, TH>) > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(k_mask_raster<LAYOUT, S, TH>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
     dim3 grid((b.w + 32 - 1) / 32, (b.h + TH - 1) / TH, nframes);
-    k_mask_raster<LAYOUT, S, TH><<<grid, 256, smem, s>>>(b, lut);
+    k_mask_raster<LAYOUT, S, TH><<<grid, kRT, smem, s>>>(b, lut);
     return cudaGetLastError();
 }
 
 // ---- uneven batches: the raster as a persistent kernel over a tile queue
 
-// three blocks per SM: the persistent loop would otherwise hold the kernel at
-// 116 registers and two blocks (12 % slower on 4096 sprites at x4)
 template <int S, int TW, int TH>
-__global__ void __launch_bounds__(256, 3) k_raster_queue(QueueBatch q)
+__global__ void __launch_bounds__(kRT, raster_blocks(S)) k_raster_queue(QueueBatch q)
 {
-    __shared__ MaskTile<TW, TH> M;
+    __shared__ MaskTile<S, TW, TH> M;
     extern __shared__ uint32_t masks[];
     const QueueHeader* H = q.hdr;
     const int n = H->n;
@@ -1336,18 +1524,12 @@ __global__ void __launch_bounds__(256, 3) k_raster_queue(QueueBatch q)
 }
 
 template <int S, int TW, int TH>
-static size_t raster_queue_smem(int scale)
-{
-    return (size_t)MaskTile<TW, TH>::GN * mask_geom(scale).F * sizeof(uint32_t);
-}
-
-template <int S, int TW, int TH>
 static cudaError_t queue_raster_t(const QueueBatch& q, int blocks, cudaStream_t s)
 {
     // the shared-memory opt-in is made by raster_queue_occupancy, which the
     // host calls on each device before any launch or stream capture
-    const size_t smem = raster_queue_smem<S, TW, TH>(q.scale);
-    k_raster_queue<S, TW, TH><<<blocks, 256, smem, s>>>(q);
+    const size_t smem = mask_smem<S, TW, TH>(q.scale);
+    k_raster_queue<S, TW, TH><<<blocks, kRT, smem, s>>>(q);
     return cudaGetLastError();
 }
 
@@ -1355,33 +1537,32 @@ template <int S, int TW, int TH>
 static int raster_queue_occupancy(int scale)
 {
     int nb = 0;
-    const size_t smem = raster_queue_smem<S, TW, TH>(scale);
-    if (smem + sizeof(MaskTile<TW, TH>) > 48 * 1024 &&
+    const size_t smem = mask_smem<S, TW, TH>(scale);
+    if (smem + sizeof(MaskTile<S, TW, TH>) > 48 * 1024 &&
         cudaFuncSetAttribute(k_raster_queue<S, TW, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
             cudaSuccess)
         return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_raster_queue<S, TW, TH>, 256, smem) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_raster_queue<S, TW, TH>, kRT, smem) != cudaSuccess)
         return 0;
     return nb;
 }
 
 // raster tile variants of the queue path: 32x32, 32x16, 16x16 cells
+#define DEPIX_RQ_SCALES(FN, TW, TH, ...)                                                                \
+    switch (raster_mode(q.scale)) {                                                                     \
+    case 1: return FN<1, TW, TH>(__VA_ARGS__);                                                          \
+    case 2: return FN<2, TW, TH>(__VA_ARGS__);                                                          \
+    case 3: return FN<3, TW, TH>(__VA_ARGS__);                                                          \
+    case 4: return FN<4, TW, TH>(__VA_ARGS__);                                                          \
+    case 8: return FN<8, TW, TH>(__VA_ARGS__);                                                          \
+    case 0: return FN<0, TW, TH>(__VA_ARGS__);                                                          \
+    default: return FN<-1, TW, TH>(__VA_ARGS__);                                                        \
+    }
 #define DEPIX_RQ_DISPATCH(FN, ...)                                                                      \
     do {                                                                                                \
-        const int sc = q.scale == 4 ? 4 : (q.scale == 8 ? 8 : 0);                                       \
-        if (q.rtw == 32 && q.rth == 32) {                                                               \
-            if (sc == 4) return FN<4, 32, 32>(__VA_ARGS__);                                             \
-            if (sc == 8) return FN<8, 32, 32>(__VA_ARGS__);                                             \
-            return FN<0, 32, 32>(__VA_ARGS__);                                                          \
-        }                                                                                               \
-        if (q.rtw == 32) {                                                                              \
-            if (sc == 4) return FN<4, 32, 16>(__VA_ARGS__);                                             \
-            if (sc == 8) return FN<8, 32, 16>(__VA_ARGS__);                                             \
-            return FN<0, 32, 16>(__VA_ARGS__);                                                          \
-        }                                                                                               \
-        if (sc == 4) return FN<4, 16, 16>(__VA_ARGS__);                                                 \
-        if (sc == 8) return FN<8, 16, 16>(__VA_ARGS__);                                                 \
-        return FN<0, 16, 16>(__VA_ARGS__);                                                              \
+        if (q.rtw == 32 && q.rth == 32) DEPIX_RQ_SCALES(FN, 32, 32, __VA_ARGS__)                        \
+        if (q.rtw == 32) DEPIX_RQ_SCALES(FN, 32, 16, __VA_ARGS__)                                       \
+        DEPIX_RQ_SCALES(FN, 16, 16, __VA_ARGS__)                                                        \
     } while (0)
 
 cudaError_t queue_raster(const QueueBatch& q, int blocks, cudaStream_t s)
@@ -1395,22 +1576,26 @@ int queue_raster_blocks_per_sm(const QueueBatch& q) { DEPIX_RQ_DISPATCH(raster_q
 // the work), 32x16 above (the footprint masks grow with the scale)
 // A single frame fills a fraction of the SMs, so it takes tiles half as high
 // at x4 (twice the blocks, each half as long); batches keep the 32-row tiles.
+template <int LAYOUT>
+static cudaError_t launch_mask_raster_l(const RasterBatch& b, int nframes, const uint32_t* lut, cudaStream_t s)
+{
+    switch (raster_mode(b.scale)) {
+    case 1: return launch_mask_raster_t<LAYOUT, 1, 32>(b, nframes, lut, s);
+    case 2: return launch_mask_raster_t<LAYOUT, 2, 32>(b, nframes, lut, s);
+    case 3: return launch_mask_raster_t<LAYOUT, 3, 32>(b, nframes, lut, s);
+    case 4:
+        return nframes == 1 ? launch_mask_raster_t<LAYOUT, 4, 16>(b, nframes, lut, s)
+                            : launch_mask_raster_t<LAYOUT, 4, 32>(b, nframes, lut, s);
+    case 8: return launch_mask_raster_t<LAYOUT, 8, 16>(b, nframes, lut, s);
+    case 0: return launch_mask_raster_t<LAYOUT, 0, 16>(b, nframes, lut, s);
+    default: return launch_mask_raster_t<LAYOUT, -1, 16>(b, nframes, lut, s);
+    }
+}
+
 cudaError_t launch_mask_raster(const RasterBatch& b, int nframes, const uint32_t* lut, cudaStream_t s)
 {
-    if (b.layout == DEPIX_LAYOUT_RGBA) {
-        if (b.scale == 4)
-            return nframes == 1 ? launch_mask_raster_t<DEPIX_LAYOUT_RGBA, 4, 16>(b, nframes, lut, s)
-                                : launch_mask_raster_t<DEPIX_LAYOUT_RGBA, 4, 32>(b, nframes, lut, s);
-        if (b.scale == 8) return launch_mask_raster_t<DEPIX_LAYOUT_RGBA, 8, 16>(b, nframes, lut, s);
-        if (b.scale < 4) return launch_mask_raster_t<DEPIX_LAYOUT_RGBA, 0, 32>(b, nframes, lut, s);
-        return launch_mask_raster_t<DEPIX_LAYOUT_RGBA, 0, 16>(b, nframes, lut, s);
-    }
-    if (b.scale == 4)
-        return nframes == 1 ? launch_mask_raster_t<DEPIX_LAYOUT_BGR, 4, 16>(b, nframes, lut, s)
-                            : launch_mask_raster_t<DEPIX_LAYOUT_BGR, 4, 32>(b, nframes, lut, s);
-    if (b.scale == 8) return launch_mask_raster_t<DEPIX_LAYOUT_BGR, 8, 16>(b, nframes, lut, s);
-    if (b.scale < 4) return launch_mask_raster_t<DEPIX_LAYOUT_BGR, 0, 32>(b, nframes, lut, s);
-    return launch_mask_raster_t<DEPIX_LAYOUT_BGR, 0, 16>(b, nframes, lut, s);
+    return b.layout == DEPIX_LAYOUT_RGBA ? launch_mask_raster_l<DEPIX_LAYOUT_RGBA>(b, nframes, lut, s)
+                                         : launch_mask_raster_l<DEPIX_LAYOUT_BGR>(b, nframes, lut, s);
 }
 
 cudaError_t take_raster_fault(int* out)
@@ -1420,7 +1605,5 @@ cudaError_t take_raster_fault(int* out)
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_raster_fault, &zero, sizeof(int));
     return e;
 }
-
-size_t scale_mask_words(int s) { return (size_t)4096 * mask_geom(s).HF; }
 
 }  // namespace depix
