@@ -9,9 +9,6 @@ namespace depix {
 
 // ------------------------------------------------------------ graph stage
 
-// Pair bits of one pixel p inside the tile region: similarity with the
-// right (bit 0), upper (bit 1), upper-right (bit 2) pixel, and of the pair
-// (right, upper) (bit 3), each only when both pixels are in the image.
 // set when a bounded wait for a TMA tile load gave up (that tile of the
 // graph was left unwritten); read and cleared by depix_take_device_faults
 __device__ int g_graph_fault;
@@ -21,121 +18,235 @@ __device__ int g_heur_fault; // the same for the heuristics stage
 __device__ int g_graph_tma_timeout_test;
 constexpr int kTestPolls = 16;
 
-constexpr int kGTW = 64;  // graph tile width (pixels)
-constexpr int kGTH = 16;  // graph tile height
+// A block of kGThreads threads makes a tile of 64 x (4 GH) nodes: it turns the
+// tile's pixel window (one pixel around it, more on the sides for the 16-byte
+// alignment of the TMA box) into comparable words in shared memory, once a
+// pixel; then each group of 16 lanes marches up a strip of GH rows, four
+// columns a lane, holding two rows of words in registers, the pairs of four
+// columns as the bytes of one register and the node bytes of four columns as
+// another.
+//
+// Bound: issue. What a pixel costs is its word (about 25 instructions), four
+// pair tests of three instructions and a quarter of the packed node assembly;
+// a thread per pixel over byte arrays in shared memory took five times as
+// many. 1024 frames of 256x224: 512 us before, 175 us now (85 instructions a pixel).
+constexpr int kGTW = 64;          // tile width (pixels): 16 lanes of four columns
+constexpr int kGThreads = 64;     // four groups of 16 lanes, strips of GH rows above each other
+constexpr int kGBoxW = kGTW + 8;  // window from x0 - 4
+// rows of a strip: 8 in large batches (the pairs of the row below a strip are
+// made twice, 1/8 of them), 4 up to 2^21 pixels and 1 up to 2^18, where blocks
+// are what is missing (8 frames of 256x224: 10.5 us with 8 rows, 9.9 with 4; one
+// frame: 7.8 us with 2 rows, 7.1 with 1; 1024 frames: 198 us with 4 rows, 175
+// with 8), 4 in the tile queue (its 64x16 tiles); the left column's pairs take
+// a lane a row, so at most 15
+constexpr int kGStrip = 8, kGStripSmall = 4, kGStripFrame = 1, kGStripQueue = 4;
 
-// the pixel window of a graph tile as one TMA box: RGBA words from x0 - 4
-// (16-byte aligned), y0 - 1, (kGTW + 8) x (kGTH + 2)
-constexpr int kGBoxW = kGTW + 8, kGBoxH = kGTH + 2;
+// Comparable form of a packed Y/U/V word (yuv_word): its byte fields in slots
+// of 10 bits, whose bit 9 is a guard. With A = a + guards + thresholds, the
+// slots of E = A - b hold 512 + t + (a - b) and those of C - E, C = 2 (guards
+// + thresholds), 512 + t - (a - b): a and b are similar (every field within
+// its threshold) when both keep all guard bits. kNoPixel, outside the image,
+// is similar to no pixel: its lowest slot is further from any byte than any
+// threshold reaches.
+constexpr uint32_t kGuards = 1u << 9 | 1u << 19 | 1u << 29;
+constexpr uint32_t kNoPixel = 511u;
 
-template <int LAYOUT, bool TMA = false>
+__device__ __forceinline__ uint32_t spread_fields(uint32_t w)
+{
+    return (w & 0xFFu) + ((w & 0xFF00u) << 2) + ((w & 0xFF0000u) << 4);
+}
+
+// Spread words of four RGBA pixels, yuv_word's arithmetic on integers, exact
+// over every input: the quotient of 0..255000 by 1000; 0.492f and 0.877f
+// times -255..255 rounded to float and truncated (no product of a negative
+// difference is whole, so truncation is the floor plus one). Negative fields
+// borrow from the next slot as they do from the next byte of the word. The
+// double evaluation only where a luma sum leaves no remainder, as yuv_word
+// explains; one branch for the four.
+__device__ __forceinline__ void pixel_fields(const uint32_t (&px)[4], int mode, uint32_t (&out)[4])
+{
+    int y[4], sum[4];
+    bool whole = false;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        // in the reference's byte order B plays r and R plays b: 299 B + 587 G + 114 R
+        sum[q] = (int)__dp4a(px[q], 0x002B4B72u, 256u * __dp4a(px[q], 0x00010200u, 0u));
+        y[q] = (int)__umulhi((unsigned)sum[q], 4294968u);
+        whole |= sum[q] == y[q] * 1000;
+    }
+    if (whole) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (sum[q] != y[q] * 1000 || sum[q] == 0) continue;
+            const double r = (double)(int)((px[q] >> 16) & 0xFFu), g = (double)(int)((px[q] >> 8) & 0xFFu);
+            const double b = (double)(int)(px[q] & 0xFFu);
+            const double t = mode == DEPIX_YUV_HOST
+                                 ? __dadd_rn(__dadd_rn(__dmul_rn(0.299, r), __dmul_rn(0.587, g)), __dmul_rn(0.114, b))
+                                 : __fma_rn(0.114, b, __fma_rn(0.299, r, __dmul_rn(0.587, g)));
+            y[q] = __double2int_rz(t);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const int du = (int)(px[q] & 0xFFu) - y[q], dv = (int)((px[q] >> 16) & 0xFFu) - y[q];
+        const int u = ((du * 32245) >> 16) + (int)((unsigned)du >> 31);
+        const int v = ((dv * 57475) >> 16) + (int)((unsigned)dv >> 31);
+        out[q] = (uint32_t)(y[q] * (1 << 20) + u * (1 << 10) + v) & 0x0FF3FCFFu;
+    }
+}
+
+// bit k set in the packed bytes when a (as A) and b are similar
+__device__ __forceinline__ uint32_t pair_bit(uint32_t A, uint32_t b, uint32_t C, uint32_t bit)
+{
+    const uint32_t E = A - b;
+    return (~(E & (C - E)) & kGuards) == 0 ? bit : 0u;
+}
+
+template <int LAYOUT, int GH, bool TMA = false>
 __device__ __forceinline__ void graph_tile(const FrameRef f, int x0, int y0, uint32_t thr, bool fuse_trivial,
                                            const CUtensorMap* pix_map = nullptr, int frame = 0)
 {
-    constexpr int RW = kGTW + 2, RH = kGTH + 2;
-    __shared__ uint32_t words[RH][RW];
-    __shared__ uint8_t pairs[RH][RW];
-    const int w = f.w, h = f.h;
+    static_assert(GH < 16, "a lane for each row's left pair");
+    constexpr int TH = GH * (kGThreads / 16), RH = TH + 2, RW = kGBoxW;
+    __shared__ __align__(128) uint32_t win[RH][RW]; // pixel (x, y) at win[y - y0 + 1][x - x0 + 4]
+    const int w = f.w, h = f.h, mode = yuv_mode_of(thr);
     if constexpr (TMA) {
-        __shared__ __align__(128) uint32_t box[kGBoxH][kGBoxW];
         __shared__ uint64_t bar;
         __shared__ int ok;
         if (threadIdx.x == 0) {
             const bool test_timeout = *(volatile int*)&g_graph_tma_timeout_test != 0;
             mbar_init(&bar, 1);
-            mbar_expect_tx(&bar, (uint32_t)sizeof(box));
-            if (!test_timeout) tma_load_3d(&box[0][0], pix_map, x0 - 4, y0 - 1, frame, &bar);
+            mbar_expect_tx(&bar, (uint32_t)sizeof(win));
+            if (!test_timeout) tma_load_3d(&win[0][0], pix_map, x0 - 4, y0 - 1, frame, &bar);
             ok = tma_wait_or_flag(&bar, &g_graph_fault, test_timeout ? kTestPolls : kTmaPolls) ? 1 : 0;
         }
         __syncthreads();
         if (!ok) return;
-        for (int k = threadIdx.x; k < RW * RH; k += blockDim.x) {
-            const int rx = k % RW, ry = k / RW;
-            const uint32_t p = box[ry][rx + 3]; // window column rx is image column x0 - 1 + rx
-            // RGBA -> the reference's byte order (b0, b1, b2) = (B, G, R); zero outside the image
-            const uint32_t c = ((p >> 16) & 0xFFu) | (p & 0xFF00u) | ((p & 0xFFu) << 16);
-            const int gx = x0 - 1 + rx, gy = y0 - 1 + ry;
-            words[ry][rx] = (gx >= 0 && gy >= 0 && gx < w && gy < h) ? word_of_bgr(c, thr) : 0u;
+    }
+    // ---- words of the window, four a thread (outer columns of the box that no
+    // pair reads are made too: they keep the rows 16-byte aligned)
+    const bool inside = x0 >= 4 && y0 >= 1 && x0 + kGTW + 4 <= w && y0 + TH + 1 <= h;
+    for (int k = threadIdx.x; k < RH * (RW / 4); k += kGThreads) {
+        const int ry = k / (RW / 4), rx = 4 * (k % (RW / 4));
+        const int gx = x0 - 4 + rx, gy = y0 - 1 + ry;
+        uint32_t px[4];
+        if constexpr (TMA) {
+            const uint4 v = *reinterpret_cast<const uint4*>(&win[ry][rx]);
+            px[0] = v.x; px[1] = v.y; px[2] = v.z; px[3] = v.w;
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                px[q] = 0;
+                if (gx + q < 0 || gx + q >= w || gy < 0 || gy >= h) continue;
+                if (LAYOUT == DEPIX_LAYOUT_RGBA) {
+                    px[q] = __ldg(reinterpret_cast<const uint32_t*>(f.img + (size_t)gy * f.ws) + gx + q);
+                } else {
+                    const uint32_t c = load_bgr(f.img, f.ws, LAYOUT, gx + q, gy);
+                    px[q] = ((c >> 16) & 0xFFu) | (c & 0xFF00u) | ((c & 0xFFu) << 16);
+                }
+            }
         }
-    } else {
-        for (int k = threadIdx.x; k < RW * RH; k += blockDim.x) {
-            int rx = k % RW, ry = k / RW;
-            int gx = x0 - 1 + rx, gy = y0 - 1 + ry;
-            uint32_t wd = 0;
-            if (gx >= 0 && gy >= 0 && gx < w && gy < h) wd = word_of_bgr(load_bgr(f.img, f.ws, LAYOUT, gx, gy), thr);
-            words[ry][rx] = wd;
+        uint32_t fd[4];
+        pixel_fields(px, mode, fd);
+        if (!inside) {
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (gx + q < 0 || gx + q >= w || gy < 0 || gy >= h) fd[q] = kNoPixel;
         }
+        *reinterpret_cast<uint4*>(&win[ry][rx]) = make_uint4(fd[0], fd[1], fd[2], fd[3]);
     }
     __syncthreads();
-    for (int k = threadIdx.x; k < RW * RH; k += blockDim.x) {
-        int rx = k % RW, ry = k / RW;
-        int gx = x0 - 1 + rx, gy = y0 - 1 + ry;
-        unsigned pb = 0;
-        bool in = gx >= 0 && gy >= 0 && gx < w && gy < h;
-        bool rin = rx + 1 < RW && gx + 1 < w && gx + 1 >= 0 && in;
-        bool uin = ry + 1 < RH && gy + 1 < h && gy + 1 >= 0 && in;
-        if (rin && similar(words[ry][rx], words[ry][rx + 1], thr)) pb |= 1u;
-        if (uin && similar(words[ry][rx], words[ry + 1][rx], thr)) pb |= 2u;
-        if (rin && uin) {
-            if (similar(words[ry][rx], words[ry + 1][rx + 1], thr)) pb |= 4u;
-            if (similar(words[ry][rx + 1], words[ry + 1][rx], thr)) pb |= 8u;
-        }
-        pairs[ry][rx] = (uint8_t)pb;
+    // ---- strips
+    const uint32_t GT = kGuards + spread_fields(thr & 0x00FFFFFFu), C = 2u * GT;
+    const int gl = threadIdx.x & 15, base = GH * (threadIdx.x >> 4); // window row of y0 - 1 + base
+    // pairs of a column c with the row above (words lo: row, hi: row above): bit
+    // 0 right, 1 up, 2 up-right, 3 right's up-left, 4 the block's four sides
+    // all similar (its trivial crossing goes, crossCheck_4)
+    // the column left of the tile, a row a lane
+    uint32_t edge = 0;
+    if (gl <= GH) {
+        const uint32_t* lo = &win[base + gl][3];
+        const uint32_t* hi = &win[base + gl + 1][3];
+        const uint32_t a0 = lo[0] + GT, a1 = lo[1] + GT;
+        edge = pair_bit(a0, lo[1], C, 1u) | pair_bit(a0, hi[0], C, 2u) | pair_bit(a0, hi[1], C, 4u) |
+               pair_bit(a1, hi[0], C, 8u);
+        if (fuse_trivial && (edge & 3u) == 3u && pair_bit(a1, hi[1], C, 1u) && pair_bit(hi[0] + GT, hi[1], C, 1u)) edge |= 16u;
     }
-    __syncthreads();
-    // fused trivial removal (crossCheck_4): a diagonal goes when the 2x2 block
-    // it crosses has all four sides similar; each block decided once (bit 4
-    // of the pairs byte of its lower-left node)
-    if (fuse_trivial) {
-        for (int k = threadIdx.x; k < (kGTW + 1) * (kGTH + 1); k += blockDim.x) {
-            const int bx = k % (kGTW + 1), by = k / (kGTW + 1);
-            const unsigned full = pairs[by][bx] & pairs[by + 1][bx] & (pairs[by][bx] >> 1) & (pairs[by][bx + 1] >> 1) & 1u;
-            pairs[by][bx] |= (uint8_t)(full << 4);
+    auto row_words = [&](int r, uint32_t (&v)[5]) {
+        const uint4 q = *reinterpret_cast<const uint4*>(&win[r][4 + 4 * gl]);
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+        v[4] = win[r][8 + 4 * gl];
+    };
+    auto right_pairs = [&](const uint32_t (&A)[5], const uint32_t (&v)[5]) {
+        return pair_bit(A[0], v[1], C, 1u) | pair_bit(A[1], v[2], C, 1u << 8) | pair_bit(A[2], v[3], C, 1u << 16) |
+               pair_bit(A[3], v[4], C, 1u << 24);
+    };
+    uint32_t A[5], n[5];
+    row_words(base, n);
+#pragma unroll
+    for (int q = 0; q < 5; q++) A[q] = n[q] + GT;
+    uint32_t R = right_pairs(A, n), below = 0, below_left = 0;
+    const int gx = x0 + 4 * gl;
+    uint8_t* out = f.graph + (ptrdiff_t)(y0 + base - 1) * w + gx;
+    const bool wide = gx + 3 < w && ((w | (int)reinterpret_cast<uintptr_t>(f.graph)) & 3) == 0;
+#pragma unroll
+    for (int r = 0; r <= GH; r++) {
+        row_words(base + r + 1, n);
+        uint32_t P = R, U = 0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            U |= pair_bit(A[q], n[q], C, 1u << (8 * q));
+            P |= pair_bit(A[q], n[q + 1], C, 4u << (8 * q)) | pair_bit(A[q + 1], n[q], C, 8u << (8 * q));
         }
-        __syncthreads();
-    }
-    // node bits (graph_Kernel)
-    for (int k = threadIdx.x; k < kGTW * kGTH; k += blockDim.x) {
-        int tx = k % kGTW, ty = k / kGTW;
-        int gx = x0 + tx, gy = y0 + ty;
-        if (gx >= w || gy >= h) continue;
-        int rx = tx + 1, ry = ty + 1;
-        unsigned c = pairs[ry][rx], l = pairs[ry][rx - 1], d = pairs[ry - 1][rx], dl = pairs[ry - 1][rx - 1];
-        unsigned node = 0;
-        node |= (unsigned)bitof(c, 1) << 1;   // up
-        node |= (unsigned)bitof(d, 1) << 6;   // down
-        node |= (unsigned)bitof(c, 0) << 4;   // right
-        node |= (unsigned)bitof(l, 0) << 3;   // left
-        node |= (unsigned)bitof(c, 2) << 2;   // up-right
-        node |= (unsigned)bitof(l, 3) << 0;   // up-left: pair (right of l = c, up of l)
-        node |= (unsigned)bitof(dl, 2) << 5;  // down-left
-        node |= (unsigned)bitof(d, 3) << 7;   // down-right: pair (right of d, up of d = c)
-        if (fuse_trivial) {
-            // blocks with lower-left (rx, ry), (rx-1, ry), (rx-1, ry-1), (rx, ry-1)
-            if (bitof(c, 4)) node &= ~4u;
-            if (bitof(l, 4)) node &= ~1u;
-            if (bitof(dl, 4)) node &= ~32u;
-            if (bitof(d, 4)) node &= ~128u;
+        const uint32_t U4 = pair_bit(A[4], n[4], C, 1u << 24);
+#pragma unroll
+        for (int q = 0; q < 5; q++) A[q] = n[q] + GT;
+        const uint32_t Rn = right_pairs(A, n);
+        P |= U << 1;
+        if (fuse_trivial) P |= (R & Rn & U & (U >> 8 | U4)) << 4;
+        R = Rn;
+        uint32_t left = __shfl_up_sync(0xFFFFFFFFu, P, 1, 16) >> 24;
+        const uint32_t e = __shfl_sync(0xFFFFFFFFu, edge, r, 16);
+        if (gl == 0) left = e;
+        const uint32_t L = P << 8 | left; // the pairs of the column to the left
+        if (r > 0) {
+            constexpr uint32_t k1 = 0x01010101u;
+            uint32_t node = (L >> 3 & k1) | (P & 2 * k1) | (P & 4 * k1) | (L & k1) << 3 | (P & k1) << 4 |
+                            (below_left & 4 * k1) << 3 | (below & 2 * k1) << 5 | (below & 8 * k1) << 4;
+            // the blocks at whose corners the node is lose their crossing diagonals
+            node &= ~((L >> 4 & k1) | (P >> 2 & 4 * k1) | (below_left & 16 * k1) << 1 | (below & 16 * k1) << 3);
+            if (y0 + base + r - 1 < h) {
+                uint8_t* o = out + (size_t)r * w;
+                if (wide) {
+                    *reinterpret_cast<uint32_t*>(o) = node;
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        if (gx + q < w) o[q] = (uint8_t)(node >> (8 * q));
+                }
+            }
         }
-        f.graph[(size_t)gy * w + gx] = (uint8_t)node;
+        below = P;
+        below_left = L;
     }
 }
 
-template <int LAYOUT>
-__global__ void __launch_bounds__(256) k_graph(FrameBatch b, uint32_t thr, int fuse_trivial)
+template <int LAYOUT, int GH>
+__global__ void __launch_bounds__(kGThreads) k_graph(FrameBatch b, uint32_t thr, int fuse_trivial)
 {
     FrameRef f = b.frame(blockIdx.z);
-    graph_tile<LAYOUT>(f, blockIdx.x * kGTW, blockIdx.y * kGTH, thr, fuse_trivial != 0);
+    graph_tile<LAYOUT, GH>(f, blockIdx.x * kGTW, blockIdx.y * 4 * GH, thr, fuse_trivial != 0);
 }
 
 // RGBA frames whose base, rows and frame stride are 16-byte aligned: the
 // pixel windows come by TMA
-__global__ void __launch_bounds__(256) k_graph_tma(FrameBatch b, uint32_t thr, int fuse_trivial,
-                                                   const __grid_constant__ CUtensorMap pix_map)
+template <int GH>
+__global__ void __launch_bounds__(kGThreads) k_graph_tma(FrameBatch b, uint32_t thr, int fuse_trivial,
+                                                         const __grid_constant__ CUtensorMap pix_map)
 {
     FrameRef f = b.frame(blockIdx.z);
-    graph_tile<DEPIX_LAYOUT_RGBA, true>(f, blockIdx.x * kGTW, blockIdx.y * kGTH, thr, fuse_trivial != 0, &pix_map,
-                                        (int)blockIdx.z);
+    graph_tile<DEPIX_LAYOUT_RGBA, GH, true>(f, blockIdx.x * kGTW, blockIdx.y * 4 * GH, thr, fuse_trivial != 0, &pix_map,
+                                            (int)blockIdx.z);
 }
 
 // Trivial removal on a graph in place (crossCheck_4, graph_functions.cu:1211-1274).
@@ -887,7 +998,7 @@ __global__ void k_cc_flatten(int32_t* L, int n, size_t frame_stride)
 
 // ------------------------------------------------ uneven batches (queue)
 
-__global__ void __launch_bounds__(256) k_graph_queue(QueueBatch q)
+__global__ void __launch_bounds__(kGThreads) k_graph_queue(QueueBatch q)
 {
     const QueueHeader* H = q.hdr;
     const int n = H->n;
@@ -897,7 +1008,7 @@ __global__ void __launch_bounds__(256) k_graph_queue(QueueBatch q)
         const QueueFrame fr = H->frames[f];
         const int lt = t - (int)base[f], tx = (fr.w + kGTW - 1) / kGTW;
         FrameRef ref{H->img + fr.in_off, fr.w, fr.h, 4 * fr.w, q.graph_a + fr.px_off};
-        graph_tile<DEPIX_LAYOUT_RGBA>(ref, (lt % tx) * kGTW, (lt / tx) * kGTH, H->thr, true);
+        graph_tile<DEPIX_LAYOUT_RGBA, kGStripQueue>(ref, (lt % tx) * kGTW, (lt / tx) * 4 * kGStripQueue, H->thr, true);
     });
 }
 
@@ -951,7 +1062,7 @@ __global__ void __launch_bounds__(256) k_label_flatten_queue(QueueBatch q)
 
 cudaError_t queue_graph(const QueueBatch& q, int blocks, cudaStream_t s)
 {
-    k_graph_queue<<<blocks, 256, 0, s>>>(q);
+    k_graph_queue<<<blocks, kGThreads, 0, s>>>(q);
     return cudaGetLastError();
 }
 
@@ -970,7 +1081,7 @@ cudaError_t queue_labels(const QueueBatch& q, int blocks, cudaStream_t s)
     return cudaGetLastError();
 }
 
-static_assert(kQGraphTW == kGTW && kQGraphTH == kGTH, "graph queue tile");
+static_assert(kQGraphTW == kGTW && kQGraphTH == 4 * kGStripQueue, "graph queue tile");
 static_assert(kQHeurTW == kHTW && kQHeurTH == kHTH, "heuristics queue tile");
 static_assert(kQLabelT == kLT, "label queue tile");
 
@@ -985,7 +1096,7 @@ static int occupancy(K kernel, int threads)
 int queue_blocks_per_sm(int stage, const QueueBatch& q)
 {
     switch (stage) {
-    case QS_GRAPH: return occupancy(k_graph_queue, 256);
+    case QS_GRAPH: return occupancy(k_graph_queue, kGThreads);
     case QS_HEUR: return q.vote ? occupancy(k_heur_queue<true>, 256) : occupancy(k_heur_queue<false>, 256);
     case QS_LABEL: return occupancy(k_label_flatten_queue, 256);
     default: return queue_raster_blocks_per_sm(q);
@@ -1022,18 +1133,27 @@ cudaError_t take_graph_fault(int* out)
     return e;
 }
 
-cudaError_t launch_graph(const FrameBatch& b, int nframes, uint32_t thr, bool fuse_trivial, cudaStream_t s)
+template <int GH>
+static cudaError_t launch_graph_t(const FrameBatch& b, int nframes, uint32_t thr, bool fuse_trivial, cudaStream_t s)
 {
-    dim3 grid((b.w + kGTW - 1) / kGTW, (b.h + kGTH - 1) / kGTH, nframes);
+    dim3 grid((b.w + kGTW - 1) / kGTW, (b.h + 4 * GH - 1) / (4 * GH), nframes);
     CUtensorMap map;
     if (b.layout == DEPIX_LAYOUT_RGBA &&
-        rgba_tensor_map(b.img, b.w, b.h, b.ws, b.img_stride, nframes, kGBoxW, kGBoxH, &map))
-        k_graph_tma<<<grid, 256, 0, s>>>(b, thr, fuse_trivial ? 1 : 0, map);
+        rgba_tensor_map(b.img, b.w, b.h, b.ws, b.img_stride, nframes, kGBoxW, 4 * GH + 2, &map))
+        k_graph_tma<GH><<<grid, kGThreads, 0, s>>>(b, thr, fuse_trivial ? 1 : 0, map);
     else if (b.layout == DEPIX_LAYOUT_RGBA)
-        k_graph<DEPIX_LAYOUT_RGBA><<<grid, 256, 0, s>>>(b, thr, fuse_trivial ? 1 : 0);
+        k_graph<DEPIX_LAYOUT_RGBA, GH><<<grid, kGThreads, 0, s>>>(b, thr, fuse_trivial ? 1 : 0);
     else
-        k_graph<DEPIX_LAYOUT_BGR><<<grid, 256, 0, s>>>(b, thr, fuse_trivial ? 1 : 0);
+        k_graph<DEPIX_LAYOUT_BGR, GH><<<grid, kGThreads, 0, s>>>(b, thr, fuse_trivial ? 1 : 0);
     return cudaGetLastError();
+}
+
+cudaError_t launch_graph(const FrameBatch& b, int nframes, uint32_t thr, bool fuse_trivial, cudaStream_t s)
+{
+    const long long px = (long long)b.w * b.h * nframes;
+    if (px <= 1 << 18) return launch_graph_t<kGStripFrame>(b, nframes, thr, fuse_trivial, s);
+    if (px <= 1 << 21) return launch_graph_t<kGStripSmall>(b, nframes, thr, fuse_trivial, s);
+    return launch_graph_t<kGStrip>(b, nframes, thr, fuse_trivial, s);
 }
 
 cudaError_t launch_trivial(uint8_t* g, int w, int h, cudaStream_t s)
