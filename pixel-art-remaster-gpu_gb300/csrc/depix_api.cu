@@ -303,7 +303,7 @@ depix_status depix_resolve_heuristics(const uint8_t* d_snapshot, int w, int h, u
     if (!d_snapshot || !d_out) return arg_fail("graph pointer is NULL");
     if (d_snapshot == d_out) return arg_fail("snapshot and output must be distinct buffers");
     GraphBatch b{d_snapshot, d_out, 0, w, h};
-    DEPIX_CK(launch_heuristics(b, 1, S(s)));
+    DEPIX_CK(launch_heuristics(b, 1, nullptr, S(s)));
     return DEPIX_OK;
 }
 
@@ -313,7 +313,7 @@ depix_status depix_resolve_heuristics_vote(const uint8_t* d_snapshot, int w, int
     if (!d_snapshot || !d_out) return arg_fail("graph pointer is NULL");
     if (d_snapshot == d_out) return arg_fail("snapshot and output must be distinct buffers");
     GraphBatch b{d_snapshot, d_out, 0, w, h, 1};
-    DEPIX_CK(launch_heuristics(b, 1, S(s)));
+    DEPIX_CK(launch_heuristics(b, 1, nullptr, S(s)));
     return DEPIX_OK;
 }
 
@@ -579,8 +579,7 @@ depix_status run_batch(depix_context* ctx, int n, const int* w, const int* h, co
             // with labels, each heuristics tile also makes its local labels
             StageTimer t(ctx, DEPIX_STAGE_HEURISTICS, 1, s);
             GraphBatch hb{ctx->graph_a, ctx->graph_b, px, w[0], h[0], p->vote};
-            if (d_labels) DEPIX_CK(launch_heuristics_labels(hb, n, d_labels, s));
-            else DEPIX_CK(launch_heuristics(hb, n, s));
+            DEPIX_CK(launch_heuristics(hb, n, d_labels, s));
         }
         if (d_labels) {
             StageTimer t(ctx, DEPIX_STAGE_LABELS, 2, s);
@@ -629,8 +628,7 @@ depix_status run_batch(depix_context* ctx, int n, const int* w, const int* h, co
         {
             StageTimer t(ctx, DEPIX_STAGE_HEURISTICS, 1, s);
             GraphBatch hb{ctx->graph_a + goff, ctx->graph_b + goff, 0, w[k], h[k], p->vote};
-            if (d_labels) DEPIX_CK(launch_heuristics_labels(hb, 1, d_labels + loff, s));
-            else DEPIX_CK(launch_heuristics(hb, 1, s));
+            DEPIX_CK(launch_heuristics(hb, 1, d_labels ? d_labels + loff : nullptr, s));
         }
         if (d_labels) {
             StageTimer t(ctx, DEPIX_STAGE_LABELS, 2, s);
@@ -846,8 +844,7 @@ depix_status depix_frame(depix_context* ctx, const uint8_t* d_img, int w, int h,
     {
         StageTimer t(ctx, DEPIX_STAGE_HEURISTICS, 1, s);
         GraphBatch hb{ctx->graph_a, resolved, 0, w, h, p->vote};
-        if (d_labels) DEPIX_CK(launch_heuristics_labels(hb, 1, d_labels, s));
-        else DEPIX_CK(launch_heuristics(hb, 1, s));
+        DEPIX_CK(launch_heuristics(hb, 1, d_labels, s));
     }
     if (d_labels) {
         StageTimer t(ctx, DEPIX_STAGE_LABELS, 2, s);
@@ -980,7 +977,7 @@ depix_status compat_run(void* pos, void* colorPos, char* img_data, int w, int h,
     FrameBatch gb{c.img, 0, c.g0, 0, w, h, ws, DEPIX_LAYOUT_BGR};
     DEPIX_CK(launch_graph(gb, 1, pack_thresholds(p->tr_y, p->tr_u, p->tr_v, p->yuv), true, s));
     GraphBatch hb{c.g0, c.g1, 0, w, h, p->vote};
-    DEPIX_CK(launch_heuristics(hb, 1, s));
+    DEPIX_CK(launch_heuristics(hb, 1, nullptr, s));
     DEPIX_CK(launch_cells(c.g1, w, h, c.diag, c.ec, s));
     if (subdivide) {
         DEPIX_CK(cudaMemcpyAsync(c.snap, c.diag, px * kCell * sizeof(float2), cudaMemcpyDeviceToDevice, s));

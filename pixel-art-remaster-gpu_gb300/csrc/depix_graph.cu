@@ -279,13 +279,26 @@ __global__ void k_trivial(uint8_t* g, int w, int h)
 // ------------------------------------------------------- heuristics stage
 
 constexpr int kHTW = 64, kHTH = 16;
-constexpr int kHalo = 32; // a curve-length walk moves at most 31 steps from a block node
-constexpr int kHRW = kHTW + 2 * kHalo, kHRH = kHTH + 2 * kHalo;
+// Window of a tile: 16 columns (TMA's alignment) and 8 rows around it, which
+// hold the 8x8 windows of the vote and nearly all curve-length walks; a walk
+// moves at most 31 steps from its block, and one that leaves the window reads
+// the snapshot in global memory. (A halo of 32 that held every walk was 10 KB
+// to load and keep for the tile's 1 KB.)
+constexpr int kHaloX = 16, kHaloY = 8;
+constexpr int kHRW = kHTW + 2 * kHaloX, kHRH = kHTH + 2 * kHaloY;
+constexpr int kHThreads = 128;
 
 struct SnapTile {
     const uint8_t (*s)[kHRW];
     int ox, oy; // image coordinates of s[0][0]
-    __device__ __forceinline__ unsigned at(int x, int y) const { return s[y - oy][x - ox]; }
+    const uint8_t* g;
+    int w, h;
+    __device__ __forceinline__ unsigned at(int x, int y) const { return s[y - oy][x - ox]; } // inside the window
+    __device__ __forceinline__ unsigned far(int x, int y) const
+    {
+        if ((unsigned)(x - ox) < (unsigned)kHRW && (unsigned)(y - oy) < (unsigned)kHRH) return s[y - oy][x - ox];
+        return (unsigned)x < (unsigned)w && (unsigned)y < (unsigned)h ? __ldg(g + (size_t)y * w + x) : 0u;
+    }
 };
 
 // set bits of node other than bit e; last = the highest such bit in the
@@ -308,7 +321,7 @@ __device__ __forceinline__ void walk_len(const SnapTile& t, int i, int j, int e,
 {
     for (;;) {
         int k_n = 0;
-        int s = others(t.at(i, j), e, k_n);
+        int s = others(t.far(i, j), e, k_n);
         if (result > 30) return;
         if (s != 1) return;
         result++;
@@ -374,9 +387,8 @@ __device__ __forceinline__ int window_component(const uint64_t (&m)[8], uint64_t
 // sparser one is kept), islands with weight 5 for a diagonal whose removal
 // would leave one of its ends without edges. The diagonal with fewer votes
 // is removed; a tie removes both.
-__device__ unsigned vote_decision(const uint8_t (*s)[kHRW], int ox, int oy, int i, int j)
+__device__ unsigned vote_decision(const SnapTile& t, int i, int j)
 {
-    const SnapTile t{s, ox, oy};
     unsigned n1 = t.at(i, j), n2 = t.at(i, j + 1), n3 = t.at(i + 1, j), n4 = t.at(i + 1, j + 1);
     int dummy;
     int o1 = others(n1, 2, dummy), o4 = others(n4, 5, dummy), o3 = others(n3, 0, dummy), o2 = others(n2, 7, dummy);
@@ -393,7 +405,7 @@ __device__ unsigned vote_decision(const uint8_t (*s)[kHRW], int ox, int oy, int 
     // window columns i-3 .. i+4, rows j-3 .. j+4 (inside the snapshot halo)
     uint64_t m[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int r = 0; r < 8; r++) {
-        const uint8_t* row = &s[j - 3 + r - oy][i - 3 - ox];
+        const uint8_t* row = &t.s[j - 3 + r - t.oy][i - 3 - t.ox];
         for (int c = 0; c < 8; c++) {
             const unsigned nd = row[c];
             const uint64_t bit = 1ull << (r * 8 + c);
@@ -411,135 +423,161 @@ __device__ unsigned vote_decision(const uint8_t (*s)[kHRW], int ox, int oy, int 
     return kDecCross | kDecSlash | kDecBack;
 }
 
-template <int TW, int TH>
-__device__ void cc_local_core(const uint8_t* sg, int* sl, uint16_t* run, int32_t* L, int w, int h, int x0, int y0);
-template <int TW, int TH>
-__device__ void cc_sym_unions(const uint8_t* sg, int* sl);
-template <int TW, int TH>
-__device__ void cc_sym_store(const uint8_t* sg, int* sl, int32_t* L, int w, int h, int x0, int y0);
+constexpr int kMaxJoins = (kHTH - 1) * 3 * kHTW; // every upward edge of a tile
+__device__ void tile_labels(const uint8_t (*node)[kHTW], uint16_t* joins, int32_t* L, int w, int h, int x0, int y0);
 
 // Heuristic resolution of one 64x16 tile; with L set, the tile's local
 // component labels too (union-find over the resolved bytes, still in shared
 // memory), which leaves the label stage only the merge across tile borders
 // and the flattening.
+//
+// Crossings are few, so four 2x2 blocks a thread are tested for one at a time
+// in packed bytes, the crossings go to a list, and a lane decides each (once:
+// its four corner nodes each lose a bit of the decision). Bound: issue (79 %);
+// 1024 frames of 256x224 with labels: 636 us when every node tested its four
+// blocks over bytes and every lane ran a row's join masks, 254 us now (the
+// vote on 32 frames of 159x143: 68 us before, 33 now).
 template <bool TMA = false, bool VOTE = false>
 __device__ __forceinline__ void heuristics_tile(const uint8_t* snap, uint8_t* out, int w, int h, int x0, int y0,
                                                 int32_t* L = nullptr, const CUtensorMap* map = nullptr,
                                                 int frame = 0)
 {
-    __shared__ __align__(128) uint8_t s[kHRH][kHRW];
-    const int ox = x0 - kHalo, oy = y0 - kHalo;
+    // the window, later the labels' list of joins
+    __shared__ __align__(128) uint8_t buf[kHRH * kHRW > 2 * kMaxJoins ? kHRH * kHRW : 2 * kMaxJoins];
+    uint8_t(*s)[kHRW] = reinterpret_cast<uint8_t(*)[kHRW]>(buf);
+    __shared__ __align__(16) uint8_t res[kHTH][kHTW]; // resolved nodes
+    // blocks touching the tile that hold a crossing: column - (x0 - 1) | row - (y0 - 1) << 8
+    __shared__ uint16_t list[(kHTW + 1) * (kHTH + 1)];
+    __shared__ int count;
+    const int ox = x0 - kHaloX, oy = y0 - kHaloY;
     if constexpr (TMA) {
-        // the window as one TMA box (x0 - 32 is a multiple of 16 bytes);
+        // the window as one TMA box (x0 - 16 is a multiple of 16 bytes);
         // bytes outside the image read as zero
         __shared__ uint64_t bar;
         __shared__ int ok;
         if (threadIdx.x == 0) {
+            count = 0;
             mbar_init(&bar, 1);
-            mbar_expect_tx(&bar, (uint32_t)sizeof(s));
+            mbar_expect_tx(&bar, (uint32_t)(kHRH * kHRW));
             tma_load_3d(&s[0][0], map, ox, oy, frame, &bar);
             ok = tma_wait_or_flag(&bar, &g_heur_fault) ? 1 : 0;
         }
         __syncthreads();
         if (!ok) return;
-    } else
-    // 4-byte loads where a row is word aligned in memory, else bytes
-    for (int k = threadIdx.x; k < kHRH * (kHRW / 4); k += blockDim.x) {
-        int ry = k / (kHRW / 4), rx = 4 * (k % (kHRW / 4));
-        int gy = oy + ry, gx = ox + rx;
-        uint32_t v = 0;
-        if (gy >= 0 && gy < h) {
-            const uint8_t* row = snap + (size_t)gy * w;
-            if (gx >= 0 && gx + 3 < w && ((reinterpret_cast<uintptr_t>(row + gx) & 3) == 0)) {
-                v = __ldg(reinterpret_cast<const uint32_t*>(row + gx));
-            } else {
-                for (int q = 0; q < 4; q++)
-                    if (gx + q >= 0 && gx + q < w) v |= (uint32_t)__ldg(row + gx + q) << (8 * q);
+    } else {
+        if (threadIdx.x == 0) count = 0;
+        // 4-byte loads where a row is word aligned in memory, else bytes
+        for (int k = threadIdx.x; k < kHRH * (kHRW / 4); k += kHThreads) {
+            int ry = k / (kHRW / 4), rx = 4 * (k % (kHRW / 4));
+            int gy = oy + ry, gx = ox + rx;
+            uint32_t v = 0;
+            if (gy >= 0 && gy < h) {
+                const uint8_t* row = snap + (size_t)gy * w;
+                if (gx >= 0 && gx + 3 < w && ((reinterpret_cast<uintptr_t>(row + gx) & 3) == 0)) {
+                    v = __ldg(reinterpret_cast<const uint32_t*>(row + gx));
+                } else {
+                    for (int q = 0; q < 4; q++)
+                        if (gx + q >= 0 && gx + q < w) v |= (uint32_t)__ldg(row + gx + q) << (8 * q);
+                }
+            }
+            *reinterpret_cast<uint32_t*>(&s[ry][rx]) = v;
+        }
+        __syncthreads();
+    }
+    const SnapTile t{s, ox, oy, snap, w, h};
+    // ---- crossings, four blocks of a row at a time: rows y0 - 1 .. y0 + 15,
+    // columns x0 - 4 .. x0 + 63 of which the first word gives x0 - 1 only.
+    // Blocks reaching outside the image read zeros and are never crossings.
+    constexpr int NW = kHTW / 4 + 1;
+    for (int k = threadIdx.x; k < NW * (kHTH + 1); k += kHThreads) {
+        const int wc = k % NW, by = k / NW;
+        const uint32_t* a = reinterpret_cast<const uint32_t*>(&s[by + kHaloY - 1][kHaloX - 4 + 4 * wc]);
+        const uint32_t* b = a + kHRW / 4;
+        const uint32_t a0 = a[0], b0 = b[0];
+        const uint32_t a1 = __funnelshift_r(a0, a[1], 8), b1 = __funnelshift_r(b0, b[1], 8); // one column on
+        uint32_t cross = (a0 >> 2) & (b0 >> 7) & a1 & (b1 >> 5) & 0x01010101u;
+        if (wc == 0) cross &= 0x01000000u;
+        if (wc > 0 && by > 0) *reinterpret_cast<uint32_t*>(&res[by - 1][4 * wc - 4]) = a0;
+        if (cross) {
+            int slot = atomicAdd(&count, __popc(cross));
+            while (cross) {
+                const int q = (__ffs(cross) - 1) >> 3;
+                cross &= cross - 1;
+                list[slot++] = (uint16_t)((4 * wc + q - 3) | by << 8);
             }
         }
-        *reinterpret_cast<uint32_t*>(&s[ry][rx]) = v;
     }
-    SnapTile t{s, ox, oy};
-    // each 2x2 block touching the tile decided once (the four corner nodes
-    // each clear their own bit of it), as a kDec* code; blocks reaching
-    // outside the image read the zero halo and are never crossings
-    __shared__ uint8_t dec[kHTH + 1][kHTW + 1];
     __syncthreads();
-    for (int k = threadIdx.x; k < (kHTW + 1) * (kHTH + 1); k += blockDim.x) {
-        const int bx = k % (kHTW + 1), by = k / (kHTW + 1);
-        const int bi = x0 - 1 + bx, bj = y0 - 1 + by;
-        unsigned d = 0;
-        if (bitof(t.at(bi, bj), 2) && bitof(t.at(bi, bj + 1), 7) && bitof(t.at(bi + 1, bj), 0) &&
-            bitof(t.at(bi + 1, bj + 1), 5))
-        {
-            if constexpr (VOTE) d = vote_decision(s, ox, oy, bi, bj);
-            else d = kDecCross | (block_decision(t, bi, bj) ? kDecSlash : kDecBack);
+    const int n = count;
+    for (int k = threadIdx.x; k < n; k += kHThreads) {
+        const int bx = list[k] & 0xFF, by = list[k] >> 8;
+        const int i = x0 - 1 + bx, j = y0 - 1 + by;
+        unsigned d;
+        if constexpr (VOTE) d = vote_decision(t, i, j);
+        else d = block_decision(t, i, j) ? kDecSlash : kDecBack;
+        // the block's nodes lose their bits of it, those inside the tile
+        auto drop = [&](int tx, int ty, unsigned bit) {
+            if ((unsigned)tx < (unsigned)kHTW && (unsigned)ty < (unsigned)kHTH)
+                atomicAnd(reinterpret_cast<unsigned*>(&res[ty][tx & ~3]), ~(bit << (8 * (tx & 3))));
+        };
+        if (d & kDecSlash) {
+            drop(bx - 1, by - 1, 4u);
+            drop(bx, by, 32u);
         }
-        dec[by][bx] = (uint8_t)d;
+        if (d & kDecBack) {
+            drop(bx, by - 1, 1u);
+            drop(bx - 1, by, 128u);
+        }
     }
     __syncthreads();
-    // With L, each pixel's union-find parent starts at the leftmost pixel of
-    // its horizontal run, from one ballot of the warp that resolves the
-    // pixel's 32-pixel row segment (a warp's 32 values of k are one segment:
-    // blockDim.x is a multiple of 32 and a row is two segments); a run that
-    // comes into the second segment from the first hangs from the first
-    // segment's last pixel.
-    __shared__ uint8_t res[kHTW * kHTH];
-    __shared__ int sl[kHTW * kHTH];
-    for (int k = threadIdx.x; k < kHTW * kHTH; k += blockDim.x) {
-        const int tx = k % kHTW, ty = k / kHTW;
+    // ---- output, four nodes a thread; for the labels the nodes on the image's
+    // edge lose their bits toward outside
+    const bool edge = x0 == 0 || y0 == 0 || x0 + kHTW >= w || y0 + kHTH >= h;
+    for (int k = threadIdx.x; k < kHTW / 4 * kHTH; k += kHThreads) {
+        const int tx = 4 * (k % (kHTW / 4)), ty = k / (kHTW / 4);
         const int i = x0 + tx, j = y0 + ty;
-        unsigned v = 0;
-        if (i < w && j < h) {
-            unsigned o = t.at(i, j);
-            // the node is the lower-right corner of block (i-1, j), the upper-right
-            // of (i-1, j-1), the upper-left of (i, j-1), the lower-left of (i, j)
-            const unsigned a = dec[ty + 1][tx], b = dec[ty][tx], c = dec[ty][tx + 1], d = dec[ty + 1][tx + 1];
-            if (a & kDecBack) o &= ~1u;
-            if (b & kDecSlash) o &= ~32u;
-            if (c & kDecBack) o &= ~128u;
-            if (d & kDecSlash) o &= ~4u;
-            out[(size_t)j * w + i] = (uint8_t)o;
-            v = o & inside_mask(i, j, w, h);
+        const uint32_t v = *reinterpret_cast<const uint32_t*>(&res[ty][tx]);
+        if (j < h && i < w) {
+            uint8_t* o = out + (size_t)j * w + i;
+            if (i + 3 < w && (reinterpret_cast<uintptr_t>(o) & 3) == 0) {
+                *reinterpret_cast<uint32_t*>(o) = v;
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if (i + q < w) o[q] = (uint8_t)(v >> (8 * q));
+            }
         }
-        res[k] = (uint8_t)v;
-        if (L) {
-            const int lane = tx & 31;
-            const unsigned starts = __ballot_sync(0xFFFFFFFFu, tx == 0 || !bitof(v, 3));
-            const unsigned upto = starts & (0xFFFFFFFFu >> (31 - lane));
-            sl[k] = upto ? (k - lane) + 31 - __clz(upto) : k - lane - 1;
+        if (L && edge) {
+            uint32_t m = 0;
+            if (j < h) {
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if (i + q < w) m |= inside_mask(i + q, j, w, h) << (8 * q);
+            }
+            *reinterpret_cast<uint32_t*>(&res[ty][tx]) = v & m;
         }
     }
     if (L) {
-        __syncthreads();
-        cc_sym_unions<kHTW, kHTH>(res, sl);
-        __syncthreads();
-        cc_sym_store<kHTW, kHTH>(res, sl, L, w, h, x0, y0);
+        if (edge) __syncthreads();
+        tile_labels(res, reinterpret_cast<uint16_t*>(buf), L, w, h, x0, y0);
     }
 }
 
-// VOTE: the weighted vote instead of the reference's ordered tests
+// VOTE: the weighted vote instead of the reference's ordered tests; L may be
+// NULL
 template <bool VOTE>
-__global__ void __launch_bounds__(256) k_heuristics(GraphBatch b)
-{
-    const uint8_t* snap = b.snap + b.frame_stride * blockIdx.z;
-    uint8_t* out = b.out + b.frame_stride * blockIdx.z;
-    heuristics_tile<false, VOTE>(snap, out, b.w, b.h, blockIdx.x * kHTW, blockIdx.y * kHTH);
-}
-
-template <bool VOTE>
-__global__ void __launch_bounds__(256) k_heuristics_labels(GraphBatch b, int32_t* L)
+__global__ void __launch_bounds__(kHThreads) k_heuristics(GraphBatch b, int32_t* L)
 {
     const uint8_t* snap = b.snap + b.frame_stride * blockIdx.z;
     uint8_t* out = b.out + b.frame_stride * blockIdx.z;
     heuristics_tile<false, VOTE>(snap, out, b.w, b.h, blockIdx.x * kHTW, blockIdx.y * kHTH,
-                                 L + b.frame_stride * blockIdx.z);
+                                 L ? L + b.frame_stride * blockIdx.z : nullptr);
 }
 
 // the same with the graph windows by TMA (width and frame stride multiples of
-// 16 bytes, 16-byte aligned base); L may be NULL
+// 16 bytes, 16-byte aligned base)
 template <bool VOTE>
-__global__ void __launch_bounds__(256) k_heuristics_tma(GraphBatch b, int32_t* L, const __grid_constant__ CUtensorMap map)
+__global__ void __launch_bounds__(kHThreads) k_heuristics_tma(GraphBatch b, int32_t* L, const __grid_constant__ CUtensorMap map)
 {
     const uint8_t* snap = b.snap + b.frame_stride * blockIdx.z;
     uint8_t* out = b.out + b.frame_stride * blockIdx.z;
@@ -582,7 +620,7 @@ __device__ __forceinline__ void uf_unite(int32_t* L, int a, int b)
 // (local roots are the tile-local minima, which are also the minima in global
 // index order), then unions across tile borders on the global label array,
 // then one flattening pass. The frame and batch paths make the tile-local
-// labels inside the 64x16 heuristics tiles (cc_sym_unions, cc_sym_store) and
+// labels inside the 64x16 heuristics tiles (tile_labels) and
 // merge with merge_tile_borders; the stage API (depix_label_components) runs
 // its own 32x32 tiles over a graph in global memory (cc_local_core: a warp
 // owns a row, horizontal runs from one ballot, one union per pair of touching
@@ -662,13 +700,18 @@ __device__ __forceinline__ int run_start(uint64_t S, int c) { return 63 - __clzl
 // deferrals ends at an edge that is kept (e = 0 and e = 1 edges defer only
 // to lower positions, and an e = 2 edge to a lower position or to an e = 1
 // edge), so the kept edges join the same sets as all of them.
+__device__ __forceinline__ uint64_t join_mask(int e, uint64_t Sr, uint64_t Sq, uint64_t E0, uint64_t E1, uint64_t E2,
+                                              uint64_t q_end)
+{
+    if (e == 0) return E0 & ~(~Sr & (((E0 & ~Sq) << 1) | (E1 << 1)));
+    if (e == 1) return E1 & ~((E1 << 1) & ~Sr & ~Sq);
+    return E2 & ~(((E2 << 1) & ~Sr & ~((Sq >> 1) | q_end)) | ((E1 & ~Sr) >> 1));
+}
 __device__ __forceinline__ void join_masks(uint64_t Sr, uint64_t Sq, uint64_t E0, uint64_t E1, uint64_t E2,
                                            uint64_t q_end, uint64_t (&need)[3])
 {
-    const uint64_t nSr = ~Sr, nSq = ~Sq;
-    need[0] = E0 & ~(nSr & (((E0 & nSq) << 1) | (E1 << 1)));
-    need[1] = E1 & ~((E1 << 1) & nSr & nSq);
-    need[2] = E2 & ~(((E2 << 1) & nSr & ~((Sq >> 1) | q_end)) | ((E1 & nSr) >> 1));
+#pragma unroll
+    for (int e = 0; e < 3; e++) need[e] = join_mask(e, Sr, Sq, E0, E1, E2, q_end);
 }
 
 // fn(e, c) for every set bit c of need[e], spread over the warp's lanes
@@ -685,85 +728,102 @@ __device__ __forceinline__ void for_each_join(const uint64_t (&need)[3], Fn fn)
     }
 }
 
-// Joins of a 64-pixel-wide tile of a symmetric graph (each edge held by
-// both of its nodes, as in the resolved graph) whose parents start at the
-// run roots (a run's leftmost pixel, see heuristics_tile). Warp w owns the
-// row pairs (r, r + 1) for r = w and w + 8 (edges up-left, up, up-right as
-// e = 0, 1, 2): it parks each pair's run starts and the edges join_masks
-// keeps, then spreads the unions of both pairs over its lanes at once (one
-// round of unions for up to 32 of them, not one per pair). Blocks of 256
-// threads (8 warps).
-template <int TW, int TH>
-__device__ void cc_sym_unions(const uint8_t* sg, int* sl)
+// Component labels of a 64x16 tile of a symmetric graph (each edge held by
+// both of its nodes, as in the resolved graph; 0 outside the image), as global
+// indices of the tile-local roots. A run's parent is kept at its leftmost
+// pixel. The rows' run starts and upward edges become 64-bit masks by ballot;
+// a lane then lists the edges of one kind between half a row and the row above
+// it that join_masks keeps (three warps, one a kind); all threads unite along
+// the listed edges, one each (a lane that united its own edges in turn waited
+// for a chain of finds per edge: 8.4 k cycles of a tile's 26 k); then the
+// listed runs, which are all that are not their own root, are pointed at their
+// roots, and each pixel reads its run's parent (following the chains from
+// there cost 6.8 k cycles).
+__device__ void tile_labels(const uint8_t (*node)[kHTW], uint16_t* joins, int32_t* L, int w, int h, int x0, int y0)
 {
-    static_assert(TW == 64 && TH <= 17, "two 32-pixel segments per row, at most two row pairs per warp");
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    __shared__ uint64_t pm[8][2][5]; // per warp and pair: Sr, Sq, kept edges e = 0, 1, 2
-    __shared__ int pcnt[8][7];       // per warp: prefix of the kept-edge counts
-    int npairs = 0;
-    for (int r = warp; r < TH - 1; r += nwarp, npairs++) {
-        const int p0 = r * TW + lane;
-        const unsigned a0 = sg[p0], a1 = sg[p0 + 32], b0 = sg[p0 + TW], b1 = sg[p0 + TW + 32];
-        const uint64_t Sr = ballot64(lane == 0 || !bitof(a0, 3), !bitof(a1, 3));
-        const uint64_t Sq = ballot64(lane == 0 || !bitof(b0, 3), !bitof(b1, 3));
-        uint64_t need[3];
-        join_masks(Sr, Sq, ballot64(bitof(a0, 0), bitof(a1, 0)) & ~1ull, ballot64(bitof(a0, 1), bitof(a1, 1)),
-                   ballot64(bitof(a0, 2), bitof(a1, 2)) & ~(1ull << 63), 1ull << 63, need);
-        if (lane == 0) {
-            pm[warp][npairs][0] = Sr;
-            pm[warp][npairs][1] = Sq;
-            pm[warp][npairs][2] = need[0];
-            pm[warp][npairs][3] = need[1];
-            pm[warp][npairs][4] = need[2];
+    static_assert(kHTW == 64 && kHTH == 16 && kHThreads == 128, "lanes of the joins");
+    __shared__ __align__(16) int sl[kHTH * kHTW];
+    __shared__ uint64_t rows[4][kHTH]; // run starts, up-left, up, up-right edges
+    __shared__ int njoins;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) njoins = 0;
+    {
+        // eight columns a thread: bit planes of its two words as bytes of the
+        // row masks (the product gathers a word's four bits in its top byte)
+        const int r = threadIdx.x >> 3, g = threadIdx.x & 7;
+        const uint2 v = *reinterpret_cast<const uint2*>(&node[r][8 * g]);
+        auto plane = [&](int bit) -> unsigned {
+            return ((v.x >> bit & 0x01010101u) * 0x01020408u >> 24) | ((v.y >> bit & 0x01010101u) * 0x01020408u >> 24) << 4;
+        };
+        const unsigned first = g == 0, last = g == 7 ? 0x80u : 0u;
+        auto put = [&](int k, unsigned m) { reinterpret_cast<uint8_t*>(&rows[k][r])[g] = (uint8_t)m; };
+        put(0, ~plane(3) | first);
+        put(1, plane(0) & ~first); // edges within the tile
+        put(2, plane(1));
+        put(3, plane(2) & ~last);
+        const int p = 8 * threadIdx.x;
+        int4* q = reinterpret_cast<int4*>(&sl[p]);
+        q[0] = make_int4(p, p + 1, p + 2, p + 3);
+        q[1] = make_int4(p + 4, p + 5, p + 6, p + 7);
+    }
+    __syncthreads();
+    // joins as position in the tile | kind << 10
+    if (warp < 3 && lane < 2 * (kHTH - 1)) {
+        const int r = lane >> 1, half = lane & 1;
+        const uint64_t need = join_mask(warp, rows[0][r], rows[0][r + 1], rows[1][r], rows[2][r], rows[3][r], 1ull << 63);
+        uint32_t m = (uint32_t)(need >> (32 * half));
+        int slot = m ? atomicAdd(&njoins, __popc(m)) : 0;
+        while (m) {
+            joins[slot++] = (uint16_t)(r * kHTW + 32 * half + __ffs(m) - 1 | warp << 10);
+            m &= m - 1;
         }
     }
-    __syncwarp();
-    if (lane == 0) {
-        int t = 0;
-        for (int k = 0; k < 6; k++) {
-            pcnt[warp][k] = t;
-            t += k / 3 < npairs ? __popcll(pm[warp][k / 3][2 + k % 3]) : 0;
-        }
-        pcnt[warp][6] = t;
+    __syncthreads();
+    const int n = njoins;
+    auto runs = [&](int i, int& a, int& b) {
+        const int p = joins[i] & 1023, e = joins[i] >> 10, r = p / kHTW, c = p % kHTW;
+        a = r * kHTW + run_start(rows[0][r], c);
+        b = (r + 1) * kHTW + run_start(rows[0][r + 1], c + e - 1);
+    };
+    for (int i = threadIdx.x; i < n; i += kHThreads) {
+        int a, b;
+        runs(i, a, b);
+        s_unite(sl, a, b);
     }
-    __syncwarp();
-    const int n = pcnt[warp][6];
-    for (int i = lane; i < n; i += 32) {
-        int k = 0;
-        while (k < 5 && pcnt[warp][k + 1] <= i) k++;
-        const int pr = k / 3, e = k % 3, r = warp + pr * nwarp;
-        const uint64_t* m = pm[warp][pr];
-        const int c = nth_set_bit64(m[2 + e], i - pcnt[warp][k]);
-        s_unite(sl, r * TW + run_start(m[0], c), (r + 1) * TW + run_start(m[1], c + e - 1));
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += kHThreads) {
+        int a, b;
+        runs(i, a, b);
+        // no union in flight: both ends have one root, and a store only ever
+        // shortens another thread's way to it
+        const int root = s_root(sl, a);
+        sl[a] = root;
+        sl[b] = root;
     }
-}
-
-// Labels of a tile after cc_sym_unions: one find per run (at its leftmost
-// pixel), shuffled to the run's other pixels (a run that comes into the
-// second segment takes the first segment's last label), stored as global
-// indices of the tile-local roots.
-template <int TW, int TH>
-__device__ void cc_sym_store(const uint8_t* sg, int* sl, int32_t* L, int w, int h, int x0, int y0)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    for (int r = warp; r < TH; r += nwarp) {
-        int carry = 0;
+    __syncthreads();
+    // four pixels a thread: their runs' roots, stored at once where the row allows
+    const bool wide = ((w | x0 | (int)(reinterpret_cast<uintptr_t>(L) >> 2)) & 3) == 0;
 #pragma unroll
-        for (int sgm = 0; sgm < TW / 32; sgm++) {
-            const int c = sgm * 32 + lane, p = r * TW + c;
-            const unsigned starts = __ballot_sync(0xFFFFFFFFu, c == 0 || !bitof(sg[p], 3));
-            const unsigned upto = starts & (0xFFFFFFFFu >> (31 - lane));
-            const int src = upto ? 31 - __clz(upto) : 0;
-            int g = 0;
-            if (upto && src == lane) {
-                const int root = s_find(sl, p);
-                g = (y0 + root / TW) * w + (x0 + root % TW);
-            }
-            g = __shfl_sync(0xFFFFFFFFu, g, src);
-            if (!upto) g = carry;
-            carry = __shfl_sync(0xFFFFFFFFu, g, 31);
-            const int x = x0 + c, y = y0 + r;
-            if (x < w && y < h) L[(size_t)y * w + x] = g;
+    for (int k = threadIdx.x; k < kHTW / 4 * kHTH; k += kHThreads) {
+        const int r = k / (kHTW / 4), c = 4 * (k % (kHTW / 4)), x = x0 + c, y = y0 + r;
+        const uint64_t S = rows[0][r];
+        int run = run_start(S, c);
+        const unsigned s4 = (unsigned)(S >> c);
+        int lab[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (q && (s4 >> q & 1u)) run = c + q;
+            const int root = sl[r * kHTW + run];
+            lab[q] = (y0 + root / kHTW) * w + x0 + root % kHTW;
+        }
+        if (y >= h || x >= w) continue;
+        int32_t* o = L + (size_t)y * w + x;
+        if (wide) {
+            *reinterpret_cast<int4*>(o) = make_int4(lab[0], lab[1], lab[2], lab[3]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (x + q < w) o[q] = lab[q];
         }
     }
 }
@@ -954,31 +1014,29 @@ __global__ void k_cc_merge(const uint8_t* g, int32_t* L, int w, int h, size_t fr
     cc_merge_border(g + frame_stride * blockIdx.z, L + frame_stride * blockIdx.z, w, h, t / kLBorder, t % kLBorder);
 }
 
-// Four consecutive pixels per thread, their labels in one 16-byte load where
-// aligned and their four finds interleaved, so that each thread keeps four
-// independent loads in flight (one find per pixel is bound by load latency).
-__global__ void k_cc_flatten(int32_t* L, int n, size_t frame_stride)
+// Roots of up to four consecutive labels q[0..n): one 16-byte load where
+// aligned, the finds interleaved, so that their loads are in flight together
+// (one find per pixel is bound by load latency; settling groups of one label
+// by one find measured slower, 217 against 194 us for 1024 frames with the
+// merge: the warp then runs both ways one after the other). Only labels that
+// change are written.
+__device__ __forceinline__ void flatten4(int32_t* L, int32_t* q, int n)
 {
-    const int k = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
-    if (k >= n) return;
-    L += frame_stride * blockIdx.z;
-    int32_t* q = L + k;
-    int p[4], x[4];
-    if (k + 3 < n && (reinterpret_cast<uintptr_t>(q) & 15) == 0) {
+    int x[4], p[4], first[4];
+    if (n == 4 && (reinterpret_cast<uintptr_t>(q) & 15) == 0) {
         const int4 v = *reinterpret_cast<const int4*>(q);
-        p[0] = v.x;
-        p[1] = v.y;
-        p[2] = v.z;
-        p[3] = v.w;
+        x[0] = v.x;
+        x[1] = v.y;
+        x[2] = v.z;
+        x[3] = v.w;
     } else {
 #pragma unroll
-        for (int i = 0; i < 4; i++) p[i] = k + i < n ? q[i] : k + i;
+        for (int i = 0; i < 4; i++) x[i] = q[i < n ? i : 0];
     }
-    int first[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        x[i] = k + i;
-        first[i] = p[i];
+        first[i] = x[i];
+        p[i] = L[x[i]];
     }
     for (;;) {
         bool more = false;
@@ -993,7 +1051,15 @@ __global__ void k_cc_flatten(int32_t* L, int n, size_t frame_stride)
     }
 #pragma unroll
     for (int i = 0; i < 4; i++)
-        if (k + i < n && first[i] != x[i]) q[i] = x[i];
+        if (i < n && first[i] != x[i]) q[i] = x[i];
+}
+
+__global__ void k_cc_flatten(int32_t* L, int n, size_t frame_stride)
+{
+    const int k = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (k >= n) return;
+    L += frame_stride * blockIdx.z;
+    flatten4(L, L + k, min(4, n - k));
 }
 
 // ------------------------------------------------ uneven batches (queue)
@@ -1013,7 +1079,7 @@ __global__ void __launch_bounds__(kGThreads) k_graph_queue(QueueBatch q)
 }
 
 template <bool VOTE>
-__global__ void __launch_bounds__(256) k_heur_queue(QueueBatch q)
+__global__ void __launch_bounds__(kHThreads) k_heur_queue(QueueBatch q)
 {
     const QueueHeader* H = q.hdr;
     const int n = H->n;
@@ -1053,9 +1119,9 @@ __global__ void __launch_bounds__(256) k_label_flatten_queue(QueueBatch q)
         const int lt = t - (int)base[f], tx = (fr.w + kLT - 1) / kLT;
         const int x0 = (lt % tx) * kLT, y0 = (lt / tx) * kLT;
         int32_t* L = H->labels + fr.px_off;
-        for (int p = threadIdx.x; p < kLT * kLT; p += blockDim.x) {
-            const int x = x0 + p % kLT, y = y0 + p / kLT;
-            if (x < fr.w && y < fr.h) L[y * fr.w + x] = uf_find(L, y * fr.w + x);
+        for (int p = threadIdx.x; p < kLT / 4 * kLT; p += blockDim.x) {
+            const int x = x0 + 4 * (p % (kLT / 4)), y = y0 + p / (kLT / 4);
+            if (x < fr.w && y < fr.h) flatten4(L, L + y * fr.w + x, min(4, fr.w - x));
         }
     });
 }
@@ -1068,8 +1134,8 @@ cudaError_t queue_graph(const QueueBatch& q, int blocks, cudaStream_t s)
 
 cudaError_t queue_heuristics(const QueueBatch& q, int blocks, cudaStream_t s)
 {
-    if (q.vote) k_heur_queue<true><<<blocks, 256, 0, s>>>(q);
-    else k_heur_queue<false><<<blocks, 256, 0, s>>>(q);
+    if (q.vote) k_heur_queue<true><<<blocks, kHThreads, 0, s>>>(q);
+    else k_heur_queue<false><<<blocks, kHThreads, 0, s>>>(q);
     return cudaGetLastError();
 }
 
@@ -1097,7 +1163,7 @@ int queue_blocks_per_sm(int stage, const QueueBatch& q)
 {
     switch (stage) {
     case QS_GRAPH: return occupancy(k_graph_queue, kGThreads);
-    case QS_HEUR: return q.vote ? occupancy(k_heur_queue<true>, 256) : occupancy(k_heur_queue<false>, 256);
+    case QS_HEUR: return q.vote ? occupancy(k_heur_queue<true>, kHThreads) : occupancy(k_heur_queue<false>, kHThreads);
     case QS_LABEL: return occupancy(k_label_flatten_queue, 256);
     default: return queue_raster_blocks_per_sm(q);
     }
@@ -1163,27 +1229,15 @@ cudaError_t launch_trivial(uint8_t* g, int w, int h, cudaStream_t s)
     return cudaGetLastError();
 }
 
-cudaError_t launch_heuristics(const GraphBatch& b, int nframes, cudaStream_t s)
+cudaError_t launch_heuristics(const GraphBatch& b, int nframes, int32_t* labels, cudaStream_t s)
 {
     dim3 grid((b.w + kHTW - 1) / kHTW, (b.h + kHTH - 1) / kHTH, nframes);
     CUtensorMap map;
     const bool tma = u8_tensor_map(b.snap, b.w, b.h, b.frame_stride, nframes, kHRW, kHRH, &map);
-    if (tma && b.vote) k_heuristics_tma<true><<<grid, 256, 0, s>>>(b, nullptr, map);
-    else if (tma) k_heuristics_tma<false><<<grid, 256, 0, s>>>(b, nullptr, map);
-    else if (b.vote) k_heuristics<true><<<grid, 256, 0, s>>>(b);
-    else k_heuristics<false><<<grid, 256, 0, s>>>(b);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_heuristics_labels(const GraphBatch& b, int nframes, int32_t* labels, cudaStream_t s)
-{
-    dim3 grid((b.w + kHTW - 1) / kHTW, (b.h + kHTH - 1) / kHTH, nframes);
-    CUtensorMap map;
-    const bool tma = u8_tensor_map(b.snap, b.w, b.h, b.frame_stride, nframes, kHRW, kHRH, &map);
-    if (tma && b.vote) k_heuristics_tma<true><<<grid, 256, 0, s>>>(b, labels, map);
-    else if (tma) k_heuristics_tma<false><<<grid, 256, 0, s>>>(b, labels, map);
-    else if (b.vote) k_heuristics_labels<true><<<grid, 256, 0, s>>>(b, labels);
-    else k_heuristics_labels<false><<<grid, 256, 0, s>>>(b, labels);
+    if (tma && b.vote) k_heuristics_tma<true><<<grid, kHThreads, 0, s>>>(b, labels, map);
+    else if (tma) k_heuristics_tma<false><<<grid, kHThreads, 0, s>>>(b, labels, map);
+    else if (b.vote) k_heuristics<true><<<grid, kHThreads, 0, s>>>(b, labels);
+    else k_heuristics<false><<<grid, kHThreads, 0, s>>>(b, labels);
     return cudaGetLastError();
 }
 

@@ -1285,7 +1285,7 @@ depix_status depix_refine_setup(depix_refiner* r, const uint8_t* d_img, int w, i
         RF_CK(r->own_snap.reserve(n));
         const FrameBatch fb{d_img, 0, r->own_snap.p, 0, w, h, widthstep, (int)layout};
         RF_CK(launch_graph(fb, 1, pack_thresholds(p->tr_y, p->tr_u, p->tr_v, p->yuv), true, s));
-        RF_CK(launch_heuristics(GraphBatch{r->own_snap.p, r->own_graph.p, 0, w, h, p->vote}, 1, s));
+        RF_CK(launch_heuristics(GraphBatch{r->own_snap.p, r->own_graph.p, 0, w, h, p->vote}, 1, nullptr, s));
         d_graph = r->own_graph.p;
     }
     Geo G{d_img, widthstep, (int)layout, d_graph, w, h, gw, gh, r->lut, r->box.p,

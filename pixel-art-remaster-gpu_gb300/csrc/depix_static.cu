@@ -101,7 +101,7 @@ depix_status depix_resolve_heuristics_static(uint8_t* d_graph, int w, int h, dep
     // the copy overwrites every snapshot byte the kernel reads: nothing has
     // to start at zero, whatever an earlier call left in the array
     cudaError_t e = cudaMemcpyAsync(snap, d_graph, n, cudaMemcpyDeviceToDevice, cs);
-    if (e == cudaSuccess) e = depix::launch_heuristics(depix::GraphBatch{snap, d_graph, 0, w, h}, 1, cs);
+    if (e == cudaSuccess) e = depix::launch_heuristics(depix::GraphBatch{snap, d_graph, 0, w, h}, 1, nullptr, cs);
     if (e != cudaSuccess) {
         depix::set_last_error(std::string("snapshot copy or launch: ") + cudaGetErrorString(e));
         return DEPIX_ERR_CUDA;
