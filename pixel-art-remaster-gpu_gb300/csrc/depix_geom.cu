@@ -11,6 +11,7 @@
 #include <map>
 #include <memory>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "depix_internal.h"
@@ -674,15 +675,15 @@ __host__ __device__ __forceinline__ MaskGeom mask_geom(int s)
 }
 
 enum MaskLayout { ML_U16, ML_U64, ML_ROWS };
-__host__ __device__ constexpr MaskLayout mask_layout(int s) { return s <= 4 ? ML_U16 : (s <= 8 ? ML_U64 : ML_ROWS); }
+__host__ __device__ constexpr MaskLayout mask_layout(int s) { return s <= 4 ? ML_U16 : (s == 8 ? ML_U64 : ML_ROWS); }
 // words of a mask, of a table entry (mask, then 16 flag bits: above part 8
 // for ML_U16, in a word of their own else) and between masks in shared memory
 // (odd, so that a warp's cells fall into different banks)
 __host__ __device__ __forceinline__ int mask_words(int s)
 {
-    return s <= 4 ? 5 : (s <= 8 ? 18 : mask_geom(s).F);
+    return s <= 4 ? 5 : (s == 8 ? 18 : mask_geom(s).F);
 }
-__host__ __device__ __forceinline__ int entry_words(int s) { return s <= 4 ? 8 : (s <= 8 ? 20 : ((mask_geom(s).F + 4) & ~3)); }
+__host__ __device__ __forceinline__ int entry_words(int s) { return s <= 4 ? 8 : (s == 8 ? 20 : ((mask_geom(s).F + 4) & ~3)); }
 __host__ __device__ __forceinline__ int mask_stride(int s) { return mask_words(s) | 1; }
 
 // a scale's table: plain hulls, cut cells' own pieces (per pattern), paths
@@ -864,9 +865,9 @@ cudaError_t build_scale_masks(int s, uint32_t* lut, cudaStream_t st)
 __device__ int g_raster_fault;
 
 // Compile-time scale of a raster kernel: 1..4 and 8 themselves, 0 the scales
-// 5 to 7 (64-bit parts), -1 the scales above 8 (rows).
+// 5 to 7, -1 the scales above 8.
 __host__ __device__ constexpr int raster_mode(int s) { return (s <= 4 || s == 8) ? s : (s < 8 ? 0 : -1); }
-__host__ __device__ constexpr MaskLayout mode_layout(int S) { return S < 0 ? ML_ROWS : (S == 0 ? ML_U64 : mask_layout(S)); }
+__host__ __device__ constexpr MaskLayout mode_layout(int S) { return S <= 0 ? ML_ROWS : mask_layout(S); }
 
 // Threads of a raster block, and the blocks per SM that its registers leave
 // room for: 48 registers and five blocks up to x4, whose masks take 23 KB of a
@@ -927,7 +928,8 @@ __device__ __forceinline__ int list_slot(int* counter, bool pred)
 // and ear-clipped as the reference does, triangle by triangle. g: the cell's
 // graph byte in the tile window (rows of `pitch` bytes); keep: bit c the
 // corner test at corner c (as CutTables::corners), bit 4 every vertex kept.
-__device__ __noinline__ void ear_clip_cell_mask(const uint8_t* g, int pitch, unsigned keep, int s, uint32_t* dst)
+__device__ __noinline__ void ear_clip_cell_mask(const uint8_t* g, int pitch, unsigned keep, int s, uint32_t* dst,
+                                                uint16_t* info)
 {
     const MaskGeom G = mask_geom(s);
     auto pattern = [&](const uint8_t* q) { return cell_pattern(q[0], q[-1], q[1]); };
@@ -954,17 +956,28 @@ __device__ __noinline__ void ear_clip_cell_mask(const uint8_t* g, int pitch, uns
         tri_mask(p.x[a] * u, p.y[a] * u, p.x[b] * u, p.y[b] * u, p.x[d] * u, p.y[d] * u, G.mlo, G.F, rows);
     }
     pack_mask(G, rows, dst);
+    if (mask_layout(s) == ML_ROWS) {
+        const uint32_t blockbits = (1u << s) - 1u;
+        unsigned touched = 512u;
+        for (int r = 0; r < G.F; r++) {
+            const int m = r + G.mlo, dj = m < 0 ? 0 : (m >= s ? 2 : 1);
+            const uint64_t x = (uint64_t)rows[r] << (s + G.mlo);
+            for (int di = 0; di < 3; di++)
+                if ((x >> (di * s)) & blockbits) touched |= 1u << (dj * 3 + di);
+            if (dj == 1 && ((rows[r] >> -G.mlo) & blockbits) != blockbits) touched &= ~512u;
+        }
+        *info = (uint16_t)touched;
+    }
 }
 
-// XOR of table entries: in registers for the part layouts, straight in the
-// cell's mask for the rows
+// XOR of table entries in registers
 template <MaskLayout ML>
 struct MaskAcc {
     static constexpr int W = ML == ML_U16 ? 5 : 18;
     uint32_t w[W];
     unsigned flags;
     uint32_t* dst;
-    __device__ __forceinline__ MaskAcc(uint32_t* d, int) : flags(0), dst(d)
+    __device__ __forceinline__ MaskAcc(uint32_t* d, const MaskGeom&, uint16_t*) : flags(0), dst(d)
     {
 #pragma unroll
         for (int k = 0; k < W; k++) w[k] = 0;
@@ -995,29 +1008,65 @@ struct MaskAcc {
         for (int k = 0; k < W; k++) dst[k] = w[k];
     }
 };
-template <>
-struct MaskAcc<ML_ROWS> {
+// rows: store() also notes the parts that the mask touches (bits 0-8) and
+// whether it covers its own block (bit 9)
+template <int MODE>
+struct MaskAccRows {
+    static constexpr int NQ = MODE == 0 ? 5 : 8; // row quads: F + 1 is at most 18 up to x7, 31 up to x12
+    uint32_t w[4 * NQ];
     uint32_t* dst;
-    int F;
+    uint16_t* info;
+    MaskGeom G;
     unsigned flags;
-    __device__ __forceinline__ MaskAcc(uint32_t* d, int F_) : dst(d), F(F_), flags(0)
+    __device__ __forceinline__ MaskAccRows(uint32_t* d, const MaskGeom& G_, uint16_t* i) : dst(d), info(i), G(G_), flags(0)
     {
-        for (int r = 0; r < F; r++) dst[r] = 0;
+#pragma unroll
+        for (int k = 0; k < 4 * NQ; k++) w[k] = 0;
     }
     __device__ __forceinline__ void add(const uint32_t* e)
     {
-        for (int r = 0; r < F; r++) dst[r] ^= __ldg(e + r);
-        flags += __ldg(e + F);
+#pragma unroll
+        for (int k = 0; k < NQ; k++)
+            if (4 * k < G.F) {
+                const uint4 a = __ldg(reinterpret_cast<const uint4*>(e) + k);
+                w[4 * k] ^= a.x; w[4 * k + 1] ^= a.y; w[4 * k + 2] ^= a.z; w[4 * k + 3] ^= a.w;
+            }
+        flags += __ldg(e + G.F);
     }
-    __device__ __forceinline__ void store() const {}
+    __device__ __forceinline__ void store() const
+    {
+        const uint32_t blockbits = (1u << G.s) - 1u;
+        uint32_t lo = 0, mid = 0, hi = 0, all = blockbits;
+#pragma unroll
+        for (int r = 0; r < 4 * NQ; r++) {
+            const int m = r + G.mlo;
+            if (r >= G.F) break;
+            dst[r] = w[r];
+            if (m < 0) lo |= w[r];
+            else if (m >= G.s) hi |= w[r];
+            else {
+                mid |= w[r];
+                all &= w[r] >> -G.mlo;
+            }
+        }
+        *info = (uint16_t)(mask_columns(G, lo) | mask_columns(G, mid) << 3 | mask_columns(G, hi) << 6 |
+                           (all == blockbits ? 512u : 0u));
+    }
+    // bit di + 1 set when a footprint row's bits reach the block column di
+    static __device__ __forceinline__ unsigned mask_columns(const MaskGeom& G, uint32_t row)
+    {
+        const uint64_t x = (uint64_t)row << (G.s + G.mlo);
+        const uint32_t blockbits = (1u << G.s) - 1u;
+        return ((x & blockbits) ? 1u : 0u) | ((x >> G.s & blockbits) ? 2u : 0u) | ((x >> (2 * G.s)) ? 4u : 0u);
+    }
 };
 
 // Mask of a subdivided cell as the XOR of its pieces. pat, g: its pattern and
 // its graph byte in the tile window (rows of `pitch` bytes); keep_of(corner
 // classes) the corners (bits 0-3, as CutTables::corners) that the T-junction
 // test keeps, bit 4 when it keeps every vertex.
-template <MaskLayout ML, typename Keep>
-__device__ __forceinline__ void cut_cell_mask(MaskAcc<ML>& acc, int pat, const uint8_t* g, int pitch, const uint32_t* lut,
+template <typename Acc, typename Keep>
+__device__ __forceinline__ void cut_cell_mask(Acc& acc, int pat, const uint8_t* g, int pitch, const uint32_t* lut,
                                               int ES, Keep keep_of)
 {
     const uint4 ed = __ldg(&g_cut.edges[pat]);
@@ -1117,8 +1166,12 @@ __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const 
 {
     using T = MaskTile<S, TW, TH>;
     constexpr MaskLayout ML = mode_layout(S);
+    using Acc = std::conditional_t<ML == ML_ROWS, MaskAccRows<S>, MaskAcc<ML == ML_ROWS ? ML_U16 : ML>>;
     const int s = S > 0 ? S : scale;
+    const MaskGeom G = mask_geom(s);
     const int MS = mask_stride(s), ES = entry_words(s), MW = mask_words(s);
+    // rows layout: after the masks the cells' touched parts
+    uint16_t* info = reinterpret_cast<uint16_t*>(masks + T::GN * MS);
     constexpr uint32_t kAlpha = 0xFF000000u;
     // ---- phase A
     if constexpr (TMA) {
@@ -1180,17 +1233,27 @@ __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const 
             uint32_t* dst = masks + k * MS;
             if (ci < 0 || cj < 0 || ci >= w || cj >= h) {
                 for (int r = 0; r < MW; r++) dst[r] = 0;
+                if (ML == ML_ROWS) info[k] = 0;
             } else {
                 const uint8_t* gb = &M.graph[ly + 2][lx + 2 + T::kGOff];
                 const unsigned node = gb[0];
                 cut = subdivide && node != 90;
                 if (!cut) {
-                    if (ML == ML_U16 && node == 90) {
-                        // linked on its four sides only: its own square
-                        dst[0] = dst[1] = dst[3] = dst[4] = 0;
-                        dst[2] = T::kFull; // part 4
+                    if (node == 90) {
+                        // linked on its four sides only: its own square, part 4
+                        if constexpr (ML == ML_U16) {
+                            dst[0] = dst[1] = dst[3] = dst[4] = 0;
+                            dst[2] = T::kFull;
+                        } else if constexpr (ML == ML_U64) {
+#pragma unroll
+                            for (int r = 0; r < 18; r++) dst[r] = r == 8 || r == 9 ? 0xFFFFFFFFu : 0u;
+                        } else {
+                            for (int r = 0; r < G.F; r++)
+                                dst[r] = r + G.mlo >= 0 && r + G.mlo < s ? ((1u << s) - 1u) << -G.mlo : 0u;
+                            info[k] = 512 | 16;
+                        }
                     } else {
-                        MaskAcc<ML> acc(dst, MW);
+                        Acc acc(dst, G, info + k);
                         acc.add(lut + (size_t)(kPlainEntry + cell_pattern(node, gb[-1], gb[1])) * ES);
                         acc.store();
                     }
@@ -1213,13 +1276,13 @@ __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const 
         const int pat = cell_pattern(gb[0], gb[-1], gb[1]);
         const bool edge = ci == 0 || cj == 0 || ci == w - 1 || cj == h - 1;
         unsigned keep = edge ? edge_corner_tests<LAYOUT>(px, PW, img, ws, w, h, ci, cj) : 0u;
-        MaskAcc<ML> acc(masks + k * MS, MW);
+        Acc acc(masks + k * MS, G, info + k);
         cut_cell_mask(acc, pat, gb, T::GRW, lut, ES, [&](uint32_t corners) {
             if (!edge && corners != 0xFFFFFFFFu) keep = corner_tests(px, PW);
             return keep;
         });
         if ((acc.flags & 0xFFFFu) == 1u) acc.store();
-        else ear_clip_cell_mask(gb, T::GRW, keep, s, masks + k * MS); // not star-shaped
+        else ear_clip_cell_mask(gb, T::GRW, keep, s, masks + k * MS, info + k); // not star-shaped
     }
     __syncthreads();
 
@@ -1229,23 +1292,96 @@ __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const 
     // block is part q of its mask.
     const int ow = w * s;
     const bool vec = (S == 4 || S == 8) && (ow % 4) == 0 && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
-    const uint32_t blockbits = (1u << s) - 1u;
-    auto cand = [&](int k, int q) -> const uint32_t* { return masks + (k + (1 - q / 3) * T::GW + 1 - q % 3) * MS; };
-    // row r of the block as candidate q covers it
-    auto part_row = [&](int k, int q, int r) -> uint32_t {
-        const uint32_t* m = cand(k, q);
-        if constexpr (ML == ML_U16) {
-            return (reinterpret_cast<const uint16_t*>(m)[q] >> (r * s)) & blockbits;
-        } else if constexpr (ML == ML_U64) {
-            return (uint32_t)(((uint64_t)m[2 * q + 1] << 32 | m[2 * q]) >> (r * s)) & blockbits;
-        } else {
-            const MaskGeom G = mask_geom(s);
-            const int rr = r - s * (1 - q / 3) - G.mlo, sh = s * (1 - q % 3) + G.mlo;
-            if (rr < 0 || rr >= G.F) return 0u;
-            const uint64_t b = m[rr];
-            return (uint32_t)(sh >= 0 ? b << sh : b >> -sh) & blockbits;
+    if constexpr (ML == ML_ROWS) {
+        // A warp takes 32 blocks of the tile (one or two of its rows) and
+        // writes the output rows of those that their own cell fills in order,
+        // four pixels a lane, so that the stores are contiguous whatever s is;
+        // the rows of the other blocks follow, one a thread. (Resolving each
+        // row of the 32 blocks in the warp and writing it whole: 132 us for 100
+        // frames of 152x102 at x5, 96 us now; one thread a block, which stores
+        // every pixel apart: 171.)
+        constexpr int CM = S == 0 ? 7 : 12; // most samples of a row
+        const uint32_t blockbits = (1u << s) - 1u;
+        const unsigned inv = (1u << 20) / (unsigned)s + 1u; // x / s = x inv >> 20 for x up to a tile's rows (12 k)
+        const int lane = threadIdx.x & 31;
+        const bool quads = (ow % 4) == 0 && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
+        for (int b0 = threadIdx.x & ~31; b0 < TW * TH; b0 += kRT) {
+            const int tx = lane % TW, ty = (b0 + lane) / TW, k = (ty + 1) * T::GW + tx + 1;
+            const bool in = x0 + tx < w && y0 + ty < h;
+            auto touch = [&](int q) { return (unsigned)info[k + (1 - q / 3) * T::GW + 1 - q % 3] >> q & 1u; };
+            const bool fill = (info[k] & 512u) && !(touch(0) | touch(1) | touch(2) | touch(3));
+            const uint32_t own = M.pix[ty + 2][tx + 4] | kAlpha;
+            const int slot = list_slot(&M.slow, in && !fill);
+            if (in && !fill) M.list[slot] = (uint16_t)(b0 + lane);
+            const unsigned filled = __ballot_sync(0xFFFFFFFFu, in && fill);
+            if (!filled) continue;
+            const int per = quads ? 4 : 1;
+            for (int i0 = 0; i0 < 32 * s; i0 += 32 * per) {
+                const int i = i0 + per * lane;
+                const bool live = i < 32 * s;
+                // a lane's pixels lie in at most two blocks (s > 4)
+                const int ba = live ? (int)(i * inv >> 20) : 0, bb = live ? (int)((i + per - 1) * inv >> 20) : 0;
+                const uint32_t ca = __shfl_sync(0xFFFFFFFFu, own, ba), cb = __shfl_sync(0xFFFFFFFFu, own, bb);
+                const bool fa = filled >> ba & 1u, fb = filled >> bb & 1u;
+                if (!live || !(fa || fb)) continue;
+                const int row = TW == 32 ? 0 : (i >= TW * s);
+                uint32_t* o = reinterpret_cast<uint32_t*>(out) + (size_t)((y0 + b0 / TW + row) * s) * ow +
+                              (x0 * s + i - row * TW * s);
+                const int left = bb * s - i; // pixels of the lane in block ba, when the blocks differ
+                if (!quads) {
+                    for (int r = 0; r < s; r++) o[(size_t)r * ow] = ca;
+                } else if (fa && fb) {
+                    const uint4 v = ba == bb ? make_uint4(ca, ca, ca, ca)
+                                             : make_uint4(ca, left > 1 ? ca : cb, left > 2 ? ca : cb, cb);
+                    for (int r = 0; r < s; r++) __stcs(reinterpret_cast<uint4*>(o + (size_t)r * ow), v);
+                } else {
+                    for (int r = 0; r < s; r++)
+#pragma unroll
+                        for (int c = 0; c < 4; c++)
+                            if ((ba == bb || c < left) ? fa : fb) o[(size_t)r * ow + c] = (ba == bb || c < left) ? ca : cb;
+                }
+            }
         }
-    };
+        __syncthreads();
+        const int rows = M.slow * s;
+        for (int i = threadIdx.x; i < rows; i += kRT) {
+            const int bi = (int)((unsigned)i * inv >> 20), r = i - bi * s, q0 = M.list[bi];
+            const int tx = q0 % TW, ty = q0 / TW, k = (ty + 1) * T::GW + tx + 1;
+            const uint32_t* px = &M.pix[ty + 2][tx + 4];
+            uint32_t col[CM], claimed = 0;
+#pragma unroll
+            for (int c = 0; c < CM; c++) col[c] = kAlpha; // no owner: the clear colour
+            unsigned owners = 0; // candidates that touch the block
+#pragma unroll
+            for (int q = 0; q < 9; q++)
+                owners |= (unsigned)info[k + (1 - q / 3) * T::GW + 1 - q % 3] & 1u << q;
+            while (owners && claimed != blockbits) {
+                const int q = __ffs(owners) - 1, dj = 1 - q / 3, di = 1 - q % 3;
+                owners &= owners - 1;
+                const int rr = r - s * dj - G.mlo, sh = s * di + G.mlo; // block column = footprint column + sh
+                if (rr < 0 || rr >= G.F) continue;
+                const uint64_t m = masks[(k + dj * T::GW + di) * MS + rr];
+                const uint32_t take = (uint32_t)(sh >= 0 ? m << sh : m >> -sh) & blockbits & ~claimed;
+                const uint32_t c0 = px[dj * (T::CW + 4) + di] | kAlpha;
+                claimed |= take;
+#pragma unroll
+                for (int c = 0; c < CM; c++)
+                    if (take >> c & 1u) col[c] = c0;
+            }
+            uint32_t* o = reinterpret_cast<uint32_t*>(out) + (size_t)((y0 + ty) * s + r) * ow + (size_t)(x0 + tx) * s;
+            if (S < 0 && quads && s % 4 == 0) {
+#pragma unroll
+                for (int c = 0; c < CM; c += 4)
+                    if (c < s) __stcs(reinterpret_cast<uint4*>(o + c), make_uint4(col[c], col[c + 1], col[c + 2], col[c + 3]));
+            } else {
+#pragma unroll
+                for (int c = 0; c < CM; c++)
+                    if (c < s) o[c] = col[c];
+            }
+        }
+        return;
+    }
+    auto cand = [&](int k, int q) -> const uint32_t* { return masks + (k + (1 - q / 3) * T::GW + 1 - q % 3) * MS; };
     constexpr int NG = T::NG;
     constexpr int GR = S == 8 ? 2 : (S > 0 ? S : 1); // rows of a group
     constexpr uint32_t kFull = T::kFull;
@@ -1261,25 +1397,16 @@ __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const 
         const int k = (ty + 1) * T::GW + tx + 1;
         // filled at once: its own cell covers all of it and no later one any
         bool fill = false;
-        if (in) {
-            if constexpr (S > 0) {
-                fill = group(k, 4, gr) == kFull &&
-                       (group(k, 0, gr) | group(k, 1, gr) | group(k, 2, gr) | group(k, 3, gr)) == 0;
-            } else {
-                fill = true;
-                for (int r = 0; r < s && fill; r++)
-                    fill = part_row(k, 4, r) == blockbits &&
-                           (part_row(k, 0, r) | part_row(k, 1, r) | part_row(k, 2, r) | part_row(k, 3, r)) == 0;
-            }
-        }
+        if (in)
+            fill = group(k, 4, gr) == kFull &&
+                   (group(k, 0, gr) | group(k, 1, gr) | group(k, 2, gr) | group(k, 3, gr)) == 0;
         const int slot = list_slot(&M.slow, in && !fill);
         if (in && !fill) M.list[slot] = (uint16_t)i; // resolved after the barrier, over a compacted list
         if (!fill) continue;
         const uint32_t col = M.pix[ty + 2][tx + 4] | kAlpha;
         uint8_t* orow = out + (((size_t)cj * s + gr * GR) * ow + (size_t)ci * s) * 4;
-        const int rows = S > 0 ? GR : s;
 #pragma unroll
-        for (int r = 0; r < rows; r++) {
+        for (int r = 0; r < GR; r++) {
             uint32_t* o = reinterpret_cast<uint32_t*>(orow + (size_t)r * ow * 4);
             if (vec) {
 #pragma unroll
@@ -1298,68 +1425,44 @@ __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const 
         const int k = (ty + 1) * T::GW + tx + 1;
         uint8_t* orow = out + (((size_t)cj * s + gr * GR) * ow + (size_t)ci * s) * 4;
         const uint32_t* px = &M.pix[ty + 2][tx + 4];
-        auto colour = [&](int q) -> uint32_t { return px[(1 - q / 3) * (T::CW + 4) + 1 - q % 3] | kAlpha; };
-        if constexpr (S > 0) {
-            // candidates from the latest on until every sample has its owner
-            // (each lane walks its own block's owners, so that a warp's trips
-            // are the most owners of a block, not the nine candidates)
-            constexpr int NS = S == 8 ? 16 : S * S, RL = S;
-            uint32_t col[NS], claimed = 0;
-            unsigned owners = 0;
+        // candidates from the latest on until every sample has its owner
+        // (each lane walks its own block's owners, so that a warp's trips
+        // are the most owners of a block, not the nine candidates)
+        constexpr int NS = S == 8 ? 16 : (S > 0 ? S * S : 1), RL = S;
+        uint32_t col[NS], claimed = 0;
+        unsigned owners = 0;
 #pragma unroll
-            for (int q = 0; q < 9; q++) {
-                const uint32_t m = group(k, q, gr);
-                if (m & ~claimed) owners |= 1u << q;
-                claimed |= m;
-            }
+        for (int q = 0; q < 9; q++) {
+            const uint32_t m = group(k, q, gr);
+            if (m & ~claimed) owners |= 1u << q;
+            claimed |= m;
+        }
 #pragma unroll
-            for (int c = 0; c < NS; c++) col[c] = kAlpha; // no owner: the clear colour
-            claimed = 0;
-            while (owners) {
-                const int q = __ffs(owners) - 1;
-                owners &= owners - 1;
-                const int dj = 1 - q / 3, di = 1 - q % 3;
-                const uint16_t* mp = reinterpret_cast<const uint16_t*>(masks + (k + dj * T::GW + di) * MS);
-                const uint32_t m = mp[S == 8 ? 4 * q + gr : q], take = m & ~claimed;
-                const uint32_t c0 = px[dj * (T::CW + 4) + di] | kAlpha;
-                claimed |= m;
+        for (int c = 0; c < NS; c++) col[c] = kAlpha; // no owner: the clear colour
+        claimed = 0;
+        while (owners) {
+            const int q = __ffs(owners) - 1;
+            owners &= owners - 1;
+            const int dj = 1 - q / 3, di = 1 - q % 3;
+            const uint16_t* mp = reinterpret_cast<const uint16_t*>(masks + (k + dj * T::GW + di) * MS);
+            const uint32_t m = mp[S == 8 ? 4 * q + gr : q], take = m & ~claimed;
+            const uint32_t c0 = px[dj * (T::CW + 4) + di] | kAlpha;
+            claimed |= m;
 #pragma unroll
-                for (int c = 0; c < NS; c++)
-                    if ((take >> c) & 1u) col[c] = c0;
-            }
+            for (int c = 0; c < NS; c++)
+                if ((take >> c) & 1u) col[c] = c0;
+        }
 #pragma unroll
-            for (int r = 0; r < GR; r++) {
-                uint32_t* o = reinterpret_cast<uint32_t*>(orow + (size_t)r * ow * 4);
-                if (vec) {
+        for (int r = 0; r < GR; r++) {
+            uint32_t* o = reinterpret_cast<uint32_t*>(orow + (size_t)r * ow * 4);
+            if (vec) {
 #pragma unroll
-                    for (int c4 = 0; c4 + 3 < RL; c4 += 4)
-                        __stcs(reinterpret_cast<uint4*>(o + c4), make_uint4(col[r * RL + c4], col[r * RL + c4 + 1],
-                                                                            col[r * RL + c4 + 2], col[r * RL + c4 + 3]));
-                } else {
+                for (int c4 = 0; c4 + 3 < RL; c4 += 4)
+                    __stcs(reinterpret_cast<uint4*>(o + c4), make_uint4(col[r * RL + c4], col[r * RL + c4 + 1],
+                                                                        col[r * RL + c4 + 2], col[r * RL + c4 + 3]));
+            } else {
 #pragma unroll
-                    for (int c = 0; c < RL; c++) o[c] = col[r * RL + c];
-                }
-            }
-        } else {
-            for (int r = 0; r < s; r++) {
-                uint32_t col[12], claimed = 0;
-#pragma unroll
-                for (int c = 0; c < 12; c++) col[c] = kAlpha;
-#pragma unroll 1
-                for (int q = 0; q < 9; q++) {
-                    const uint32_t m = part_row(k, q, r), take = m & ~claimed;
-                    if (!take) continue;
-                    const uint32_t c0 = colour(q);
-#pragma unroll
-                    for (int c = 0; c < 12; c++)
-                        if ((take >> c) & 1u) col[c] = c0;
-                    claimed |= m;
-                    if (claimed == blockbits) break;
-                }
-                uint32_t* o = reinterpret_cast<uint32_t*>(orow + (size_t)r * ow * 4);
-#pragma unroll
-                for (int c = 0; c < 12; c++)
-                    if (c < s) o[c] = col[c];
+                for (int c = 0; c < RL; c++) o[c] = col[r * RL + c];
             }
         }
     }
@@ -1462,11 +1565,15 @@ static bool pixel_tensor_map(const RasterBatch& b, int nframes, int TH, CUtensor
     return rgba_tensor_map(b.img, b.w, b.h, b.ws, b.img_stride, nframes, 32 + 8, TH + 4, map);
 }
 
-// dynamic shared memory: the cells' masks
+// dynamic shared memory: the cells' masks, in the rows layout also what they
+// touch
 template <int S, int TW, int TH>
 static size_t mask_smem(int scale)
 {
-    return (size_t)MaskTile<S, TW, TH>::GN * mask_stride(scale) * sizeof(uint32_t);
+    constexpr size_t GN = MaskTile<S, TW, TH>::GN;
+    size_t words = GN * mask_stride(scale);
+    if (mode_layout(S) == ML_ROWS) words += (GN + 1) / 2;
+    return words * sizeof(uint32_t);
 }
 
 template <int LAYOUT, int S, int TH>

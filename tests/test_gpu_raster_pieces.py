@@ -69,3 +69,34 @@ def test_raster_of_random_graphs(cuda, scale, layout):
                          torch.from_numpy(g.reshape(-1).copy()).cuda(), depix.params(48, 7, 6, sub, scale), out)
             got = out.cpu().numpy().reshape(h * scale, w * scale, 4)
             assert np.array_equal(got, want), (w, h, kind, sub)
+
+
+@pytest.mark.parametrize("tile", [(32, 32), (32, 16), (16, 16)])
+@pytest.mark.parametrize("scale", [1, 3, 4, 5, 7, 8, 9, 12])
+def test_queue_tiles_of_every_layout(cuda, scale, tile):
+    """Uneven batches through each raster tile, on images of mostly shared
+    blocks (a random colour per pixel of three) and flat ones."""
+    import depix
+    torch = cuda
+    rng = np.random.default_rng([scale, *tile])
+    sizes = [(1, 1), (33, 31), (16, 17), (40, 64), (64, 33)]
+    imgs = [rng.integers(0, 3 if k % 2 else 1, size=(h, w, 4)).astype(np.uint8) * 90 for k, (w, h) in enumerate(sizes)]
+    io = np.concatenate([[0], np.cumsum([(4 * w * h + 15) // 16 * 16 for w, h in sizes])])
+    oo = np.concatenate([[0], np.cumsum([(4 * w * h * scale * scale + 15) // 16 * 16 for w, h in sizes])])
+    buf = np.zeros(int(io[-1]), np.uint8)
+    for k, img in enumerate(imgs):
+        buf[io[k]:io[k] + img.size] = img.reshape(-1)
+    ctx = depix.Context(max(w * h for w, h in sizes), len(sizes))
+    ctx.set_launch_shape(2, *tile)
+    out = torch.zeros(int(oo[-1]), dtype=torch.uint8, device="cuda")
+    ctx.batch([w for w, _ in sizes], [h for _, h in sizes], io[:-1].astype(np.uint64), oo[:-1].astype(np.uint64),
+              torch.from_numpy(buf).cuda(), depix.params(48, 7, 6, True, scale), out)
+    out = out.cpu().numpy()
+    ctx.close()
+    for k, (w, h) in enumerate(sizes):
+        ws = (3 * w + 3) & ~3
+        ref = np.zeros((h, ws), np.uint8)
+        ref[:, :3 * w] = imgs[k][..., 2::-1].reshape(h, -1)
+        f = O.frame(ref.reshape(-1), w, h, ws, True)
+        want = O.raster(f.pos, f.col, w, h, scale)
+        assert np.array_equal(out[oo[k]:oo[k] + want.size].reshape(want.shape), want), (w, h)
