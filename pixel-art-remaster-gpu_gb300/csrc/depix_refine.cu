@@ -19,8 +19,8 @@
 //     3e+1), the piece from a pinned end to the first cut point (3e, 3e+2)
 //     and the cut corner of each free node (3E + node);
 //   * every output sample within 1.5 output pixels of a segment is assigned
-//     to the nearest one (exact integer distances, one rounded division;
-//     ties to the lower slot).
+//     to the nearest one (distances in whole numbers; ties to the lower
+//     slot).
 // Energy (every term a mean): w_curv * 1/F sum_free |a - 2p + b|^2 / 8
 //   + w_dev * 1/F sum_free |p - p0|^2
 //   + w_cov * 1/(3 Ws Hs) sum_samples sum_rgb ((r - t)/255)^2,
@@ -59,8 +59,102 @@ static_assert(seg_wb(1, 1) == 3 && seg_wb(2, 0) == 3 && seg_wb(2, 1) == 1 && seg
 // vertex grid word: bit 0 a hull vertex, bit 1 on an edge without a twin,
 // bits 8.. the number of curve edges
 constexpr uint32_t kVUsed = 1, kVFrame = 2;
-constexpr int kNoSeg = 0x7F7F7F7F; // a byte fill of 0x7F: no segment
 constexpr int kDegShift = 8;
+
+// ---------------------------------------------------------------- scans
+
+constexpr int kScanBlock = 1024, kScanItems = 4, kScanTile = kScanBlock * kScanItems;
+
+template <typename T>
+__device__ __forceinline__ T block_exclusive_scan(T v, T* warp_sums)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) warp_sums[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+        T s = lane < (int)(blockDim.x >> 5) ? warp_sums[lane] : T(0);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const T y = __shfl_up_sync(0xFFFFFFFFu, s, o);
+            if (lane >= o) s += y;
+        }
+        warp_sums[lane] = s; // inclusive
+    }
+    __syncthreads();
+    const T base = warp > 0 ? warp_sums[warp - 1] : T(0);
+    __syncthreads();
+    return base + x - v;
+}
+
+// An exclusive scan left in two parts: out within tiles of kScanTile, and the
+// tiles' own sums before them. Readers add the two (at), which spares a pass
+// over the array.
+template <typename T>
+struct Scan {
+    T* out;
+    T* tiles;
+    T* total;
+    int* ticket; // zero between scans
+    __device__ __forceinline__ T at(int k) const { return out[k] + tiles[k / kScanTile]; }
+};
+
+// Exclusive scan of load(0) .. load(n - 1) in one launch: every block scans its
+// tile, the last one to finish scans the tiles' sums (none waits for another).
+template <typename T, typename Load>
+__global__ void __launch_bounds__(kScanBlock) k_scan(Load load, int n, Scan<T> S)
+{
+    __shared__ T ws[32];
+    __shared__ int last;
+    const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+    T v[kScanItems], s = T(0);
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        v[k] = base + k < n ? load(base + k) : T(0);
+        s += v[k];
+    }
+    T ex = block_exclusive_scan(s, ws);
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        if (base + k < n) S.out[base + k] = ex;
+        ex += v[k];
+    }
+    if (threadIdx.x == blockDim.x - 1) {
+        S.tiles[blockIdx.x] = ex;
+        __threadfence();
+        last = atomicAdd(S.ticket, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    T carry = T(0);
+    for (int b = 0; b < (int)gridDim.x; b += kScanBlock) {
+        const int k = b + threadIdx.x;
+        const T t = k < (int)gridDim.x ? __ldcg(S.tiles + k) : T(0);
+        const T e = block_exclusive_scan(t, ws);
+        if (k < (int)gridDim.x) S.tiles[k] = carry + e;
+        if (threadIdx.x == blockDim.x - 1) ws[0] = e + t;
+        __syncthreads();
+        carry += ws[0];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        *S.total = carry;
+        *S.ticket = 0;
+    }
+}
+
+template <typename T, typename Load>
+cudaError_t exclusive_scan(Load load, int n, const Scan<T>& S, cudaStream_t s)
+{
+    k_scan<T><<<std::max(1, (n + kScanTile - 1) / kScanTile), kScanBlock, 0, s>>>(load, n, S);
+    return cudaGetLastError();
+}
 
 struct Geo {
     const uint8_t* img;
@@ -87,16 +181,26 @@ __device__ __forceinline__ int qvx(uint64_t e, int t, int i) { return 4 * i + (i
 __device__ __forceinline__ int qvy(uint64_t e, int t, int j) { return 4 * j + (int)((e >> (7 + 6 * t)) & 7u) - 1; }
 __device__ __forceinline__ int vindex(const Geo& G, int x, int y) { return (y + 1) * G.gw + (x + 1); }
 
-__device__ __forceinline__ int igcd(int a, int b)
+// the unit step of a hull edge on the quarter grid and how many it takes
+__device__ __forceinline__ int edge_steps(int dx, int dy, int& sx, int& sy)
 {
-    a = abs(a);
-    b = abs(b);
-    while (b) {
-        int t = a % b;
-        a = b;
-        b = t;
+    const int ax = abs(dx), ay = abs(dy);
+    int g = max(ax, ay);
+    if (ax && ay && ax != ay) { // neither along an axis nor a diagonal
+        int u = ax, v = ay;
+        while (v) {
+            const int t = u % v;
+            u = v;
+            v = t;
+        }
+        g = u;
+        sx = dx / g;
+        sy = dy / g;
+        return g;
     }
-    return a;
+    sx = (dx > 0) - (dx < 0);
+    sy = (dy > 0) - (dy < 0);
+    return g;
 }
 
 // v -> u lies on p -> q in the same direction
@@ -115,66 +219,52 @@ __device__ __forceinline__ uint32_t cell_word(const Geo& G, int i, int j)
     return word_of_bgr(load_bgr(G.img, G.ws, G.layout, i, j), G.thr);
 }
 
-// Walks the split edges of cell idx; for each, the twin's owner: the first
-// 8-neighbour (in bit order) with a hull edge that holds the reversed split
-// edge. A neighbour is only searched when its hull's bounding box (the
-// per-pattern box table) holds the split edge. fn(ux, uy, vx, vy, owner, B).
+// Walks the split edges of hull edge t of cell idx; for each, the twin's owner:
+// the first 8-neighbour (in bit order) with a hull edge that holds the reversed
+// split edge. A neighbour is only searched when its hull's bounding box (the
+// per-pattern box table) holds the split edge. npat, nbox: the neighbours'
+// patterns (-1 outside the frame) and boxes, in shared memory (in registers,
+// with the loop over them unrolled, they left room for 16 warps an SM).
+// fn(ux, uy, vx, vy, owner, B).
 template <typename Fn>
-__device__ void walk_split_edges(const Geo& G, const uint32_t* vgrid, int idx, Fn fn)
+__device__ __forceinline__ void walk_split_edges(const Geo& G, const uint32_t* vgrid, int i, int j, uint64_t e, int t,
+                                                 const int* npat, const uint32_t* nbox, Fn fn)
 {
-    const int i = idx % G.w, j = idx / G.w;
-    const uint64_t e = cell_hull(G, idx);
-    const int k = (int)(e & 0xF);
-    int npat[8];
-    uint32_t nbox[8]; // x0, x1, y0, y1 in global quarter units, 8 bits each after a +8 bias
-#pragma unroll
-    for (int d = 0; d < 8; d++) {
-        const int ni = i + dir_di(d), nj = j + dir_dj(d);
-        npat[d] = -1;
-        nbox[d] = 0;
-        if (ni >= 0 && ni < G.w && nj >= 0 && nj < G.h) {
-            const int nidx = nj * G.w + ni;
-            const int n = G.w * G.h;
-            npat[d] = cell_pattern(G.g[nidx], nidx > 0 ? G.g[nidx - 1] : 0u, nidx + 1 < n ? G.g[nidx + 1] : 0u);
-            nbox[d] = __ldg(&G.box[npat[d]]);
-        }
-    }
-    for (int t = 0; t < k; t++) {
-        const int t1 = t + 1 == k ? 0 : t + 1;
-        const int ax = qvx(e, t, i), ay = qvy(e, t, j), bx = qvx(e, t1, i), by = qvy(e, t1, j);
-        const int gcd = igcd(bx - ax, by - ay);
-        const int sx = (bx - ax) / gcd, sy = (by - ay) / gcd;
-        int px = ax, py = ay;
-        for (int st = 1; st <= gcd; st++) {
-            const int cx = ax + st * sx, cy = ay + st * sy;
-            if (st < gcd && !(vgrid[vindex(G, cx, cy)] & kVUsed)) continue;
-            int owner = -1;
-            // the split edge relative to the cell's own quarter origin
-            const int lx0 = min(px, cx) - 4 * i, lx1 = max(px, cx) - 4 * i;
-            const int ly0 = min(py, cy) - 4 * j, ly1 = max(py, cy) - 4 * j;
-            for (int d = 0; d < 8 && owner < 0; d++) {
-                if (npat[d] < 0) continue;
-                const uint32_t bb = nbox[d];
-                const int ox = 4 * dir_di(d), oy = 4 * dir_dj(d);
-                if (lx0 < (int)(bb & 0xFF) - 8 + ox || lx1 > (int)((bb >> 8) & 0xFF) - 8 + ox ||
-                    ly0 < (int)((bb >> 16) & 0xFF) - 8 + oy || ly1 > (int)(bb >> 24) - 8 + oy)
-                    continue;
-                const int ni = i + dir_di(d), nj = j + dir_dj(d);
-                const uint64_t ne = __ldg(&G.lut[npat[d]]);
-                const int nk = (int)(ne & 0xF);
-                for (int s = 0; s < nk; s++) {
-                    const int s1 = s + 1 == nk ? 0 : s + 1;
-                    if (reversed_on(qvx(ne, s, ni), qvy(ne, s, nj), qvx(ne, s1, ni), qvy(ne, s1, nj), px, py, cx, cy)) {
-                        owner = d;
-                        break;
-                    }
+    const int k = (int)(e & 0xF), t1 = t + 1 == k ? 0 : t + 1;
+    const int ax = qvx(e, t, i), ay = qvy(e, t, j), bx = qvx(e, t1, i), by = qvy(e, t1, j);
+    int sx, sy;
+    const int gcd = edge_steps(bx - ax, by - ay, sx, sy);
+    int px = ax, py = ay;
+    for (int st = 1; st <= gcd; st++) {
+        const int cx = ax + st * sx, cy = ay + st * sy;
+        if (st < gcd && !(vgrid[vindex(G, cx, cy)] & kVUsed)) continue;
+        int owner = -1;
+        // the split edge relative to the cell's own quarter origin
+        const int lx0 = min(px, cx) - 4 * i, lx1 = max(px, cx) - 4 * i;
+        const int ly0 = min(py, cy) - 4 * j, ly1 = max(py, cy) - 4 * j;
+#pragma unroll 1
+        for (int d = 0; d < 8 && owner < 0; d++) {
+            if (npat[d] < 0) continue;
+            const uint32_t bb = nbox[d];
+            const int ox = 4 * dir_di(d), oy = 4 * dir_dj(d);
+            if (lx0 < (int)(bb & 0xFF) - 8 + ox || lx1 > (int)((bb >> 8) & 0xFF) - 8 + ox ||
+                ly0 < (int)((bb >> 16) & 0xFF) - 8 + oy || ly1 > (int)(bb >> 24) - 8 + oy)
+                continue;
+            const int ni = i + dir_di(d), nj = j + dir_dj(d);
+            const uint64_t ne = __ldg(&G.lut[npat[d]]);
+            const int nk = (int)(ne & 0xF);
+            for (int s = 0; s < nk; s++) {
+                const int s1 = s + 1 == nk ? 0 : s + 1;
+                if (reversed_on(qvx(ne, s, ni), qvy(ne, s, nj), qvx(ne, s1, ni), qvy(ne, s1, nj), px, py, cx, cy)) {
+                    owner = d;
+                    break;
                 }
             }
-            const int B = owner < 0 ? -1 : (j + dir_dj(owner)) * G.w + (i + dir_di(owner));
-            fn(px, py, cx, cy, owner, B);
-            px = cx;
-            py = cy;
         }
+        const int B = owner < 0 ? -1 : (j + dir_dj(owner)) * G.w + (i + dir_di(owner));
+        fn(px, py, cx, cy, owner, B);
+        px = cx;
+        py = cy;
     }
 }
 
@@ -207,38 +297,119 @@ __global__ void k_rf_mark_vertices(Geo G, uint32_t* vgrid)
     for (int t = 0; t < k; t++) atomicOr(&vgrid[vindex(G, qvx(e, t, i), qvy(e, t, j))], kVUsed);
 }
 
-// pass 0: curve edges per cell, and the frame marks
-__global__ void k_rf_count_edges(Geo G, uint32_t* vgrid, int* count)
+// A cell whose node and neighbours all link their four sides and no diagonal
+// (byte 90) is a square among squares: its edges are shared whole with the
+// four cells beside it.
+__device__ __forceinline__ bool square_among_squares(const Geo& G, int i, int j)
 {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= G.w * G.h) return;
-    const int i = idx % G.w, j = idx / G.w;
-    const uint32_t me = cell_word(G, i, j);
-    int c = 0;
-    walk_split_edges(G, vgrid, idx, [&](int ux, int uy, int vx, int vy, int owner, int B) {
-        if (owner < 0) {
-            atomicOr(&vgrid[vindex(G, ux, uy)], kVFrame);
-            atomicOr(&vgrid[vindex(G, vx, vy)], kVFrame);
-        } else if (B > idx && !similar(me, cell_word(G, B % G.w, B / G.w), G.thr)) {
-            c++;
-        }
-    });
-    count[idx] = c;
+    if (i == 0 || j == 0 || i == G.w - 1 || j == G.h - 1) return false;
+    const uint8_t* q = G.g + (size_t)j * G.w + i;
+    bool all = true;
+#pragma unroll
+    for (int dj = -1; dj <= 1; dj++)
+#pragma unroll
+        for (int di = -1; di <= 1; di++) all &= q[dj * G.w + di] == 90;
+    return all;
 }
 
-// pass 1: the curve edges at their offsets; degrees and up to two
-// neighbours (vertex, edge) per vertex
-__global__ void k_rf_emit_edges(Geo G, uint32_t* vgrid, const int* off, int4* edges, int2* nb_v, int2* nb_e)
+// Curve edges per cell, the frame marks, and the edges themselves, 16 bits each
+// at slots + cell * max_split: the ends relative to the cell's corner (quarter
+// units + 1, 3 bits a coordinate: u, v) and the owner's direction (bits 12-14).
+// A block takes kEdgeCells cells; those that are not squares among similar
+// squares go to a list (about four in ten), of which eight lanes take a cell, a
+// hull edge each (a hull has at most eight): one cell's walk is a long chain,
+// and a lane per cell spent 38 us on a 256x224 frame, once to count and once
+// more to emit (57 us with the list and a lane per cell: too few warps). It is
+// 33 us now and the emission, from the slots, 5.
+constexpr int kEdgeCells = 32, kEdgeThreads = 128;
+__global__ void __launch_bounds__(kEdgeThreads) k_rf_count_edges(Geo G, uint32_t* vgrid, int max_split, int* count,
+                                                                 uint16_t* slots)
+{
+    __shared__ int list[kEdgeCells], n;
+    __shared__ int npat[kEdgeThreads];
+    __shared__ uint32_t nbox[kEdgeThreads];
+    if (threadIdx.x == 0) n = 0;
+    __syncthreads();
+    if (threadIdx.x < kEdgeCells) {
+        const int idx = blockIdx.x * kEdgeCells + threadIdx.x;
+        if (idx < G.w * G.h) {
+            const int i = idx % G.w, j = idx / G.w;
+            bool flat = square_among_squares(G, i, j);
+            if (flat) {
+                // the later of its neighbours are to the right and above
+                const uint32_t me = cell_word(G, i, j);
+                flat = similar(me, cell_word(G, i + 1, j), G.thr) && similar(me, cell_word(G, i, j + 1), G.thr);
+            }
+            if (flat) count[idx] = 0;
+            else list[atomicAdd(&n, 1)] = idx;
+        }
+    }
+    __syncthreads();
+    const int t = threadIdx.x & 7;
+    for (int k0 = 0; k0 < n; k0 += kEdgeThreads / 8) {
+        const int k = k0 + (threadIdx.x >> 3);
+        if (k0 + ((int)threadIdx.x & ~31) / 8 >= n) break; // whole warps
+        const bool have = k < n;
+        const int idx = list[have ? k : n - 1], i = idx % G.w, j = idx / G.w;
+        // a neighbour's pattern and box a lane
+        {
+            const int ni = i + dir_di(t), nj = j + dir_dj(t);
+            int mine = -1;
+            if (ni >= 0 && ni < G.w && nj >= 0 && nj < G.h) {
+                const int nidx = nj * G.w + ni, last = G.w * G.h;
+                mine = cell_pattern(G.g[nidx], nidx > 0 ? G.g[nidx - 1] : 0u, nidx + 1 < last ? G.g[nidx + 1] : 0u);
+                nbox[threadIdx.x] = __ldg(&G.box[mine]);
+            }
+            npat[threadIdx.x] = mine;
+        }
+        __syncwarp();
+        const uint64_t e = cell_hull(G, idx);
+        const uint32_t me = cell_word(G, i, j);
+        uint64_t found = 0; // up to four split edges of a hull edge, 16 bits each
+        int c = 0;
+        if (have && t < (int)(e & 0xF))
+            walk_split_edges(G, vgrid, i, j, e, t, npat + (threadIdx.x & ~7), nbox + (threadIdx.x & ~7), [&](int ux, int uy, int vx, int vy, int owner, int B) {
+                if (owner < 0) {
+                    atomicOr(&vgrid[vindex(G, ux, uy)], kVFrame);
+                    atomicOr(&vgrid[vindex(G, vx, vy)], kVFrame);
+                } else if (B > idx && !similar(me, cell_word(G, i + dir_di(owner), j + dir_dj(owner)), G.thr)) {
+                    found |= (uint64_t)((ux - 4 * i + 1) | (uy - 4 * j + 1) << 3 | (vx - 4 * i + 1) << 6 |
+                                        (vy - 4 * j + 1) << 9 | owner << 12)
+                             << (16 * c++);
+                }
+            });
+        int upto = c;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const int y = __shfl_up_sync(0xFFFFFFFFu, upto, o, 8);
+            if (t >= o) upto += y;
+        }
+        if (have) {
+            uint16_t* slot = slots + (size_t)idx * max_split + (upto - c);
+            for (int q = 0; q < c; q++) slot[q] = (uint16_t)(found >> (16 * q));
+            if (t == 7) count[idx] = upto;
+        }
+        __syncwarp();
+    }
+}
+
+// the curve edges at their offsets; degrees and up to two neighbours (vertex,
+// edge) per vertex
+__global__ void k_rf_emit_edges(Geo G, uint32_t* vgrid, int max_split, const int* count, Scan<int> off,
+                                const uint16_t* slots, int4* edges, int2* nb_v, int2* nb_e)
 {
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= G.w * G.h) return;
-    const int i = idx % G.w, j = idx / G.w;
-    const uint32_t me = cell_word(G, i, j);
-    int o = off[idx];
-    walk_split_edges(G, vgrid, idx, [&](int ux, int uy, int vx, int vy, int owner, int B) {
-        if (owner < 0 || B <= idx || similar(me, cell_word(G, B % G.w, B / G.w), G.thr)) return;
-        const int u = vindex(G, ux, uy), v = vindex(G, vx, vy);
-        edges[o] = make_int4(u, v, idx, B);
+    const int c = count[idx];
+    if (!c) return;
+    const int i = idx % G.w, j = idx / G.w, o0 = off.at(idx);
+    const uint16_t* slot = slots + (size_t)idx * max_split;
+    for (int k = 0; k < c; k++) {
+        const unsigned e = slot[k];
+        const int u = vindex(G, 4 * i + (int)(e & 7u) - 1, 4 * j + (int)(e >> 3 & 7u) - 1);
+        const int v = vindex(G, 4 * i + (int)(e >> 6 & 7u) - 1, 4 * j + (int)(e >> 9 & 7u) - 1);
+        const int d = (int)(e >> 12), o = o0 + k;
+        edges[o] = make_int4(u, v, idx, (j + dir_dj(d)) * G.w + i + dir_di(d));
         const uint32_t su = atomicAdd(&vgrid[u], 1u << kDegShift) >> kDegShift;
         const uint32_t sv = atomicAdd(&vgrid[v], 1u << kDegShift) >> kDegShift;
         if (su < 2) {
@@ -249,15 +420,31 @@ __global__ void k_rf_emit_edges(Geo G, uint32_t* vgrid, const int* off, int4* ed
             (&nb_v[v].x)[sv] = u;
             (&nb_e[v].x)[sv] = o;
         }
-        o++;
-    });
+    }
 }
 
-__global__ void k_rf_node_flags(const uint32_t* vgrid, int nv, int* is_node)
-{
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < nv) is_node[v] = (vgrid[v] >> kDegShift) > 0;
-}
+// scan inputs: vertices with curve edges, free nodes
+struct NodeFlag {
+    const uint32_t* vgrid;
+    __device__ __forceinline__ int operator()(int v) const { return (vgrid[v] >> kDegShift) > 0; }
+};
+struct FreeFlag {
+    const int* flags;
+    __device__ __forceinline__ int operator()(int k) const { return !(flags[k] & 1); }
+};
+struct CellCount {
+    const int* count;
+    __device__ __forceinline__ int operator()(int k) const { return count[k]; }
+};
+// samples of a slot (low word) and whether it has any (high word)
+struct SampleCount {
+    const int* count;
+    __device__ __forceinline__ unsigned long long operator()(int k) const
+    {
+        const unsigned c = (unsigned)count[k];
+        return c | (unsigned long long)(c > 0) << 32;
+    }
+};
 
 struct NodeOut {
     int2* q;        // quarter coordinates
@@ -265,22 +452,23 @@ struct NodeOut {
     int2* nbr;      // neighbours of degree-2 nodes (ascending), else -1
     int2* nbr_edge; // the edges to them
     float2* pos0;
+    float2* gcov;   // zeroed
 };
 
-__global__ void k_rf_nodes(Geo G, const uint32_t* vgrid, const int* nid, const int2* nb_v, const int2* nb_e, NodeOut N)
+__global__ void k_rf_make_nodes(Geo G, const uint32_t* vgrid, Scan<int> nid, const int2* nb_v, const int2* nb_e, NodeOut N)
 {
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= G.gw * G.gh) return;
     const uint32_t word = vgrid[v];
     const int deg = (int)(word >> kDegShift);
     if (deg == 0) return;
-    const int k = nid[v];
+    const int k = nid.at(v);
     const int x = v % G.gw - 1, y = v / G.gw - 1;
     int f = min(deg, 15) << 4;
     if (word & kVFrame) f |= 2;
     int2 nb = make_int2(-1, -1), ne = make_int2(-1, -1);
     if (deg == 2) {
-        int a = nid[nb_v[v].x], b = nid[nb_v[v].y];
+        int a = nid.at(nb_v[v].x), b = nid.at(nb_v[v].y);
         int ea = nb_e[v].x, eb = nb_e[v].y;
         const int va = nb_v[v].x, vb = nb_v[v].y;
         int vax = va % G.gw - 1, vay = va / G.gw - 1, vbx = vb % G.gw - 1, vby = vb / G.gw - 1;
@@ -300,6 +488,7 @@ __global__ void k_rf_nodes(Geo G, const uint32_t* vgrid, const int* nid, const i
     N.nbr[k] = nb;
     N.nbr_edge[k] = ne;
     N.pos0[k] = make_float2(0.25f * x, 0.25f * y);
+    N.gcov[k] = make_float2(0.f, 0.f);
 }
 
 struct SegOut {
@@ -307,21 +496,22 @@ struct SegOut {
     uint2* col;   // left, right RGB (0xBBGGRR)
 };
 
-__device__ __forceinline__ uint32_t cell_rgb(const Geo& G, int idx)
+__device__ __forceinline__ uint32_t pixel_rgb(const Geo& G, int i, int j)
 {
-    const uint32_t c = load_bgr(G.img, G.ws, G.layout, idx % G.w, idx / G.w); // b0 | b1 << 8 | b2 << 16
+    const uint32_t c = load_bgr(G.img, G.ws, G.layout, i, j); // b0 | b1 << 8 | b2 << 16
     // reference bytes (b0, b1, b2) = (B, G, R) -> R | G << 8 | B << 16
     return ((c >> 16) & 0xFFu) | (c & 0xFF00u) | ((c & 0xFFu) << 16);
 }
+__device__ __forceinline__ uint32_t cell_rgb(const Geo& G, int idx) { return pixel_rgb(G, idx % G.w, idx / G.w); }
 
 // segment slots: 3 per edge, then one per node
-__global__ void k_rf_segments(Geo G, const int* nid, int4* edges, int E, int Nn, const int* flags, const int2* nbr,
+__global__ void k_rf_segments(Geo G, Scan<int> nid, int4* edges, int E, int Nn, const int* flags, const int2* nbr,
                               const int2* nbr_edge, SegOut S)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < E) {
         int4 ed = edges[t];
-        const int u = nid[ed.x], v = nid[ed.y];
+        const int u = nid.at(ed.x), v = nid.at(ed.y);
         const uint2 col = make_uint2(cell_rgb(G, ed.z), cell_rgb(G, ed.w));
         const bool pu = flags[u] & 1, pv = flags[v] & 1;
         S.seg[3 * t] = pu ? make_int4(u, v, -1, SEG_PIN_U) : make_int4(-1, -1, -1, SEG_NONE);
@@ -340,7 +530,7 @@ __global__ void k_rf_segments(Geo G, const int* nid, int4* edges, int E, int Nn,
         const int e = nbr_edge[p].x; // the edge between a and p
         const int4 ed = edges[e];
         const uint32_t l = cell_rgb(G, ed.z), r = cell_rgb(G, ed.w);
-        const bool flip = nid[ed.x] != a; // stored as p -> a
+        const bool flip = nid.at(ed.x) != a; // stored as p -> a
         S.seg[s] = make_int4(a, p, b, SEG_CORNER);
         S.col[s] = flip ? make_uint2(r, l) : make_uint2(l, r);
     }
@@ -368,167 +558,232 @@ __device__ __forceinline__ void seg_ends(const int4 sg, const int2* q, int scale
     by *= m;
 }
 
-// squared distance, or -1 beyond the band (decided in integers first, so the
-// rounded division only runs for samples inside it)
-__device__ __forceinline__ double seg_dist2(long long ax, long long ay, long long bx, long long by, long long X,
-                                            long long Y)
-{
-    const long long band2 = (long long)kBand * kBand;
-    const long long ex = bx - ax, ey = by - ay, wx = X - ax, wy = Y - ay;
-    const long long L = ex * ex + ey * ey, dot = ex * wx + ey * wy;
-    if (dot <= 0) {
-        const long long d = wx * wx + wy * wy;
-        return d <= band2 ? (double)d : -1.0;
-    }
-    if (dot >= L) {
-        const long long d = (X - bx) * (X - bx) + (Y - by) * (Y - by);
-        return d <= band2 ? (double)d : -1.0;
-    }
-    const long long cr = ex * wy - ey * wx;
-    if (cr * cr > band2 * L) return -1.0;
-    return __ddiv_rn((double)(cr * cr), (double)L);
-}
+// A segment and the output samples of its box (with the band), numbered row by
+// row: sample Xo sits at 16 (2 Xo + 1). Coordinates relative to the first end
+// fit 32 bits (a segment spans a few source pixels of 32 s units).
+struct SegBox {
+    int x0, y0, nx, ny; // first sample, samples
+    int ex, ey, wx, wy; // second end, and the first sample's position, from the first end
+    __device__ __forceinline__ int count() const { return nx > 0 && ny > 0 ? nx * ny : 0; }
+};
 
 __device__ __forceinline__ long long floor_div_ll(long long a, long long b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 
-// samples of a segment's box (+ band): fn(sample index, d2)
-template <typename Fn>
-__device__ void seg_samples(const int4 sg, const int2* q, int scale, int ow, int oh, Fn fn)
+__device__ __forceinline__ SegBox seg_box(const int4 sg, const int2* q, int scale, int ow, int oh)
 {
     long long ax, ay, bx, by;
     seg_ends(sg, q, scale, ax, ay, bx, by);
-    // sample Xo sits at 16 (2 Xo + 1)
     const long long x0 = max(0LL, -floor_div_ll(-(min(ax, bx) - kBand - 16), 32));
     const long long x1 = min((long long)ow - 1, floor_div_ll(max(ax, bx) + kBand - 16, 32));
     const long long y0 = max(0LL, -floor_div_ll(-(min(ay, by) - kBand - 16), 32));
     const long long y1 = min((long long)oh - 1, floor_div_ll(max(ay, by) + kBand - 16, 32));
-    for (long long yo = y0; yo <= y1; yo++)
-        for (long long xo = x0; xo <= x1; xo++) {
-            const double d2 = seg_dist2(ax, ay, bx, by, 16 * (2 * xo + 1), 16 * (2 * yo + 1));
-            if (d2 >= 0.0) fn((int)(yo * ow + xo), d2);
-        }
+    return SegBox{(int)x0, (int)y0, (int)(x1 - x0 + 1), (int)(y1 - y0 + 1), (int)(bx - ax), (int)(by - ay),
+                  (int)(16 * (2 * x0 + 1) - ax), (int)(16 * (2 * y0 + 1) - ay)};
 }
 
-__global__ void k_rf_assign_dist(const int4* seg, int S, const int2* q, int scale, int ow, int oh,
-                                 unsigned long long* best)
+// Order of the squared distances of the box's samples (i, j), without their
+// rounded quotients: in the middle of a segment the squared distance is
+// cr^2 / L in whole numbers, L the segment's squared length, at most 512 s^2
+// (half a hull edge, or a quarter of two, of 4 sqrt 2 quarter pixels at most).
+// Two different ones lie 1 / (512 s^2)^2 apart or more, so that their floors to
+// frac_bits = 2 log2(512 s^2) binary digits keep their order and tell them
+// apart (as their quotients rounded to double do). At most band^2 < 2^12.
+// kFar beyond the band. The digits come 15 at a time from a float quotient,
+// which is off by at most one, corrected in whole numbers. (64-bit float
+// quotients, on a unit of two lanes a cycle, were most of the two passes' 34 us
+// each over a 256x224 frame at x4.)
+constexpr unsigned long long kFar = ~0ull;
+__host__ __device__ __forceinline__ int frac_bits(int scale)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    const int4 sg = seg[s];
-    if (sg.w == SEG_NONE) return;
-    seg_samples(sg, q, scale, ow, oh, [&](int x, double d2) {
-        atomicMin(&best[x], (unsigned long long)__double_as_longlong(d2));
-    });
+    int b = 0;
+    while ((1 << b) < 512 * scale * scale) b++;
+    return 2 * b;
 }
-
-__global__ void k_rf_assign_seg(const int4* seg, int S, const int2* q, int scale, int ow, int oh,
-                                const unsigned long long* best, int* bseg)
+__device__ __forceinline__ uint32_t divide(uint32_t a, uint32_t L, float inv, uint32_t& rem)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    const int4 sg = seg[s];
-    if (sg.w == SEG_NONE) return;
-    seg_samples(sg, q, scale, ow, oh, [&](int x, double d2) {
-        if ((unsigned long long)__double_as_longlong(d2) == best[x]) atomicMin(&bseg[x], s);
-    });
-}
-
-__global__ void k_rf_count_samples(const int* bseg, int n, int* seg_count)
-{
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x < n && bseg[x] != kNoSeg) atomicAdd(&seg_count[bseg[x]], 1);
-}
-
-__global__ void k_rf_scatter_samples(const int* bseg, int n, const int* seg_off, int* cursor, int* samp)
-{
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= n || bseg[x] == kNoSeg) return;
-    const int s = bseg[x];
-    samp[seg_off[s] + atomicAdd(&cursor[s], 1)] = x;
-}
-
-// each segment's samples in ascending order (summation order fixed)
-__global__ void k_rf_sort_samples(const int* seg_off, int S, int* samp)
-{
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    const int a = seg_off[s], b = seg_off[s + 1];
-    for (int i = a + 1; i < b; i++) {
-        const int v = samp[i];
-        int j = i - 1;
-        while (j >= a && samp[j] > v) {
-            samp[j + 1] = samp[j];
-            j--;
-        }
-        samp[j + 1] = v;
+    uint32_t q = (uint32_t)__float2uint_rz((float)a * inv);
+    int r = (int)(a - q * L);
+    if (r < 0) {
+        q--;
+        r += (int)L;
+    } else if (r >= (int)L) {
+        q++;
+        r -= (int)L;
     }
+    rem = (uint32_t)r;
+    return q;
+}
+__device__ __forceinline__ unsigned long long seg_key(const SegBox& B, int i, int j, float inv, int bits)
+{
+    constexpr int band2 = kBand * kBand;
+    const int wx = B.wx + 32 * i, wy = B.wy + 32 * j;
+    const int L = B.ex * B.ex + B.ey * B.ey, dot = B.ex * wx + B.ey * wy;
+    if (dot <= 0 || dot >= L) {
+        const int ux = dot <= 0 ? wx : wx - B.ex, uy = dot <= 0 ? wy : wy - B.ey;
+        const int d = ux * ux + uy * uy;
+        return d <= band2 ? (unsigned long long)d << bits : kFar;
+    }
+    const long long cr = (long long)B.ex * wy - (long long)B.ey * wx;
+    if (cr * cr > (long long)band2 * L) return kFar;
+    uint32_t r;
+    unsigned long long key = divide((uint32_t)(cr * cr), (uint32_t)L, inv, r);
+    for (int left = bits; left > 0; left -= 15) {
+        const int n = min(left, 15);
+        key = key << n | divide(r << n, (uint32_t)L, inv, r);
+    }
+    return key;
+}
+
+// The samples of each slot's box, kBoxLanes lanes a slot: fn(slot, box, live,
+// output sample, column, row) for every sample, the lanes of the warp together
+// (live: the lane has one); a box's samples come in ascending order. (One lane a
+// slot, with 64-bit coordinates, spent 39 us on each pass over the boxes of a
+// 256x224 frame at x4; eight lanes take 15 to assign and 12 to fill.)
+constexpr int kBoxLanes = 8;
+template <typename Fn>
+__device__ __forceinline__ void box_samples(const SegBox& B, int ow, Fn fn)
+{
+    const int n = B.count(), gl = threadIdx.x & (kBoxLanes - 1);
+    int most = n;
+#pragma unroll
+    for (int o = kBoxLanes; o < 32; o <<= 1) most = max(most, __shfl_xor_sync(0xFFFFFFFFu, most, o));
+    int i = gl, j = 0; // column and row of the lane's sample
+    for (int k = gl; k - gl < most; k += kBoxLanes, i += kBoxLanes) {
+        const bool live = k < n;
+        if (live)
+            while (i >= B.nx) {
+                i -= B.nx;
+                j++;
+            }
+        fn(live, live ? (B.y0 + j) * ow + B.x0 + i : 0, i, j);
+    }
+}
+
+// the lane's slot and its box (empty for slots without a segment)
+__device__ __forceinline__ SegBox slot_box(const int4* seg, int S, const int2* q, int scale, int ow, int oh, int& slot)
+{
+    slot = (blockIdx.x * blockDim.x + threadIdx.x) / kBoxLanes;
+    const int4 sg = slot < S ? seg[slot] : make_int4(-1, -1, -1, SEG_NONE);
+    if (sg.w == SEG_NONE) return SegBox{0, 0, 0, 0, 0, 0, 0, 0};
+    return seg_box(sg, q, scale, ow, oh);
+}
+
+// The slot nearest to each output sample, ties to the lower one. Where distance
+// and slot fit one 64-bit key (slot_bits > 0, any frame of up to 2^18 slots at
+// any scale), its minimum is all; else the least distance, then the lowest slot
+// that has it.
+struct Owner {
+    unsigned long long* best;
+    int* bseg;     // NULL with keys that hold the slot
+    int slot_bits;
+    __device__ __forceinline__ int operator()(int x) const
+    {
+        return bseg ? bseg[x] : (int)(best[x] & ((1ull << slot_bits) - 1ull)); // none: no slot's number
+    }
+};
+
+template <bool SLOT_PASS>
+__global__ void k_rf_assign(const int4* seg, int S, const int2* q, int scale, int ow, int oh, Owner own)
+{
+    int slot;
+    const SegBox B = slot_box(seg, S, q, scale, ow, oh, slot);
+    const float inv = 1.f / (float)max(B.ex * B.ex + B.ey * B.ey, 1);
+    const int bits = frac_bits(scale);
+    box_samples(B, ow, [&](bool live, int x, int i, int j) {
+        if (!live) return;
+        const unsigned long long key = seg_key(B, i, j, inv, bits);
+        if (key == kFar) return;
+        if constexpr (SLOT_PASS) {
+            if (key == own.best[x]) atomicMin(&own.bseg[x], slot);
+        } else {
+            atomicMin(&own.best[x], own.slot_bits ? key << own.slot_bits | (unsigned)slot : key);
+        }
+    });
+}
+
+// samples assigned to each slot
+__global__ void k_rf_count_samples(const int4* seg, int S, const int2* q, int scale, int ow, int oh, Owner own,
+                                   int* seg_count)
+{
+    int slot, c = 0;
+    const SegBox B = slot_box(seg, S, q, scale, ow, oh, slot);
+    box_samples(B, ow, [&](bool live, int x, int, int) { c += live && own(x) == slot; });
+#pragma unroll
+    for (int o = kBoxLanes / 2; o > 0; o >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
+    if (slot < S && (threadIdx.x & (kBoxLanes - 1)) == 0) seg_count[slot] = c;
 }
 
 // the nearest-neighbour target under the coverage Gaussian, per sample
-// (separable: three column and three row weights)
-__global__ void k_rf_targets(Geo G, int scale, float sig, const int* samp, const int* pM, float4* tgt)
+// (separable: three column and three row weights), and its position
+__global__ void k_rf_targets(Geo G, int scale, float sig, const int* samp, const int* pM, float4* tgt,
+                             float2* sxy)
 {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= *pM) return;
-    const int ow = G.w * scale;
-    const int yo = samp[m] / ow, xo = samp[m] - yo * ow;
-    const float x = ((float)xo + 0.5f) / (float)scale, y = ((float)yo + 0.5f) / (float)scale;
-    const int ix = xo / scale, iy = yo / scale;
-    const float inv = 1.f / sig;
-    float cx[3], cy[3];
+    const int M = *pM, ow = G.w * scale;
+    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
+        const int yo = samp[m] / ow, xo = samp[m] - yo * ow;
+        const float x = ((float)xo + 0.5f) / (float)scale, y = ((float)yo + 0.5f) / (float)scale;
+        const int ix = xo / scale, iy = yo / scale;
+        const float inv = 1.f / sig;
+        float cx[3], cy[3];
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-        const int ii = ix + d - 1, jj = iy + d - 1;
-        cx[d] = (ii >= 0 && ii < G.w) ? normcdff((x - (float)ii) * inv) - normcdff((x - (float)ii - 1.f) * inv) : 0.f;
-        cy[d] = (jj >= 0 && jj < G.h) ? normcdff((y - (float)jj) * inv) - normcdff((y - (float)jj - 1.f) * inv) : 0.f;
-    }
-    float r = 0.f, g = 0.f, b = 0.f;
-#pragma unroll
-    for (int dj = 0; dj < 3; dj++) {
-        const int jj = iy + dj - 1;
-        if (jj < 0 || jj >= G.h) continue;
-#pragma unroll
-        for (int di = 0; di < 3; di++) {
-            const int ii = ix + di - 1;
-            if (ii < 0 || ii >= G.w) continue;
-            const float wgt = cx[di] * cy[dj];
-            const uint32_t c = cell_rgb(G, jj * G.w + ii);
-            r += wgt * (float)(c & 0xFF);
-            g += wgt * (float)((c >> 8) & 0xFF);
-            b += wgt * (float)((c >> 16) & 0xFF);
+        for (int d = 0; d < 3; d++) {
+            const int ii = ix + d - 1, jj = iy + d - 1;
+            cx[d] = (ii >= 0 && ii < G.w) ? normcdff((x - (float)ii) * inv) - normcdff((x - (float)ii - 1.f) * inv) : 0.f;
+            cy[d] = (jj >= 0 && jj < G.h) ? normcdff((y - (float)jj) * inv) - normcdff((y - (float)jj - 1.f) * inv) : 0.f;
         }
+        float r = 0.f, g = 0.f, b = 0.f;
+#pragma unroll
+        for (int dj = 0; dj < 3; dj++) {
+            const int jj = iy + dj - 1;
+            if (jj < 0 || jj >= G.h) continue;
+#pragma unroll
+            for (int di = 0; di < 3; di++) {
+                const int ii = ix + di - 1;
+                if (ii < 0 || ii >= G.w) continue;
+                const float wgt = cx[di] * cy[dj];
+                const uint32_t c = pixel_rgb(G, ii, jj);
+                r += wgt * (float)(c & 0xFF);
+                g += wgt * (float)((c >> 8) & 0xFF);
+                b += wgt * (float)((c >> 16) & 0xFF);
+            }
+        }
+        tgt[m] = make_float4(r, g, b, 0.f);
+        sxy[m] = make_float2(x, y);
     }
-    tgt[m] = make_float4(r, g, b, 0.f);
 }
 
 // ------------------------------------------------------------ warm start
 
 constexpr int kWarmTile = 16; // source pixels per tile side
 
-// Tile signature: FNV-1a (64-bit) over the resolved graph byte and the RGB of
-// every pixel of the tile and its one-pixel ring (row-major, pixels outside
-// the frame skipped): everything the tile's cells, curve edges and targets
-// depend on.
+// Tile signature, a warp per tile: the sum over the pixels of the tile and its
+// one-pixel ring (those inside the frame) of a 64-bit mix of the pixel's place,
+// resolved graph byte and RGB: everything the tile's cells, curve edges and
+// targets depend on. Only compared, frame against frame of one size. (A
+// byte-by-byte FNV-1a, a lane per tile, was one chain of 1296 products: 57 us.)
 __global__ void k_rf_tile_hash(Geo G, int tiles_x, int tiles, uint64_t* hash)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (t >= tiles) return;
     const int x0 = (t % tiles_x) * kWarmTile - 1, y0 = (t / tiles_x) * kWarmTile - 1;
-    uint64_t hsh = 0xcbf29ce484222325ull;
-    auto mix = [&](uint32_t byte) {
-        hsh ^= byte;
-        hsh *= 0x100000001b3ull;
-    };
-    for (int y = max(y0, 0); y < min(y0 + kWarmTile + 2, G.h); y++)
-        for (int x = max(x0, 0); x < min(x0 + kWarmTile + 2, G.w); x++) {
-            const int idx = y * G.w + x;
-            const uint32_t c = cell_rgb(G, idx);
-            mix(G.g[idx]);
-            mix(c & 0xFF);
-            mix((c >> 8) & 0xFF);
-            mix((c >> 16) & 0xFF);
-        }
-    hash[t] = hsh;
+    constexpr int W = kWarmTile + 2;
+    unsigned long long sum = 0;
+    for (int k = lane; k < W * W; k += 32) {
+        const int x = x0 + k % W, y = y0 + k / W;
+        if (x < 0 || y < 0 || x >= G.w || y >= G.h) continue;
+        // the finaliser of MurmurHash3 (Appleby, public domain)
+        unsigned long long z = (unsigned long long)pixel_rgb(G, x, y) | (unsigned long long)G.g[y * G.w + x] << 24 |
+                               (unsigned long long)(k + 1) << 32;
+        z ^= z >> 33;
+        z *= 0xFF51AFD7ED558CCDull;
+        z ^= z >> 33;
+        z *= 0xC4CEB9FE1A85EC53ull;
+        z ^= z >> 33;
+        sum += z;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+    if (lane == 0) hash[t] = sum;
 }
 
 __global__ void k_rf_warm_scatter(const int2* q, const float2* pos, int N, int gw, float2* grid, int* stamp, int epoch)
@@ -559,89 +814,6 @@ __global__ void k_rf_same_tiles(const uint64_t* a, const uint64_t* b, int tiles,
     const bool same = t < tiles && a[t] == b[t];
     const unsigned m = __ballot_sync(0xFFFFFFFFu, same);
     if ((threadIdx.x & 31) == 0 && m) atomicAdd(count, __popc(m));
-}
-
-// ---------------------------------------------------------------- scans
-
-constexpr int kScanBlock = 1024, kScanItems = 4, kScanTile = kScanBlock * kScanItems;
-
-__device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_sums[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        int s = lane < (blockDim.x >> 5) ? warp_sums[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xFFFFFFFFu, s, o);
-            if (lane >= o) s += y;
-        }
-        warp_sums[lane] = s; // inclusive
-    }
-    __syncthreads();
-    const int base = warp > 0 ? warp_sums[warp - 1] : 0;
-    return base + x - v;
-}
-
-__global__ void __launch_bounds__(kScanBlock) k_scan_tiles(const int* in, int* out, int n, int* tile_sums)
-{
-    __shared__ int ws[32];
-    const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    int v[kScanItems], s = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; k++) {
-        v[k] = base + k < n ? in[base + k] : 0;
-        s += v[k];
-    }
-    int ex = block_exclusive_scan(s, ws);
-#pragma unroll
-    for (int k = 0; k < kScanItems; k++) {
-        if (base + k < n) out[base + k] = ex;
-        ex += v[k];
-    }
-    if (threadIdx.x == blockDim.x - 1) tile_sums[blockIdx.x] = ex;
-}
-
-__global__ void __launch_bounds__(kScanBlock) k_scan_sums(int* tile_sums, int tiles, int* total)
-{
-    __shared__ int ws[32];
-    __shared__ int carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int b = 0; b < tiles; b += kScanBlock) {
-        const int k = b + threadIdx.x;
-        const int v = k < tiles ? tile_sums[k] : 0;
-        const int ex = block_exclusive_scan(v, ws);
-        const int c = carry;
-        if (k < tiles) tile_sums[k] = c + ex;
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) carry = c + ex + v;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *total = carry;
-}
-
-__global__ void k_scan_add(int* out, int n, const int* tile_sums)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) out[k] += tile_sums[k / kScanTile];
-}
-
-// exclusive scan of n ints; the sum lands in *total (device)
-cudaError_t exclusive_scan(const int* in, int* out, int n, int* tile_sums, int* total, cudaStream_t s)
-{
-    const int tiles = (n + kScanTile - 1) / kScanTile;
-    if (tiles > 0) k_scan_tiles<<<tiles, kScanBlock, 0, s>>>(in, out, n, tile_sums);
-    k_scan_sums<<<1, kScanBlock, 0, s>>>(tile_sums, tiles, total);
-    if (n > 0) k_scan_add<<<(n + 255) / 256, 256, 0, s>>>(out, n, tile_sums);
-    return cudaGetLastError();
 }
 
 // ------------------------------------------------------- energy and adjoint
@@ -695,12 +867,13 @@ struct StepArgs {
     float sigma;         // output pixels
     float w_curv, w_dev, w_cov;
     float lr, bc1, bc2;  // Adam step and bias corrections 1 - beta^t
-    int update;
 };
 
 constexpr float kBeta1 = 0.9f, kBeta2 = 0.999f, kEps = 1e-8f;
 constexpr float kInvSqrt2Pi = 0.3989422804014327f;
-constexpr int kSegLanes = 4; // lanes per segment in the coverage pass
+// Lanes per segment in the coverage pass: three push a node's gradient each, and
+// 8 lanes took 6.7 us per step of a 256x224 x4 frame where 4 take 5.9.
+constexpr int kSegLanes = 4;
 
 __device__ __forceinline__ float warp_sum(float v)
 {
@@ -716,11 +889,75 @@ __device__ __forceinline__ float group_sum(float v, unsigned mask)
     return v;
 }
 
-// Four lanes per live segment: Chaikin ends recomputed from the nodes, each
-// assigned sample's soft colour, loss and d loss / d ends, reduced in the
-// group and pushed to the segment's free nodes.
+// A live segment's line at positions x, its Chaikin ends recomputed from the
+// nodes, and its colours.
+struct Edge {
+    float2 A, B;
+    float cr[3], dl[3], ex, ey, invL;
+};
+__device__ __forceinline__ Edge live_edge(const LiveSeg& ls, const float2* x)
+{
+    Edge E;
+    const int4 sg = ls.nodes;
+    const int nodes[3] = {sg.x, sg.y, sg.z};
+    E.A = E.B = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        if (nodes[k] < 0) continue;
+        const float2 p = x[nodes[k]];
+        const float wa = 0.25f * seg_wa(sg.w, k), wb = 0.25f * seg_wb(sg.w, k);
+        E.A.x += wa * p.x;
+        E.A.y += wa * p.y;
+        E.B.x += wb * p.x;
+        E.B.y += wb * p.y;
+    }
+    const uint32_t left = (uint32_t)ls.range.z, right = (uint32_t)ls.range.w;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        E.cr[c] = (float)((right >> (8 * c)) & 0xFF);
+        E.dl[c] = (float)(int)((left >> (8 * c)) & 0xFF) - (float)(int)((right >> (8 * c)) & 0xFF);
+    }
+    E.ex = E.B.x - E.A.x;
+    E.ey = E.B.y - E.A.y;
+    E.invL = rsqrtf(E.ex * E.ex + E.ey * E.ey);
+    return E;
+}
+
+// One sample's soft colour against its target: adds d loss / d ends to g (A.x,
+// A.y, B.x, B.y) and returns the squared error.
+__device__ __forceinline__ float sample_loss(const Edge& E, float2 X, float4 t, float inv_sig, float cov_norm, float (&g)[4])
+{
+    const float wx = X.x - E.A.x, wy = X.y - E.A.y;
+    const float d = (E.ex * wy - E.ey * wx) * E.invL;
+    const float z = d * inv_sig;
+    const float Phi = normcdff(z);
+    const float r0 = (E.cr[0] + E.dl[0] * Phi - t.x) * (1.f / 255.f);
+    const float r1 = (E.cr[1] + E.dl[1] * Phi - t.y) * (1.f / 255.f);
+    const float r2 = (E.cr[2] + E.dl[2] * Phi - t.z) * (1.f / 255.f);
+    const float phi = expf(-0.5f * z * z) * kInvSqrt2Pi * inv_sig;
+    const float dEdd = 2.f * cov_norm * (1.f / 255.f) * (r0 * E.dl[0] + r1 * E.dl[1] + r2 * E.dl[2]) * phi;
+    // d d / d e = (wy, -wx) / L - d e / L^2 ; d d / d w = (-ey, ex) / L
+    const float dex = wy * E.invL - d * E.ex * E.invL * E.invL, dey = -wx * E.invL - d * E.ey * E.invL * E.invL;
+    const float dwx = -E.ey * E.invL, dwy = E.ex * E.invL;
+    g[0] += dEdd * (-dex - dwx);
+    g[1] += dEdd * (-dey - dwy);
+    g[2] += dEdd * dex;
+    g[3] += dEdd * dey;
+    return r0 * r0 + r1 * r1 + r2 * r2;
+}
+
+// A launch of the step kernels may start while the one before it still runs;
+// what the steps do not change is loaded before the wait for it (early_start
+// lets the next one start).
+__device__ __forceinline__ void early_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void wait_for_last() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Coverage: kSegLanes lanes per live segment, the samples' gradients reduced in
+// the group and pushed to the segment's free nodes.
+template <bool ENERGY>
 __global__ void __launch_bounds__(256) k_rf_coverage(StepArgs a)
 {
+    early_start();
     const RefineFrame F = *a.fr;
     const float inv_sig = (float)F.scale / a.sigma;
     const float cov_norm = a.w_cov * F.inv_samples3;
@@ -728,107 +965,100 @@ __global__ void __launch_bounds__(256) k_rf_coverage(StepArgs a)
     const unsigned gmask = ((1u << kSegLanes) - 1u) << (lane & ~(kSegLanes - 1));
     const int groups = (gridDim.x * blockDim.x) / kSegLanes;
     float eloss = 0.f;
+    bool waited = false;
     for (int l = (blockIdx.x * blockDim.x + threadIdx.x) / kSegLanes; l < F.L; l += groups) {
         const LiveSeg ls = a.live[l];
+        const int m0 = ls.range.x + gl;
+        const bool have = m0 < ls.range.y;
+        float2 X = make_float2(0.f, 0.f);
+        float4 T = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (have) {
+            X = a.sxy[m0];
+            T = a.tgt[m0];
+        }
         const int4 sg = ls.nodes;
-        const int b0 = ls.range.x, b1 = ls.range.y;
-        const int nodes[3] = {sg.x, sg.y, sg.z};
-        float2 A = make_float2(0.f, 0.f), B = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            if (nodes[k] < 0) continue;
-            const float2 p = a.x[nodes[k]];
-            const float wa = 0.25f * seg_wa(sg.w, k), wb = 0.25f * seg_wb(sg.w, k);
-            A.x += wa * p.x;
-            A.y += wa * p.y;
-            B.x += wb * p.x;
-            B.y += wb * p.y;
-        }
-        const uint32_t cl = (uint32_t)ls.range.z, crr = (uint32_t)ls.range.w;
-        const float dl[3] = {(float)(int)(cl & 0xFF) - (float)(int)(crr & 0xFF),
-                             (float)(int)((cl >> 8) & 0xFF) - (float)(int)((crr >> 8) & 0xFF),
-                             (float)(int)((cl >> 16) & 0xFF) - (float)(int)((crr >> 16) & 0xFF)};
-        const float cr[3] = {(float)(crr & 0xFF), (float)((crr >> 8) & 0xFF), (float)((crr >> 16) & 0xFF)};
-        const float ex = B.x - A.x, ey = B.y - A.y;
-        const float invL = rsqrtf(ex * ex + ey * ey);
-        float gax = 0.f, gay = 0.f, gbx = 0.f, gby = 0.f;
-        for (int m = b0 + gl; m < b1; m += kSegLanes) {
-            const float2 X = a.sxy[m];
-            const float wx = X.x - A.x, wy = X.y - A.y;
-            const float d = (ex * wy - ey * wx) * invL;
-            const float z = d * inv_sig;
-            const float Phi = normcdff(z);
-            const float4 t = a.tgt[m];
-            const float r0 = (cr[0] + dl[0] * Phi - t.x) * (1.f / 255.f);
-            const float r1 = (cr[1] + dl[1] * Phi - t.y) * (1.f / 255.f);
-            const float r2 = (cr[2] + dl[2] * Phi - t.z) * (1.f / 255.f);
-            eloss += r0 * r0 + r1 * r1 + r2 * r2;
-            const float phi = expf(-0.5f * z * z) * kInvSqrt2Pi * inv_sig;
-            const float dEdd = 2.f * cov_norm * (1.f / 255.f) * (r0 * dl[0] + r1 * dl[1] + r2 * dl[2]) * phi;
-            // d d / d e = (wy, -wx) / L - d e / L^2 ; d d / d w = (-ey, ex) / L
-            const float dex = wy * invL - d * ex * invL * invL, dey = -wx * invL - d * ey * invL * invL;
-            const float dwx = -ey * invL, dwy = ex * invL;
-            gbx += dEdd * dex;
-            gby += dEdd * dey;
-            gax += dEdd * (-dex - dwx);
-            gay += dEdd * (-dey - dwy);
-        }
-        gax = group_sum(gax, gmask);
-        gay = group_sum(gay, gmask);
-        gbx = group_sum(gbx, gmask);
-        gby = group_sum(gby, gmask);
         const int my = gl == 0 ? sg.x : (gl == 1 ? sg.y : (gl == 2 ? sg.z : -1));
-        if (my >= 0 && !(a.flags[my] & 1)) {
+        const bool push = my >= 0 && !(a.flags[my] & 1);
+        if (!waited) wait_for_last();
+        waited = true;
+        const Edge E = live_edge(ls, a.x);
+        float g[4] = {0.f, 0.f, 0.f, 0.f};
+        if (have) eloss += sample_loss(E, X, T, inv_sig, cov_norm, g);
+        for (int m = m0 + kSegLanes; m < ls.range.y; m += kSegLanes)
+            eloss += sample_loss(E, a.sxy[m], a.tgt[m], inv_sig, cov_norm, g);
+#pragma unroll
+        for (int k = 0; k < 4; k++) g[k] = group_sum(g[k], gmask);
+        if (push) {
             const float wa = 0.25f * seg_wa(sg.w, gl), wb = 0.25f * seg_wb(sg.w, gl);
-            atomicAdd(&a.gcov[my].x, wa * gax + wb * gbx);
-            atomicAdd(&a.gcov[my].y, wa * gay + wb * gby);
+            atomicAdd(&a.gcov[my].x, wa * g[0] + wb * g[2]);
+            atomicAdd(&a.gcov[my].y, wa * g[1] + wb * g[3]);
         }
     }
-    if (a.energy) {
+    if (!waited) wait_for_last(); // a grid that ended without it could overtake the one before
+    if constexpr (ENERGY) {
         eloss = warp_sum(eloss);
         if (lane == 0 && eloss != 0.f) atomicAdd(&a.energy[2], (double)eloss * (double)cov_norm);
     }
 }
 
-// One thread per node: curvature and deviation gradients (gathered from the
-// node's own and its free neighbours' second differences), the coverage
-// gradient, then an Adam step (or the gradient written out).
-__global__ void __launch_bounds__(256) k_rf_nodes_step(StepArgs a)
+// The curvature stencil of a free node p: its second difference t and the sum g
+// of what its own and its free neighbours' second differences give p. nb, qn:
+// the neighbours' neighbours (-1 where the neighbour is pinned).
+struct Stencil {
+    float2 t, g;
+};
+__device__ __forceinline__ Stencil node_stencil(float2 p, float2 pa, float2 pb, const int (&nb)[4], const float2 (&qn)[4])
 {
+    const float tx = pa.x - 2.f * p.x + pb.x, ty = pa.y - 2.f * p.y + pb.y;
+    float gx = -2.f * tx, gy = -2.f * ty;
+    if (nb[0] >= 0) { // a is free: its second difference reads p
+        gx += qn[0].x - 2.f * pa.x + qn[1].x;
+        gy += qn[0].y - 2.f * pa.y + qn[1].y;
+    }
+    if (nb[2] >= 0) {
+        gx += qn[2].x - 2.f * pb.x + qn[3].x;
+        gy += qn[2].y - 2.f * pb.y + qn[3].y;
+    }
+    return Stencil{make_float2(tx, ty), make_float2(gx, gy)};
+}
+
+// One thread per free node: curvature and deviation gradients, the coverage
+// gradient that k_rf_coverage left (zeroed for the next one), then an Adam step,
+// or the energy and the gradient written out.
+template <bool ENERGY>
+__global__ void __launch_bounds__(64) k_rf_nodes(StepArgs a)
+{
+    early_start();
     const RefineFrame F = *a.fr;
     const float curv_k = a.w_curv / (float)max(F.F, 1), dev_k = a.w_dev / (float)max(F.F, 1);
     float ec = 0.f, ed = 0.f;
+    bool waited = false;
     for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < F.F; f += gridDim.x * blockDim.x) {
         const FreeNode fn = a.fnodes[f];
         const int k = fn.k_a_b_aa.x;
-        const float2 p = a.x[k], pa = a.x[fn.k_a_b_aa.y], pb = a.x[fn.k_a_b_aa.z];
-        const int q_nb[4] = {fn.k_a_b_aa.w, fn.ab_ba_bb.x, fn.ab_ba_bb.y, fn.ab_ba_bb.z};
+        const float2 p0 = a.x0[k];
+        if (!waited) wait_for_last();
+        waited = true;
+        const int nb[4] = {fn.k_a_b_aa.w, fn.ab_ba_bb.x, fn.ab_ba_bb.y, fn.ab_ba_bb.z};
         float2 qn[4];
 #pragma unroll
-        for (int t = 0; t < 4; t++) qn[t] = q_nb[t] >= 0 ? a.x[q_nb[t]] : make_float2(0.f, 0.f);
-        const float tx = pa.x - 2.f * p.x + pb.x, ty = pa.y - 2.f * p.y + pb.y;
-        float gx = -2.f * tx, gy = -2.f * ty;
-        if (q_nb[0] >= 0) { // a is free: its second difference reads p
-            gx += qn[0].x - 2.f * pa.x + qn[1].x;
-            gy += qn[0].y - 2.f * pa.y + qn[1].y;
+        for (int t = 0; t < 4; t++) qn[t] = nb[t] >= 0 ? a.x[nb[t]] : make_float2(0.f, 0.f);
+        const float2 p = a.x[k], pa = a.x[fn.k_a_b_aa.y], pb = a.x[fn.k_a_b_aa.z], gc = a.gcov[k];
+        float2 m = make_float2(0.f, 0.f), v = m;
+        if constexpr (!ENERGY) {
+            m = a.m[f];
+            v = a.v[f];
         }
-        if (q_nb[2] >= 0) {
-            gx += qn[2].x - 2.f * pb.x + qn[3].x;
-            gy += qn[2].y - 2.f * pb.y + qn[3].y;
-        }
-        const float2 p0 = a.x0[k];
+        const Stencil S = node_stencil(p, pa, pb, nb, qn);
         const float dx = p.x - p0.x, dy = p.y - p0.y;
-        const float2 gc = a.gcov[k];
-        gx = 0.25f * curv_k * gx + 2.f * dev_k * dx + gc.x;
-        gy = 0.25f * curv_k * gy + 2.f * dev_k * dy + gc.y;
+        const float gx = 0.25f * curv_k * S.g.x + 2.f * dev_k * dx + gc.x;
+        const float gy = 0.25f * curv_k * S.g.y + 2.f * dev_k * dy + gc.y;
         a.gcov[k] = make_float2(0.f, 0.f);
-        if (a.energy) {
-            ec += 0.125f * (tx * tx + ty * ty);
+        if constexpr (ENERGY) {
+            ec += 0.125f * (S.t.x * S.t.x + S.t.y * S.t.y);
             ed += dx * dx + dy * dy;
-        }
-        if (a.gout) a.gout[k] = make_float2(gx, gy);
-        if (a.update) {
-            float2 m = a.m[f], v = a.v[f];
+            if (a.gout) a.gout[k] = make_float2(gx, gy);
+        } else {
             m.x = kBeta1 * m.x + (1.f - kBeta1) * gx;
             m.y = kBeta1 * m.y + (1.f - kBeta1) * gy;
             v.x = kBeta2 * v.x + (1.f - kBeta2) * gx * gx;
@@ -839,7 +1069,8 @@ __global__ void __launch_bounds__(256) k_rf_nodes_step(StepArgs a)
                                  p.y - a.lr * (m.y / a.bc1) / (sqrtf(v.y / a.bc2) + kEps));
         }
     }
-    if (a.energy) {
+    if (!waited) wait_for_last();
+    if constexpr (ENERGY) {
         ec = warp_sum(ec);
         ed = warp_sum(ed);
         if ((threadIdx.x & 31) == 0) {
@@ -849,27 +1080,33 @@ __global__ void __launch_bounds__(256) k_rf_nodes_step(StepArgs a)
     }
 }
 
-// live segments: a slot with a type and at least one sample
-__global__ void k_rf_live_flags(const int4* seg, const int* seg_off, int S, int* flag)
+// The samples of each slot in ascending order (summation order fixed) at its
+// offset, the live segments (those with samples) packed, and the offsets.
+__global__ void k_rf_fill_samples(const int4* seg, int S, const int2* q, int scale, int ow, int oh, Owner own,
+                                  const int* seg_count, Scan<unsigned long long> off, const uint2* col, int* samp,
+                                  int* seg_off, LiveSeg* live)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < S) flag[s] = seg[s].w != SEG_NONE && seg_off[s + 1] > seg_off[s];
-}
-
-__global__ void k_rf_live_scatter(const int* flag, const int* pos, int S, const int4* seg, const int* seg_off,
-                                  const uint2* col, LiveSeg* live)
-{
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < S && flag[s])
-        live[pos[s]] = LiveSeg{seg[s], make_int4(seg_off[s], seg_off[s + 1], (int)col[s].x, (int)col[s].y)};
-}
-
-__global__ void k_rf_sample_xy(const int* samp, const int* pM, int ow, int scale, float2* sxy)
-{
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= *pM) return;
-    const int yo = samp[m] / ow, xo = samp[m] - yo * ow;
-    sxy[m] = make_float2(((float)xo + 0.5f) / (float)scale, ((float)yo + 0.5f) / (float)scale);
+    int slot;
+    SegBox B = slot_box(seg, S, q, scale, ow, oh, slot);
+    const int gl = threadIdx.x & (kBoxLanes - 1), shift = threadIdx.x & 31 & ~(kBoxLanes - 1);
+    const unsigned long long o = slot < S ? off.at(slot) : 0ull;
+    int at = (int)(unsigned)o;
+    const int c = slot < S ? seg_count[slot] : 0;
+    if (slot < S && gl == 0) {
+        seg_off[slot] = at;
+        if (slot == S - 1) seg_off[S] = at + c;
+        if (c) {
+            const uint2 lr = col[slot];
+            live[o >> 32] = LiveSeg{seg[slot], make_int4(at, at + c, (int)lr.x, (int)lr.y)};
+        }
+    }
+    if (!c) B.nx = 0;
+    box_samples(B, ow, [&](bool have, int x, int, int) {
+        const bool mine = have && own(x) == slot;
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, mine) >> shift & ((1u << kBoxLanes) - 1u);
+        if (mine) samp[at + __popc(m & ((1u << gl) - 1u))] = x;
+        at += __popc(m);
+    });
 }
 
 // start of an Adam run: both position buffers from src, moments zeroed
@@ -884,28 +1121,24 @@ __global__ void k_rf_begin(const float2* src, float2* x, float2* y, float2* m, f
     }
 }
 
-// the step kernels' frame record, from the scan totals on the device (F in
-// slot 3, L in slot 4)
-__global__ void k_rf_frame(const int* totals, int N, int ow, int oh, int scale, float inv_samples3, RefineFrame* fr)
-{
-    *fr = RefineFrame{N, totals[4], ow, oh, scale, totals[3], inv_samples3};
-}
-
-__global__ void k_rf_free_flags(const int* flags, int N, int* is_free)
+// the free nodes packed with their curvature stencils; and the step kernels'
+// frame record (F the free nodes, L the live segments)
+__global__ void k_rf_free_nodes(const int* flags, const int2* nbr, Scan<int> pos, int N, FreeNode* out,
+                                const unsigned long long* samples_live, int* totals, int ow, int oh, int scale,
+                                float inv_samples3, RefineFrame* fr)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < N) is_free[k] = !(flags[k] & 1);
-}
-
-__global__ void k_rf_free_nodes(const int* flags, const int2* nbr, const int* is_free, const int* pos, int N,
-                                FreeNode* out)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= N || !is_free[k]) return;
+    if (k == 0) {
+        const unsigned long long t = *samples_live;
+        totals[2] = (int)(unsigned)t;  // M
+        totals[4] = (int)(t >> 32);    // L
+        *fr = RefineFrame{N, (int)(t >> 32), ow, oh, scale, *pos.total, inv_samples3};
+    }
+    if (k >= N || (flags[k] & 1)) return;
     const int2 nb = nbr[k];
     const int2 na = (flags[nb.x] & 1) ? make_int2(-1, -1) : nbr[nb.x];
     const int2 nbb = (flags[nb.y] & 1) ? make_int2(-1, -1) : nbr[nb.y];
-    out[pos[k]] = FreeNode{make_int4(k, nb.x, nb.y, na.x), make_int4(na.y, nbb.x, nbb.y, 0)};
+    out[pos.at(k)] = FreeNode{make_int4(k, nb.x, nb.y, na.x), make_int4(na.y, nbb.x, nbb.y, 0)};
 }
 
 template <typename T>
@@ -956,7 +1189,10 @@ struct depix_refiner {
     DevBuf<float2> warm_grid;
     DevBuf<int> warm_stamp;
     int tiles_x = 0, tiles = 0, warm_epoch = 0;
-    DevBuf<int> cell_count, cell_off, is_node, nid, tile_sums, scalars;
+    DevBuf<int> cell_count, cell_off, cell_tiles, nid, nid_tiles, free_pos, free_tiles, scalars;
+    DevBuf<uint16_t> edge_slots;
+    DevBuf<unsigned long long> samp_off, samp_tiles, samp_total;
+    DevBuf<int> tickets; // of the four scans
     DevBuf<int2> nb_v, nb_e;
     DevBuf<int4> edges;
     DevBuf<int2> node_q, node_nbr, node_nbr_edge;
@@ -965,16 +1201,16 @@ struct depix_refiner {
     DevBuf<int4> seg;
     DevBuf<uint2> seg_col;
     DevBuf<unsigned long long> best;
-    DevBuf<int> bseg, seg_count, seg_off, cursor, samp;
+    DevBuf<int> bseg, seg_count, seg_off, samp;
     DevBuf<float4> tgt;
     DevBuf<double> energy;
     DevBuf<LiveSeg> live;
-    DevBuf<int> live_flag, live_pos, free_flag, free_pos;
     DevBuf<FreeNode> fnodes;
     DevBuf<float2> sxy;
     DevBuf<RefineFrame> frame;
     int L = 0;
     int* h_scalars = nullptr; // pinned
+    cudaEvent_t counted = nullptr; // E and N are on the host
     double* h_energy = nullptr;
     bool ready = false;
     // the Adam loop as a graph, replayed while its parameters and buffers stay
@@ -1087,20 +1323,24 @@ depix_status check_sigma(const depix_refiner* r, const depix_refine_params* p)
     return DEPIX_OK;
 }
 
-// grids: enough blocks for the frame rounded up to a power of two (the
-// kernels stride over the sizes they read on the device, so a captured loop
-// serves every frame whose rounded grids match), at most 8 blocks per SM
-int pow2_at_least(long long n)
+// grids: enough blocks for the frame, rounded up in eighths of a power of two
+// (the kernels stride over the sizes they read on the device, so a captured
+// loop serves every frame whose rounded grids match), at most 8 blocks of 256
+// threads per SM. The live segments are about the edges' middles and the nodes'
+// corners.
+int grid_for(long long threads, int block, int most)
 {
-    int p = 1;
+    const long long n = std::max<long long>(1, (threads + block - 1) / block);
+    long long p = 1;
     while (p < n) p <<= 1;
-    return p;
+    const long long g = std::max<long long>(1, p / 8);
+    return (int)std::min<long long>(most, (n + g - 1) / g * g);
 }
 int cov_blocks(const depix_refiner* r)
 {
-    return std::min(r->sms * 8, pow2_at_least(((long long)r->S * kSegLanes + 255) / 256)); // L <= S
+    return grid_for(((long long)r->E + r->N) * kSegLanes, 256, r->sms * 8);
 }
-int node_blocks(const depix_refiner* r) { return std::min(r->sms * 8, pow2_at_least(((long long)r->N + 255) / 256)); } // F <= N
+int node_blocks(const depix_refiner* r) { return grid_for(r->N, 64, r->sms * 32); } // F <= N
 
 bool same_loop(const StepArgs& a, const StepArgs& b)
 {
@@ -1110,27 +1350,47 @@ bool same_loop(const StepArgs& a, const StepArgs& b)
            a.w_dev == b.w_dev && a.w_cov == b.w_cov && a.lr == b.lr;
 }
 
+// a kernel that may start while the one before it on the stream ends
+template <typename... P, typename... A>
+cudaError_t launch_early(void (*kernel)(P...), int blocks, int threads, cudaStream_t s, A... args)
+{
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cfg.attrs = &early;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // launches the Adam steps from pos_a (result in pos_a after an even number
-// of steps, pos_b after an odd one)
+// of steps, pos_b after an odd one). A step is two short kernels, bound by the
+// latency of their launches and loads (one of a 256x224 frame touches 4 MB in
+// L2): 7.5 us when each waited for the other before its first load, 5.9 us with
+// early starts. (One kernel that gathers a node's gradient over the five
+// segments that read it, evaluating each 2.7 times: 7.2 us.)
 cudaError_t launch_steps(depix_refiner* r, const StepArgs& base, int steps, cudaStream_t s)
 {
     StepArgs a = base;
-    a.update = 1;
     float2* x = r->pos_a.p;
     float2* y = r->pos_b.p;
     double b1 = 1.0, b2 = 1.0;
-    for (int t = 1; t <= steps; t++) {
+    cudaError_t e = cudaSuccess;
+    for (int t = 1; t <= steps && e == cudaSuccess; t++) {
         b1 *= (double)kBeta1;
         b2 *= (double)kBeta2;
         a.x = x;
         a.y = y;
         a.bc1 = (float)(1.0 - b1);
         a.bc2 = (float)(1.0 - b2);
-        k_rf_coverage<<<cov_blocks(r), 256, 0, s>>>(a);
-        k_rf_nodes_step<<<node_blocks(r), 256, 0, s>>>(a);
+        e = launch_early(k_rf_coverage<false>, cov_blocks(r), 256, s, a);
+        if (e == cudaSuccess) e = launch_early(k_rf_nodes<false>, node_blocks(r), 64, s, a);
         std::swap(x, y);
     }
-    return cudaGetLastError();
+    return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 // energy (and gradient when gout) at positions x, without an update
@@ -1141,12 +1401,10 @@ depix_status eval(depix_refiner* r, const depix_refine_params* p, const float2* 
     a.x = x;
     a.gout = gout;
     a.energy = r->energy.p;
-    a.update = 0;
     RF_CK(cudaMemsetAsync(r->energy.p, 0, 3 * sizeof(double), s));
     if (gout) RF_CK(cudaMemsetAsync(gout, 0, (size_t)r->N * sizeof(float2), s)); // pinned nodes stay zero
-    k_rf_coverage<<<cov_blocks(r), 256, 0, s>>>(a);
-    k_rf_nodes_step<<<node_blocks(r), 256, 0, s>>>(a);
-    RF_CK(cudaGetLastError());
+    RF_CK(launch_early(k_rf_coverage<true>, cov_blocks(r), 256, s, a));
+    RF_CK(launch_early(k_rf_nodes<true>, node_blocks(r), 64, s, a));
     RF_CK(cudaMemcpyAsync(r->h_energy, r->energy.p, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
     RF_CK(cudaStreamSynchronize(s));
     out[0] = r->h_energy[0];
@@ -1210,6 +1468,10 @@ depix_status depix_refiner_create(depix_refiner** out, size_t max_pixels)
         r->max_split = std::max(r->max_split, 1);
     }
     if (e == cudaSuccess) e = r->scalars.reserve(8);
+    if (e == cudaSuccess) e = r->samp_total.reserve(1);
+    if (e == cudaSuccess) e = r->tickets.reserve(4);
+    if (e == cudaSuccess) e = cudaMemset(r->tickets.p, 0, 4 * sizeof(int));
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&r->counted, cudaEventDisableTiming);
     if (e == cudaSuccess) e = r->energy.reserve(3);
     if (e == cudaSuccess) e = cudaHostAlloc(&r->h_scalars, 8 * sizeof(int), cudaHostAllocDefault);
     if (e == cudaSuccess) e = cudaHostAlloc(&r->h_energy, 4 * sizeof(double), cudaHostAllocDefault);
@@ -1232,17 +1494,18 @@ depix_status depix_refiner_destroy(depix_refiner* r)
     r->box.release();
     r->own_graph.release(); r->own_snap.release(); r->tile_hash.release(); r->warm_grid.release();
     r->warm_stamp.release();
-    r->cell_count.release(); r->cell_off.release(); r->is_node.release(); r->nid.release();
-    r->tile_sums.release(); r->scalars.release();
+    r->cell_count.release(); r->cell_off.release(); r->cell_tiles.release(); r->nid.release(); r->nid_tiles.release();
+    r->free_pos.release(); r->free_tiles.release(); r->scalars.release(); r->edge_slots.release();
+    r->samp_off.release(); r->samp_tiles.release(); r->samp_total.release(); r->tickets.release();
     r->nb_v.release(); r->nb_e.release(); r->edges.release();
     r->node_q.release(); r->node_nbr.release(); r->node_nbr_edge.release(); r->node_flags.release();
     r->pos0.release(); r->pos_a.release(); r->pos_b.release(); r->gcov.release();
     r->adam_m.release(); r->adam_v.release();
     r->seg.release(); r->seg_col.release(); r->best.release(); r->bseg.release();
-    r->seg_count.release(); r->seg_off.release(); r->cursor.release(); r->samp.release(); r->tgt.release();
+    r->seg_count.release(); r->seg_off.release(); r->samp.release(); r->tgt.release();
     r->energy.release();
-    r->live.release(); r->live_flag.release(); r->live_pos.release(); r->frame.release();
-    r->free_flag.release(); r->free_pos.release(); r->fnodes.release(); r->sxy.release();
+    r->live.release(); r->frame.release(); r->fnodes.release(); r->sxy.release();
+    if (r->counted) cudaEventDestroy(r->counted);
     if (r->loop) cudaGraphExecDestroy(r->loop);
     if (r->capture_stream) cudaStreamDestroy(r->capture_stream);
     cudaFreeHost(r->h_scalars);
@@ -1290,30 +1553,44 @@ depix_status depix_refine_setup(depix_refiner* r, const uint8_t* d_img, int w, i
     }
     Geo G{d_img, widthstep, (int)layout, d_graph, w, h, gw, gh, r->lut, r->box.p,
           pack_thresholds(p->tr_y, p->tr_u, p->tr_v, p->yuv)};
+    const int ow = w * p->scale, oh = h * p->scale, no_px = ow * oh;
     RF_CK(r->vgrid.reserve(nv));
     RF_CK(r->cell_count.reserve(n));
     RF_CK(r->cell_off.reserve(n));
-    RF_CK(r->is_node.reserve(nv));
+    RF_CK(r->cell_tiles.reserve(n / kScanTile + 1));
+    RF_CK(r->edge_slots.reserve((size_t)n * r->max_split));
     RF_CK(r->nid.reserve(nv));
+    RF_CK(r->nid_tiles.reserve(nv / kScanTile + 1));
     RF_CK(r->nb_v.reserve(nv));
     RF_CK(r->nb_e.reserve(nv));
-    RF_CK(r->tile_sums.reserve((size_t)nv / kScanTile + 2));
+    RF_CK(r->best.reserve(no_px));
+    r->tiles_x = (w + kWarmTile - 1) / kWarmTile;
+    r->tiles = r->tiles_x * ((h + kWarmTile - 1) / kWarmTile);
+    RF_CK(r->tile_hash.reserve(r->tiles));
+    const Scan<int> cells{r->cell_off.p, r->cell_tiles.p, r->scalars.p + 0, r->tickets.p + 0};
+    const Scan<int> nid{r->nid.p, r->nid_tiles.p, r->scalars.p + 1, r->tickets.p + 1};
     RF_CK(cudaMemsetAsync(r->vgrid.p, 0, (size_t)nv * sizeof(uint32_t), s));
     k_rf_mark_vertices<<<blocks_for(n), 256, 0, s>>>(G, r->vgrid.p);
-    k_rf_count_edges<<<blocks_for(n, 128), 128, 0, s>>>(G, r->vgrid.p, r->cell_count.p);
+    k_rf_count_edges<<<blocks_for(n, kEdgeCells), kEdgeThreads, 0, s>>>(G, r->vgrid.p, r->max_split, r->cell_count.p,
+                                                                        r->edge_slots.p);
     RF_CK(cudaGetLastError());
-    RF_CK(exclusive_scan(r->cell_count.p, r->cell_off.p, n, r->tile_sums.p, r->scalars.p + 0, s));
+    RF_CK(exclusive_scan(CellCount{r->cell_count.p}, n, cells, s));
     // edges reserved for the most a frame can have, so that E and N come
     // back together: the one read back of the setup (they size the node and
     // segment arrays; the later counts stay on the device)
     RF_CK(r->edges.reserve((size_t)n * r->max_split));
-    k_rf_emit_edges<<<blocks_for(n, 128), 128, 0, s>>>(G, r->vgrid.p, r->cell_off.p, r->edges.p, r->nb_v.p, r->nb_e.p);
-    k_rf_node_flags<<<blocks_for(nv), 256, 0, s>>>(r->vgrid.p, nv, r->is_node.p);
+    k_rf_emit_edges<<<blocks_for(n, 128), 128, 0, s>>>(G, r->vgrid.p, r->max_split, r->cell_count.p, cells,
+                                                       r->edge_slots.p, r->edges.p, r->nb_v.p, r->nb_e.p);
     RF_CK(cudaGetLastError());
-    RF_CK(exclusive_scan(r->is_node.p, r->nid.p, nv, r->tile_sums.p, r->scalars.p + 1, s));
-    int EN[2];
-    DEPIX_TRY_RF(read_totals(r, 0, 2, EN, s));
-    const int E = EN[0], N = EN[1];
+    RF_CK(exclusive_scan(NodeFlag{r->vgrid.p}, nv, nid, s));
+    RF_CK(cudaMemcpyAsync(r->h_scalars, r->scalars.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+    RF_CK(cudaEventRecord(r->counted, s));
+    // what needs neither runs while the host waits for them
+    RF_CK(cudaMemsetAsync(r->best.p, 0xFF, (size_t)no_px * sizeof(unsigned long long), s));
+    k_rf_tile_hash<<<blocks_for(32LL * r->tiles), 256, 0, s>>>(G, r->tiles_x, r->tiles, r->tile_hash.p);
+    RF_CK(cudaGetLastError());
+    RF_CK(cudaEventSynchronize(r->counted));
+    const int E = r->h_scalars[0], N = r->h_scalars[1];
     RF_CK(r->node_q.reserve(N));
     RF_CK(r->node_flags.reserve(N));
     RF_CK(r->node_nbr.reserve(N));
@@ -1324,54 +1601,58 @@ depix_status depix_refine_setup(depix_refiner* r, const uint8_t* d_img, int w, i
     RF_CK(r->gcov.reserve(N));
     RF_CK(r->adam_m.reserve(N));
     RF_CK(r->adam_v.reserve(N));
-    NodeOut no{r->node_q.p, r->node_flags.p, r->node_nbr.p, r->node_nbr_edge.p, r->pos0.p};
-    k_rf_nodes<<<blocks_for(nv), 256, 0, s>>>(G, r->vgrid.p, r->nid.p, r->nb_v.p, r->nb_e.p, no);
-    RF_CK(cudaGetLastError());
     const int S = 3 * E + N;
     RF_CK(r->seg.reserve(S));
     RF_CK(r->seg_col.reserve(S));
-    k_rf_segments<<<blocks_for((long long)E + N), 256, 0, s>>>(G, r->nid.p, r->edges.p, E, N, r->node_flags.p,
-                                                              r->node_nbr.p, r->node_nbr_edge.p,
-                                                              SegOut{r->seg.p, r->seg_col.p});
-    // sample assignment
-    const int ow = w * p->scale, oh = h * p->scale, no_px = ow * oh;
-    RF_CK(r->best.reserve(no_px));
-    RF_CK(r->bseg.reserve(no_px));
     RF_CK(r->seg_count.reserve((size_t)S + 1));
     RF_CK(r->seg_off.reserve((size_t)S + 1));
-    RF_CK(r->cursor.reserve((size_t)S + 1));
-    RF_CK(r->tile_sums.reserve((size_t)std::max(nv, S + 1) / kScanTile + 2));
-    RF_CK(cudaMemsetAsync(r->best.p, 0xFF, (size_t)no_px * sizeof(unsigned long long), s));
-    RF_CK(cudaMemsetAsync(r->bseg.p, 0x7F, (size_t)no_px * sizeof(int), s)); // kNoSeg
-    k_rf_assign_dist<<<blocks_for(S, 128), 128, 0, s>>>(r->seg.p, S, r->node_q.p, p->scale, ow, oh, r->best.p);
-    k_rf_assign_seg<<<blocks_for(S, 128), 128, 0, s>>>(r->seg.p, S, r->node_q.p, p->scale, ow, oh, r->best.p,
-                                                       r->bseg.p);
-    RF_CK(cudaMemsetAsync(r->seg_count.p, 0, ((size_t)S + 1) * sizeof(int), s));
-    k_rf_count_samples<<<blocks_for(no_px), 256, 0, s>>>(r->bseg.p, no_px, r->seg_count.p);
-    RF_CK(cudaGetLastError());
-    RF_CK(exclusive_scan(r->seg_count.p, r->seg_off.p, S + 1, r->tile_sums.p, r->scalars.p + 2, s));
+    RF_CK(r->samp_off.reserve((size_t)S + 1));
+    RF_CK(r->samp_tiles.reserve((size_t)S / kScanTile + 1));
+    RF_CK(r->free_pos.reserve(N));
+    RF_CK(r->free_tiles.reserve((size_t)N / kScanTile + 1));
+    RF_CK(r->fnodes.reserve(N));
+    RF_CK(r->live.reserve(S));
     // samples (M on the device): at most one per output pixel
     RF_CK(r->samp.reserve(no_px));
     RF_CK(r->tgt.reserve(no_px));
-    RF_CK(cudaMemsetAsync(r->cursor.p, 0, ((size_t)S + 1) * sizeof(int), s));
-    k_rf_scatter_samples<<<blocks_for(no_px), 256, 0, s>>>(r->bseg.p, no_px, r->seg_off.p, r->cursor.p, r->samp.p);
-    k_rf_sort_samples<<<blocks_for(S), 256, 0, s>>>(r->seg_off.p, S, r->samp.p);
-    k_rf_targets<<<blocks_for(no_px), 256, 0, s>>>(G, p->scale, rp->sigma / (float)p->scale, r->samp.p,
-                                                   r->scalars.p + 2, r->tgt.p);
-    RF_CK(cudaGetLastError());
     RF_CK(r->sxy.reserve(no_px));
-    k_rf_sample_xy<<<blocks_for(no_px), 256, 0, s>>>(r->samp.p, r->scalars.p + 2, ow, p->scale, r->sxy.p);
-    // free nodes and their curvature stencils
-    RF_CK(r->free_flag.reserve(N));
-    RF_CK(r->free_pos.reserve(N));
-    RF_CK(r->fnodes.reserve(N));
-    k_rf_free_flags<<<blocks_for(N), 256, 0, s>>>(r->node_flags.p, N, r->free_flag.p);
+    NodeOut no{r->node_q.p, r->node_flags.p, r->node_nbr.p, r->node_nbr_edge.p, r->pos0.p, r->gcov.p};
+    k_rf_make_nodes<<<blocks_for(nv), 256, 0, s>>>(G, r->vgrid.p, nid, r->nb_v.p, r->nb_e.p, no);
+    k_rf_segments<<<blocks_for((long long)E + N), 256, 0, s>>>(G, nid, r->edges.p, E, N, r->node_flags.p, r->node_nbr.p,
+                                                              r->node_nbr_edge.p, SegOut{r->seg.p, r->seg_col.p});
     RF_CK(cudaGetLastError());
-    RF_CK(exclusive_scan(r->free_flag.p, r->free_pos.p, N, r->tile_sums.p, r->scalars.p + 3, s));
-    k_rf_free_nodes<<<blocks_for(N), 256, 0, s>>>(r->node_flags.p, r->node_nbr.p, r->free_flag.p, r->free_pos.p, N,
-                                                  r->fnodes.p);
+    // sample assignment
+    const Scan<unsigned long long> soff{r->samp_off.p, r->samp_tiles.p, r->samp_total.p, r->tickets.p + 2};
+    const int box_blocks = blocks_for((long long)S * kBoxLanes);
+    Owner own{r->best.p, nullptr, 0};
+    int bits = 1;
+    while (((long long)1 << bits) <= S) bits++;
+    if (12 + frac_bits(p->scale) + bits <= 64) {
+        own.slot_bits = bits;
+    } else {
+        RF_CK(r->bseg.reserve(no_px));
+        RF_CK(cudaMemsetAsync(r->bseg.p, 0x7F, (size_t)no_px * sizeof(int), s)); // above every slot
+    }
+    k_rf_assign<false><<<box_blocks, 256, 0, s>>>(r->seg.p, S, r->node_q.p, p->scale, ow, oh, own);
+    if (!own.slot_bits) {
+        own.bseg = r->bseg.p;
+        k_rf_assign<true><<<box_blocks, 256, 0, s>>>(r->seg.p, S, r->node_q.p, p->scale, ow, oh, own);
+    }
+    k_rf_count_samples<<<box_blocks, 256, 0, s>>>(r->seg.p, S, r->node_q.p, p->scale, ow, oh, own,
+                                                  r->seg_count.p);
     RF_CK(cudaGetLastError());
-    RF_CK(cudaMemsetAsync(r->gcov.p, 0, (size_t)std::max(N, 1) * sizeof(float2), s));
+    RF_CK(exclusive_scan(SampleCount{r->seg_count.p}, S, soff, s));
+    k_rf_fill_samples<<<box_blocks, 256, 0, s>>>(r->seg.p, S, r->node_q.p, p->scale, ow, oh, own, r->seg_count.p,
+                                                 soff, r->seg_col.p, r->samp.p, r->seg_off.p, r->live.p);
+    // free nodes and their curvature stencils, and the frame record
+    const Scan<int> free_pos{r->free_pos.p, r->free_tiles.p, r->scalars.p + 3, r->tickets.p + 3};
+    RF_CK(exclusive_scan(FreeFlag{r->node_flags.p}, N, free_pos, s));
+    k_rf_free_nodes<<<blocks_for(N), 256, 0, s>>>(r->node_flags.p, r->node_nbr.p, free_pos, N, r->fnodes.p,
+                                                  r->samp_total.p, r->scalars.p, ow, oh, p->scale,
+                                                  (float)(1.0 / (3.0 * (double)ow * (double)oh)), r->frame.p);
+    k_rf_targets<<<std::min(blocks_for(no_px), r->sms * 8), 256, 0, s>>>(
+        G, p->scale, rp->sigma / (float)p->scale, r->samp.p, r->scalars.p + 2, r->tgt.p, r->sxy.p);
+    RF_CK(cudaGetLastError());
     r->w = w;
     r->h = h;
     r->scale = p->scale;
@@ -1382,24 +1663,6 @@ depix_status depix_refine_setup(depix_refiner* r, const uint8_t* d_img, int w, i
     r->S = S;
     r->F = r->M = r->L = -1; // on the device until fetch_counts
     r->sigma = rp->sigma;
-    // live segments
-    RF_CK(r->live_flag.reserve(S));
-    RF_CK(r->live_pos.reserve(S));
-    RF_CK(r->live.reserve(S));
-    k_rf_live_flags<<<blocks_for(S), 256, 0, s>>>(r->seg.p, r->seg_off.p, S, r->live_flag.p);
-    RF_CK(cudaGetLastError());
-    RF_CK(exclusive_scan(r->live_flag.p, r->live_pos.p, S, r->tile_sums.p, r->scalars.p + 4, s));
-    k_rf_live_scatter<<<blocks_for(S), 256, 0, s>>>(r->live_flag.p, r->live_pos.p, S, r->seg.p, r->seg_off.p,
-                                                    r->seg_col.p, r->live.p);
-    RF_CK(cudaGetLastError());
-    r->tiles_x = (w + kWarmTile - 1) / kWarmTile;
-    r->tiles = r->tiles_x * ((h + kWarmTile - 1) / kWarmTile);
-    RF_CK(r->tile_hash.reserve(r->tiles));
-    k_rf_tile_hash<<<blocks_for(r->tiles, 64), 64, 0, s>>>(G, r->tiles_x, r->tiles, r->tile_hash.p);
-    RF_CK(cudaGetLastError());
-    k_rf_frame<<<1, 1, 0, s>>>(r->scalars.p, N, ow, oh, p->scale, (float)(1.0 / (3.0 * (double)ow * (double)oh)),
-                               r->frame.p);
-    RF_CK(cudaGetLastError());
     r->ready = true; // the rest is ordered on s: later calls on s see the frame, others wait on an event of s
     return DEPIX_OK;
 }
@@ -1431,9 +1694,11 @@ depix_status depix_refine_export(depix_refiner* r, int32_t* node_q, int32_t* nod
     if (edges) {
         // vertex indices -> node ids on the host copy
         std::vector<int4> ev(r->E);
-        std::vector<int> nid((size_t)(4 * r->w + 3) * (4 * r->h + 3));
+        std::vector<int> nid((size_t)(4 * r->w + 3) * (4 * r->h + 3)), tiles(nid.size() / kScanTile + 1);
         RF_CK(cudaMemcpy(ev.data(), r->edges.p, (size_t)r->E * sizeof(int4), cudaMemcpyDeviceToHost));
         RF_CK(cudaMemcpy(nid.data(), r->nid.p, nid.size() * sizeof(int), cudaMemcpyDeviceToHost));
+        RF_CK(cudaMemcpy(tiles.data(), r->nid_tiles.p, tiles.size() * sizeof(int), cudaMemcpyDeviceToHost));
+        for (size_t v = 0; v < nid.size(); v++) nid[v] += tiles[v / kScanTile];
         for (int e = 0; e < r->E; e++) {
             edges[4 * e] = nid[ev[e].x];
             edges[4 * e + 1] = nid[ev[e].y];
