@@ -924,12 +924,10 @@ struct CompatScratch {
     uint8_t* g0 = nullptr;
     uint8_t* g1 = nullptr;
     float* diag = nullptr;
-    float* snap = nullptr;
     int* ec = nullptr;
-    int* ec_snap = nullptr;
     void release()
     {
-        dev_free(img); dev_free(g0); dev_free(g1); dev_free(diag); dev_free(snap); dev_free(ec); dev_free(ec_snap);
+        dev_free(img); dev_free(g0); dev_free(g1); dev_free(diag); dev_free(ec);
         *this = CompatScratch();
     }
     bool reserve(size_t ib, size_t px)
@@ -939,9 +937,7 @@ struct CompatScratch {
         bool ok = dev_alloc(&img, ib) == cudaSuccess && dev_alloc(&g0, px) == cudaSuccess &&
                   dev_alloc(&g1, px) == cudaSuccess &&
                   dev_alloc(&diag, px * kCell * sizeof(float2)) == cudaSuccess &&
-                  dev_alloc(&snap, px * kCell * sizeof(float2)) == cudaSuccess &&
-                  dev_alloc(&ec, px * sizeof(int)) == cudaSuccess &&
-                  dev_alloc(&ec_snap, px * sizeof(int)) == cudaSuccess;
+                  dev_alloc(&ec, px * sizeof(int)) == cudaSuccess;
         if (!ok) {
             cudaGetLastError();
             release();
@@ -978,16 +974,8 @@ depix_status compat_run(void* pos, void* colorPos, char* img_data, int w, int h,
     DEPIX_CK(launch_graph(gb, 1, pack_thresholds(p->tr_y, p->tr_u, p->tr_v, p->yuv), true, s));
     GraphBatch hb{c.g0, c.g1, 0, w, h, p->vote};
     DEPIX_CK(launch_heuristics(hb, 1, nullptr, s));
-    DEPIX_CK(launch_cells(c.g1, w, h, c.diag, c.ec, s));
-    if (subdivide) {
-        DEPIX_CK(cudaMemcpyAsync(c.snap, c.diag, px * kCell * sizeof(float2), cudaMemcpyDeviceToDevice, s));
-        DEPIX_CK(cudaMemcpyAsync(c.ec_snap, c.ec, px * sizeof(int), cudaMemcpyDeviceToDevice, s));
-        DEPIX_CK(launch_subdivide(c.img, w, h, ws, DEPIX_LAYOUT_BGR, c.g1, c.snap, c.ec_snap, c.diag, c.ec, s));
-    }
-    DEPIX_CK(launch_triangulate(c.diag, c.ec, w, h, s));
-    if (pos || colorPos)
-        DEPIX_CK(launch_emit(c.img, w, h, ws, DEPIX_LAYOUT_BGR, c.diag, c.ec, static_cast<float*>(pos),
-                             static_cast<uint8_t*>(colorPos), s));
+    DEPIX_CK(launch_vbo(c.img, w, h, ws, DEPIX_LAYOUT_BGR, c.g1, subdivide != 0, c.diag, c.ec,
+                        static_cast<float*>(pos), static_cast<uint8_t*>(colorPos), s));
     if (edge_count_h) DEPIX_CK(cudaMemcpyAsync(edge_count_h, c.ec, px * sizeof(int), cudaMemcpyDeviceToHost, s));
     if (graph_h) DEPIX_CK(cudaMemcpyAsync(graph_h, c.g1, px, cudaMemcpyDeviceToHost, s));
     depix_point* out = static_cast<depix_point*>(malloc(px * kCell * sizeof(depix_point)));

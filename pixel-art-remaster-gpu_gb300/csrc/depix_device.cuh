@@ -131,13 +131,16 @@ __device__ __forceinline__ int ref_stride(int w, int ws, int layout)
     return layout == DEPIX_LAYOUT_BGR ? ws : ((3 * w + 3) & ~3);
 }
 
-// 3-byte colour equality at two linear offsets (isColorEqual, subdivision_functions.cu:157-167)
-__device__ __forceinline__ bool ref_color_eq(const uint8_t* img, int w, int h, int ws, int layout, long long a,
-                                             long long b)
+// The three bytes at a linear offset (isColorEqual compares them,
+// subdivision_functions.cu:157-167).
+__device__ __forceinline__ uint32_t ref_color(const uint8_t* img, int w, int h, int ws, int layout, long long off)
 {
-    return ref_byte(img, w, h, ws, layout, a) == ref_byte(img, w, h, ws, layout, b) &&
-           ref_byte(img, w, h, ws, layout, a + 1) == ref_byte(img, w, h, ws, layout, b + 1) &&
-           ref_byte(img, w, h, ws, layout, a + 2) == ref_byte(img, w, h, ws, layout, b + 2);
+    if (layout == DEPIX_LAYOUT_BGR && off >= 0 && off + 2 < (long long)h * ws) {
+        const uint8_t* q = img + off;
+        return (uint32_t)__ldg(q) | (uint32_t)__ldg(q + 1) << 8 | (uint32_t)__ldg(q + 2) << 16;
+    }
+    return (uint32_t)ref_byte(img, w, h, ws, layout, off) | (uint32_t)ref_byte(img, w, h, ws, layout, off + 1) << 8 |
+           (uint32_t)ref_byte(img, w, h, ws, layout, off + 2) << 16;
 }
 
 // T-junction test at vertex (cx, cy) of cell (i, j) (checkTJunction,
@@ -150,15 +153,12 @@ static __device__ __noinline__ bool t_junction_global(const uint8_t* img, int w,
     long long st = ref_stride(w, ws, layout);
     long long index = (long long)j * st + (long long)i * 3;
     if ((index - st - 1) < 0 || (index + w + 1) > ((long long)h * st - 1)) return true;
-    long long c0 = index + st - 3, c1 = index + st, c2 = index + st + 3, c3 = index - 3, c4 = index + 3;
-    long long c5 = index - st - 3, c6 = index - st, c7 = index - st + 3;
-#define EQ(a, b) ref_color_eq(img, w, h, ws, layout, a, b)
-    if (cx == 0 && cy == 0 && (!EQ(c3, c5) || !EQ(c5, c6))) return true;
-    if (cx == kUnit && cy == 0 && (!EQ(c4, c7) || !EQ(c7, c6))) return true;
-    if (cx == kUnit && cy == kUnit && (!EQ(c1, c2) || !EQ(c2, c4))) return true;
-    if (cx == 0 && cy == kUnit && (!EQ(c0, c1) || !EQ(c1, c3))) return true;
-#undef EQ
-    return false;
+    if ((cx != 0 && cx != kUnit) || (cy != 0 && cy != kUnit)) return false;
+    // the neighbours beside, across and above or below the corner
+    const long long dx = cx == 0 ? -3 : 3, dy = cy == 0 ? -st : st;
+    const uint32_t across = ref_color(img, w, h, ws, layout, index + dy + dx);
+    const uint32_t beside = ref_color(img, w, h, ws, layout, index + dx);
+    return (beside != across) | (across != ref_color(img, w, h, ws, layout, index + dy));
 }
 
 // ------------------------------------------------------- cell pattern tables

@@ -420,6 +420,224 @@ __global__ void k_emit(const uint8_t* img, int w, int h, int ws, int layout, con
     }
 }
 
+// ------------------------------------------------------ a frame's VBO whole
+//
+// What the stage kernels above do one after the other over a frame (cells,
+// snapshot, subdivision, triangulation, emission), in one pass: a block takes
+// kVboCells cells, keeps their polygons and triangles in shared memory and
+// writes the three buffers a slot per lane, in order. The stages moved the
+// 45-slot buffers seven times, a cell's 360 bytes by one lane, and clipped ears
+// with the polygon in local memory: 15 + 8 (snapshot) + 39 + 44 + 31 us of a
+// 256x224 frame, where this takes 25 (10 without subdivision, about the 52 MB
+// written; the rest is the latency of the longest ear clips).
+//
+// A cell whose edges are all linked (or with no subdivision every cell) keeps
+// its hull, whose triangles are in the table; the others, about one in five, go
+// to a list. Eight lanes cut a cell, a hull vertex each (a hull has at most
+// eight); then a lane clips its ears, the lanes of a warp side by side (28 us
+// with the list dealt out to all warps; 33 us at 32 cells a block, 30 at 128).
+constexpr int kVboCells = 64, kVboThreads = 128;
+
+struct VboShared {
+    char2 xy[kVboCells][kMaxPoly + 2]; // nine words, for lanes that read a cell each
+    uint64_t hull[kVboCells];
+    uint8_t tri[kVboCells][3 * kMaxPoly + 4];
+    int origin[kVboCells][2];
+    uint32_t color[kVboCells];
+    uint8_t node[kVboCells], n[kVboCells], nt[kVboCells], list[kVboCells];
+    int listed;
+};
+
+// hull entry of cell idx, neighbours read linearly; a single point at the
+// origin outside the frame
+__device__ __forceinline__ uint64_t linear_hull(const uint8_t* g, int n, int idx)
+{
+    if (idx < 0 || idx >= n) return 1 | 1 << 4 | 1 << 7;
+    return __ldg(&g_hull_lut[cell_pattern(__ldg(g + idx), linear_at(g, n, idx - 1), linear_at(g, n, idx + 1))]);
+}
+
+// Q (or R) of the linked neighbour's hull nb around vertex (px, py)
+// (get{Q,R}_i_from_linked_cell), in this cell's coordinates
+__device__ __forceinline__ int2 hull_linked_qr(uint64_t nb, int link, int px, int py, bool want_r)
+{
+    const int n = (int)(nb & 15), bx = kUnit * dir_di(link), by = kUnit * dir_dj(link);
+    int at = 0;
+    for (int t = n - 1; t >= 0; t--)
+        if (hx(nb, t) == px - bx && hy(nb, t) == py - by) at = t;
+    int2 o;
+    hull_qr(nb, n, want_r ? at - 1 : at, want_r, o.x, o.y);
+    return make_int2(o.x + bx, o.y + by);
+}
+
+// ear_clip on a polygon in shared memory, without the places it tests in vain:
+// it clips the first ear after the place it stands at, an ear being a convex
+// corner with no other vertex in or on its triangle. Vertices are their places
+// in its list, which runs counter-clockwise; corners that are not convex are
+// kept in a mask, of which a clip changes two. (Eight lanes a cell that test
+// place after place, or that keep the vertices in each corner's triangle, take
+// 37 and 36 us for the whole kernel on a 256x224 frame, where a lane a cell
+// takes 25: they issue several times as many instructions.)
+__device__ __forceinline__ int clip_ears(const char2* xy, int n, uint8_t* tri)
+{
+    if (n < 3) return 0;
+    int area = 0;
+    for (int q = 0; q < n; q++) {
+        const char2 p = xy[q > 0 ? q - 1 : n - 1], r = xy[q];
+        area += p.x * r.y - r.x * p.y;
+    }
+    const bool turned = area <= 0;
+    auto at = [&](int k) { return turned ? n - 1 - k : k; };
+    unsigned alive = (1u << n) - 1u;
+    auto next = [](unsigned set, int k) { // of a set that is not empty: its first place from k on, around
+        const unsigned up = set >> k << k;
+        return __ffs(up != 0 ? up : set) - 1;
+    };
+    auto before = [&](int k) {
+        const unsigned down = alive & ((1u << k) - 1u);
+        return 31 - __clz(down != 0 ? down : alive);
+    };
+    auto convex = [](char2 A, char2 B, char2 C) {
+        return (B.x - A.x) * (C.y - A.y) - (B.y - A.y) * (C.x - A.x) > 0;
+    };
+    unsigned corners = 0; // the convex ones
+    char2 A = xy[at(n - 1)], B = xy[at(0)];
+    for (int q = 0; q < n; q++) {
+        const char2 C = xy[at(q + 1 < n ? q + 1 : 0)];
+        if (convex(A, B, C)) corners |= 1u << q;
+        A = B;
+        B = C;
+    }
+    int nt = 0, from = 0;
+    unsigned left = corners; // not tested since the last clip
+    for (int nv = n; nv > 2 && left != 0;) {
+        const int b = next(left, from), u = before(b), d = next(alive, b + 1);
+        const char2 U = xy[at(u)], V = xy[at(b)], D = xy[at(d)];
+        bool ear = true;
+        for (unsigned o = alive & ~(1u << u | 1u << b | 1u << d); o != 0 && ear; o &= o - 1) {
+            const char2 P = xy[at(__ffs(o) - 1)];
+            ear = !inside_tri(U.x, U.y, V.x, V.y, D.x, D.y, P.x, P.y);
+        }
+        if (!ear) {
+            left &= ~(1u << b);
+            from = b + 1;
+            continue;
+        }
+        tri[3 * nt] = (uint8_t)at(u);
+        tri[3 * nt + 1] = (uint8_t)at(b);
+        tri[3 * nt + 2] = (uint8_t)at(d);
+        nt++;
+        nv--;
+        alive &= ~(1u << b);
+        const int uu = before(u), dd = next(alive, d + 1);
+        corners &= ~(1u << u | 1u << b | 1u << d);
+        if (convex(xy[at(uu)], U, D)) corners |= 1u << u;
+        if (convex(U, D, xy[at(dd)])) corners |= 1u << d;
+        left = corners;
+        from = dd;
+    }
+    return nt;
+}
+
+__global__ void __launch_bounds__(kVboThreads) k_vbo(const uint8_t* img, int w, int h, int ws, int layout,
+                                                     const uint8_t* g, int subdivide, float2* diagram, int* ec,
+                                                     float2* pos, uchar4* col)
+{
+    __shared__ VboShared S;
+    constexpr unsigned kAll = 0xFFFFFFFFu;
+    const int frame = w * h, first = blockIdx.x * kVboCells, cells = min(kVboCells, frame - first);
+    if (threadIdx.x == 0) S.listed = 0;
+    __syncthreads();
+    for (int c = threadIdx.x; c < cells; c += kVboThreads) {
+        const int idx = first + c, j = idx / w, i = idx - j * w;
+        const unsigned node = __ldg(g + idx);
+        const int pat = cell_pattern(node, linear_at(g, frame, idx - 1), linear_at(g, frame, idx + 1));
+        const uint64_t e = __ldg(&g_hull_lut[pat]);
+        const int n = (int)(e & 15);
+        // all edges linked: no vertex between border edges, no linked edge beside one
+        const bool whole = __ldg(&g_cut.verts[pat]) == ~0ull && (__ldg(&g_cut.edges[pat].x) >> 23 & 1) == 0;
+        if (!subdivide || node == 90 || whole) {
+            const uint64_t te = __ldg(&g_tri_lut[pat]);
+            int nt = 0;
+            for (; nt < n - 2 && ((te >> (9 * nt)) & 511u) != 0; nt++)
+#pragma unroll
+                for (int k = 0; k < 3; k++) S.tri[c][3 * nt + k] = (uint8_t)((te >> (9 * nt + 3 * k)) & 7u);
+            for (int v = 0; v < n; v++) S.xy[c][v] = make_char2((signed char)hx(e, v), (signed char)hy(e, v));
+            S.n[c] = (uint8_t)n;
+            S.nt[c] = (uint8_t)nt;
+        } else {
+            S.list[atomicAdd(&S.listed, 1)] = (uint8_t)c;
+            S.hull[c] = e;
+            S.node[c] = (uint8_t)node;
+        }
+        S.origin[c][0] = i;
+        S.origin[c][1] = j;
+        if (col) {
+            const uint32_t p = load_bgr(img, ws, layout, i, j);
+            S.color[c] = (p >> 16 & 0xFFu) | (p & 0xFF00u) | (p & 0xFFu) << 16 | 0xFF000000u;
+        }
+    }
+    __syncthreads();
+
+    const int lane = threadIdx.x & 31, base = lane & 24, v = lane & 7, listed = S.listed;
+    for (int q0 = 4 * (threadIdx.x >> 5); q0 < listed; q0 += kVboThreads / 8) {
+        const bool live = q0 + (base >> 3) < listed;
+        const int c = S.list[live ? q0 + (base >> 3) : q0], idx = first + c;
+        const unsigned node = S.node[c];
+        const uint64_t e = live ? S.hull[c] : 0;
+        const int n = (int)(e & 15);
+        const int link = v < n ? hull_edge_link(e, n, node, v) : -1;
+        const int before = __shfl_sync(kAll, link, base + (v > 0 ? v - 1 : max(n - 1, 0)));
+        // the vertex stays, or a point on each side of it takes its place
+        int x0 = hx(e, v), y0 = hy(e, v), x1 = 0, y1 = 0;
+        bool two = false;
+        if (v < n && (link < 0 || before < 0)) {
+            const int px = x0, py = y0, i = S.origin[c][0], j = S.origin[c][1];
+            if (link >= 0 || before >= 0 || !t_junction_global(img, w, h, ws, layout, i, j, px, py)) {
+                two = true;
+                int2 r, t;
+                hull_qr(e, n, v - 1, true, r.x, r.y);
+                hull_qr(e, n, v, false, t.x, t.y);
+                if (link >= 0 || before >= 0) {
+                    const int l = max(link, before);
+                    const uint64_t nb = linear_hull(g, frame, idx + dir_dj(l) * w + dir_di(l));
+                    const int2 a = hull_linked_qr(nb, l, px, py, before >= 0);
+                    if (before >= 0) r = make_int2((t.x + a.x) / 2, (t.y + a.y) / 2);
+                    else t = make_int2((r.x + a.x) / 2, (r.y + a.y) / 2);
+                }
+                x0 = r.x, y0 = r.y, x1 = t.x, y1 = t.y;
+            }
+        }
+        const unsigned twos = __ballot_sync(kAll, two) >> base & 0xFFu;
+        const int m = n + __popc(twos), at = v + __popc(twos & ((1u << v) - 1u));
+        if (v < n) {
+            S.xy[c][at] = make_char2((signed char)x0, (signed char)y0);
+            if (two) S.xy[c][at + 1] = make_char2((signed char)x1, (signed char)y1);
+        }
+        if (live && v == 0) S.n[c] = (uint8_t)m;
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < listed; q += kVboThreads) {
+        const int c = S.list[q];
+        S.nt[c] = (uint8_t)clip_ears(S.xy[c], S.n[c], S.tri[c]);
+    }
+    __syncthreads();
+
+    for (int c = threadIdx.x; c < cells; c += kVboThreads) ec[first + c] = S.n[c];
+    const size_t base_slot = (size_t)first * kCell;
+    for (int k = threadIdx.x; k < cells * kCell; k += kVboThreads) {
+        const int c = k / kCell, t = k - c * kCell;
+        float2 o = make_float2(-100.f, -100.f);
+        if (t < 3 * S.nt[c]) {
+            const char2 p = S.xy[c][S.tri[c][t]];
+            o = make_float2((float)p.x * (1.0f / kUnit) + (float)S.origin[c][0],
+                            (float)p.y * (1.0f / kUnit) + (float)S.origin[c][1]);
+        }
+        diagram[base_slot + k] = o;
+        if (pos) pos[base_slot + k] = o;
+        if (col) reinterpret_cast<uint32_t*>(col)[base_slot + k] = S.color[c];
+    }
+}
+
 static dim3 grid1(int n, int b) { return dim3((n + b - 1) / b); }
 
 cudaError_t launch_cells(const uint8_t* g, int w, int h, float* diagram, int* ec, cudaStream_t s)
@@ -447,6 +665,16 @@ cudaError_t launch_emit(const uint8_t* img, int w, int h, int ws, int layout, co
 {
     k_emit<<<grid1(w * h, 128), 128, 0, s>>>(img, w, h, ws, layout, reinterpret_cast<const float2*>(diagram), ec,
                                              reinterpret_cast<float2*>(pos), reinterpret_cast<uchar4*>(col));
+    return cudaGetLastError();
+}
+
+cudaError_t launch_vbo(const uint8_t* img, int w, int h, int ws, int layout, const uint8_t* g, bool subdivide,
+                       float* diagram, int* ec, float* pos, uint8_t* col, cudaStream_t s)
+{
+    k_vbo<<<grid1(w * h, kVboCells), kVboThreads, 0, s>>>(img, w, h, ws, layout, g, subdivide ? 1 : 0,
+                                                          reinterpret_cast<float2*>(diagram), ec,
+                                                          reinterpret_cast<float2*>(pos),
+                                                          reinterpret_cast<uchar4*>(col));
     return cudaGetLastError();
 }
 

@@ -205,6 +205,9 @@ cudaError_t launch_subdivide(const uint8_t* img, int w, int h, int ws, int layou
 cudaError_t launch_triangulate(float* diagram, const int* ec, int w, int h, cudaStream_t s);
 cudaError_t launch_emit(const uint8_t* img, int w, int h, int ws, int layout, const float* diagram, const int* ec,
                         float* pos, uint8_t* col, cudaStream_t s);
+// the four stages above in one pass over a resolved graph (pos and col may be null)
+cudaError_t launch_vbo(const uint8_t* img, int w, int h, int ws, int layout, const uint8_t* g, bool subdivide,
+                       float* diagram, int* ec, float* pos, uint8_t* col, cudaStream_t s);
 cudaError_t launch_raster(const RasterBatch& b, int nframes, cudaStream_t s);
 // coverage-mask raster (scale <= kMaxMaskScale) and its per-scale pattern table
 constexpr int kMaxMaskScale = 12;
