@@ -1063,12 +1063,15 @@ __global__ void k_cc_merge(const uint8_t* g, int32_t* L, int w, int h, size_t fr
 // aligned, the finds interleaved, so that their loads are in flight together
 // (one find per pixel is bound by load latency; settling groups of one label
 // by one find measured slower, 217 against 194 us for 1024 frames with the
-// merge: the warp then runs both ways one after the other). Only labels that
-// change are written.
+// merge: the warp then runs both ways one after the other; two or four groups of
+// four a thread 177 and 282 against 176: fewer warps). Groups in which nothing
+// changes are not written, the others by one 16-byte store where aligned (a
+// store per label: 184 us).
 __device__ __forceinline__ void flatten4(int32_t* L, int32_t* q, int n)
 {
     int x[4], p[4], first[4];
-    if (n == 4 && (reinterpret_cast<uintptr_t>(q) & 15) == 0) {
+    const bool whole = n == 4 && (reinterpret_cast<uintptr_t>(q) & 15) == 0;
+    if (whole) {
         const int4 v = *reinterpret_cast<const int4*>(q);
         x[0] = v.x;
         x[1] = v.y;
@@ -1094,9 +1097,14 @@ __device__ __forceinline__ void flatten4(int32_t* L, int32_t* q, int n)
             }
         if (!more) break;
     }
+    if (!((first[0] ^ x[0]) | (first[1] ^ x[1]) | (first[2] ^ x[2]) | (first[3] ^ x[3]))) return;
+    if (whole) {
+        *reinterpret_cast<int4*>(q) = make_int4(x[0], x[1], x[2], x[3]);
+    } else {
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-        if (i < n && first[i] != x[i]) q[i] = x[i];
+        for (int i = 0; i < 4; i++)
+            if (i < n && first[i] != x[i]) q[i] = x[i];
+    }
 }
 
 __global__ void k_cc_flatten(int32_t* L, int n, size_t frame_stride)
