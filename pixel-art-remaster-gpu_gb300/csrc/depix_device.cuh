@@ -94,12 +94,12 @@ __device__ __forceinline__ bool similar(uint32_t a, uint32_t b, uint32_t thr)
 __device__ __forceinline__ uint32_t load_bgr(const uint8_t* img, int ws, int layout, int i, int j)
 {
     if (layout == DEPIX_LAYOUT_RGBA) {
-        uint32_t p = __ldg(reinterpret_cast<const uint32_t*>(img + (size_t)j * ws) + i);
+        uint32_t p = reinterpret_cast<const uint32_t*>(img + (size_t)j * ws)[i];
         // RGBA -> B,G,R
         return ((p >> 16) & 0xFFu) | (p & 0xFF00u) | ((p & 0xFFu) << 16);
     }
     const uint8_t* q = img + (size_t)j * ws + 3 * i;
-    return (uint32_t)__ldg(q) | ((uint32_t)__ldg(q + 1) << 8) | ((uint32_t)__ldg(q + 2) << 16);
+    return (uint32_t)q[0] | ((uint32_t)q[1] << 8) | ((uint32_t)q[2] << 16);
 }
 
 // word of packed bytes c = b0 | b1 << 8 | b2 << 16 under the y arithmetic
@@ -116,14 +116,14 @@ __device__ __forceinline__ int ref_byte(const uint8_t* img, int w, int h, int ws
 {
     if (layout == DEPIX_LAYOUT_BGR) {
         if (off < 0 || off >= (long long)h * ws) return 0;
-        return __ldg(img + off);
+        return img[off];
     }
     int vws = (3 * w + 3) & ~3;
     if (off < 0 || off >= (long long)h * vws) return 0;
     int row = (int)(off / vws), col = (int)(off % vws);
     if (col >= 3 * w) return 0;
     int px = col / 3, ch = col % 3; // ch 0 = B, 1 = G, 2 = R
-    return __ldg(img + (size_t)row * ws + 4 * px + (2 - ch));
+    return img[(size_t)row * ws + 4 * px + (2 - ch)];
 }
 
 __device__ __forceinline__ int ref_stride(int w, int ws, int layout)
@@ -137,7 +137,7 @@ __device__ __forceinline__ uint32_t ref_color(const uint8_t* img, int w, int h, 
 {
     if (layout == DEPIX_LAYOUT_BGR && off >= 0 && off + 2 < (long long)h * ws) {
         const uint8_t* q = img + off;
-        return (uint32_t)__ldg(q) | (uint32_t)__ldg(q + 1) << 8 | (uint32_t)__ldg(q + 2) << 16;
+        return (uint32_t)q[0] | (uint32_t)q[1] << 8 | (uint32_t)q[2] << 16;
     }
     return (uint32_t)ref_byte(img, w, h, ws, layout, off) | (uint32_t)ref_byte(img, w, h, ws, layout, off + 1) << 8 |
            (uint32_t)ref_byte(img, w, h, ws, layout, off + 2) << 16;
@@ -498,6 +498,19 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
 }  // namespace depix
 
 namespace depix {
+
+// A kernel launched by launch_early may start while the one before it on the
+// stream still runs: it waits for its end, with all that it wrote, before its
+// first access to memory (buffers that the one before may have written are then
+// read with plain loads, not through the non-coherent path), and only then lets
+// the next one start, so that no more than two kernels of a stream overlap.
+__device__ __forceinline__ void early_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void wait_for_last() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void follow_last()
+{
+    wait_for_last();
+    early_start();
+}
 
 // Persistent work loop: the block pulls `gran` tile indices at a time from
 // *counter until `total` is reached and runs body(t) on each; a barrier

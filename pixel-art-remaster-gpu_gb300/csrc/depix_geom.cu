@@ -453,7 +453,7 @@ struct VboShared {
 __device__ __forceinline__ uint64_t linear_hull(const uint8_t* g, int n, int idx)
 {
     if (idx < 0 || idx >= n) return 1 | 1 << 4 | 1 << 7;
-    return __ldg(&g_hull_lut[cell_pattern(__ldg(g + idx), linear_at(g, n, idx - 1), linear_at(g, n, idx + 1))]);
+    return __ldg(&g_hull_lut[cell_pattern(g[idx], linear_at(g, n, idx - 1), linear_at(g, n, idx + 1))]);
 }
 
 // Q (or R) of the linked neighbour's hull nb around vertex (px, py)
@@ -542,6 +542,7 @@ __global__ void __launch_bounds__(kVboThreads) k_vbo(const uint8_t* img, int w, 
                                                      const uint8_t* g, int subdivide, float2* diagram, int* ec,
                                                      float2* pos, uchar4* col)
 {
+    follow_last();
     __shared__ VboShared S;
     constexpr unsigned kAll = 0xFFFFFFFFu;
     const int frame = w * h, first = blockIdx.x * kVboCells, cells = min(kVboCells, frame - first);
@@ -549,7 +550,7 @@ __global__ void __launch_bounds__(kVboThreads) k_vbo(const uint8_t* img, int w, 
     __syncthreads();
     for (int c = threadIdx.x; c < cells; c += kVboThreads) {
         const int idx = first + c, j = idx / w, i = idx - j * w;
-        const unsigned node = __ldg(g + idx);
+        const unsigned node = g[idx];
         const int pat = cell_pattern(node, linear_at(g, frame, idx - 1), linear_at(g, frame, idx + 1));
         const uint64_t e = __ldg(&g_hull_lut[pat]);
         const int n = (int)(e & 15);
@@ -671,11 +672,9 @@ cudaError_t launch_emit(const uint8_t* img, int w, int h, int ws, int layout, co
 cudaError_t launch_vbo(const uint8_t* img, int w, int h, int ws, int layout, const uint8_t* g, bool subdivide,
                        float* diagram, int* ec, float* pos, uint8_t* col, cudaStream_t s)
 {
-    k_vbo<<<grid1(w * h, kVboCells), kVboThreads, 0, s>>>(img, w, h, ws, layout, g, subdivide ? 1 : 0,
-                                                          reinterpret_cast<float2*>(diagram), ec,
-                                                          reinterpret_cast<float2*>(pos),
-                                                          reinterpret_cast<uchar4*>(col));
-    return cudaGetLastError();
+    return launch_early(true, k_vbo, grid1(w * h, kVboCells), kVboThreads, 0, s, img, w, h, ws, layout, g, subdivide ? 1 : 0,
+                        reinterpret_cast<float2*>(diagram), ec, reinterpret_cast<float2*>(pos),
+                        reinterpret_cast<uchar4*>(col));
 }
 
 // ------------------------------------------------------------------ raster
@@ -1135,7 +1134,7 @@ struct MaskTile {
 template <int LAYOUT>
 __device__ __forceinline__ uint32_t load_rgba(const uint8_t* img, int ws, int i, int j)
 {
-    if (LAYOUT == DEPIX_LAYOUT_RGBA) return __ldg(reinterpret_cast<const uint32_t*>(img + (size_t)j * ws) + i);
+    if (LAYOUT == DEPIX_LAYOUT_RGBA) return reinterpret_cast<const uint32_t*>(img + (size_t)j * ws)[i];
     const uint32_t p = load_bgr(img, ws, LAYOUT, i, j);
     return ((p >> 16) & 0xFFu) | (p & 0xFF00u) | ((p & 0xFFu) << 16);
 }
@@ -1358,7 +1357,7 @@ __device__ uint32_t wrapped_colour(const uint8_t* img, int ws, int w, int h, int
         uint32_t c = 0;
         const long long off = (long long)j * ws + 3LL * i, end = (long long)h * ws;
         for (int b = 0; b < 3; b++)
-            if (off + b >= 0 && off + b < end) c |= (uint32_t)__ldg(img + off + b) << (8 * b);
+            if (off + b >= 0 && off + b < end) c |= (uint32_t)img[off + b] << (8 * b);
         return c;
     }
     const int pad = 8 * (((3 * w + 3) & ~3) - 3 * w); // bits of padding after a row
@@ -1425,7 +1424,7 @@ __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const 
         for (int k = threadIdx.x; k < T::BW * T::BH; k += blockDim.x) {
             int gx = x0 - 3 + k % T::BW, gy = y0 - 3 + k / T::BW;
             unsigned v = 0;
-            if (gx >= 0 && gy >= 0 && gx < w && gy < h) v = __ldg(g + (size_t)gy * w + gx) & inside_mask(gx, gy, w, h);
+            if (gx >= 0 && gy >= 0 && gx < w && gy < h) v = g[(size_t)gy * w + gx] & inside_mask(gx, gy, w, h);
             M.graph[k / T::BW][k % T::BW + T::kGOff] = (uint8_t)v;
         }
     }
@@ -1705,6 +1704,7 @@ __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const 
 template <int LAYOUT, int S, int TH>
 __global__ void __launch_bounds__(kRT, raster_blocks(S)) k_mask_raster(RasterBatch b, const uint32_t* lut)
 {
+    follow_last();
     __shared__ MaskTile<S, 32, TH> M;
     extern __shared__ uint32_t masks[];
     size_t z = blockIdx.z;
@@ -1720,6 +1720,7 @@ __global__ void __launch_bounds__(kRT, raster_blocks(S)) k_mask_raster_tma(Raste
                                                          const __grid_constant__ CUtensorMap pix_map,
                                                          const __grid_constant__ CUtensorMap graph_map, int with_graph)
 {
+    follow_last();
     __shared__ MaskTile<S, 32, TH> M;
     extern __shared__ uint32_t masks[];
     size_t z = blockIdx.z;
@@ -1813,6 +1814,7 @@ static size_t mask_smem(int scale)
 template <int LAYOUT, int S, int TH>
 static cudaError_t launch_mask_raster_t(const RasterBatch& b, int nframes, const uint32_t* lut, cudaStream_t s)
 {
+    const bool early = early_stages((long long)b.w * b.h * nframes);
     if constexpr (LAYOUT == DEPIX_LAYOUT_RGBA) {
         CUtensorMap map;
         if (pixel_tensor_map(b, nframes, TH, &map)) {
@@ -1827,8 +1829,7 @@ static cudaError_t launch_mask_raster_t(const RasterBatch& b, int nframes, const
             const bool with_graph = u8_tensor_map(b.graph, b.w, b.h, b.graph_stride, nframes, 32 + 32, TH + 6, &gmap);
             if (!with_graph) gmap = map; // unused
             dim3 grid((b.w + 32 - 1) / 32, (b.h + TH - 1) / TH, nframes);
-            k_mask_raster_tma<S, TH><<<grid, kRT, smem, s>>>(b, lut, map, gmap, with_graph ? 1 : 0);
-            return cudaGetLastError();
+            return launch_early(early, k_mask_raster_tma<S, TH>, grid, kRT, smem, s, b, lut, map, gmap, with_graph ? 1 : 0);
         }
     }
     size_t smem = mask_smem<S, 32, TH>(b.scale);
@@ -1838,8 +1839,7 @@ static cudaError_t launch_mask_raster_t(const RasterBatch& b, int nframes, const
         if (e != cudaSuccess) return e;
     }
     dim3 grid((b.w + 32 - 1) / 32, (b.h + TH - 1) / TH, nframes);
-    k_mask_raster<LAYOUT, S, TH><<<grid, kRT, smem, s>>>(b, lut);
-    return cudaGetLastError();
+    return launch_early(early, k_mask_raster<LAYOUT, S, TH>, grid, kRT, smem, s, b, lut);
 }
 
 // ---- uneven batches: the raster as a persistent kernel over a tile queue
@@ -1847,6 +1847,7 @@ static cudaError_t launch_mask_raster_t(const RasterBatch& b, int nframes, const
 template <int S, int TW, int TH>
 __global__ void __launch_bounds__(kRT, raster_blocks(S)) k_raster_queue(QueueBatch q)
 {
+    follow_last();
     __shared__ MaskTile<S, TW, TH> M;
     extern __shared__ uint32_t masks[];
     const QueueHeader* H = q.hdr;
@@ -1870,8 +1871,7 @@ static cudaError_t queue_raster_t(const QueueBatch& q, int blocks, cudaStream_t 
     // the shared-memory opt-in is made by raster_queue_occupancy, which the
     // host calls on each device before any launch or stream capture
     const size_t smem = mask_smem<S, TW, TH>(q.scale);
-    k_raster_queue<S, TW, TH><<<blocks, kRT, smem, s>>>(q);
-    return cudaGetLastError();
+    return launch_early(true, k_raster_queue<S, TW, TH>, blocks, kRT, smem, s, q);
 }
 
 template <int S, int TW, int TH>

@@ -234,6 +234,7 @@ __device__ __forceinline__ void graph_tile(const FrameRef f, int x0, int y0, uin
 template <int LAYOUT, int GH>
 __global__ void __launch_bounds__(kGThreads) k_graph(FrameBatch b, uint32_t thr, int fuse_trivial)
 {
+    early_start();
     FrameRef f = b.frame(blockIdx.z);
     graph_tile<LAYOUT, GH>(f, blockIdx.x * kGTW, blockIdx.y * 4 * GH, thr, fuse_trivial != 0);
 }
@@ -244,6 +245,7 @@ template <int GH>
 __global__ void __launch_bounds__(kGThreads) k_graph_tma(FrameBatch b, uint32_t thr, int fuse_trivial,
                                                          const __grid_constant__ CUtensorMap pix_map)
 {
+    early_start();
     FrameRef f = b.frame(blockIdx.z);
     graph_tile<DEPIX_LAYOUT_RGBA, GH, true>(f, blockIdx.x * kGTW, blockIdx.y * 4 * GH, thr, fuse_trivial != 0, &pix_map,
                                             (int)blockIdx.z);
@@ -297,7 +299,7 @@ struct SnapTile {
     __device__ __forceinline__ unsigned far(int x, int y) const
     {
         if ((unsigned)(x - ox) < (unsigned)kHRW && (unsigned)(y - oy) < (unsigned)kHRH) return s[y - oy][x - ox];
-        return (unsigned)x < (unsigned)w && (unsigned)y < (unsigned)h ? __ldg(g + (size_t)y * w + x) : 0u;
+        return (unsigned)x < (unsigned)w && (unsigned)y < (unsigned)h ? g[(size_t)y * w + x] : 0u;
     }
 };
 
@@ -483,10 +485,10 @@ __device__ __forceinline__ void heuristics_tile(const uint8_t* snap, uint8_t* ou
             if (gy >= 0 && gy < h) {
                 const uint8_t* row = snap + (size_t)gy * w;
                 if (gx >= 0 && gx + 3 < w && ((reinterpret_cast<uintptr_t>(row + gx) & 3) == 0)) {
-                    v = __ldg(reinterpret_cast<const uint32_t*>(row + gx));
+                    v = *reinterpret_cast<const uint32_t*>(row + gx);
                 } else {
                     for (int q = 0; q < 4; q++)
-                        if (gx + q >= 0 && gx + q < w) v |= (uint32_t)__ldg(row + gx + q) << (8 * q);
+                        if (gx + q >= 0 && gx + q < w) v |= (uint32_t)row[gx + q] << (8 * q);
                 }
             }
             *reinterpret_cast<uint32_t*>(&s[ry][rx]) = v;
@@ -603,6 +605,7 @@ __device__ __forceinline__ void heuristics_tile(const uint8_t* snap, uint8_t* ou
 template <bool VOTE>
 __global__ void __launch_bounds__(kHThreads) k_heuristics(GraphBatch b, int32_t* L)
 {
+    follow_last();
     const uint8_t* snap = b.snap + b.frame_stride * blockIdx.z;
     uint8_t* out = b.out + b.frame_stride * blockIdx.z;
     heuristics_tile<false, VOTE>(snap, out, b.w, b.h, blockIdx.x * kHTW, blockIdx.y * kHTH,
@@ -614,6 +617,7 @@ __global__ void __launch_bounds__(kHThreads) k_heuristics(GraphBatch b, int32_t*
 template <bool VOTE>
 __global__ void __launch_bounds__(kHThreads) k_heuristics_tma(GraphBatch b, int32_t* L, const __grid_constant__ CUtensorMap map)
 {
+    follow_last();
     const uint8_t* snap = b.snap + b.frame_stride * blockIdx.z;
     uint8_t* out = b.out + b.frame_stride * blockIdx.z;
     heuristics_tile<true, VOTE>(snap, out, b.w, b.h, blockIdx.x * kHTW, blockIdx.y * kHTH,
@@ -1044,6 +1048,7 @@ __device__ __forceinline__ void cc_merge_tile_warp(const uint8_t* g, int32_t* L,
 // warp did both and each union's finds ran one after the other, 8.5 now)
 __global__ void __launch_bounds__(128) k_cc_merge_tiles(const uint8_t* g, int32_t* L, int w, int h, size_t frame_stride)
 {
+    follow_last();
     const int tiles_x = (w + kHTW - 1) / kHTW, tiles = tiles_x * ((h + kHTH - 1) / kHTH);
     const int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), t = k >> 1;
     if (t >= tiles) return;
@@ -1109,6 +1114,7 @@ __device__ __forceinline__ void flatten4(int32_t* L, int32_t* q, int n)
 
 __global__ void k_cc_flatten(int32_t* L, int n, size_t frame_stride)
 {
+    follow_last();
     const int k = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (k >= n) return;
     L += frame_stride * blockIdx.z;
@@ -1119,6 +1125,7 @@ __global__ void k_cc_flatten(int32_t* L, int n, size_t frame_stride)
 
 __global__ void __launch_bounds__(kGThreads) k_graph_queue(QueueBatch q)
 {
+    early_start();
     const QueueHeader* H = q.hdr;
     const int n = H->n;
     queue_loop(q.counters + QC_GRAPH, (int)H->total[QS_GRAPH], q.gran[QS_GRAPH], [&](int t) {
@@ -1134,6 +1141,7 @@ __global__ void __launch_bounds__(kGThreads) k_graph_queue(QueueBatch q)
 template <bool VOTE>
 __global__ void __launch_bounds__(kHThreads) k_heur_queue(QueueBatch q)
 {
+    follow_last();
     const QueueHeader* H = q.hdr;
     const int n = H->n;
     queue_loop(q.counters + QC_HEUR, (int)H->total[QS_HEUR], q.gran[QS_HEUR], [&](int t) {
@@ -1149,6 +1157,7 @@ __global__ void __launch_bounds__(kHThreads) k_heur_queue(QueueBatch q)
 
 __global__ void __launch_bounds__(128) k_label_merge_queue(QueueBatch q)
 {
+    follow_last();
     // the local labels came with the heuristics stage: its tiles, its prefix
     const QueueHeader* H = q.hdr;
     const int n = H->n;
@@ -1163,6 +1172,7 @@ __global__ void __launch_bounds__(128) k_label_merge_queue(QueueBatch q)
 
 __global__ void __launch_bounds__(256) k_label_flatten_queue(QueueBatch q)
 {
+    follow_last();
     const QueueHeader* H = q.hdr;
     const int n = H->n;
     queue_loop(q.counters + QC_FLATTEN, (int)H->total[QS_LABEL], q.gran[QS_LABEL], [&](int t) {
@@ -1187,17 +1197,14 @@ cudaError_t queue_graph(const QueueBatch& q, int blocks, cudaStream_t s)
 
 cudaError_t queue_heuristics(const QueueBatch& q, int blocks, cudaStream_t s)
 {
-    if (q.vote) k_heur_queue<true><<<blocks, kHThreads, 0, s>>>(q);
-    else k_heur_queue<false><<<blocks, kHThreads, 0, s>>>(q);
-    return cudaGetLastError();
+    return launch_early(true, q.vote ? k_heur_queue<true> : k_heur_queue<false>, blocks, kHThreads, 0, s, q);
 }
 
 cudaError_t queue_labels(const QueueBatch& q, int blocks, cudaStream_t s)
 {
     // local labels were made by the heuristics stage
-    k_label_merge_queue<<<blocks, 128, 0, s>>>(q);
-    k_label_flatten_queue<<<blocks, 256, 0, s>>>(q);
-    return cudaGetLastError();
+    const cudaError_t e = launch_early(true, k_label_merge_queue, blocks, 128, 0, s, q);
+    return e == cudaSuccess ? launch_early(true, k_label_flatten_queue, blocks, 256, 0, s, q) : e;
 }
 
 static_assert(kQGraphTW == kGTW && kQGraphTH == 4 * kGStripQueue, "graph queue tile");
@@ -1285,13 +1292,11 @@ cudaError_t launch_trivial(uint8_t* g, int w, int h, cudaStream_t s)
 cudaError_t launch_heuristics(const GraphBatch& b, int nframes, int32_t* labels, cudaStream_t s)
 {
     dim3 grid((b.w + kHTW - 1) / kHTW, (b.h + kHTH - 1) / kHTH, nframes);
+    const bool early = early_stages((long long)b.w * b.h * nframes);
     CUtensorMap map;
     const bool tma = u8_tensor_map(b.snap, b.w, b.h, b.frame_stride, nframes, kHRW, kHRH, &map);
-    if (tma && b.vote) k_heuristics_tma<true><<<grid, kHThreads, 0, s>>>(b, labels, map);
-    else if (tma) k_heuristics_tma<false><<<grid, kHThreads, 0, s>>>(b, labels, map);
-    else if (b.vote) k_heuristics<true><<<grid, kHThreads, 0, s>>>(b, labels);
-    else k_heuristics<false><<<grid, kHThreads, 0, s>>>(b, labels);
-    return cudaGetLastError();
+    if (tma) return launch_early(early, b.vote ? k_heuristics_tma<true> : k_heuristics_tma<false>, grid, kHThreads, 0, s, b, labels, map);
+    return launch_early(early, b.vote ? k_heuristics<true> : k_heuristics<false>, grid, kHThreads, 0, s, b, labels);
 }
 
 cudaError_t take_heuristics_fault(int* out)
@@ -1307,9 +1312,12 @@ cudaError_t launch_labels_after_heuristics(const uint8_t* g, int32_t* labels, in
 {
     const int n = w * h;
     const int tiles = ((w + kHTW - 1) / kHTW) * ((h + kHTH - 1) / kHTH);
-    k_cc_merge_tiles<<<dim3((tiles + 1) / 2, 1, nframes), 128, 0, s>>>(g, labels, w, h, frame_stride);
-    k_cc_flatten<<<dim3((n + 1023) / 1024, 1, nframes), 256, 0, s>>>(labels, n, frame_stride);
-    return cudaGetLastError();
+    const bool early = early_stages((long long)n * nframes);
+    const cudaError_t e =
+        launch_early(early, k_cc_merge_tiles, dim3((tiles + 1) / 2, 1, nframes), 128, 0, s, g, labels, w, h, frame_stride);
+    return e == cudaSuccess
+               ? launch_early(early, k_cc_flatten, dim3((n + 1023) / 1024, 1, nframes), 256, 0, s, labels, n, frame_stride)
+               : e;
 }
 
 cudaError_t launch_labels(const uint8_t* g, int32_t* labels, int w, int h, int nframes, size_t frame_stride,

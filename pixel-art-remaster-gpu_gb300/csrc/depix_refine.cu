@@ -946,18 +946,11 @@ __device__ __forceinline__ float sample_loss(const Edge& E, float2 X, float4 t, 
     return r0 * r0 + r1 * r1 + r2 * r2;
 }
 
-// A launch of the step kernels may start while the one before it still runs;
-// what the steps do not change is loaded before the wait for it (early_start
-// lets the next one start).
-__device__ __forceinline__ void early_start() { asm volatile("griddepcontrol.launch_dependents;"); }
-__device__ __forceinline__ void wait_for_last() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // Coverage: kSegLanes lanes per live segment, the samples' gradients reduced in
 // the group and pushed to the segment's free nodes.
 template <bool ENERGY>
 __global__ void __launch_bounds__(256) k_rf_coverage(StepArgs a)
 {
-    early_start();
     const RefineFrame F = *a.fr;
     const float inv_sig = (float)F.scale / a.sigma;
     const float cov_norm = a.w_cov * F.inv_samples3;
@@ -979,7 +972,7 @@ __global__ void __launch_bounds__(256) k_rf_coverage(StepArgs a)
         const int4 sg = ls.nodes;
         const int my = gl == 0 ? sg.x : (gl == 1 ? sg.y : (gl == 2 ? sg.z : -1));
         const bool push = my >= 0 && !(a.flags[my] & 1);
-        if (!waited) wait_for_last();
+        if (!waited) follow_last();
         waited = true;
         const Edge E = live_edge(ls, a.x);
         float g[4] = {0.f, 0.f, 0.f, 0.f};
@@ -994,7 +987,7 @@ __global__ void __launch_bounds__(256) k_rf_coverage(StepArgs a)
             atomicAdd(&a.gcov[my].y, wa * g[1] + wb * g[3]);
         }
     }
-    if (!waited) wait_for_last(); // a grid that ended without it could overtake the one before
+    if (!waited) follow_last(); // a grid that ended without it could overtake the one before
     if constexpr (ENERGY) {
         eloss = warp_sum(eloss);
         if (lane == 0 && eloss != 0.f) atomicAdd(&a.energy[2], (double)eloss * (double)cov_norm);
@@ -1028,7 +1021,6 @@ __device__ __forceinline__ Stencil node_stencil(float2 p, float2 pa, float2 pb, 
 template <bool ENERGY>
 __global__ void __launch_bounds__(64) k_rf_nodes(StepArgs a)
 {
-    early_start();
     const RefineFrame F = *a.fr;
     const float curv_k = a.w_curv / (float)max(F.F, 1), dev_k = a.w_dev / (float)max(F.F, 1);
     float ec = 0.f, ed = 0.f;
@@ -1037,7 +1029,7 @@ __global__ void __launch_bounds__(64) k_rf_nodes(StepArgs a)
         const FreeNode fn = a.fnodes[f];
         const int k = fn.k_a_b_aa.x;
         const float2 p0 = a.x0[k];
-        if (!waited) wait_for_last();
+        if (!waited) follow_last();
         waited = true;
         const int nb[4] = {fn.k_a_b_aa.w, fn.ab_ba_bb.x, fn.ab_ba_bb.y, fn.ab_ba_bb.z};
         float2 qn[4];
@@ -1069,7 +1061,7 @@ __global__ void __launch_bounds__(64) k_rf_nodes(StepArgs a)
                                  p.y - a.lr * (m.y / a.bc1) / (sqrtf(v.y / a.bc2) + kEps));
         }
     }
-    if (!waited) wait_for_last();
+    if (!waited) follow_last();
     if constexpr (ENERGY) {
         ec = warp_sum(ec);
         ed = warp_sum(ed);
@@ -1350,22 +1342,6 @@ bool same_loop(const StepArgs& a, const StepArgs& b)
            a.w_dev == b.w_dev && a.w_cov == b.w_cov && a.lr == b.lr;
 }
 
-// a kernel that may start while the one before it on the stream ends
-template <typename... P, typename... A>
-cudaError_t launch_early(void (*kernel)(P...), int blocks, int threads, cudaStream_t s, A... args)
-{
-    cudaLaunchAttribute early{};
-    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    early.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(threads);
-    cfg.stream = s;
-    cfg.attrs = &early;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 // launches the Adam steps from pos_a (result in pos_a after an even number
 // of steps, pos_b after an odd one). A step is two short kernels, bound by the
 // latency of their launches and loads (one of a 256x224 frame touches 4 MB in
@@ -1386,8 +1362,8 @@ cudaError_t launch_steps(depix_refiner* r, const StepArgs& base, int steps, cuda
         a.y = y;
         a.bc1 = (float)(1.0 - b1);
         a.bc2 = (float)(1.0 - b2);
-        e = launch_early(k_rf_coverage<false>, cov_blocks(r), 256, s, a);
-        if (e == cudaSuccess) e = launch_early(k_rf_nodes<false>, node_blocks(r), 64, s, a);
+        e = launch_early(true, k_rf_coverage<false>, cov_blocks(r), 256, 0, s, a);
+        if (e == cudaSuccess) e = launch_early(true, k_rf_nodes<false>, node_blocks(r), 64, 0, s, a);
         std::swap(x, y);
     }
     return e == cudaSuccess ? cudaGetLastError() : e;
@@ -1403,8 +1379,8 @@ depix_status eval(depix_refiner* r, const depix_refine_params* p, const float2* 
     a.energy = r->energy.p;
     RF_CK(cudaMemsetAsync(r->energy.p, 0, 3 * sizeof(double), s));
     if (gout) RF_CK(cudaMemsetAsync(gout, 0, (size_t)r->N * sizeof(float2), s)); // pinned nodes stay zero
-    RF_CK(launch_early(k_rf_coverage<true>, cov_blocks(r), 256, s, a));
-    RF_CK(launch_early(k_rf_nodes<true>, node_blocks(r), 64, s, a));
+    RF_CK(launch_early(true, k_rf_coverage<true>, cov_blocks(r), 256, 0, s, a));
+    RF_CK(launch_early(true, k_rf_nodes<true>, node_blocks(r), 64, 0, s, a));
     RF_CK(cudaMemcpyAsync(r->h_energy, r->energy.p, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
     RF_CK(cudaStreamSynchronize(s));
     out[0] = r->h_energy[0];
