@@ -1421,12 +1421,15 @@ __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const 
         M.slow = 0;
     }
     if (!(TMA && graph_map)) {
-        for (int k = threadIdx.x; k < T::BW * T::BH; k += blockDim.x) {
-            int gx = x0 - 3 + k % T::BW, gy = y0 - 3 + k / T::BW;
-            unsigned v = 0;
-            if (gx >= 0 && gy >= 0 && gx < w && gy < h) v = g[(size_t)gy * w + gx] & inside_mask(gx, gy, w, h);
-            M.graph[k / T::BW][k % T::BW + T::kGOff] = (uint8_t)v;
-        }
+        // the window's words, from the one that holds its first byte
+        constexpr int C0 = T::kGOff / 4, NC = (T::kGOff + T::BW + 3) / 4 - C0;
+        for_each_batched<2>(
+            NC * T::BH,
+            [&](int k) {
+                const int gx = x0 - 3 - T::kGOff + 4 * (C0 + k % NC), gy = y0 - 3 + k / NC;
+                return row_bytes4(g, w, h, gx, gy) & inside_mask4(gx, gy, w, h);
+            },
+            [&](int k, uint32_t v) { *reinterpret_cast<uint32_t*>(&M.graph[k / NC][4 * (C0 + k % NC)]) = v; });
     }
     if constexpr (TMA) {
         if (threadIdx.x == 0) {
@@ -1445,12 +1448,13 @@ __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const 
             __syncthreads();
         }
     } else {
-        for (int k = threadIdx.x; k < T::CW * T::CH; k += blockDim.x) {
-            int gx = x0 - 2 + k % T::CW, gy = y0 - 2 + k / T::CW;
-            uint32_t v = 0;
-            if (gx >= 0 && gy >= 0 && gx < w && gy < h) v = load_rgba<LAYOUT>(img, ws, gx, gy);
-            M.pix[k / T::CW][k % T::CW + 2] = v;
-        }
+        for_each_batched<3>(
+            T::CW * T::CH,
+            [&](int k) {
+                const int gx = x0 - 2 + k % T::CW, gy = y0 - 2 + k / T::CW;
+                return gx >= 0 && gy >= 0 && gx < w && gy < h ? load_rgba<LAYOUT>(img, ws, gx, gy) : 0u;
+            },
+            [&](int k, uint32_t v) { M.pix[k / T::CW][k % T::CW + 2] = v; });
         __syncthreads();
     }
 

@@ -477,22 +477,10 @@ __device__ __forceinline__ void heuristics_tile(const uint8_t* snap, uint8_t* ou
         if (!ok) return;
     } else {
         if (threadIdx.x == 0) count = count2 = 0;
-        // 4-byte loads where a row is word aligned in memory, else bytes
-        for (int k = threadIdx.x; k < kHRH * (kHRW / 4); k += kHThreads) {
-            int ry = k / (kHRW / 4), rx = 4 * (k % (kHRW / 4));
-            int gy = oy + ry, gx = ox + rx;
-            uint32_t v = 0;
-            if (gy >= 0 && gy < h) {
-                const uint8_t* row = snap + (size_t)gy * w;
-                if (gx >= 0 && gx + 3 < w && ((reinterpret_cast<uintptr_t>(row + gx) & 3) == 0)) {
-                    v = *reinterpret_cast<const uint32_t*>(row + gx);
-                } else {
-                    for (int q = 0; q < 4; q++)
-                        if (gx + q >= 0 && gx + q < w) v |= (uint32_t)row[gx + q] << (8 * q);
-                }
-            }
-            *reinterpret_cast<uint32_t*>(&s[ry][rx]) = v;
-        }
+        constexpr int RW4 = kHRW / 4;
+        for_each_batched<2>(
+            kHRH * RW4, [&](int k) { return row_bytes4(snap, w, h, ox + 4 * (k % RW4), oy + k / RW4); },
+            [&](int k, uint32_t v) { *reinterpret_cast<uint32_t*>(&s[k / RW4][4 * (k % RW4)]) = v; });
         __syncthreads();
     }
     const SnapTile t{s, ox, oy, snap, w, h};
