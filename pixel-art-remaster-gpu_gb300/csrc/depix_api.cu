@@ -192,7 +192,8 @@ depix_status check_out_size(int w, int h, const depix_params* p)
 
 inline cudaStream_t S(depix_stream s) { return reinterpret_cast<cudaStream_t>(s); }
 
-// Coverage-mask raster up to scale 12, per-pixel gather beyond.
+// Coverage-mask raster up to scale 12, per-pixel gather beyond (which leaves
+// the labels alone).
 depix_status raster_launch(const RasterBatch& b, int nframes, cudaStream_t s)
 {
     DEPIX_TRY(ensure_tables(s));
@@ -565,6 +566,7 @@ depix_status run_batch(depix_context* ctx, int n, const int* w, const int* h, co
                        int32_t* d_labels, const BatchShape& shape, cudaStream_t s)
 {
     const uint32_t thr = pack_thresholds(p->tr_y, p->tr_u, p->tr_v, p->yuv);
+    const bool flatten = p->scale > kMaxMaskScale; // else the raster does it
     if (shape.uniform && shape.strided) {
         // equal sizes at equal strides: one launch per stage for the batch
         size_t px = (size_t)w[0] * h[0];
@@ -582,12 +584,12 @@ depix_status run_batch(depix_context* ctx, int n, const int* w, const int* h, co
             DEPIX_CK(launch_heuristics(hb, n, d_labels, s));
         }
         if (d_labels) {
-            StageTimer t(ctx, DEPIX_STAGE_LABELS, 2, s);
-            DEPIX_CK(launch_labels_after_heuristics(ctx->graph_b, d_labels, w[0], h[0], n, px, s));
+            StageTimer t(ctx, DEPIX_STAGE_LABELS, flatten ? 2 : 1, s);
+            DEPIX_CK(launch_labels_after_heuristics(ctx->graph_b, d_labels, w[0], h[0], n, px, flatten, s));
         }
         {
             RasterBatch rb{img0, (size_t)is, ctx->graph_b, px, d_out + out_offset[0], (size_t)os, w[0], h[0],
-                           4 * w[0], DEPIX_LAYOUT_RGBA, p->scale, p->subdivide};
+                           4 * w[0], DEPIX_LAYOUT_RGBA, p->scale, p->subdivide, flatten ? nullptr : d_labels, px};
             DEPIX_TRY(ctx_raster(ctx, rb, n, s));
         }
         return DEPIX_OK;
@@ -610,7 +612,7 @@ depix_status run_batch(depix_context* ctx, int n, const int* w, const int* h, co
                                              DEPIX_STAGE_RASTER};
         for (int st = 0; st < QS_COUNT; st++) {
             if (st == QS_LABEL && !d_labels) continue;
-            StageTimer t(ctx, kStage[st], st == QS_LABEL ? 2 : 1, s);
+            StageTimer t(ctx, kStage[st], 1, s);
             DEPIX_TRY(queue_launch_stage(ctx->queue, st, s));
         }
         return DEPIX_OK;
@@ -631,12 +633,12 @@ depix_status run_batch(depix_context* ctx, int n, const int* w, const int* h, co
             DEPIX_CK(launch_heuristics(hb, 1, d_labels ? d_labels + loff : nullptr, s));
         }
         if (d_labels) {
-            StageTimer t(ctx, DEPIX_STAGE_LABELS, 2, s);
-            DEPIX_CK(launch_labels_after_heuristics(ctx->graph_b + goff, d_labels + loff, w[k], h[k], 1, 0, s));
+            StageTimer t(ctx, DEPIX_STAGE_LABELS, flatten ? 2 : 1, s);
+            DEPIX_CK(launch_labels_after_heuristics(ctx->graph_b + goff, d_labels + loff, w[k], h[k], 1, 0, flatten, s));
         }
         {
             RasterBatch rb{img, 0, ctx->graph_b + goff, 0, d_out + out_offset[k], 0, w[k], h[k], 4 * w[k],
-                           DEPIX_LAYOUT_RGBA, p->scale, p->subdivide};
+                           DEPIX_LAYOUT_RGBA, p->scale, p->subdivide, flatten || !d_labels ? nullptr : d_labels + loff};
             DEPIX_TRY(ctx_raster(ctx, rb, 1, s));
         }
         goff += ctx->max_pixels;
@@ -836,6 +838,7 @@ depix_status depix_frame(depix_context* ctx, const uint8_t* d_img, int w, int h,
     if (d_out) DEPIX_TRY(check_out_size(w, h, p));
     cudaStream_t s = S(s_);
     uint8_t* resolved = d_graph_out ? d_graph_out : ctx->graph_b;
+    const bool flatten = !d_out || p->scale > kMaxMaskScale; // else the raster does it
     {
         StageTimer t(ctx, DEPIX_STAGE_GRAPH, 1, s);
         FrameBatch gb{d_img, 0, ctx->graph_a, 0, w, h, widthstep, (int)layout};
@@ -847,11 +850,12 @@ depix_status depix_frame(depix_context* ctx, const uint8_t* d_img, int w, int h,
         DEPIX_CK(launch_heuristics(hb, 1, d_labels, s));
     }
     if (d_labels) {
-        StageTimer t(ctx, DEPIX_STAGE_LABELS, 2, s);
-        DEPIX_CK(launch_labels_after_heuristics(resolved, d_labels, w, h, 1, 0, s));
+        StageTimer t(ctx, DEPIX_STAGE_LABELS, flatten ? 2 : 1, s);
+        DEPIX_CK(launch_labels_after_heuristics(resolved, d_labels, w, h, 1, 0, flatten, s));
     }
     if (d_out) {
-        RasterBatch rb{d_img, 0, resolved, 0, d_out, 0, w, h, widthstep, (int)layout, p->scale, p->subdivide};
+        RasterBatch rb{d_img, 0, resolved, 0, d_out, 0, w, h, widthstep, (int)layout, p->scale, p->subdivide,
+                       flatten ? nullptr : d_labels};
         DEPIX_TRY(ctx_raster(ctx, rb, 1, s));
     }
     return DEPIX_OK;

@@ -432,6 +432,64 @@ __device__ __forceinline__ bool covers(int ax, int ay, int bx, int by, int cx, i
     return true;
 }
 
+// Roots of up to four consecutive labels q[0..n): one 16-byte load where
+// aligned, the finds interleaved, so that their loads are in flight together
+// (one find per pixel is bound by load latency; settling groups of one label
+// by one find measured slower, 217 against 194 us for 1024 frames with the
+// merge: the warp then runs both ways one after the other; two or four groups of
+// four a thread 177 and 282 against 176: fewer warps). Groups in which nothing
+// changes are not written, the others by one 16-byte store where aligned (a
+// store per label: 184 us).
+__device__ __forceinline__ void flatten4(int32_t* L, int32_t* q, int n)
+{
+    int x[4], p[4], first[4];
+    const bool whole = n == 4 && (reinterpret_cast<uintptr_t>(q) & 15) == 0;
+    if (whole) {
+        const int4 v = *reinterpret_cast<const int4*>(q);
+        x[0] = v.x;
+        x[1] = v.y;
+        x[2] = v.z;
+        x[3] = v.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++) x[i] = q[i < n ? i : 0];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        first[i] = x[i];
+        p[i] = L[x[i]];
+    }
+    for (;;) {
+        bool more = false;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (p[i] != x[i]) {
+                x[i] = p[i];
+                p[i] = L[x[i]];
+                more = true;
+            }
+        if (!more) break;
+    }
+    if (!((first[0] ^ x[0]) | (first[1] ^ x[1]) | (first[2] ^ x[2]) | (first[3] ^ x[3]))) return;
+    if (whole) {
+        *reinterpret_cast<int4*>(q) = make_int4(x[0], x[1], x[2], x[3]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (i < n && first[i] != x[i]) q[i] = x[i];
+    }
+}
+
+// flatten4 over a tile of TW x TH labels
+template <int TW, int TH>
+__device__ __forceinline__ void flatten_tile(int32_t* L, int w, int h, int x0, int y0)
+{
+    for (int k = threadIdx.x; k < TW / 4 * TH; k += blockDim.x) {
+        const int x = x0 + 4 * (k % (TW / 4)), y = y0 + k / (TW / 4);
+        if (x < w && y < h) flatten4(L, L + (size_t)y * w + x, min(4, w - x));
+    }
+}
+
 }  // namespace depix
 
 namespace depix {

@@ -1392,7 +1392,7 @@ __device__ __noinline__ unsigned edge_corner_tests(const uint32_t* px, int PW, c
 template <int LAYOUT, int S, int TW, int TH, bool TMA = false>
 __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const uint8_t* img, int ws, const uint8_t* g,
                                  uint8_t* out, int w, int h, int scale, bool subdivide, const uint32_t* lut, int x0,
-                                 int y0, const CUtensorMap* pix_map = nullptr, int frame = 0,
+                                 int y0, int32_t* labels, const CUtensorMap* pix_map = nullptr, int frame = 0,
                                  const CUtensorMap* graph_map = nullptr)
 {
     using T = MaskTile<S, TW, TH>;
@@ -1420,6 +1420,10 @@ __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const 
         M.count = 0;
         M.slow = 0;
     }
+    // the roots of the tile's labels, while the loads are under way (1024 frames
+    // of 256x224 at x4: 120 us as a kernel of its own, 85 here; 156 when the
+    // warps do it at the tile's end; 4096 sprites 33 and 10)
+    if (labels) flatten_tile<TW, TH>(labels, w, h, x0, y0);
     if (!(TMA && graph_map)) {
         // the window's words, from the one that holds its first byte
         constexpr int C0 = T::kGOff / 4, NC = (T::kGOff + T::BW + 3) / 4 - C0;
@@ -1714,7 +1718,8 @@ __global__ void __launch_bounds__(kRT, raster_blocks(S)) k_mask_raster(RasterBat
     size_t z = blockIdx.z;
     mask_raster_tile<LAYOUT, S, 32, TH>(M, masks, b.img + b.img_stride * z, b.ws, b.graph + b.graph_stride * z,
                                         b.out + b.out_stride * z, b.w, b.h, b.scale, b.subdivide != 0, lut,
-                                        blockIdx.x * 32, blockIdx.y * TH);
+                                        blockIdx.x * 32, blockIdx.y * TH,
+                                        b.labels ? b.labels + b.label_stride * z : nullptr);
 }
 
 // The equal-size batch raster with its pixel windows loaded by TMA (RGBA
@@ -1731,7 +1736,8 @@ __global__ void __launch_bounds__(kRT, raster_blocks(S)) k_mask_raster_tma(Raste
     mask_raster_tile<DEPIX_LAYOUT_RGBA, S, 32, TH, true>(M, masks, b.img + b.img_stride * z, b.ws,
                                                          b.graph + b.graph_stride * z, b.out + b.out_stride * z, b.w,
                                                          b.h, b.scale, b.subdivide != 0, lut, blockIdx.x * 32,
-                                                         blockIdx.y * TH, &pix_map, (int)z,
+                                                         blockIdx.y * TH,
+                                                         b.labels ? b.labels + b.label_stride * z : nullptr, &pix_map, (int)z,
                                                          with_graph ? &graph_map : nullptr);
 }
 
@@ -1865,7 +1871,8 @@ __global__ void __launch_bounds__(kRT, raster_blocks(S)) k_raster_queue(QueueBat
         const int lt = t - (int)base[f], tx = (fr.w + TW - 1) / TW;
         mask_raster_tile<DEPIX_LAYOUT_RGBA, S, TW, TH>(M, masks, H->img + fr.in_off, 4 * fr.w, q.graph_b + fr.px_off,
                                                        H->out + fr.out_off, fr.w, fr.h, q.scale, H->subdivide != 0,
-                                                       q.lut, (lt % tx) * TW, (lt / tx) * TH);
+                                                       q.lut, (lt % tx) * TW, (lt / tx) * TH,
+                                                       H->labels ? H->labels + fr.px_off : nullptr);
     });
 }
 

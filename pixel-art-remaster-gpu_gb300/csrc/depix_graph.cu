@@ -1052,54 +1052,7 @@ __global__ void k_cc_merge(const uint8_t* g, int32_t* L, int w, int h, size_t fr
     cc_merge_border(g + frame_stride * blockIdx.z, L + frame_stride * blockIdx.z, w, h, t / kLBorder, t % kLBorder);
 }
 
-// Roots of up to four consecutive labels q[0..n): one 16-byte load where
-// aligned, the finds interleaved, so that their loads are in flight together
-// (one find per pixel is bound by load latency; settling groups of one label
-// by one find measured slower, 217 against 194 us for 1024 frames with the
-// merge: the warp then runs both ways one after the other; two or four groups of
-// four a thread 177 and 282 against 176: fewer warps). Groups in which nothing
-// changes are not written, the others by one 16-byte store where aligned (a
-// store per label: 184 us).
-__device__ __forceinline__ void flatten4(int32_t* L, int32_t* q, int n)
-{
-    int x[4], p[4], first[4];
-    const bool whole = n == 4 && (reinterpret_cast<uintptr_t>(q) & 15) == 0;
-    if (whole) {
-        const int4 v = *reinterpret_cast<const int4*>(q);
-        x[0] = v.x;
-        x[1] = v.y;
-        x[2] = v.z;
-        x[3] = v.w;
-    } else {
-#pragma unroll
-        for (int i = 0; i < 4; i++) x[i] = q[i < n ? i : 0];
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        first[i] = x[i];
-        p[i] = L[x[i]];
-    }
-    for (;;) {
-        bool more = false;
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-            if (p[i] != x[i]) {
-                x[i] = p[i];
-                p[i] = L[x[i]];
-                more = true;
-            }
-        if (!more) break;
-    }
-    if (!((first[0] ^ x[0]) | (first[1] ^ x[1]) | (first[2] ^ x[2]) | (first[3] ^ x[3]))) return;
-    if (whole) {
-        *reinterpret_cast<int4*>(q) = make_int4(x[0], x[1], x[2], x[3]);
-    } else {
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-            if (i < n && first[i] != x[i]) q[i] = x[i];
-    }
-}
-
+// the roots of all labels, where no raster follows that makes them
 __global__ void k_cc_flatten(int32_t* L, int n, size_t frame_stride)
 {
     follow_last();
@@ -1146,34 +1099,15 @@ __global__ void __launch_bounds__(kHThreads) k_heur_queue(QueueBatch q)
 __global__ void __launch_bounds__(128) k_label_merge_queue(QueueBatch q)
 {
     follow_last();
-    // the local labels came with the heuristics stage: its tiles, its prefix
+    // the local labels came with the heuristics stage: its tiles
     const QueueHeader* H = q.hdr;
     const int n = H->n;
-    warp_queue_loop(q.counters + QC_MERGE, (int)H->total[QS_HEUR], q.gran[QS_LABEL], [&](int t) {
-        const uint32_t* base = H->base + QS_HEUR * (n + 1);
+    warp_queue_loop(q.counters + QC_MERGE, (int)H->total[QS_LABEL], q.gran[QS_LABEL], [&](int t) {
+        const uint32_t* base = H->base + QS_LABEL * (n + 1);
         const int f = queue_frame(base, n, (uint32_t)t);
         const QueueFrame fr = H->frames[f];
         const int lt = t - (int)base[f], tx = (fr.w + kHTW - 1) / kHTW;
         cc_merge_tile_warp(q.graph_b + fr.px_off, H->labels + fr.px_off, fr.w, fr.h, lt % tx, lt / tx, true, true);
-    });
-}
-
-__global__ void __launch_bounds__(256) k_label_flatten_queue(QueueBatch q)
-{
-    follow_last();
-    const QueueHeader* H = q.hdr;
-    const int n = H->n;
-    queue_loop(q.counters + QC_FLATTEN, (int)H->total[QS_LABEL], q.gran[QS_LABEL], [&](int t) {
-        const uint32_t* base = H->base + QS_LABEL * (n + 1);
-        const int f = queue_frame(base, n, (uint32_t)t);
-        const QueueFrame fr = H->frames[f];
-        const int lt = t - (int)base[f], tx = (fr.w + kLT - 1) / kLT;
-        const int x0 = (lt % tx) * kLT, y0 = (lt / tx) * kLT;
-        int32_t* L = H->labels + fr.px_off;
-        for (int p = threadIdx.x; p < kLT / 4 * kLT; p += blockDim.x) {
-            const int x = x0 + 4 * (p % (kLT / 4)), y = y0 + p / (kLT / 4);
-            if (x < fr.w && y < fr.h) flatten4(L, L + y * fr.w + x, min(4, fr.w - x));
-        }
     });
 }
 
@@ -1190,14 +1124,12 @@ cudaError_t queue_heuristics(const QueueBatch& q, int blocks, cudaStream_t s)
 
 cudaError_t queue_labels(const QueueBatch& q, int blocks, cudaStream_t s)
 {
-    // local labels were made by the heuristics stage
-    const cudaError_t e = launch_early(true, k_label_merge_queue, blocks, 128, 0, s, q);
-    return e == cudaSuccess ? launch_early(true, k_label_flatten_queue, blocks, 256, 0, s, q) : e;
+    // local labels were made by the heuristics stage; the raster makes the roots
+    return launch_early(true, k_label_merge_queue, blocks, 128, 0, s, q);
 }
 
 static_assert(kQGraphTW == kGTW && kQGraphTH == 4 * kGStripQueue, "graph queue tile");
 static_assert(kQHeurTW == kHTW && kQHeurTH == kHTH, "heuristics queue tile");
-static_assert(kQLabelT == kLT, "label queue tile");
 
 template <typename K>
 static int occupancy(K kernel, int threads)
@@ -1212,7 +1144,7 @@ int queue_blocks_per_sm(int stage, const QueueBatch& q)
     switch (stage) {
     case QS_GRAPH: return occupancy(k_graph_queue, kGThreads);
     case QS_HEUR: return q.vote ? occupancy(k_heur_queue<true>, kHThreads) : occupancy(k_heur_queue<false>, kHThreads);
-    case QS_LABEL: return occupancy(k_label_flatten_queue, 256);
+    case QS_LABEL: return occupancy(k_label_merge_queue, 128);
     default: return queue_raster_blocks_per_sm(q);
     }
 }
@@ -1296,14 +1228,14 @@ cudaError_t take_heuristics_fault(int* out)
 }
 
 cudaError_t launch_labels_after_heuristics(const uint8_t* g, int32_t* labels, int w, int h, int nframes,
-                                          size_t frame_stride, cudaStream_t s)
+                                          size_t frame_stride, bool flatten, cudaStream_t s)
 {
     const int n = w * h;
     const int tiles = ((w + kHTW - 1) / kHTW) * ((h + kHTH - 1) / kHTH);
     const bool early = early_stages((long long)n * nframes);
     const cudaError_t e =
         launch_early(early, k_cc_merge_tiles, dim3((tiles + 1) / 2, 1, nframes), 128, 0, s, g, labels, w, h, frame_stride);
-    return e == cudaSuccess
+    return e == cudaSuccess && flatten
                ? launch_early(early, k_cc_flatten, dim3((n + 1023) / 1024, 1, nframes), 256, 0, s, labels, n, frame_stride)
                : e;
 }

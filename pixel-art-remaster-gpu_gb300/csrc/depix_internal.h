@@ -49,6 +49,9 @@ struct RasterBatch {
     int w, h, ws, layout;
     int scale;
     int subdivide;
+    // merged labels whose roots the mask raster makes on the way (may be null)
+    int32_t* labels = nullptr;
+    size_t label_stride = 0;
 };
 
 // Whether the stages of so many pixels are launched early: a frame of 24x24
@@ -85,7 +88,7 @@ inline cudaError_t launch_early(bool early_start, void (*kernel)(P...), dim3 gri
 // tile's frame by binary search over the prefix.
 enum QueueStage { QS_GRAPH = 0, QS_HEUR = 1, QS_LABEL = 2, QS_RASTER = 3, QS_COUNT = 4 };
 // the raster has one counter per tile shape (QC_RASTER + shape index)
-enum QueueCounter { QC_GRAPH = 0, QC_HEUR, QC_MERGE, QC_FLATTEN, QC_RASTER, QC_COUNT = QC_RASTER + 3 };
+enum QueueCounter { QC_GRAPH = 0, QC_HEUR, QC_MERGE, QC_RASTER, QC_COUNT = QC_RASTER + 3 };
 
 struct QueueFrame {
     uint64_t in_off;  // bytes into the batch input (RGBA8, rows 4*w bytes)
@@ -129,7 +132,7 @@ struct QueueBatch {
 // every shape without new descriptors, and three more prefixes in which each
 // frame counts only in the shape assigned to it (kQMixedBase + shape index:
 // the shape with the fewest cells to process, ring included)
-constexpr int kQGraphTW = 64, kQGraphTH = 16, kQHeurTW = 64, kQHeurTH = 16, kQLabelT = 32;
+constexpr int kQGraphTW = 64, kQGraphTH = 16, kQHeurTW = 64, kQHeurTH = 16;
 constexpr int kQRasterShapes = 3;
 constexpr int kQMixedBase = QS_RASTER + kQRasterShapes;
 constexpr int kQPrefixes = kQMixedBase + kQRasterShapes;
@@ -194,11 +197,11 @@ cudaError_t launch_border_walks(const uint8_t* graph, int w, int h, int nframes,
                                 int8_t* edges, int32_t* offsets, int max_nodes, int max_walks, int32_t* counts,
                                 cudaStream_t s);
 // heuristics, with each tile's local component labels fused in when labels is
-// set, then the label stage's remainder (merge across the 64x16 tile borders,
-// flatten)
+// set, then the label stage's remainder (merge across the 64x16 tile borders;
+// flatten where no mask raster follows, which then makes the roots)
 cudaError_t launch_heuristics(const GraphBatch& b, int nframes, int32_t* labels, cudaStream_t s);
 cudaError_t launch_labels_after_heuristics(const uint8_t* g, int32_t* labels, int w, int h, int nframes,
-                                          size_t frame_stride, cudaStream_t s);
+                                          size_t frame_stride, bool flatten, cudaStream_t s);
 cudaError_t launch_labels(const uint8_t* g, int32_t* labels, int w, int h, int nframes, size_t frame_stride,
                           cudaStream_t s);
 

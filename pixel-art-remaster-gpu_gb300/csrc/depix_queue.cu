@@ -359,7 +359,7 @@ depix_status queue_prepare(QueueRunner* r, const QueueCall& c, cudaStream_t s)
         const int w = c.w[f], hh = c.h[f];
         F[f] = QueueFrame{c.in_off[f], c.out_off[f], px, w, hh};
         uint32_t t[kQPrefixes] = {tiles(w, hh, kQGraphTW, kQGraphTH), tiles(w, hh, kQHeurTW, kQHeurTH),
-                                  tiles(w, hh, kQLabelT, kQLabelT),   tiles(w, hh, kQRasterTW[0], kQRasterTH[0]),
+                                  tiles(w, hh, kQHeurTW, kQHeurTH), tiles(w, hh, kQRasterTW[0], kQRasterTH[0]),
                                   tiles(w, hh, kQRasterTW[1], kQRasterTH[1]),
                                   tiles(w, hh, kQRasterTW[2], kQRasterTH[2]), 0, 0, 0};
         // the frame's own shape: fewest cells processed, each tile's ring included
