@@ -74,3 +74,52 @@ def test_frames_in_a_row(cuda, w, h, how):
         assert np.array_equal(labels[k].cpu().numpy(), np.asarray(lab).reshape(-1)), k
         assert np.array_equal(outs[k].cpu().numpy(), out), k
     ctx.close()
+
+
+@pytest.mark.parametrize("scale", [1, 3, 4, 5, 8, 12, 13, None])
+def test_labels_with_and_without_a_raster(cuda, scale):
+    """The labels' roots, made by the raster up to scale 12 in every layout of its
+    masks, beyond it and without an output by a kernel of their own: single frames,
+    equal batches and uneven ones in each tile shape."""
+    import depix
+    torch = cuda
+    rng = np.random.default_rng(scale or 99)
+    s = scale or 1
+    p = depix.params(48, 7, 6, True, s)
+    sizes = [(1, 1), (5, 3), (33, 17), (32, 32), (95, 70), (130, 65)]
+    want, imgs = [], []
+    for k, (w, h) in enumerate(sizes):
+        img = image(rng, w, h, k % 3)
+        ws = (3 * w + 3) & ~3
+        buf = np.zeros((h, ws), np.uint8)
+        buf[:, :3 * w] = img[..., 2::-1].reshape(h, -1)
+        want.append(np.asarray(O.label_cc(O.graph(buf.reshape(-1), w, h, ws)[2], w, h)).reshape(-1))
+        imgs.append(img)
+        ctx = depix.Context(w * h, 1)
+        d = torch.from_numpy(img).cuda()
+        out = torch.zeros(w * h * s * s * 4, dtype=torch.uint8, device="cuda") if scale else None
+        lab = torch.full((w * h,), -1, dtype=torch.int32, device="cuda")
+        ctx.frame(d, w, h, 4 * w, depix.LAYOUT_RGBA, p, out, None, lab)
+        assert np.array_equal(lab.cpu().numpy(), want[-1]), (w, h)
+        ctx.close()
+    if not scale:
+        return
+    for order, shapes in (([4] * 3, [None]), (range(len(sizes)), [(32, 32), (32, 16), (16, 16), (0, 0)])):
+        ws, hs = [sizes[k][0] for k in order], [sizes[k][1] for k in order]
+        io, oo, buf, ob = [], [], [], 0
+        for k in order:
+            io.append(sum(len(b) for b in buf))
+            b = imgs[k].tobytes()
+            buf.append(b + bytes(-len(b) % 16))
+            oo.append(ob)
+            ob += -(-len(b) * s * s // 16) * 16
+        d = torch.from_numpy(np.frombuffer(b"".join(buf), np.uint8).copy()).cuda()
+        out = torch.zeros(ob, dtype=torch.uint8, device="cuda")
+        ctx = depix.Context(max(w * h for w, h in sizes), len(ws))
+        for shape in shapes:
+            if shape:
+                ctx.set_launch_shape(1, *shape)
+            lab = torch.full((sum(w * h for w, h in zip(ws, hs)),), -1, dtype=torch.int32, device="cuda")
+            ctx.batch(ws, hs, io, oo, d, p, out, lab)
+            assert np.array_equal(lab.cpu().numpy(), np.concatenate([want[k] for k in order])), shape
+        ctx.close()
