@@ -109,6 +109,7 @@ struct Scan {
 template <typename T, typename Load>
 __global__ void __launch_bounds__(kScanBlock) k_scan(Load load, int n, Scan<T> S)
 {
+    follow_last();
     __shared__ T ws[32];
     __shared__ int last;
     const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
@@ -152,8 +153,7 @@ __global__ void __launch_bounds__(kScanBlock) k_scan(Load load, int n, Scan<T> S
 template <typename T, typename Load>
 cudaError_t exclusive_scan(Load load, int n, const Scan<T>& S, cudaStream_t s)
 {
-    k_scan<T><<<std::max(1, (n + kScanTile - 1) / kScanTile), kScanBlock, 0, s>>>(load, n, S);
-    return cudaGetLastError();
+    return launch_early(true, k_scan<T, Load>, std::max(1, (n + kScanTile - 1) / kScanTile), kScanBlock, 0, s, load, n, S);
 }
 
 struct Geo {
@@ -289,6 +289,7 @@ __global__ void k_rf_boxes(const uint64_t* lut, uint32_t* box)
 
 __global__ void k_rf_mark_vertices(Geo G, uint32_t* vgrid)
 {
+    follow_last();
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= G.w * G.h) return;
     const int i = idx % G.w, j = idx / G.w;
@@ -325,6 +326,7 @@ constexpr int kEdgeCells = 32, kEdgeThreads = 128;
 __global__ void __launch_bounds__(kEdgeThreads) k_rf_count_edges(Geo G, uint32_t* vgrid, int max_split, int* count,
                                                                  uint16_t* slots)
 {
+    follow_last();
     __shared__ int list[kEdgeCells], n;
     __shared__ int npat[kEdgeThreads];
     __shared__ uint32_t nbox[kEdgeThreads];
@@ -398,6 +400,7 @@ __global__ void __launch_bounds__(kEdgeThreads) k_rf_count_edges(Geo G, uint32_t
 __global__ void k_rf_emit_edges(Geo G, uint32_t* vgrid, int max_split, const int* count, Scan<int> off,
                                 const uint16_t* slots, int4* edges, int2* nb_v, int2* nb_e)
 {
+    follow_last();
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= G.w * G.h) return;
     const int c = count[idx];
@@ -457,6 +460,7 @@ struct NodeOut {
 
 __global__ void k_rf_make_nodes(Geo G, const uint32_t* vgrid, Scan<int> nid, const int2* nb_v, const int2* nb_e, NodeOut N)
 {
+    follow_last();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= G.gw * G.gh) return;
     const uint32_t word = vgrid[v];
@@ -508,6 +512,7 @@ __device__ __forceinline__ uint32_t cell_rgb(const Geo& G, int idx) { return pix
 __global__ void k_rf_segments(Geo G, Scan<int> nid, int4* edges, int E, int Nn, const int* flags, const int2* nbr,
                               const int2* nbr_edge, SegOut S)
 {
+    follow_last();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < E) {
         int4 ed = edges[t];
@@ -685,6 +690,7 @@ struct Owner {
 template <bool SLOT_PASS>
 __global__ void k_rf_assign(const int4* seg, int S, const int2* q, int scale, int ow, int oh, Owner own)
 {
+    follow_last();
     int slot;
     const SegBox B = slot_box(seg, S, q, scale, ow, oh, slot);
     const float inv = 1.f / (float)max(B.ex * B.ex + B.ey * B.ey, 1);
@@ -705,6 +711,7 @@ __global__ void k_rf_assign(const int4* seg, int S, const int2* q, int scale, in
 __global__ void k_rf_count_samples(const int4* seg, int S, const int2* q, int scale, int ow, int oh, Owner own,
                                    int* seg_count)
 {
+    follow_last();
     int slot, c = 0;
     const SegBox B = slot_box(seg, S, q, scale, ow, oh, slot);
     box_samples(B, ow, [&](bool live, int x, int, int) { c += live && own(x) == slot; });
@@ -718,6 +725,7 @@ __global__ void k_rf_count_samples(const int4* seg, int S, const int2* q, int sc
 __global__ void k_rf_targets(Geo G, int scale, float sig, const int* samp, const int* pM, float4* tgt,
                              float2* sxy)
 {
+    follow_last();
     const int M = *pM, ow = G.w * scale;
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
         const int yo = samp[m] / ow, xo = samp[m] - yo * ow;
@@ -763,6 +771,7 @@ constexpr int kWarmTile = 16; // source pixels per tile side
 // byte-by-byte FNV-1a, a lane per tile, was one chain of 1296 products: 57 us.)
 __global__ void k_rf_tile_hash(Geo G, int tiles_x, int tiles, uint64_t* hash)
 {
+    follow_last();
     const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (t >= tiles) return;
     const int x0 = (t % tiles_x) * kWarmTile - 1, y0 = (t / tiles_x) * kWarmTile - 1;
@@ -788,6 +797,7 @@ __global__ void k_rf_tile_hash(Geo G, int tiles_x, int tiles, uint64_t* hash)
 
 __global__ void k_rf_warm_scatter(const int2* q, const float2* pos, int N, int gw, float2* grid, int* stamp, int epoch)
 {
+    follow_last();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= N) return;
     const int v = (q[k].y + 1) * gw + (q[k].x + 1);
@@ -799,6 +809,7 @@ __global__ void k_rf_warm_gather(const int2* q, const float2* pos0, int N, int w
                                  const uint64_t* hash, const uint64_t* prev_hash, const float2* grid,
                                  const int* stamp, int epoch, float2* out)
 {
+    follow_last();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= N) return;
     const int2 c = q[k];
@@ -810,6 +821,7 @@ __global__ void k_rf_warm_gather(const int2* q, const float2* pos0, int N, int w
 
 __global__ void k_rf_same_tiles(const uint64_t* a, const uint64_t* b, int tiles, int* count)
 {
+    follow_last();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const bool same = t < tiles && a[t] == b[t];
     const unsigned m = __ballot_sync(0xFFFFFFFFu, same);
@@ -1078,6 +1090,7 @@ __global__ void k_rf_fill_samples(const int4* seg, int S, const int2* q, int sca
                                   const int* seg_count, Scan<unsigned long long> off, const uint2* col, int* samp,
                                   int* seg_off, LiveSeg* live)
 {
+    follow_last();
     int slot;
     SegBox B = slot_box(seg, S, q, scale, ow, oh, slot);
     const int gl = threadIdx.x & (kBoxLanes - 1), shift = threadIdx.x & 31 & ~(kBoxLanes - 1);
@@ -1104,6 +1117,7 @@ __global__ void k_rf_fill_samples(const int4* seg, int S, const int2* q, int sca
 // start of an Adam run: both position buffers from src, moments zeroed
 __global__ void k_rf_begin(const float2* src, float2* x, float2* y, float2* m, float2* v, int N)
 {
+    follow_last();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
         const float2 q = src[i];
         x[i] = q;
@@ -1119,6 +1133,7 @@ __global__ void k_rf_free_nodes(const int* flags, const int2* nbr, Scan<int> pos
                                 const unsigned long long* samples_live, int* totals, int ow, int oh, int scale,
                                 float inv_samples3, RefineFrame* fr)
 {
+    follow_last();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k == 0) {
         const unsigned long long t = *samples_live;
@@ -1546,24 +1561,27 @@ depix_status depix_refine_setup(depix_refiner* r, const uint8_t* d_img, int w, i
     const Scan<int> cells{r->cell_off.p, r->cell_tiles.p, r->scalars.p + 0, r->tickets.p + 0};
     const Scan<int> nid{r->nid.p, r->nid_tiles.p, r->scalars.p + 1, r->tickets.p + 1};
     RF_CK(cudaMemsetAsync(r->vgrid.p, 0, (size_t)nv * sizeof(uint32_t), s));
-    k_rf_mark_vertices<<<blocks_for(n), 256, 0, s>>>(G, r->vgrid.p);
-    k_rf_count_edges<<<blocks_for(n, kEdgeCells), kEdgeThreads, 0, s>>>(G, r->vgrid.p, r->max_split, r->cell_count.p,
-                                                                        r->edge_slots.p);
+    // the topology is some twenty short kernels, each started while the one
+    // before it ends (256x224 at x4: 166 us one after the other, 135 so)
+    RF_CK(launch_early(true, k_rf_mark_vertices, blocks_for(n), 256, 0, s, G, r->vgrid.p));
+    RF_CK(launch_early(true, k_rf_count_edges, blocks_for(n, kEdgeCells), kEdgeThreads, 0, s, G, r->vgrid.p,
+                       r->max_split, r->cell_count.p, r->edge_slots.p));
     RF_CK(cudaGetLastError());
     RF_CK(exclusive_scan(CellCount{r->cell_count.p}, n, cells, s));
     // edges reserved for the most a frame can have, so that E and N come
     // back together: the one read back of the setup (they size the node and
     // segment arrays; the later counts stay on the device)
     RF_CK(r->edges.reserve((size_t)n * r->max_split));
-    k_rf_emit_edges<<<blocks_for(n, 128), 128, 0, s>>>(G, r->vgrid.p, r->max_split, r->cell_count.p, cells,
-                                                       r->edge_slots.p, r->edges.p, r->nb_v.p, r->nb_e.p);
+    RF_CK(launch_early(true, k_rf_emit_edges, blocks_for(n, 128), 128, 0, s, G, r->vgrid.p, r->max_split,
+                       r->cell_count.p, cells, r->edge_slots.p, r->edges.p, r->nb_v.p, r->nb_e.p));
     RF_CK(cudaGetLastError());
     RF_CK(exclusive_scan(NodeFlag{r->vgrid.p}, nv, nid, s));
     RF_CK(cudaMemcpyAsync(r->h_scalars, r->scalars.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
     RF_CK(cudaEventRecord(r->counted, s));
     // what needs neither runs while the host waits for them
     RF_CK(cudaMemsetAsync(r->best.p, 0xFF, (size_t)no_px * sizeof(unsigned long long), s));
-    k_rf_tile_hash<<<blocks_for(32LL * r->tiles), 256, 0, s>>>(G, r->tiles_x, r->tiles, r->tile_hash.p);
+    RF_CK(launch_early(true, k_rf_tile_hash, blocks_for(32LL * r->tiles), 256, 0, s, G, r->tiles_x, r->tiles,
+                       r->tile_hash.p));
     RF_CK(cudaGetLastError());
     RF_CK(cudaEventSynchronize(r->counted));
     const int E = r->h_scalars[0], N = r->h_scalars[1];
@@ -1593,9 +1611,10 @@ depix_status depix_refine_setup(depix_refiner* r, const uint8_t* d_img, int w, i
     RF_CK(r->tgt.reserve(no_px));
     RF_CK(r->sxy.reserve(no_px));
     NodeOut no{r->node_q.p, r->node_flags.p, r->node_nbr.p, r->node_nbr_edge.p, r->pos0.p, r->gcov.p};
-    k_rf_make_nodes<<<blocks_for(nv), 256, 0, s>>>(G, r->vgrid.p, nid, r->nb_v.p, r->nb_e.p, no);
-    k_rf_segments<<<blocks_for((long long)E + N), 256, 0, s>>>(G, nid, r->edges.p, E, N, r->node_flags.p, r->node_nbr.p,
-                                                              r->node_nbr_edge.p, SegOut{r->seg.p, r->seg_col.p});
+    RF_CK(launch_early(true, k_rf_make_nodes, blocks_for(nv), 256, 0, s, G, r->vgrid.p, nid, r->nb_v.p, r->nb_e.p,
+                       no));
+    RF_CK(launch_early(true, k_rf_segments, blocks_for((long long)E + N), 256, 0, s, G, nid, r->edges.p, E, N,
+                       r->node_flags.p, r->node_nbr.p, r->node_nbr_edge.p, SegOut{r->seg.p, r->seg_col.p}));
     RF_CK(cudaGetLastError());
     // sample assignment
     const Scan<unsigned long long> soff{r->samp_off.p, r->samp_tiles.p, r->samp_total.p, r->tickets.p + 2};
@@ -1609,25 +1628,27 @@ depix_status depix_refine_setup(depix_refiner* r, const uint8_t* d_img, int w, i
         RF_CK(r->bseg.reserve(no_px));
         RF_CK(cudaMemsetAsync(r->bseg.p, 0x7F, (size_t)no_px * sizeof(int), s)); // above every slot
     }
-    k_rf_assign<false><<<box_blocks, 256, 0, s>>>(r->seg.p, S, r->node_q.p, p->scale, ow, oh, own);
+    RF_CK(launch_early(true, k_rf_assign<false>, box_blocks, 256, 0, s, r->seg.p, S, r->node_q.p, p->scale, ow, oh,
+                       own));
     if (!own.slot_bits) {
         own.bseg = r->bseg.p;
-        k_rf_assign<true><<<box_blocks, 256, 0, s>>>(r->seg.p, S, r->node_q.p, p->scale, ow, oh, own);
+        RF_CK(launch_early(true, k_rf_assign<true>, box_blocks, 256, 0, s, r->seg.p, S, r->node_q.p, p->scale, ow, oh,
+                           own));
     }
-    k_rf_count_samples<<<box_blocks, 256, 0, s>>>(r->seg.p, S, r->node_q.p, p->scale, ow, oh, own,
-                                                  r->seg_count.p);
+    RF_CK(launch_early(true, k_rf_count_samples, box_blocks, 256, 0, s, r->seg.p, S, r->node_q.p, p->scale, ow, oh,
+                       own, r->seg_count.p));
     RF_CK(cudaGetLastError());
     RF_CK(exclusive_scan(SampleCount{r->seg_count.p}, S, soff, s));
-    k_rf_fill_samples<<<box_blocks, 256, 0, s>>>(r->seg.p, S, r->node_q.p, p->scale, ow, oh, own, r->seg_count.p,
-                                                 soff, r->seg_col.p, r->samp.p, r->seg_off.p, r->live.p);
+    RF_CK(launch_early(true, k_rf_fill_samples, box_blocks, 256, 0, s, r->seg.p, S, r->node_q.p, p->scale, ow, oh,
+                       own, r->seg_count.p, soff, r->seg_col.p, r->samp.p, r->seg_off.p, r->live.p));
     // free nodes and their curvature stencils, and the frame record
     const Scan<int> free_pos{r->free_pos.p, r->free_tiles.p, r->scalars.p + 3, r->tickets.p + 3};
     RF_CK(exclusive_scan(FreeFlag{r->node_flags.p}, N, free_pos, s));
-    k_rf_free_nodes<<<blocks_for(N), 256, 0, s>>>(r->node_flags.p, r->node_nbr.p, free_pos, N, r->fnodes.p,
-                                                  r->samp_total.p, r->scalars.p, ow, oh, p->scale,
-                                                  (float)(1.0 / (3.0 * (double)ow * (double)oh)), r->frame.p);
-    k_rf_targets<<<std::min(blocks_for(no_px), r->sms * 8), 256, 0, s>>>(
-        G, p->scale, rp->sigma / (float)p->scale, r->samp.p, r->scalars.p + 2, r->tgt.p, r->sxy.p);
+    RF_CK(launch_early(true, k_rf_free_nodes, blocks_for(N), 256, 0, s, r->node_flags.p, r->node_nbr.p, free_pos, N,
+                       r->fnodes.p, r->samp_total.p, r->scalars.p, ow, oh, p->scale,
+                       (float)(1.0 / (3.0 * (double)ow * (double)oh)), r->frame.p));
+    RF_CK(launch_early(true, k_rf_targets, std::min(blocks_for(no_px), r->sms * 8), 256, 0, s, G, p->scale,
+                       rp->sigma / (float)p->scale, r->samp.p, r->scalars.p + 2, r->tgt.p, r->sxy.p));
     RF_CK(cudaGetLastError());
     r->w = w;
     r->h = h;
@@ -1730,16 +1751,16 @@ depix_status depix_refine_warm_start(depix_refiner* r, const depix_refiner* prev
         r->warm_epoch = 0;
     }
     const int epoch = ++r->warm_epoch;
-    k_rf_warm_scatter<<<blocks_for(prev->N), 256, 0, s>>>(prev->node_q.p, reinterpret_cast<const float2*>(d_prev_pos),
-                                                          prev->N, gw, r->warm_grid.p, r->warm_stamp.p, epoch);
-    k_rf_warm_gather<<<blocks_for(r->N), 256, 0, s>>>(r->node_q.p, r->pos0.p, r->N, r->w, r->h, gw, r->tiles_x,
-                                                      r->tile_hash.p, prev->tile_hash.p, r->warm_grid.p,
-                                                      r->warm_stamp.p, epoch, reinterpret_cast<float2*>(d_pos));
+    RF_CK(launch_early(true, k_rf_warm_scatter, blocks_for(prev->N), 256, 0, s, prev->node_q.p,
+                       reinterpret_cast<const float2*>(d_prev_pos), prev->N, gw, r->warm_grid.p, r->warm_stamp.p, epoch));
+    RF_CK(launch_early(true, k_rf_warm_gather, blocks_for(r->N), 256, 0, s, r->node_q.p, r->pos0.p, r->N, r->w, r->h,
+                       gw, r->tiles_x, r->tile_hash.p, prev->tile_hash.p, r->warm_grid.p, r->warm_stamp.p, epoch,
+                       reinterpret_cast<float2*>(d_pos)));
     RF_CK(cudaGetLastError());
     if (reused_tiles) {
         RF_CK(cudaMemsetAsync(r->scalars.p + 5, 0, sizeof(int), s));
-        k_rf_same_tiles<<<blocks_for(r->tiles), 256, 0, s>>>(r->tile_hash.p, prev->tile_hash.p, r->tiles,
-                                                             r->scalars.p + 5);
+        RF_CK(launch_early(true, k_rf_same_tiles, blocks_for(r->tiles), 256, 0, s, r->tile_hash.p, prev->tile_hash.p,
+                           r->tiles, r->scalars.p + 5));
         RF_CK(cudaGetLastError());
         DEPIX_TRY_RF(read_totals(r, 5, 1, reused_tiles, s));
     }
@@ -1770,8 +1791,8 @@ depix_status depix_refine_run(depix_refiner* r, const depix_refine_params* p, fl
     const size_t bytes = (size_t)r->N * sizeof(float2);
     float2* x = r->pos_a.p;
     float2* y = r->pos_b.p;
-    k_rf_begin<<<std::min(blocks_for(r->N), r->sms * 4), 256, 0, s>>>(
-        d_pos ? reinterpret_cast<const float2*>(d_pos) : r->pos0.p, x, y, r->adam_m.p, r->adam_v.p, r->N);
+    RF_CK(launch_early(true, k_rf_begin, std::min(blocks_for(r->N), r->sms * 4), 256, 0, s,
+                       d_pos ? reinterpret_cast<const float2*>(d_pos) : r->pos0.p, x, y, r->adam_m.p, r->adam_v.p, r->N));
     RF_CK(cudaGetLastError());
     if (before) DEPIX_TRY_RF(eval(r, p, x, nullptr, before, s));
     const StepArgs a = step_args(r, p);
