@@ -883,9 +883,9 @@ cudaError_t launch_raster(const RasterBatch& b, int nframes, cudaStream_t s)
 // short chain of shared-memory accesses; cut cells wait on table loads. 1024
 // frames of 256x224 at x4: 2605 us when a cell per distinct neighbourhood
 // built its polygon from dependent table lookups and masked it by crossing
-// number (hash tables found the distinct ones), 886 us now (4.6 TB/s of
-// input and output, 0.67 of the measured copy rate). 16 frames of 640x480 at
-// x8: 597 us before, 305 us now (4.2 TB/s).
+// number (hash tables found the distinct ones), 885 us now (4.6 TB/s of
+// input and output, 0.67 of the measured copy rate; 968 with the labels' roots).
+// 16 frames of 640x480 at x8: 597 us before, 289 us now (4.4 TB/s).
 
 struct MaskGeom {
     int s;
@@ -1536,7 +1536,7 @@ __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const 
         // four pixels a lane, so that the stores are contiguous whatever s is;
         // the rows of the other blocks follow, one a thread. (Resolving each
         // row of the 32 blocks in the warp and writing it whole: 132 us for 100
-        // frames of 152x102 at x5, 96 us now; one thread a block, which stores
+        // frames of 152x102 at x5, 96 us so; one thread a block, which stores
         // every pixel apart: 171.)
         constexpr int CM = S == 0 ? 7 : 12; // most samples of a row
         const uint32_t blockbits = (1u << s) - 1u;

@@ -439,14 +439,15 @@ __device__ void tile_labels(const uint8_t (*node)[kHTW], uint16_t* joins, int32_
 // Heuristic resolution of one 64x16 tile; with L set, the tile's local
 // component labels too (union-find over the resolved bytes, still in shared
 // memory), which leaves the label stage only the merge across tile borders
-// and the flattening.
+// and the roots.
 //
 // Crossings are few, so four 2x2 blocks a thread are tested for one at a time
 // in packed bytes, the crossings go to a list, and a lane decides each (once:
 // its four corner nodes each lose a bit of the decision). Bound: issue (79 %);
 // 1024 frames of 256x224 with labels: 636 us when every node tested its four
-// blocks over bytes and every lane ran a row's join masks, 254 us now (the
-// vote on 32 frames of 159x143: 68 us before, 33 now).
+// blocks over bytes and every lane ran a row's join masks, 244 us now (the
+// vote on 32 frames of 159x143: 68 us before, 25 now). The window by 16-byte
+// asynchronous copies instead of TMA: 255.
 template <bool TMA = false, bool VOTE = false>
 __device__ __forceinline__ void heuristics_tile(const uint8_t* snap, uint8_t* out, int w, int h, int x0, int y0,
                                                 int32_t* L = nullptr, const CUtensorMap* map = nullptr,
@@ -653,8 +654,8 @@ __device__ __forceinline__ void uf_unite(int32_t* L, int a, int b)
 // (local roots are the tile-local minima, which are also the minima in global
 // index order), then unions across tile borders on the global label array,
 // then one flattening pass. The frame and batch paths make the tile-local
-// labels inside the 64x16 heuristics tiles (tile_labels) and
-// merge with merge_tile_borders; the stage API (depix_label_components) runs
+// labels inside the 64x16 heuristics tiles (tile_labels), merge with
+// merge_tile_borders and flatten in the raster's tiles (flatten_tile); the stage API (depix_label_components) runs
 // its own 32x32 tiles over a graph in global memory (cc_local_core: a warp
 // owns a row, horizontal runs from one ballot, one union per pair of touching
 // runs).
