@@ -288,7 +288,15 @@ constexpr int kHTW = 64, kHTH = 16;
 // to load and keep for the tile's 1 KB.)
 constexpr int kHaloX = 16, kHaloY = 8;
 constexpr int kHRW = kHTW + 2 * kHaloX, kHRH = kHTH + 2 * kHaloY;
+// Threads of a tile. With few tiles a tile's time is the call's, and more threads
+// shorten its lists of crossings and joins (a call with labels at x4, us with
+// 128 / 256 / 512 threads: a 256x224 frame, 56 tiles, 36.5 / 33.6 / 28.8; 8 of
+// them 51.6 / 41.1 / 39.0; 12 of them, 672 tiles, 58.8 / 54.7 / 53.9; 16 of them
+// 61.0 / 58.6 / 62.0; 20 of them, 1120, 68.2 / 66.5 / 66.6; 24 72.4 / 72.5 / 72.5).
+// With many, blocks of 128 leave less waiting at barriers (heuristics of 1024
+// frames 244 / 309 with 256).
 constexpr int kHThreads = 128;
+constexpr long long kTiles512 = 760, kTiles256 = 1216;
 
 struct SnapTile {
     const uint8_t (*s)[kHRW];
@@ -434,6 +442,7 @@ __device__ __forceinline__ unsigned vote_decision(const SnapTile& t, int i, int 
 }
 
 constexpr int kMaxJoins = (kHTH - 1) * 3 * kHTW; // every upward edge of a tile
+template <int NT>
 __device__ void tile_labels(const uint8_t (*node)[kHTW], uint16_t* joins, int32_t* L, int w, int h, int x0, int y0);
 
 // Heuristic resolution of one 64x16 tile; with L set, the tile's local
@@ -448,7 +457,7 @@ __device__ void tile_labels(const uint8_t (*node)[kHTW], uint16_t* joins, int32_
 // blocks over bytes and every lane ran a row's join masks, 244 us now (the
 // vote on 32 frames of 159x143: 68 us before, 25 now). The window by 16-byte
 // asynchronous copies instead of TMA: 255.
-template <bool TMA = false, bool VOTE = false>
+template <int NT, bool TMA = false, bool VOTE = false>
 __device__ __forceinline__ void heuristics_tile(const uint8_t* snap, uint8_t* out, int w, int h, int x0, int y0,
                                                 int32_t* L = nullptr, const CUtensorMap* map = nullptr,
                                                 int frame = 0)
@@ -489,7 +498,7 @@ __device__ __forceinline__ void heuristics_tile(const uint8_t* snap, uint8_t* ou
     // columns x0 - 4 .. x0 + 63 of which the first word gives x0 - 1 only.
     // Blocks reaching outside the image read zeros and are never crossings.
     constexpr int NW = kHTW / 4 + 1;
-    for (int k = threadIdx.x; k < NW * (kHTH + 1); k += kHThreads) {
+    for (int k = threadIdx.x; k < NW * (kHTH + 1); k += NT) {
         const int wc = k % NW, by = k / NW;
         const uint32_t* a = reinterpret_cast<const uint32_t*>(&s[by + kHaloY - 1][kHaloX - 4 + 4 * wc]);
         const uint32_t* b = a + kHRW / 4;
@@ -532,7 +541,7 @@ __device__ __forceinline__ void heuristics_tile(const uint8_t* snap, uint8_t* ou
     int nwalks = n;
     if constexpr (!VOTE) {
         uint16_t* more = reinterpret_cast<uint16_t*>(buf + kHRH * kHRW);
-        for (int k = threadIdx.x; k < n; k += kHThreads) {
+        for (int k = threadIdx.x; k < n; k += NT) {
             const int bx = list[k] & 0xFF, by = list[k] >> 8;
             const unsigned d = block_decision(t, x0 - 1 + bx, y0 - 1 + by);
             if (d == kDecWalk) more[atomicAdd(&count2, 1)] = list[k];
@@ -542,7 +551,7 @@ __device__ __forceinline__ void heuristics_tile(const uint8_t* snap, uint8_t* ou
         walks = more;
         nwalks = count2;
     }
-    for (int k0 = 0; k0 < nwalks; k0 += kHThreads / 4) {
+    for (int k0 = 0; k0 < nwalks; k0 += NT / 4) {
         const int k = k0 + (threadIdx.x >> 2), q = threadIdx.x & 3;
         if (k0 + ((int)threadIdx.x & ~31) / 4 >= nwalks) break; // whole warps
         const int it = walks[k < nwalks ? k : nwalks - 1], bx = it & 0xFF, by = it >> 8;
@@ -559,7 +568,7 @@ __device__ __forceinline__ void heuristics_tile(const uint8_t* snap, uint8_t* ou
     // ---- output, four nodes a thread; for the labels the nodes on the image's
     // edge lose their bits toward outside
     const bool edge = x0 == 0 || y0 == 0 || x0 + kHTW >= w || y0 + kHTH >= h;
-    for (int k = threadIdx.x; k < kHTW / 4 * kHTH; k += kHThreads) {
+    for (int k = threadIdx.x; k < kHTW / 4 * kHTH; k += NT) {
         const int tx = 4 * (k % (kHTW / 4)), ty = k / (kHTW / 4);
         const int i = x0 + tx, j = y0 + ty;
         const uint32_t v = *reinterpret_cast<const uint32_t*>(&res[ty][tx]);
@@ -585,31 +594,31 @@ __device__ __forceinline__ void heuristics_tile(const uint8_t* snap, uint8_t* ou
     }
     if (L) {
         if (edge) __syncthreads();
-        tile_labels(res, reinterpret_cast<uint16_t*>(buf), L, w, h, x0, y0);
+        tile_labels<NT>(res, reinterpret_cast<uint16_t*>(buf), L, w, h, x0, y0);
     }
 }
 
 // VOTE: the weighted vote instead of the reference's ordered tests; L may be
 // NULL
-template <bool VOTE>
-__global__ void __launch_bounds__(kHThreads) k_heuristics(GraphBatch b, int32_t* L)
+template <bool VOTE, int NT>
+__global__ void __launch_bounds__(NT) k_heuristics(GraphBatch b, int32_t* L)
 {
     follow_last();
     const uint8_t* snap = b.snap + b.frame_stride * blockIdx.z;
     uint8_t* out = b.out + b.frame_stride * blockIdx.z;
-    heuristics_tile<false, VOTE>(snap, out, b.w, b.h, blockIdx.x * kHTW, blockIdx.y * kHTH,
+    heuristics_tile<NT, false, VOTE>(snap, out, b.w, b.h, blockIdx.x * kHTW, blockIdx.y * kHTH,
                                  L ? L + b.frame_stride * blockIdx.z : nullptr);
 }
 
 // the same with the graph windows by TMA (width and frame stride multiples of
 // 16 bytes, 16-byte aligned base)
-template <bool VOTE>
-__global__ void __launch_bounds__(kHThreads) k_heuristics_tma(GraphBatch b, int32_t* L, const __grid_constant__ CUtensorMap map)
+template <bool VOTE, int NT>
+__global__ void __launch_bounds__(NT) k_heuristics_tma(GraphBatch b, int32_t* L, const __grid_constant__ CUtensorMap map)
 {
     follow_last();
     const uint8_t* snap = b.snap + b.frame_stride * blockIdx.z;
     uint8_t* out = b.out + b.frame_stride * blockIdx.z;
-    heuristics_tile<true, VOTE>(snap, out, b.w, b.h, blockIdx.x * kHTW, blockIdx.y * kHTH,
+    heuristics_tile<NT, true, VOTE>(snap, out, b.w, b.h, blockIdx.x * kHTW, blockIdx.y * kHTH,
                                 L ? L + b.frame_stride * blockIdx.z : nullptr, &map, (int)blockIdx.z);
 }
 
@@ -773,15 +782,16 @@ __device__ __forceinline__ void for_each_join(const uint64_t (&need)[3], Fn fn)
 // listed runs, which are all that are not their own root, are pointed at their
 // roots, and each pixel reads its run's parent (following the chains from
 // there cost 6.8 k cycles).
+template <int NT>
 __device__ void tile_labels(const uint8_t (*node)[kHTW], uint16_t* joins, int32_t* L, int w, int h, int x0, int y0)
 {
-    static_assert(kHTW == 64 && kHTH == 16 && kHThreads == 128, "lanes of the joins");
+    static_assert(kHTW == 64 && kHTH == 16 && NT >= 128, "lanes of the joins");
     __shared__ __align__(16) int sl[kHTH * kHTW];
     __shared__ uint64_t rows[4][kHTH]; // run starts, up-left, up, up-right edges
     __shared__ int njoins;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) njoins = 0;
-    {
+    if (NT == 128 || threadIdx.x < 128) {
         // eight columns a thread: bit planes of its two words as bytes of the
         // row masks (the product gathers a word's four bits in its top byte)
         const int r = threadIdx.x >> 3, g = threadIdx.x & 7;
@@ -819,13 +829,13 @@ __device__ void tile_labels(const uint8_t (*node)[kHTW], uint16_t* joins, int32_
         a = r * kHTW + run_start(rows[0][r], c);
         b = (r + 1) * kHTW + run_start(rows[0][r + 1], c + e - 1);
     };
-    for (int i = threadIdx.x; i < n; i += kHThreads) {
+    for (int i = threadIdx.x; i < n; i += NT) {
         int a, b;
         runs(i, a, b);
         s_unite(sl, a, b);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < n; i += kHThreads) {
+    for (int i = threadIdx.x; i < n; i += NT) {
         int a, b;
         runs(i, a, b);
         // no union in flight: both ends have one root, and a store only ever
@@ -838,7 +848,7 @@ __device__ void tile_labels(const uint8_t (*node)[kHTW], uint16_t* joins, int32_
     // four pixels a thread: their runs' roots, stored at once where the row allows
     const bool wide = ((w | x0 | (int)(reinterpret_cast<uintptr_t>(L) >> 2)) & 3) == 0;
 #pragma unroll
-    for (int k = threadIdx.x; k < kHTW / 4 * kHTH; k += kHThreads) {
+    for (int k = threadIdx.x; k < kHTW / 4 * kHTH; k += NT) {
         const int r = k / (kHTW / 4), c = 4 * (k % (kHTW / 4)), x = x0 + c, y = y0 + r;
         const uint64_t S = rows[0][r];
         int run = run_start(S, c);
@@ -1091,7 +1101,7 @@ __global__ void __launch_bounds__(kHThreads) k_heur_queue(QueueBatch q)
         const int f = queue_frame(base, n, (uint32_t)t);
         const QueueFrame fr = H->frames[f];
         const int lt = t - (int)base[f], tx = (fr.w + kHTW - 1) / kHTW;
-        heuristics_tile<false, VOTE>(q.graph_a + fr.px_off, q.graph_b + fr.px_off, fr.w, fr.h, (lt % tx) * kHTW,
+        heuristics_tile<kHThreads, false, VOTE>(q.graph_a + fr.px_off, q.graph_b + fr.px_off, fr.w, fr.h, (lt % tx) * kHTW,
                                      (lt / tx) * kHTH, H->labels ? H->labels + fr.px_off : nullptr);
     });
 }
@@ -1210,14 +1220,26 @@ cudaError_t launch_trivial(uint8_t* g, int w, int h, cudaStream_t s)
     return cudaGetLastError();
 }
 
+template <int NT>
+static cudaError_t heuristics_t(bool tma, bool early, dim3 grid, cudaStream_t s, const GraphBatch& b, int32_t* labels,
+                                const CUtensorMap& map)
+{
+    if (tma)
+        return launch_early(early, b.vote ? k_heuristics_tma<true, NT> : k_heuristics_tma<false, NT>, grid, NT, 0, s, b,
+                            labels, map);
+    return launch_early(early, b.vote ? k_heuristics<true, NT> : k_heuristics<false, NT>, grid, NT, 0, s, b, labels);
+}
+
 cudaError_t launch_heuristics(const GraphBatch& b, int nframes, int32_t* labels, cudaStream_t s)
 {
     dim3 grid((b.w + kHTW - 1) / kHTW, (b.h + kHTH - 1) / kHTH, nframes);
     const bool early = early_stages((long long)b.w * b.h * nframes);
     CUtensorMap map;
     const bool tma = u8_tensor_map(b.snap, b.w, b.h, b.frame_stride, nframes, kHRW, kHRH, &map);
-    if (tma) return launch_early(early, b.vote ? k_heuristics_tma<true> : k_heuristics_tma<false>, grid, kHThreads, 0, s, b, labels, map);
-    return launch_early(early, b.vote ? k_heuristics<true> : k_heuristics<false>, grid, kHThreads, 0, s, b, labels);
+    const long long tiles = (long long)grid.x * grid.y * nframes;
+    if (tiles <= kTiles512) return heuristics_t<512>(tma, early, grid, s, b, labels, map);
+    if (tiles <= kTiles256) return heuristics_t<256>(tma, early, grid, s, b, labels, map);
+    return heuristics_t<kHThreads>(tma, early, grid, s, b, labels, map);
 }
 
 cudaError_t take_heuristics_fault(int* out)

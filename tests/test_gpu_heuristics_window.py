@@ -125,3 +125,33 @@ def test_frames_with_labels(cuda, vote):
               torch.from_numpy(buf).cuda(), p, torch.zeros(int(oo[-1]), dtype=torch.uint8, device="cuda"), lab)
     assert np.array_equal(lab.cpu().numpy(), np.concatenate([r[1] for r in refs]))
     ctx.close()
+
+
+@pytest.mark.parametrize("n", [15, 16, 25, 26])
+@pytest.mark.parametrize("vote", [False, True])
+def test_threads_by_tiles(cuda, n, vote):
+    """Equal batches on both sides of the tile counts at which the blocks change
+    their size (48 tiles a frame: 720, 768, 1200 and 1248; one frame above and
+    below each), resolved graphs by way of the labels."""
+    import depix
+    torch = cuda
+    w, h = 192, 241
+    rng = np.random.default_rng(n)
+    imgs = np.stack([lines(rng, w, h) for _ in range(3)])
+    want = []
+    for img in imgs:
+        ws = (3 * w + 3) & ~3
+        buf = np.zeros((h, ws), np.uint8)
+        buf[:, :3 * w] = img[..., 2::-1].reshape(h, -1)
+        want.append(np.asarray(O.label_cc(O.graph(buf.reshape(-1), w, h, ws, vote=vote)[2], w, h)).reshape(-1))
+    p = depix.params(48, 7, 6, True, 1, vote=vote)
+    ctx = depix.Context(w * h, n)
+    d = torch.from_numpy(imgs[np.arange(n) % 3].copy()).cuda()
+    out = torch.zeros(n * w * h * 4, dtype=torch.uint8, device="cuda")
+    lab = torch.zeros(n * w * h, dtype=torch.int32, device="cuda")
+    off = [k * w * h * 4 for k in range(n)]
+    ctx.batch([w] * n, [h] * n, off, off, d, p, out, lab)
+    got = lab.cpu().numpy().reshape(n, -1)
+    for k in range(n):
+        assert np.array_equal(got[k], want[k % 3]), k
+    ctx.close()
