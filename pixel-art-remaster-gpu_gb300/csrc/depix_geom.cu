@@ -1543,7 +1543,7 @@ __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const 
         const unsigned inv = (1u << 20) / (unsigned)s + 1u; // x / s = x inv >> 20 for x up to a tile's rows (12 k)
         const int lane = threadIdx.x & 31;
         const bool quads = (ow % 4) == 0 && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
-        for (int b0 = threadIdx.x & ~31; b0 < TW * TH; b0 += kRT) {
+        for (int b0 = threadIdx.x & ~31; b0 < TW * TH; b0 += blockDim.x) {
             const int tx = lane % TW, ty = (b0 + lane) / TW, k = (ty + 1) * T::GW + tx + 1;
             const bool in = x0 + tx < w && y0 + ty < h;
             auto touch = [&](int q) { return (unsigned)info[k + (1 - q / 3) * T::GW + 1 - q % 3] >> q & 1u; };
@@ -1582,7 +1582,7 @@ __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const 
         }
         __syncthreads();
         const int rows = M.slow * s;
-        for (int i = threadIdx.x; i < rows; i += kRT) {
+        for (int i = threadIdx.x; i < rows; i += blockDim.x) {
             const int bi = (int)((unsigned)i * inv >> 20), r = i - bi * s, q0 = M.list[bi];
             const int tx = q0 % TW, ty = q0 / TW, k = (ty + 1) * T::GW + tx + 1;
             const uint32_t* px = &M.pix[ty + 2][tx + 4];
@@ -1709,8 +1709,8 @@ __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const 
     }
 }
 
-template <int LAYOUT, int S, int TH>
-__global__ void __launch_bounds__(kRT, raster_blocks(S)) k_mask_raster(RasterBatch b, const uint32_t* lut)
+template <int LAYOUT, int S, int TH, int NT>
+__global__ void __launch_bounds__(NT, raster_blocks(S) * kRT / NT) k_mask_raster(RasterBatch b, const uint32_t* lut)
 {
     follow_last();
     __shared__ MaskTile<S, 32, TH> M;
@@ -1724,8 +1724,8 @@ __global__ void __launch_bounds__(kRT, raster_blocks(S)) k_mask_raster(RasterBat
 
 // The equal-size batch raster with its pixel windows loaded by TMA (RGBA
 // frames whose base, rows and frame stride are 16-byte aligned).
-template <int S, int TH>
-__global__ void __launch_bounds__(kRT, raster_blocks(S)) k_mask_raster_tma(RasterBatch b, const uint32_t* lut,
+template <int S, int TH, int NT>
+__global__ void __launch_bounds__(NT, raster_blocks(S) * kRT / NT) k_mask_raster_tma(RasterBatch b, const uint32_t* lut,
                                                          const __grid_constant__ CUtensorMap pix_map,
                                                          const __grid_constant__ CUtensorMap graph_map, int with_graph)
 {
@@ -1821,8 +1821,8 @@ static size_t mask_smem(int scale)
     return words * sizeof(uint32_t);
 }
 
-template <int LAYOUT, int S, int TH>
-static cudaError_t launch_mask_raster_t(const RasterBatch& b, int nframes, const uint32_t* lut, cudaStream_t s)
+template <int LAYOUT, int S, int TH, int NT>
+static cudaError_t launch_mask_raster_nt(const RasterBatch& b, int nframes, const uint32_t* lut, cudaStream_t s)
 {
     const bool early = early_stages((long long)b.w * b.h * nframes);
     if constexpr (LAYOUT == DEPIX_LAYOUT_RGBA) {
@@ -1830,7 +1830,7 @@ static cudaError_t launch_mask_raster_t(const RasterBatch& b, int nframes, const
         if (pixel_tensor_map(b, nframes, TH, &map)) {
             size_t smem = mask_smem<S, 32, TH>(b.scale);
             if (smem + sizeof(MaskTile<S, 32, TH>) > 48 * 1024) {
-                cudaError_t e = cudaFuncSetAttribute(k_mask_raster_tma<S, TH>,
+                cudaError_t e = cudaFuncSetAttribute(k_mask_raster_tma<S, TH, NT>,
                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
                 if (e != cudaSuccess) return e;
             }
@@ -1839,17 +1839,35 @@ static cudaError_t launch_mask_raster_t(const RasterBatch& b, int nframes, const
             const bool with_graph = u8_tensor_map(b.graph, b.w, b.h, b.graph_stride, nframes, 32 + 32, TH + 6, &gmap);
             if (!with_graph) gmap = map; // unused
             dim3 grid((b.w + 32 - 1) / 32, (b.h + TH - 1) / TH, nframes);
-            return launch_early(early, k_mask_raster_tma<S, TH>, grid, kRT, smem, s, b, lut, map, gmap, with_graph ? 1 : 0);
+            return launch_early(early, k_mask_raster_tma<S, TH, NT>, grid, NT, smem, s, b, lut, map, gmap, with_graph ? 1 : 0);
         }
     }
     size_t smem = mask_smem<S, 32, TH>(b.scale);
     if (smem + sizeof(MaskTile<S, 32, TH>) > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_mask_raster<LAYOUT, S, TH>,
+        cudaError_t e = cudaFuncSetAttribute(k_mask_raster<LAYOUT, S, TH, NT>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
     dim3 grid((b.w + 32 - 1) / 32, (b.h + TH - 1) / TH, nframes);
-    return launch_early(early, k_mask_raster<LAYOUT, S, TH>, grid, kRT, smem, s, b, lut);
+    return launch_early(early, k_mask_raster<LAYOUT, S, TH, NT>, grid, NT, smem, s, b, lut);
+}
+
+// With so few tiles that all are resident at once with twice the threads (two
+// blocks per SM up to x4, one above), a tile's time is the call's, and the
+// threads shorten it: a call with labels at x4 takes 26.7 us instead of 28.7 for
+// a 256x224 frame (112 tiles), 34.6 instead of 37.7 for five (280), but 44.2
+// instead of 43.2 for six (336); at x8 29.9 instead of 32.9 for one (112), 38.9
+// instead of 36.3 for two (224). 1024 threads: no better than 512 for one frame,
+// worse from four on.
+template <int S>
+constexpr long long kFewTiles = 152 * (raster_blocks(S) / 2);
+
+template <int LAYOUT, int S, int TH>
+static cudaError_t launch_mask_raster_t(const RasterBatch& b, int nframes, const uint32_t* lut, cudaStream_t s)
+{
+    const long long tiles = (long long)((b.w + 31) / 32) * ((b.h + TH - 1) / TH) * nframes;
+    return tiles <= kFewTiles<S> ? launch_mask_raster_nt<LAYOUT, S, TH, 2 * kRT>(b, nframes, lut, s)
+                                 : launch_mask_raster_nt<LAYOUT, S, TH, kRT>(b, nframes, lut, s);
 }
 
 // ---- uneven batches: the raster as a persistent kernel over a tile queue

@@ -100,3 +100,35 @@ def test_queue_tiles_of_every_layout(cuda, scale, tile):
         f = O.frame(ref.reshape(-1), w, h, ws, True)
         want = O.raster(f.pos, f.col, w, h, scale)
         assert np.array_equal(out[oo[k]:oo[k] + want.size].reshape(want.shape), want), (w, h)
+
+
+@pytest.mark.parametrize("scale,size,ns", [(2, (96, 97), (25, 26)), (3, (97, 96), (25, 26)), (4, (96, 97), (25, 26)),
+                                           (5, (64, 49), (19, 20)), (8, (64, 49), (19, 20)), (12, (65, 48), (16, 17))])
+def test_threads_by_tiles(cuda, scale, size, ns):
+    """Equal batches on both sides of the tile counts (304 up to x4, 152 above) at
+    which the raster's blocks change their size, widths with and without TMA."""
+    import depix
+    torch = cuda
+    w, h = size
+    rng = np.random.default_rng(scale)
+    imgs = [rng.integers(0, 3, size=(h, w, 4)).astype(np.uint8) * 90 for _ in range(3)]
+    want = []
+    for img in imgs:
+        ws = (3 * w + 3) & ~3
+        ref = np.zeros((h, ws), np.uint8)
+        ref[:, :3 * w] = img[..., 2::-1].reshape(h, -1)
+        f = O.frame(ref.reshape(-1), w, h, ws, True)
+        want.append(O.raster(f.pos, f.col, w, h, scale))
+    for n in ns:
+        step, ostep = (4 * w * h + 15) // 16 * 16, (4 * w * h * scale * scale + 15) // 16 * 16
+        buf = np.zeros((n, step), np.uint8)
+        for k in range(n):
+            buf[k, :4 * w * h] = imgs[k % 3].reshape(-1)
+        out = torch.zeros((n, ostep), dtype=torch.uint8, device="cuda")
+        ctx = depix.Context(w * h, n)
+        ctx.batch([w] * n, [h] * n, [k * step for k in range(n)], [k * ostep for k in range(n)],
+                  torch.from_numpy(buf).cuda(), depix.params(48, 7, 6, True, scale), out)
+        got = out.cpu().numpy()[:, :4 * w * h * scale * scale]
+        ctx.close()
+        for k in range(n):
+            assert np.array_equal(got[k].reshape(want[k % 3].shape), want[k % 3]), (n, k)
