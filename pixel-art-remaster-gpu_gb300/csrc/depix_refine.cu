@@ -1027,6 +1027,20 @@ __device__ __forceinline__ Stencil node_stencil(float2 p, float2 pa, float2 pb, 
     return Stencil{make_float2(tx, ty), make_float2(gx, gy)};
 }
 
+// The gradient and Adam's moments, with their roundings written out: where a
+// gradient should be zero, Adam makes a step of full length of its last bits, so
+// another choice of fused operations (the compiler's changed with the code around
+// them) moved nodes of some frames by hundredths of a pixel.
+__device__ __forceinline__ float node_gradient(float curv, float g, float dev, float d, float cov)
+{
+    return __fadd_rn(__fmaf_rn(curv, g, __fmul_rn(dev, d)), cov);
+}
+__device__ __forceinline__ float first_moment(float m, float g) { return __fmaf_rn(1.f - kBeta1, g, __fmul_rn(kBeta1, m)); }
+__device__ __forceinline__ float second_moment(float v, float g)
+{
+    return __fmaf_rn(__fmul_rn(1.f - kBeta2, g), g, __fmul_rn(kBeta2, v));
+}
+
 // One thread per free node: curvature and deviation gradients, the coverage
 // gradient that k_rf_coverage left (zeroed for the next one), then an Adam step,
 // or the energy and the gradient written out.
@@ -1055,18 +1069,18 @@ __global__ void __launch_bounds__(64) k_rf_nodes(StepArgs a)
         }
         const Stencil S = node_stencil(p, pa, pb, nb, qn);
         const float dx = p.x - p0.x, dy = p.y - p0.y;
-        const float gx = 0.25f * curv_k * S.g.x + 2.f * dev_k * dx + gc.x;
-        const float gy = 0.25f * curv_k * S.g.y + 2.f * dev_k * dy + gc.y;
+        const float gx = node_gradient(0.25f * curv_k, S.g.x, 2.f * dev_k, dx, gc.x);
+        const float gy = node_gradient(0.25f * curv_k, S.g.y, 2.f * dev_k, dy, gc.y);
         a.gcov[k] = make_float2(0.f, 0.f);
         if constexpr (ENERGY) {
             ec += 0.125f * (S.t.x * S.t.x + S.t.y * S.t.y);
             ed += dx * dx + dy * dy;
             if (a.gout) a.gout[k] = make_float2(gx, gy);
         } else {
-            m.x = kBeta1 * m.x + (1.f - kBeta1) * gx;
-            m.y = kBeta1 * m.y + (1.f - kBeta1) * gy;
-            v.x = kBeta2 * v.x + (1.f - kBeta2) * gx * gx;
-            v.y = kBeta2 * v.y + (1.f - kBeta2) * gy * gy;
+            m.x = first_moment(m.x, gx);
+            m.y = first_moment(m.y, gy);
+            v.x = second_moment(v.x, gx);
+            v.y = second_moment(v.y, gy);
             a.m[f] = m;
             a.v[f] = v;
             a.y[k] = make_float2(p.x - a.lr * (m.x / a.bc1) / (sqrtf(v.x / a.bc2) + kEps),
