@@ -449,13 +449,23 @@ struct SampleCount {
     }
 };
 
+// The segments that read a free node: the middles of its two edges (parts 0 and
+// 1), its own corner (2) and, across each edge, the neighbour's corner or pinned
+// piece (3 and 4). Each keeps its part of the node's coverage gradient in a place
+// of its own and the node pass sums them, so that a run's positions do not depend
+// on what else runs, or on how the steps are launched: by float atomics the sum
+// had another rounding with every order of arrival, and where it should be zero
+// Adam makes a step of full length of its last bits.
+constexpr int kParts = 5;
+
 struct NodeOut {
     int2* q;        // quarter coordinates
     int* flags;     // bit 0 pinned, 1 frame, 2 corner; degree << 4
     int2* nbr;      // neighbours of degree-2 nodes (ascending), else -1
     int2* nbr_edge; // the edges to them
     float2* pos0;
-    float2* gcov;   // zeroed
+    float2* gcov;   // kParts parts of n each, zeroed
+    int n;          // nodes
 };
 
 __global__ void k_rf_make_nodes(Geo G, const uint32_t* vgrid, Scan<int> nid, const int2* nb_v, const int2* nb_e, NodeOut N)
@@ -492,7 +502,8 @@ __global__ void k_rf_make_nodes(Geo G, const uint32_t* vgrid, Scan<int> nid, con
     N.nbr[k] = nb;
     N.nbr_edge[k] = ne;
     N.pos0[k] = make_float2(0.25f * x, 0.25f * y);
-    N.gcov[k] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < kParts; q++) N.gcov[(size_t)q * N.n + k] = make_float2(0.f, 0.f);
 }
 
 struct SegOut {
@@ -844,7 +855,7 @@ struct RefineFrame {
 // A live segment, packed for one load: its nodes and type, its sample
 // range and its colours.
 struct LiveSeg {
-    int4 nodes;  // n0, n1, n2, type
+    int4 nodes;  // n0, n1, n2, type | its part of n0 << 3, of n1 << 6, of n2 << 9
     int4 range;  // first sample, end, left colour, right colour (0xBBGGRR)
 };
 
@@ -859,7 +870,7 @@ struct FreeNode {
 struct StepArgs {
     const float2* x;     // positions read
     float2* y;           // positions written (Adam)
-    float2* gcov;        // coverage gradient (atomics), zeroed by the node pass
+    float2* gcov;        // coverage gradient: kParts parts of N nodes, zero where no live segment writes
     float2* gout;        // gradient out (energy/gradient call), or NULL
     const float2* x0;
     const int4* seg;
@@ -911,13 +922,13 @@ __device__ __forceinline__ Edge live_edge(const LiveSeg& ls, const float2* x)
 {
     Edge E;
     const int4 sg = ls.nodes;
-    const int nodes[3] = {sg.x, sg.y, sg.z};
+    const int nodes[3] = {sg.x, sg.y, sg.z}, type = sg.w & 7;
     E.A = E.B = make_float2(0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         if (nodes[k] < 0) continue;
         const float2 p = x[nodes[k]];
-        const float wa = 0.25f * seg_wa(sg.w, k), wb = 0.25f * seg_wb(sg.w, k);
+        const float wa = 0.25f * seg_wa(type, k), wb = 0.25f * seg_wb(type, k);
         E.A.x += wa * p.x;
         E.A.y += wa * p.y;
         E.B.x += wb * p.x;
@@ -959,7 +970,7 @@ __device__ __forceinline__ float sample_loss(const Edge& E, float2 X, float4 t, 
 }
 
 // Coverage: kSegLanes lanes per live segment, the samples' gradients reduced in
-// the group and pushed to the segment's free nodes.
+// the group and stored as the segment's parts of its free nodes' gradients.
 template <bool ENERGY>
 __global__ void __launch_bounds__(256) k_rf_coverage(StepArgs a)
 {
@@ -994,9 +1005,9 @@ __global__ void __launch_bounds__(256) k_rf_coverage(StepArgs a)
 #pragma unroll
         for (int k = 0; k < 4; k++) g[k] = group_sum(g[k], gmask);
         if (push) {
-            const float wa = 0.25f * seg_wa(sg.w, gl), wb = 0.25f * seg_wb(sg.w, gl);
-            atomicAdd(&a.gcov[my].x, wa * g[0] + wb * g[2]);
-            atomicAdd(&a.gcov[my].y, wa * g[1] + wb * g[3]);
+            const int type = sg.w & 7, part = sg.w >> (3 + 3 * gl) & 7;
+            const float wa = 0.25f * seg_wa(type, gl), wb = 0.25f * seg_wb(type, gl);
+            a.gcov[(size_t)part * F.N + my] = make_float2(wa * g[0] + wb * g[2], wa * g[1] + wb * g[3]);
         }
     }
     if (!waited) follow_last(); // a grid that ended without it could overtake the one before
@@ -1041,9 +1052,24 @@ __device__ __forceinline__ float second_moment(float v, float g)
     return __fmaf_rn(__fmul_rn(1.f - kBeta2, g), g, __fmul_rn(kBeta2, v));
 }
 
+// Sum of a node's parts, rounded as if once: Knuth's two-sum (The Art of Computer
+// Programming, volume 2, section 4.2.2) keeps what each addition rounds away.
+__device__ __forceinline__ float sum_parts(const float (&part)[kParts])
+{
+    float s = part[0], lost = 0.f;
+#pragma unroll
+    for (int q = 1; q < kParts; q++) {
+        const float t = __fadd_rn(s, part[q]), b = __fsub_rn(t, s);
+        lost = __fadd_rn(lost, __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(part[q], b)));
+        s = t;
+    }
+    const float sum = __fadd_rn(s, lost);
+    return sum == sum ? sum : s; // an infinite sum loses its difference to itself
+}
+
 // One thread per free node: curvature and deviation gradients, the coverage
-// gradient that k_rf_coverage left (zeroed for the next one), then an Adam step,
-// or the energy and the gradient written out.
+// gradient's parts that k_rf_coverage left, then an Adam step, or the energy and
+// the gradient written out.
 template <bool ENERGY>
 __global__ void __launch_bounds__(64) k_rf_nodes(StepArgs a)
 {
@@ -1061,7 +1087,14 @@ __global__ void __launch_bounds__(64) k_rf_nodes(StepArgs a)
         float2 qn[4];
 #pragma unroll
         for (int t = 0; t < 4; t++) qn[t] = nb[t] >= 0 ? a.x[nb[t]] : make_float2(0.f, 0.f);
-        const float2 p = a.x[k], pa = a.x[fn.k_a_b_aa.y], pb = a.x[fn.k_a_b_aa.z], gc = a.gcov[k];
+        const float2 p = a.x[k], pa = a.x[fn.k_a_b_aa.y], pb = a.x[fn.k_a_b_aa.z];
+        float cx[kParts], cy[kParts];
+#pragma unroll
+        for (int q = 0; q < kParts; q++) {
+            const float2 c = a.gcov[(size_t)q * F.N + k];
+            cx[q] = c.x;
+            cy[q] = c.y;
+        }
         float2 m = make_float2(0.f, 0.f), v = m;
         if constexpr (!ENERGY) {
             m = a.m[f];
@@ -1069,9 +1102,8 @@ __global__ void __launch_bounds__(64) k_rf_nodes(StepArgs a)
         }
         const Stencil S = node_stencil(p, pa, pb, nb, qn);
         const float dx = p.x - p0.x, dy = p.y - p0.y;
-        const float gx = node_gradient(0.25f * curv_k, S.g.x, 2.f * dev_k, dx, gc.x);
-        const float gy = node_gradient(0.25f * curv_k, S.g.y, 2.f * dev_k, dy, gc.y);
-        a.gcov[k] = make_float2(0.f, 0.f);
+        const float gx = node_gradient(0.25f * curv_k, S.g.x, 2.f * dev_k, dx, sum_parts(cx));
+        const float gy = node_gradient(0.25f * curv_k, S.g.y, 2.f * dev_k, dy, sum_parts(cy));
         if constexpr (ENERGY) {
             ec += 0.125f * (S.t.x * S.t.x + S.t.y * S.t.y);
             ed += dx * dx + dy * dy;
@@ -1098,11 +1130,23 @@ __global__ void __launch_bounds__(64) k_rf_nodes(StepArgs a)
     }
 }
 
+// Which of a free node's kParts parts a segment (slot, sg) keeps; at: the node's
+// place in the segment (0..2), nbr_edge: the nodes' edges.
+__device__ __forceinline__ int node_part(const int4 sg, int slot, int at, const int2* nbr_edge)
+{
+    const int k = at == 0 ? sg.x : (at == 1 ? sg.y : sg.z);
+    if (k < 0) return 0;
+    if (sg.w == SEG_CORNER && at == 1) return 2;
+    // the edge by which the segment reaches the node
+    const int e = sg.w != SEG_CORNER ? slot / 3 : (at == 0 ? nbr_edge[sg.y].x : nbr_edge[sg.y].y);
+    return (sg.w == SEG_MID ? 0 : 3) + (nbr_edge[k].x == e ? 0 : 1);
+}
+
 // The samples of each slot in ascending order (summation order fixed) at its
 // offset, the live segments (those with samples) packed, and the offsets.
 __global__ void k_rf_fill_samples(const int4* seg, int S, const int2* q, int scale, int ow, int oh, Owner own,
                                   const int* seg_count, Scan<unsigned long long> off, const uint2* col, int* samp,
-                                  int* seg_off, LiveSeg* live)
+                                  int* seg_off, const int2* nbr_edge, LiveSeg* live)
 {
     follow_last();
     int slot;
@@ -1114,10 +1158,19 @@ __global__ void k_rf_fill_samples(const int4* seg, int S, const int2* q, int sca
     if (slot < S && gl == 0) {
         seg_off[slot] = at;
         if (slot == S - 1) seg_off[S] = at + c;
-        if (c) {
-            const uint2 lr = col[slot];
-            live[o >> 32] = LiveSeg{seg[slot], make_int4(at, at + c, (int)lr.x, (int)lr.y)};
-        }
+    }
+    int4 sg = make_int4(-1, -1, -1, SEG_NONE);
+    int parts = 0; // of the three nodes, a lane each
+    if (c) {
+        sg = seg[slot];
+        if (gl < 3) parts = node_part(sg, slot, gl, nbr_edge) << (3 + 3 * gl);
+    }
+    parts |= __shfl_xor_sync(0xFFFFFFFFu, parts, 1);
+    parts |= __shfl_xor_sync(0xFFFFFFFFu, parts, 2);
+    if (c && gl == 0) {
+        const uint2 lr = col[slot];
+        sg.w |= parts;
+        live[o >> 32] = LiveSeg{sg, make_int4(at, at + c, (int)lr.x, (int)lr.y)};
     }
     if (!c) B.nx = 0;
     box_samples(B, ow, [&](bool have, int x, int, int) {
@@ -1606,7 +1659,7 @@ depix_status depix_refine_setup(depix_refiner* r, const uint8_t* d_img, int w, i
     RF_CK(r->pos0.reserve(N));
     RF_CK(r->pos_a.reserve(N));
     RF_CK(r->pos_b.reserve(N));
-    RF_CK(r->gcov.reserve(N));
+    RF_CK(r->gcov.reserve((size_t)kParts * N));
     RF_CK(r->adam_m.reserve(N));
     RF_CK(r->adam_v.reserve(N));
     const int S = 3 * E + N;
@@ -1624,7 +1677,7 @@ depix_status depix_refine_setup(depix_refiner* r, const uint8_t* d_img, int w, i
     RF_CK(r->samp.reserve(no_px));
     RF_CK(r->tgt.reserve(no_px));
     RF_CK(r->sxy.reserve(no_px));
-    NodeOut no{r->node_q.p, r->node_flags.p, r->node_nbr.p, r->node_nbr_edge.p, r->pos0.p, r->gcov.p};
+    NodeOut no{r->node_q.p, r->node_flags.p, r->node_nbr.p, r->node_nbr_edge.p, r->pos0.p, r->gcov.p, N};
     RF_CK(launch_early(true, k_rf_make_nodes, blocks_for(nv), 256, 0, s, G, r->vgrid.p, nid, r->nb_v.p, r->nb_e.p,
                        no));
     RF_CK(launch_early(true, k_rf_segments, blocks_for((long long)E + N), 256, 0, s, G, nid, r->edges.p, E, N,
@@ -1654,7 +1707,8 @@ depix_status depix_refine_setup(depix_refiner* r, const uint8_t* d_img, int w, i
     RF_CK(cudaGetLastError());
     RF_CK(exclusive_scan(SampleCount{r->seg_count.p}, S, soff, s));
     RF_CK(launch_early(true, k_rf_fill_samples, box_blocks, 256, 0, s, r->seg.p, S, r->node_q.p, p->scale, ow, oh,
-                       own, r->seg_count.p, soff, r->seg_col.p, r->samp.p, r->seg_off.p, r->live.p));
+                       own, r->seg_count.p, soff, r->seg_col.p, r->samp.p, r->seg_off.p, r->node_nbr_edge.p,
+                       r->live.p));
     // free nodes and their curvature stencils, and the frame record
     const Scan<int> free_pos{r->free_pos.p, r->free_tiles.p, r->scalars.p + 3, r->tickets.p + 3};
     RF_CK(exclusive_scan(FreeFlag{r->node_flags.p}, N, free_pos, s));
