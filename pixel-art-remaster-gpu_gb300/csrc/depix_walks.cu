@@ -318,6 +318,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_border_walks_smem(const uint8_
                     trunc = 1;
                     break;
                 }
+                __syncwarp(); // every lane has read done[k]
                 if (lane == 0) {
                     on[pos] = p;
                     oe[pos] = -1;
