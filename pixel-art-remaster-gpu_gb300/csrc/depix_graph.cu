@@ -1208,7 +1208,8 @@ static cudaError_t launch_graph_t(const FrameBatch& b, int nframes, uint32_t thr
 cudaError_t launch_graph(const FrameBatch& b, int nframes, uint32_t thr, bool fuse_trivial, cudaStream_t s)
 {
     const long long px = (long long)b.w * b.h * nframes;
-    if (px <= 1 << 18) return launch_graph_t<kGStripFrame>(b, nframes, thr, fuse_trivial, s);
+    // tiles of four rows only where grid.y takes them all (one column of 2^18 rows has one too many)
+    if (px <= 1 << 18 && b.h <= 65535 * 4 * kGStripFrame) return launch_graph_t<kGStripFrame>(b, nframes, thr, fuse_trivial, s);
     if (px <= 1 << 21) return launch_graph_t<kGStripSmall>(b, nframes, thr, fuse_trivial, s);
     return launch_graph_t<kGStrip>(b, nframes, thr, fuse_trivial, s);
 }
