@@ -373,6 +373,8 @@ depix_status depix_refine_energy_grad(depix_refiner* r, const depix_refine_param
  * and after when the pointers are set (those evaluations synchronise). */
 depix_status depix_refine_run(depix_refiner* r, const depix_refine_params* p, float* d_pos, double before[4],
                               double after[4], depix_stream s);
+/* Testing hook: how often the refiner captured the Adam loop as a graph. */
+depix_status depix_debug_refine_captures(const depix_refiner* r, long long* count);
 
 /* ---------------------------------------------------------------------
  * Drop-in replacement of the reference's frame driver.

@@ -1293,6 +1293,7 @@ struct depix_refiner {
     StepArgs loop_args{};
     int loop_steps = -1;
     int loop_cov_blocks = 0, loop_node_blocks = 0;
+    long long captures = 0; // of the loop
 };
 
 namespace {
@@ -1397,24 +1398,26 @@ depix_status check_sigma(const depix_refiner* r, const depix_refine_params* p)
     return DEPIX_OK;
 }
 
-// grids: enough blocks for the frame, rounded up in eighths of a power of two
-// (the kernels stride over the sizes they read on the device, so a captured
-// loop serves every frame whose rounded grids match), at most 8 blocks of 256
-// threads per SM. The live segments are about the edges' middles and the nodes'
-// corners.
+// grids: enough blocks for the frame, rounded up to a power of two, at most 8
+// blocks of 256 threads per SM. The kernels stride over the sizes they read on
+// the device, so a captured loop serves other frames too (loop_fits). The live
+// segments are about the edges' middles and the nodes' corners.
 int grid_for(long long threads, int block, int most)
 {
-    const long long n = std::max<long long>(1, (threads + block - 1) / block);
     long long p = 1;
-    while (p < n) p <<= 1;
-    const long long g = std::max<long long>(1, p / 8);
-    return (int)std::min<long long>(most, (n + g - 1) / g * g);
+    while (p < most && p * block < threads) p <<= 1;
+    return (int)std::min<long long>(p, most);
 }
 int cov_blocks(const depix_refiner* r)
 {
     return grid_for(((long long)r->E + r->N) * kSegLanes, 256, r->sms * 8);
 }
 int node_blocks(const depix_refiner* r) { return grid_for(r->N, 64, r->sms * 32); } // F <= N
+
+// A loop captured with so many blocks serves a frame that wants `want` of them or
+// as few as a quarter of that: frames whose counts move to and fro replay one
+// loop, captured for the largest.
+bool loop_fits(int blocks, int want) { return blocks >= want && blocks <= 4 * want; }
 
 bool same_loop(const StepArgs& a, const StepArgs& b)
 {
@@ -1835,6 +1838,16 @@ depix_status depix_refine_warm_start(depix_refiner* r, const depix_refiner* prev
     return DEPIX_OK;
 }
 
+depix_status depix_debug_refine_captures(const depix_refiner* r, long long* count)
+{
+    if (!r || !count) {
+        set_last_error("NULL refiner or count");
+        return DEPIX_ERR_INVALID_ARG;
+    }
+    *count = r->captures;
+    return DEPIX_OK;
+}
+
 depix_status depix_refine_energy_grad(depix_refiner* r, const depix_refine_params* p, const float* d_pos,
                                       float* d_grad, double energy[4], depix_stream s)
 {
@@ -1868,8 +1881,8 @@ depix_status depix_refine_run(depix_refiner* r, const depix_refine_params* p, fl
     RF_CK(cudaStreamIsCapturing(s, &cs));
     if (p->steps > 0 && cs == cudaStreamCaptureStatusNone) {
         if (!r->loop || r->loop_steps != p->steps || !same_loop(a, r->loop_args) ||
-            r->loop_args.x != r->pos_a.p || r->loop_args.y != r->pos_b.p || r->loop_cov_blocks != cov_blocks(r) ||
-            r->loop_node_blocks != node_blocks(r)) {
+            r->loop_args.x != r->pos_a.p || r->loop_args.y != r->pos_b.p ||
+            !loop_fits(r->loop_cov_blocks, cov_blocks(r)) || !loop_fits(r->loop_node_blocks, node_blocks(r))) {
             if (r->loop) cudaGraphExecDestroy(r->loop);
             r->loop = nullptr;
             RF_CK(cudaStreamBeginCapture(r->capture_stream, cudaStreamCaptureModeThreadLocal));
@@ -1883,6 +1896,7 @@ depix_status depix_refine_run(depix_refiner* r, const depix_refine_params* p, fl
                 r->loop = nullptr;
                 return rf_fail(e, "refine loop capture");
             }
+            r->captures++;
             r->loop_args = a;
             r->loop_args.x = r->pos_a.p;
             r->loop_args.y = r->pos_b.p;

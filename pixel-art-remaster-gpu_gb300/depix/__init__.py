@@ -80,6 +80,7 @@ def lib():
         _sig(L, "depix_debug_fail_allocations", [_i])
         _sig(L, "depix_debug_live_allocations", [_vp])
         _sig(L, "depix_debug_tma_timeout", [_i])
+        _sig(L, "depix_debug_refine_captures", [_vp, _vp])
         _sig(L, "depix_graph", [_vp, _i, _i, _i, _i, P, _i, _vp, _vp])
         _sig(L, "depix_resolve_trivial", [_vp, _i, _i, _vp])
         _sig(L, "depix_resolve_heuristics", [_vp, _i, _i, _vp, _vp])
@@ -406,6 +407,12 @@ class Refiner:
                                              ctypes.byref(n) if count else None, stream_ptr(stream)),
                "depix_refine_warm_start")
         return n.value if count else None
+
+    def debug_captures(self):
+        """Testing hook: how often the Adam loop was captured as a graph."""
+        n = ctypes.c_longlong(0)
+        _check(lib().depix_debug_refine_captures(self.handle, ctypes.byref(n)), "depix_debug_refine_captures")
+        return n.value
 
     def energy_grad(self, rp, pos, grad=None, stream=None):
         e = (ctypes.c_double * 4)()
