@@ -624,16 +624,6 @@ __global__ void __launch_bounds__(NT) k_heuristics_tma(GraphBatch b, int32_t* L,
 
 // -------------------------------------------------- component labelling
 
-__device__ __forceinline__ int uf_find(int32_t* L, int x)
-{
-    int p = L[x];
-    while (p != x) {
-        x = p;
-        p = L[x];
-    }
-    return x;
-}
-
 // lock-free union with the smaller root winning: the final root of every
 // component is its minimum index
 __device__ __forceinline__ void uf_unite(int32_t* L, int a, int b)

@@ -873,13 +873,8 @@ struct StepArgs {
     float2* gcov;        // coverage gradient: kParts parts of N nodes, zero where no live segment writes
     float2* gout;        // gradient out (energy/gradient call), or NULL
     const float2* x0;
-    const int4* seg;
-    const uint2* col;
-    const int* seg_off;
-    const int* samp;
     const float4* tgt;
     const int* flags;
-    const int2* nbr;
     const LiveSeg* live;
     const float2* sxy;   // sample positions (source pixels), in segment order
     const FreeNode* fnodes;
@@ -1358,13 +1353,8 @@ StepArgs step_args(depix_refiner* r, const depix_refine_params* p)
     StepArgs a{};
     a.gcov = r->gcov.p;
     a.x0 = r->pos0.p;
-    a.seg = r->seg.p;
-    a.col = r->seg_col.p;
-    a.seg_off = r->seg_off.p;
-    a.samp = r->samp.p;
     a.tgt = r->tgt.p;
     a.flags = r->node_flags.p;
-    a.nbr = r->node_nbr.p;
     a.live = r->live.p;
     a.sxy = r->sxy.p;
     a.fnodes = r->fnodes.p;
@@ -1421,9 +1411,8 @@ bool loop_fits(int blocks, int want) { return blocks >= want && blocks <= 4 * wa
 
 bool same_loop(const StepArgs& a, const StepArgs& b)
 {
-    return a.gcov == b.gcov && a.x0 == b.x0 && a.seg == b.seg && a.col == b.col && a.seg_off == b.seg_off &&
-           a.samp == b.samp && a.tgt == b.tgt && a.flags == b.flags && a.nbr == b.nbr && a.live == b.live && a.sxy == b.sxy && a.fnodes == b.fnodes &&
-           a.fr == b.fr && a.m == b.m && a.v == b.v && a.sigma == b.sigma && a.w_curv == b.w_curv &&
+    return a.gcov == b.gcov && a.x0 == b.x0 && a.tgt == b.tgt && a.flags == b.flags && a.live == b.live &&
+           a.sxy == b.sxy && a.fnodes == b.fnodes && a.fr == b.fr && a.m == b.m && a.v == b.v && a.sigma == b.sigma && a.w_curv == b.w_curv &&
            a.w_dev == b.w_dev && a.w_cov == b.w_cov && a.lr == b.lr;
 }
 
