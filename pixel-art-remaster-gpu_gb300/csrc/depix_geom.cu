@@ -672,7 +672,7 @@ cudaError_t launch_emit(const uint8_t* img, int w, int h, int ws, int layout, co
 cudaError_t launch_vbo(const uint8_t* img, int w, int h, int ws, int layout, const uint8_t* g, bool subdivide,
                        float* diagram, int* ec, float* pos, uint8_t* col, cudaStream_t s)
 {
-    return launch_early(true, k_vbo, grid1(w * h, kVboCells), kVboThreads, 0, s, img, w, h, ws, layout, g, subdivide ? 1 : 0,
+    return launch_early(early_stages((long long)w * h), k_vbo, grid1(w * h, kVboCells), kVboThreads, 0, s, img, w, h, ws, layout, g, subdivide ? 1 : 0,
                         reinterpret_cast<float2*>(diagram), ec, reinterpret_cast<float2*>(pos),
                         reinterpret_cast<uchar4*>(col));
 }
@@ -1875,7 +1875,6 @@ static cudaError_t launch_mask_raster_t(const RasterBatch& b, int nframes, const
 template <int S, int TW, int TH>
 __global__ void __launch_bounds__(kRT, raster_blocks(S)) k_raster_queue(QueueBatch q)
 {
-    follow_last();
     __shared__ MaskTile<S, TW, TH> M;
     extern __shared__ uint32_t masks[];
     const QueueHeader* H = q.hdr;
@@ -1900,7 +1899,8 @@ static cudaError_t queue_raster_t(const QueueBatch& q, int blocks, cudaStream_t 
     // the shared-memory opt-in is made by raster_queue_occupancy, which the
     // host calls on each device before any launch or stream capture
     const size_t smem = mask_smem<S, TW, TH>(q.scale);
-    return launch_early(true, k_raster_queue<S, TW, TH>, blocks, kRT, smem, s, q);
+    k_raster_queue<S, TW, TH><<<blocks, kRT, smem, s>>>(q);
+    return cudaGetLastError();
 }
 
 template <int S, int TW, int TH>

@@ -1067,7 +1067,6 @@ __global__ void k_cc_flatten(int32_t* L, int n, size_t frame_stride)
 
 __global__ void __launch_bounds__(kGThreads) k_graph_queue(QueueBatch q)
 {
-    early_start();
     const QueueHeader* H = q.hdr;
     const int n = H->n;
     queue_loop(q.counters + QC_GRAPH, (int)H->total[QS_GRAPH], q.gran[QS_GRAPH], [&](int t) {
@@ -1083,7 +1082,6 @@ __global__ void __launch_bounds__(kGThreads) k_graph_queue(QueueBatch q)
 template <bool VOTE>
 __global__ void __launch_bounds__(kHThreads) k_heur_queue(QueueBatch q)
 {
-    follow_last();
     const QueueHeader* H = q.hdr;
     const int n = H->n;
     queue_loop(q.counters + QC_HEUR, (int)H->total[QS_HEUR], q.gran[QS_HEUR], [&](int t) {
@@ -1099,7 +1097,6 @@ __global__ void __launch_bounds__(kHThreads) k_heur_queue(QueueBatch q)
 
 __global__ void __launch_bounds__(128) k_label_merge_queue(QueueBatch q)
 {
-    follow_last();
     // the local labels came with the heuristics stage: its tiles
     const QueueHeader* H = q.hdr;
     const int n = H->n;
@@ -1120,13 +1117,16 @@ cudaError_t queue_graph(const QueueBatch& q, int blocks, cudaStream_t s)
 
 cudaError_t queue_heuristics(const QueueBatch& q, int blocks, cudaStream_t s)
 {
-    return launch_early(true, q.vote ? k_heur_queue<true> : k_heur_queue<false>, blocks, kHThreads, 0, s, q);
+    if (q.vote) k_heur_queue<true><<<blocks, kHThreads, 0, s>>>(q);
+    else k_heur_queue<false><<<blocks, kHThreads, 0, s>>>(q);
+    return cudaGetLastError();
 }
 
 cudaError_t queue_labels(const QueueBatch& q, int blocks, cudaStream_t s)
 {
     // local labels were made by the heuristics stage; the raster makes the roots
-    return launch_early(true, k_label_merge_queue, blocks, 128, 0, s, q);
+    k_label_merge_queue<<<blocks, 128, 0, s>>>(q);
+    return cudaGetLastError();
 }
 
 static_assert(kQGraphTW == kGTW && kQGraphTH == 4 * kGStripQueue, "graph queue tile");

@@ -1419,9 +1419,10 @@ bool same_loop(const StepArgs& a, const StepArgs& b)
 // launches the Adam steps from pos_a (result in pos_a after an even number
 // of steps, pos_b after an odd one). A step is two short kernels, bound by the
 // latency of their launches and loads (one of a 256x224 frame touches 4 MB in
-// L2): 7.5 us when each waited for the other before its first load, 5.9 us with
-// early starts. (One kernel that gathers a node's gradient over the five
-// segments that read it, evaluating each 2.7 times: 7.2 us.)
+// L2): 20 steps of it take 135 us when each waits for the other before its first
+// load, 98 with early starts (64x64 112 and 82, 1500x1000 1726 and 1655). (One
+// kernel that gathers a node's gradient over the five segments that read it,
+// evaluating each 2.7 times, took 7.2 us a step where the two took 5.9.)
 cudaError_t launch_steps(depix_refiner* r, const StepArgs& base, int steps, cudaStream_t s)
 {
     StepArgs a = base;
@@ -1621,7 +1622,8 @@ depix_status depix_refine_setup(depix_refiner* r, const uint8_t* d_img, int w, i
     const Scan<int> nid{r->nid.p, r->nid_tiles.p, r->scalars.p + 1, r->tickets.p + 1};
     RF_CK(cudaMemsetAsync(r->vgrid.p, 0, (size_t)nv * sizeof(uint32_t), s));
     // the topology is some twenty short kernels, each started while the one
-    // before it ends (256x224 at x4: 166 us one after the other, 135 so)
+    // before it ends (us one after the other and so: 64x64 117 and 86, 256x224 142
+    // and 112, 640x480 436 and 402, 1500x1000 1717 and 1679)
     RF_CK(launch_early(true, k_rf_mark_vertices, blocks_for(n), 256, 0, s, G, r->vgrid.p));
     RF_CK(launch_early(true, k_rf_count_edges, blocks_for(n, kEdgeCells), kEdgeThreads, 0, s, G, r->vgrid.p,
                        r->max_split, r->cell_count.p, r->edge_slots.p));
