@@ -26,7 +26,19 @@ void depix::set_last_error(const std::string& msg) { t_last_error = msg; }
 namespace {
 std::atomic<long long> g_live_allocs{0};
 std::atomic<int> g_fail_after{-1}; // < 0: never; n: n more allocations succeed, then all fail
+std::atomic<int> g_sms[64];        // multiprocessors per device, 0 until asked for
 }  // namespace
+
+int depix::sm_count()
+{
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    const bool kept = dev >= 0 && dev < 64;
+    if (kept && (n = g_sms[dev].load(std::memory_order_relaxed)) > 0) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 152;
+    if (kept) g_sms[dev].store(n, std::memory_order_relaxed);
+    return n;
+}
 
 cudaError_t depix::dev_alloc(void** p, size_t bytes)
 {

@@ -1860,13 +1860,13 @@ static cudaError_t launch_mask_raster_nt(const RasterBatch& b, int nframes, cons
 // instead of 36.3 for two (224). 1024 threads: no better than 512 for one frame,
 // worse from four on.
 template <int S>
-constexpr long long kFewTiles = 152 * (raster_blocks(S) / 2);
+constexpr int kFewTilesPerSm = raster_blocks(S) / 2;
 
 template <int LAYOUT, int S, int TH>
 static cudaError_t launch_mask_raster_t(const RasterBatch& b, int nframes, const uint32_t* lut, cudaStream_t s)
 {
     const long long tiles = (long long)((b.w + 31) / 32) * ((b.h + TH - 1) / TH) * nframes;
-    return tiles <= kFewTiles<S> ? launch_mask_raster_nt<LAYOUT, S, TH, 2 * kRT>(b, nframes, lut, s)
+    return tiles <= (long long)kFewTilesPerSm<S> * sm_count() ? launch_mask_raster_nt<LAYOUT, S, TH, 2 * kRT>(b, nframes, lut, s)
                                  : launch_mask_raster_nt<LAYOUT, S, TH, kRT>(b, nframes, lut, s);
 }
 

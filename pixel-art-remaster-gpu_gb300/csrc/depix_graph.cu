@@ -296,7 +296,8 @@ constexpr int kHRW = kHTW + 2 * kHaloX, kHRH = kHTH + 2 * kHaloY;
 // With many, blocks of 128 leave less waiting at barriers (heuristics of 1024
 // frames 244 / 309 with 256).
 constexpr int kHThreads = 128;
-constexpr long long kTiles512 = 760, kTiles256 = 1216;
+// The lines, 760 and 1216 tiles of the 152 SMs measured, are kept per SM.
+constexpr int kTilesPerSm512 = 5, kTilesPerSm256 = 8;
 
 struct SnapTile {
     const uint8_t (*s)[kHRW];
@@ -1227,9 +1228,9 @@ cudaError_t launch_heuristics(const GraphBatch& b, int nframes, int32_t* labels,
     const bool early = early_stages((long long)b.w * b.h * nframes);
     CUtensorMap map;
     const bool tma = u8_tensor_map(b.snap, b.w, b.h, b.frame_stride, nframes, kHRW, kHRH, &map);
-    const long long tiles = (long long)grid.x * grid.y * nframes;
-    if (tiles <= kTiles512) return heuristics_t<512>(tma, early, grid, s, b, labels, map);
-    if (tiles <= kTiles256) return heuristics_t<256>(tma, early, grid, s, b, labels, map);
+    const long long tiles = (long long)grid.x * grid.y * nframes, sms = sm_count();
+    if (tiles <= kTilesPerSm512 * sms) return heuristics_t<512>(tma, early, grid, s, b, labels, map);
+    if (tiles <= kTilesPerSm256 * sms) return heuristics_t<256>(tma, early, grid, s, b, labels, map);
     return heuristics_t<kHThreads>(tma, early, grid, s, b, labels, map);
 }
 
