@@ -870,13 +870,15 @@ cudaError_t launch_raster(const RasterBatch& b, int nframes, cudaStream_t s)
 //  - an output block (the s x s samples of one cell) takes, per sample, the
 //    latest covering cell in VBO order among the 3x3 cells around it.
 //
-// Mask layouts: up to scale 8 a mask is nine parts, one per cell of the 3x3
-// around it (the cell itself is part 4), each part the s*s samples of that
-// cell in s rows of s bits, so that a block reads one part of each of its
-// nine candidates and resolves all its samples at once. A part is 16 bits up
-// to scale 4 and 64 bits up to scale 8. Above, a mask is one word per
-// footprint row (parts would need up to 144 bits each, twice the shared
-// memory of the rows).
+// Mask layouts (mask_layout): up to scale 4 and at 8 a mask is nine parts, one
+// per cell of the 3x3 around it (the cell itself is part 4), each part the s*s
+// samples of that cell in s rows of s bits, so that a block reads one part of
+// each of its nine candidates and resolves all its samples (at 8 two rows of
+// them) at once. A part is 16 bits up to scale 4, 64 bits at 8. At 5 to 7 and
+// above 8 a mask is one word per footprint row and a word on the parts that it
+// touches: parts would need up to 144 bits each, twice the shared memory of the
+// rows, and at 5 to 7 a block's rows of 5 to 7 pixels do not make whole 16-byte
+// stores, where the rows of 32 blocks do.
 //
 // What bounds it: a 32x32 tile's phases (tile load, plain cells, cut cells,
 // fills, shared blocks) take 22, 22, 28, 20 and 8 % of a block's time, each a
@@ -1536,8 +1538,8 @@ __device__ void mask_raster_tile(MaskTile<S, TW, TH>& M, uint32_t* masks, const 
         // four pixels a lane, so that the stores are contiguous whatever s is;
         // the rows of the other blocks follow, one a thread. (Resolving each
         // row of the 32 blocks in the warp and writing it whole: 132 us for 100
-        // frames of 152x102 at x5, 96 us so; one thread a block, which stores
-        // every pixel apart: 171.)
+        // frames of 152x102 at x5, 96 us so; parts of 64 bits and one thread a
+        // block, which stores every pixel apart: 171.)
         constexpr int CM = S == 0 ? 7 : 12; // most samples of a row
         const uint32_t blockbits = (1u << s) - 1u;
         const unsigned inv = (1u << 20) / (unsigned)s + 1u; // x / s = x inv >> 20 for x up to a tile's rows (12 k)

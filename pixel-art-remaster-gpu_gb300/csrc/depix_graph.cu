@@ -655,8 +655,9 @@ __device__ __forceinline__ void uf_unite(int32_t* L, int a, int b)
 // index order), then unions across tile borders on the global label array,
 // then one flattening pass. The frame and batch paths make the tile-local
 // labels inside the 64x16 heuristics tiles (tile_labels), merge with
-// merge_tile_borders and flatten in the raster's tiles (flatten_tile); the stage API (depix_label_components) runs
-// its own 32x32 tiles over a graph in global memory (cc_local_core: a warp
+// merge_tile_borders and flatten in the raster's tiles (flatten_tile), or with
+// k_cc_flatten where no mask raster follows; the stage API
+// (depix_label_components) runs its own 32x32 tiles over a graph in global memory (cc_local_core: a warp
 // owns a row, horizontal runs from one ballot, one union per pair of touching
 // runs).
 constexpr int kLT = 32;
@@ -765,10 +766,11 @@ __device__ __forceinline__ void for_each_join(const uint64_t (&need)[3], Fn fn)
 // Component labels of a 64x16 tile of a symmetric graph (each edge held by
 // both of its nodes, as in the resolved graph; 0 outside the image), as global
 // indices of the tile-local roots. A run's parent is kept at its leftmost
-// pixel. The rows' run starts and upward edges become 64-bit masks by ballot;
-// a lane then lists the edges of one kind between half a row and the row above
-// it that join_masks keeps (three warps, one a kind); all threads unite along
-// the listed edges, one each (a lane that united its own edges in turn waited
+// pixel. The rows' run starts and upward edges become 64-bit masks, eight columns
+// a thread: a product gathers a bit of four packed bytes at once. A lane then
+// lists the edges of one kind between half a row and the row above it that
+// join_mask keeps (three warps, one a kind); all threads unite along the listed
+// edges, one each (a lane that united its own edges in turn waited
 // for a chain of finds per edge: 8.4 k cycles of a tile's 26 k); then the
 // listed runs, which are all that are not their own root, are pointed at their
 // roots, and each pixel reads its run's parent (following the chains from
